@@ -453,7 +453,7 @@ int gbs_import(gbs_ctx *c, int side, const void *src, int dtype, int col_major, 
   c->vt_valid[side] = false;
   uint8_t *digits = nullptr;
   uint32_t dtab[4] = {0, 0, 0, 0};
-  if (!col_major && import_writes_digits(c)) {
+  if (import_writes_digits(c)) {
     if (ensure_digit_buffer(c, side) == cudaSuccess) {
       digits = c->digits[side];
       tc_digit_table(m, dtab);
@@ -466,13 +466,9 @@ int gbs_import(gbs_ctx *c, int side, const void *src, int dtype, int col_major, 
                          ? device_view(src, c->device, true)
                          : nullptr;
   if (view) {  // host memory the device reads directly: the pack kernel is the copy
-    if (!col_major) {
-      e = launch_pack_rows(m, view, dtype, 0, m.nrows_a, digits, dtab, s);
-      if (e == cudaSuccess && digits) c->digits_valid[side] = true;
-    } else {
-      e = launch_pack(m, view, dtype, 1, s);
-    }
+    e = launch_pack(m, view, dtype, col_major, digits, dtab, s);
     if (e != cudaSuccess) return cuda_fail(e, "gbs_import: pack kernel");
+    if (digits) c->digits_valid[side] = true;
     e = ensure_import_streams(c);
     if (e == cudaSuccess) e = cudaEventRecord(c->ev_packed[side], s);
     if (e == cudaSuccess) e = cudaEventSynchronize(c->ev_packed[side]);  // host memory may be reused once read
@@ -492,7 +488,7 @@ int gbs_import(gbs_ctx *c, int side, const void *src, int dtype, int col_major, 
       if (e == cudaSuccess) e = cudaEventRecord(c->ev_chunk[0], c->copy_stream);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(s, c->ev_chunk[0], 0);
       if (e != cudaSuccess) return cuda_fail(e, "gbs_import: host-to-device copy");
-      e = launch_pack(m, c->stage[side], dtype, 1, s);
+      e = launch_pack(m, c->stage[side], dtype, 1, digits, dtab, s);
       if (e != cudaSuccess) return cuda_fail(e, "gbs_import: pack kernel");
     } else {  // row chunks: the pack of chunk i overlaps the copy of chunk i+1
       const size_t row_bytes = m.ncols * esz;
@@ -513,10 +509,10 @@ int gbs_import(gbs_ctx *c, int side, const void *src, int dtype, int col_major, 
         if (e != cudaSuccess) return cuda_fail(e, "gbs_import: pack kernel");
         last = (int)i;
       }
-      if (digits) c->digits_valid[side] = true;
       e = cudaEventSynchronize(c->ev_chunk[last]);  // host memory may be reused once copied
       if (e != cudaSuccess) return cuda_fail(e, "gbs_import: copy wait");
     }
+    if (digits) c->digits_valid[side] = true;
     e = cudaEventRecord(c->ev_packed[side], s);
     if (e != cudaSuccess) return cuda_fail(e, "gbs_import: event record");
     c->ev_packed_set[side] = true;
@@ -524,13 +520,10 @@ int gbs_import(gbs_ctx *c, int side, const void *src, int dtype, int col_major, 
       e = cudaEventSynchronize(c->ev_chunk[0]);
       if (e != cudaSuccess) return cuda_fail(e, "gbs_import: copy wait");
     }
-  } else if (!col_major) {
-    e = launch_pack_rows(m, src, dtype, 0, m.nrows_a, digits, dtab, s);
+  } else {
+    e = launch_pack(m, src, dtype, col_major, digits, dtab, s);
     if (e != cudaSuccess) return cuda_fail(e, "gbs_import: pack kernel");
     if (digits) c->digits_valid[side] = true;
-  } else {
-    e = launch_pack(m, src, dtype, 1, s);
-    if (e != cudaSuccess) return cuda_fail(e, "gbs_import: pack kernel");
   }
   m.imported = true;
   return GBS_OK;

@@ -33,9 +33,11 @@ struct gbs_group {
   gbs::PackJob *d_rs_jobs = nullptr;
   int nrs = 0;
   uint64_t rs_warps = 0;
+  // pack jobs of the grouped import: those of the direct kernel, then those of the staged one
   gbs::PackJob *d_pack_jobs = nullptr;
-  int npack = 0;
-  uint64_t pack_warps = 0;
+  int npack[2] = {0, 0};
+  uint64_t pack_runs[2] = {0, 0};
+  uint32_t pack_run[2] = {1, 1};  // units per run
   size_t smem = 0;
   int grid = 0;
   cudaGraph_t graph = nullptr;
@@ -90,8 +92,8 @@ cudaError_t upload(T **dst, const std::vector<T> &v) {
 
 // Builds the pack-job table for (lhs_srcs[p], rhs_srcs[p]) of every problem.
 int build_pack_jobs(gbs_group *g, const void *const *lhs, const void *const *rhs, const int *dtypes) {
-  std::vector<PackJob> jobs;
-  uint64_t warps = 0;
+  std::vector<PackJob> jobs[2];  // direct, staged
+  uint64_t units[2] = {0, 0};
   size_t ti = 0;  // index among the tensor-core problems
   for (size_t p = 0; p < g->ctxs.size(); p++) {
     const uint8_t digit_sides = g->is_tc[p] ? g->tc.sides[ti++] : 0;
@@ -103,39 +105,47 @@ int build_pack_jobs(gbs_group *g, const void *const *lhs, const void *const *rhs
       if (m.nrows_a == 0 || m.wpr() == 0) continue;
       if (m.nrows && m.ncols && (!src || !device_ptr(src)))
         return fail(GBS_EINVAL, "gbs_group: sources must be device pointers (problem " + std::to_string(p) + ")");
-      PackJob j;
-      memset(&j, 0, sizeof(j));
-      j.src = src;
-      j.planes = m.planes;
-      j.nrows = m.nrows;
-      j.ncols = m.ncols;
-      j.nrows_a = m.nrows_a;
-      j.wpr = m.wpr();
-      j.nbits = (int)m.nbits;
-      j.issigned = m.issigned;
-      j.dtype = dt;
-      j.vec = (dt == GBS_I8 || dt == GBS_U8) && m.ncols % 16 == 0 && ((uintptr_t)src % 16) == 0;
-      j.segs = (uint32_t)pack_segs_per_row(m.wpr());
-      j.dcols = m.dcols;
+      uint32_t dtab[4] = {0, 0, 0, 0};
+      uint8_t *digits = nullptr, *nibbles = nullptr;
       if ((digit_sides >> side) & 1) {  // tensor-core problem: the import writes the digit matrices it reads
-        j.digits = g->ctxs[p]->digits[side];
-        tc_digit_table(m, j.dtab);
+        digits = g->ctxs[p]->digits[side];
+        tc_digit_table(m, dtab);
       }
-      if ((digit_sides >> (2 + side)) & 1) j.nibbles = g->ctxs[p]->nibbles[side];  // ... and nibble matrices
-      j.warp0 = warps;
-      warps += m.nrows_a * j.segs;
-      jobs.push_back(j);
+      if ((digit_sides >> (2 + side)) & 1) nibbles = g->ctxs[p]->nibbles[side];  // ... and nibble matrices
+      PackJob j = make_pack_job(m, src, dt, digits, dtab, nibbles);
+      const int kind = pack_job_direct(j, m) ? 0 : 1;
+      units[kind] += pack_job_units(j);
+      jobs[kind].push_back(j);
     }
   }
+  for (int k = 0; k < 2; k++) {
+    const uint32_t run = pack_run_units(units[k]);
+    uint64_t runs = 0;
+    for (PackJob &j : jobs[k]) {
+      j.warp0 = runs;
+      runs += (pack_job_units(j) + run - 1) / run;
+    }
+    g->npack[k] = (int)jobs[k].size();
+    g->pack_runs[k] = runs;
+    g->pack_run[k] = run;
+  }
+  jobs[0].insert(jobs[0].end(), jobs[1].begin(), jobs[1].end());
   if (g->d_pack_jobs) cudaFree(g->d_pack_jobs);
   g->d_pack_jobs = nullptr;
-  if (upload(&g->d_pack_jobs, jobs) != cudaSuccess) {
+  if (upload(&g->d_pack_jobs, jobs[0]) != cudaSuccess) {
     cudaGetLastError();
+    g->npack[0] = g->npack[1] = 0;
     return fail(GBS_ENOMEM, "gbs_group: pack table upload failed");
   }
-  g->npack = (int)jobs.size();
-  g->pack_warps = warps;
   return GBS_OK;
+}
+
+cudaError_t enqueue_pack(const gbs_group *g, cudaStream_t s) {
+  cudaError_t e = launch_pack_grouped(g->d_pack_jobs, g->npack[0], g->pack_runs[0], g->pack_run[0], true, s);
+  if (e == cudaSuccess)
+    e = launch_pack_grouped(g->d_pack_jobs + g->npack[0], g->npack[1], g->pack_runs[1], g->pack_run[1],
+                            false, s);
+  return e;
 }
 
 cudaError_t enqueue_gemm(gbs_group *g, cudaStream_t s) {
@@ -365,7 +375,7 @@ int gbs_group_import(gbs_group *g, const void *const *lhs_srcs, const void *cons
   if (!g || !lhs_srcs || !rhs_srcs) return fail(GBS_EINVAL, "gbs_group_import: NULL argument");
   int rc = build_pack_jobs(g, lhs_srcs, rhs_srcs, dtypes);
   if (rc != GBS_OK) return rc;
-  cudaError_t e = launch_pack_grouped(g->d_pack_jobs, g->npack, g->pack_warps, (cudaStream_t)stream);
+  cudaError_t e = enqueue_pack(g, (cudaStream_t)stream);
   if (e != cudaSuccess) return cuda_fail(e, "gbs_group_import: pack kernel");
   for (gbs_ctx *c : g->ctxs) {
     c->lhs.imported = c->rhs.imported = true;
@@ -413,14 +423,14 @@ int gbs_group_capture(gbs_group *g, const void *const *lhs_srcs, const void *con
   cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return cuda_fail(e, "gbs_group_capture: begin capture");
   cudaError_t ke = cudaSuccess;
-  if (with_pack) ke = launch_pack_grouped(g->d_pack_jobs, g->npack, g->pack_warps, s);
+  if (with_pack) ke = enqueue_pack(g, s);
   if (ke == cudaSuccess) ke = enqueue_gemm(g, s);
   e = cudaStreamEndCapture(s, &g->graph);
   if (ke != cudaSuccess) return cuda_fail(ke, "gbs_group_capture: enqueue");
   if (e != cudaSuccess) return cuda_fail(e, "gbs_group_capture: end capture");
   e = cudaGraphInstantiate(&g->exec, g->graph, 0);
   if (e != cudaSuccess) return cuda_fail(e, "gbs_group_capture: instantiate");
-  g->launches_per_replay = (with_pack && g->npack ? 1 : 0) + (g->popc_tiles ? 1 + (g->nrs ? 1 : 0) : 0) +
+  g->launches_per_replay = (with_pack ? (g->npack[0] ? 1 : 0) + (g->npack[1] ? 1 : 0) : 0) + (g->popc_tiles ? 1 + (g->nrs ? 1 : 0) : 0) +
                            (g->tc.ntiles ? 1 : 0);
   if (with_pack) {
     for (gbs_ctx *c : g->ctxs) c->lhs.imported = c->rhs.imported = true;
@@ -433,7 +443,7 @@ int gbs_group_replay(gbs_group *g, void *stream) {
   if (!g || !g->exec) return fail(GBS_ESTATE, "gbs_group_replay: capture the group first");
   cudaError_t e = cudaGraphLaunch(g->exec, (cudaStream_t)stream);
   if (e != cudaSuccess) return cuda_fail(e, "gbs_group_replay");
-  if (g->npack) {  // the replay packs new planes: cached adjoint operands and other derived copies are stale
+  if (g->npack[0] || g->npack[1]) {  // the replay packs new planes: cached adjoint operands and other derived copies are stale
     for (gbs_ctx *c : g->ctxs) c->vt_valid[0] = c->vt_valid[1] = false;
     mark_packed_digits(g);
   }

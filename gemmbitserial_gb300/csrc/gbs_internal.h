@@ -94,9 +94,10 @@ struct GroupTile {
   uint32_t p, mt, nt, cls;
 };
 
-// One operand of a grouped import / row-sum pass; warp0 = first global warp.
-// With digits set, the import also writes the operand's e4m3 digit matrix
-// [nrows_a][64 * wpr] (table dtab), the operand of the tensor-core pipe.
+// One operand of an import or of a grouped row-sum pass; warp0 = its first
+// warp run (import) or row (row sums) of a grouped pass.  With digits set, the
+// import also writes the operand's e4m3 digit matrix (table dtab), the operand
+// of the tensor-core pipe.
 struct PackJob {
   const void *src;
   uint64_t *planes;
@@ -106,7 +107,9 @@ struct PackJob {
   uint64_t nrows, ncols, nrows_a, wpr, warp0;
   uint64_t dcols;  // digit-matrix columns (a multiple of 256)
   int nbits, issigned, dtype, vec;
-  uint32_t segs;  // 512-column segments per row
+  // direct (1-byte, 16-byte-aligned rows): vec 2 when 32-byte aligned, else 1;
+  // staged kernels of a grouped import: vec 1 when four elements load as one vector
+  uint32_t cpr, magic;  // 32-column chunks per padded row, 2^32 / cpr + 1
   uint32_t dtab[4];
 };
 
@@ -251,12 +254,19 @@ void count_launch(uint64_t n = 1);
 cudaError_t dev_alloc(void **p, size_t bytes);
 
 // kernels (gbs_pack.cu)
-cudaError_t launch_pack(const Mat &m, const void *src, int dtype, int col_major, cudaStream_t s);
+// plain import (importRegular); with digits set also the e4m3 digit matrix (table dtab[4])
+cudaError_t launch_pack(const Mat &m, const void *src, int dtype, int col_major, uint8_t *digits,
+                        const uint32_t *dtab, cudaStream_t s);
 // threshold-quantising import (importRegularAndQuantize); dtype GBS_I8..GBS_F32, thr [nthres][nrows]
 cudaError_t launch_pack_quantize(const Mat &m, const void *src, const void *thr, int nthres, int dtype,
                                  int col_major, uint8_t *digits, const uint32_t *dtab, cudaStream_t s);
-// units of the row-major pack kernels: 1024-column segments per row
-inline uint64_t pack_segs_per_row(uint64_t wpr) { return (wpr * 64 + 1023) / 1024; }
+// One operand as a pack job; digits / nibbles may be null.
+PackJob make_pack_job(const Mat &m, const void *src, int dtype, uint8_t *digits, const uint32_t *dtab,
+                      uint8_t *nibbles);
+// Sets j.vec; true when the direct kernels take the job, false for the staged ones.
+bool pack_job_direct(PackJob &j, const Mat &m);
+uint64_t pack_job_units(const PackJob &j);   // units (32 chunks, one warp) of the job
+uint32_t pack_run_units(uint64_t units);    // units per warp run of a grouped import of that many
 // row-major pack of padded rows [r0, r1); with digits set also the e4m3 digit rows (table dtab[4])
 cudaError_t launch_pack_rows(const Mat &m, const void *src, int dtype, uint64_t r0, uint64_t r1, uint8_t *digits,
                              const uint32_t *dtab, cudaStream_t s);
@@ -282,7 +292,8 @@ cudaError_t prepare_gemm_popc_grouped(size_t smem);
 cudaError_t launch_gemm_popc_grouped(const GroupProblem *probs, int nprob, const GroupTile *tiles, uint32_t ntiles,
                                      uint32_t *counter, uint32_t *err, size_t smem, int grid, cudaStream_t s);
 int grouped_blocks_per_sm(size_t smem);
-cudaError_t launch_pack_grouped(const PackJob *jobs, int njobs, uint64_t total_warps, cudaStream_t s);
+cudaError_t launch_pack_grouped(const PackJob *jobs, int njobs, uint64_t runs, uint32_t run, bool direct,
+                                cudaStream_t s);
 cudaError_t launch_rowsum_grouped(const PackJob *jobs, int njobs, uint64_t total_warps, cudaStream_t s);
 cudaError_t launch_gemm_bmma(const GemmShape &g, const Epilogue &e, cudaStream_t s);
 bool bmma_supported(int wa, int wb, int use_xor);

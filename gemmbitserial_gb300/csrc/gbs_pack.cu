@@ -9,6 +9,17 @@
 //   * the low byte of x otherwise (two's complement for signed matrices; the
 //     reference's "add 2^(w-1) twice" leaves the low w bits of x unchanged).
 // Rows >= nrows and columns >= ncols are zero in every plane.
+//
+// Every import ends the same way: a lane holds the codes of one "chunk", 32
+// consecutive columns of one row (byte j%4 of q[j/4]), and emits one 32-bit
+// word per plane, 32 bytes of the digit matrix and 16 bytes of the nibble
+// matrix.  Chunks are numbered along the padded rows, so chunk c of a plane is
+// its 32-bit word c: a warp's 32 chunks store 128 contiguous bytes per plane
+// whatever the row length, and no lane idles on short rows.
+#include <algorithm>
+#include <cstring>
+#include <type_traits>
+
 #include "gbs_internal.h"
 
 namespace gbs {
@@ -16,91 +27,25 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 
-__device__ __forceinline__ int64_t load_elem(const void *src, int dtype, uint64_t idx) {
-  switch (dtype) {
-    case GBS_I8: return ((const int8_t *)src)[idx];
-    case GBS_U8: return ((const uint8_t *)src)[idx];
-    case GBS_I16: return ((const int16_t *)src)[idx];
-    default: return ((const int32_t *)src)[idx];
-  }
-}
+// ---------------------------------------------------------------- emission
 
-__device__ __forceinline__ uint32_t code_of(int64_t x, int dtype, int bipolar) {
-  if (dtype == GBS_U8) return (uint32_t)(x & 0xff);
-  if (bipolar) return x > 0 ? 1u : 0u;
-  return (uint32_t)(x & 0xff);
-}
-
-// quantize<float> (gemmbitserial.hpp:170-186): bipolar maps x > 0 to 1; a
-// negative x of a signed matrix becomes 2^(w-1) + (uint8_t)(x + 2^(w-1)), the
-// sum taken in float; otherwise (uint8_t)x.  Float -> integer casts truncate
-// toward zero, then keep the low byte.
-__device__ __forceinline__ uint32_t code_of_f32(float x, int bipolar, int issigned, int nbits) {
-  if (bipolar) return x > 0.f ? 1u : 0u;
-  if (issigned && x < 0.f) {
-    const int64_t h = (int64_t)1 << (nbits - 1);
-    return (uint32_t)(h + (int64_t)(x + (float)h)) & 0xffu;
-  }
-  return (uint32_t)(int64_t)x & 0xffu;
-}
-
-__device__ __forceinline__ uint32_t elem_code(const void *src, int dtype, uint64_t idx, int bipolar, int issigned,
-                                              int nbits) {
-  if (dtype == GBS_F32) return code_of_f32(((const float *)src)[idx], bipolar, issigned, nbits);
-  return code_of(load_elem(src, dtype, idx), dtype, bipolar);
-}
-
-// Row-major packing: a warp takes a 1024-column segment of one padded row;
-// lane l owns the 32 columns [seg*1024 + 32l, +32).  Its 32 codes (byte j%4
-// of q[j/4]) give, per plane, one whole 32-bit half of a plane word, so the
-// 32 lanes store 128 contiguous bytes per plane with no shuffles.
-constexpr int kSegCols = 1024;
-
-__host__ __device__ inline uint64_t segs_per_row(uint64_t wpr) { return (wpr * 64 + kSegCols - 1) / kSegCols; }
-
-__device__ __forceinline__ void load_codes32(const void *__restrict__ src, int dtype, int bipolar, int issigned,
-                                             int nbits, uint64_t nrows, uint64_t ncols, int vec, uint64_t r,
-                                             uint64_t col0, uint32_t (&q)[8]) {
-#pragma unroll
-  for (int i = 0; i < 8; i++) q[i] = 0u;
-  if (r >= nrows || col0 >= ncols) return;
-  const uint64_t base = r * ncols + col0;
-  if (vec) {  // 1-byte elements, 16-byte aligned rows, ncols % 16 == 0
-    const uint4 *p = reinterpret_cast<const uint4 *>((const uint8_t *)src + base);
-    const uint4 v0 = p[0];
-    q[0] = v0.x; q[1] = v0.y; q[2] = v0.z; q[3] = v0.w;
-    if (col0 + 32 <= ncols) {
-      const uint4 v1 = p[1];
-      q[4] = v1.x; q[5] = v1.y; q[6] = v1.z; q[7] = v1.w;
-    }
-    if (bipolar && dtype == GBS_I8) {
-#pragma unroll
-      for (int i = 0; i < 8; i++) q[i] = __vcmpgts4(q[i], 0u) & 0x01010101u;
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 32; j++)
-      if (col0 + j < ncols) q[j >> 2] |= elem_code(src, dtype, base + j, bipolar, issigned, nbits) << (8 * (j & 3));
-  }
-}
-
-// Bits b of the eight bytes of (hi:lo), gathered into a byte (byte i -> bit i):
-// masking leaves one bit per byte at 8i; the multiply by sum_i 2^(56-7i)
-// moves it to 56+i.  All partial products land on distinct bit positions
-// (8i - 7j is unique for i, j in 0..7), so nothing carries.
-__device__ __forceinline__ uint32_t gather8(uint32_t lo, uint32_t hi, int b) {
-  const uint64_t x = ((((uint64_t)hi << 32) | lo) >> b) & 0x0101010101010101ull;
-  return (uint32_t)((x * 0x0102040810204080ull) >> 56);
-}
-
-__device__ __forceinline__ void emit_planes32(int nbits, uint64_t nrows_a, uint64_t wpr, uint64_t *__restrict__ planes,
-                                              uint64_t r, uint64_t col0, const uint32_t (&q)[8]) {
-  uint32_t *p32 = reinterpret_cast<uint32_t *>(planes);  // little-endian halves of the u64 plane words
-  const uint64_t row32 = 2 * wpr, idx = r * row32 + (col0 >> 5), plane32 = nrows_a * row32;
+// One 32-bit word per plane from the lane's 32 codes.  Four codes at a time:
+// a mask leaves bit b of each byte and a dp4a weighs the bytes 1, 2, 4, 8 (the
+// next word's 16 .. 128), so two dp4a gather eight codes into a byte (times
+// 2^b): 21 instructions a plane, where gathering through a 64-bit multiply
+// took about 45.
+__device__ __forceinline__ void emit_planes32(int nbits, uint32_t *__restrict__ p32, uint64_t plane32, uint64_t idx,
+                                              const uint32_t (&q)[8]) {
   for (int b = 0; b < nbits; b++) {
-    const uint32_t w = gather8(q[0], q[1], b) | (gather8(q[2], q[3], b) << 8) | (gather8(q[4], q[5], b) << 16) |
-                       (gather8(q[6], q[7], b) << 24);
-    p32[b * plane32 + idx] = w;
+    const uint32_t m = 0x01010101u << b;
+    uint32_t a[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      a[i] = __dp4a(q[2 * i] & m, 0x08040201u, 0u);
+      a[i] = __dp4a(q[2 * i + 1] & m, 0x80402010u, a[i]);
+    }
+    const uint32_t lo = (a[0] + (a[1] << 8)) >> b, hi = (a[2] + (a[3] << 8)) >> b;
+    p32[(uint64_t)b * plane32 + idx] = __byte_perm(lo, hi, 0x5410u);
   }
 }
 
@@ -118,31 +63,30 @@ __device__ __forceinline__ uint32_t digits4(uint32_t x, int nbits, uint4 tab) {
   return (lo & ~m) | (hi & m);
 }
 
-// The lane's 32 digits of row r < nrows (0 past ncols) into the digit matrix
-// (dcols columns, 16-row blocks: digit_offset).  Digit rows past nrows and
-// columns past the planes' padded width stay as allocated: zero.
-__device__ __forceinline__ void write_digits32(uint8_t *__restrict__ digits, int nbits, uint64_t nrows,
-                                               uint64_t ncols, uint64_t dcols, uint4 tab, uint64_t r, uint64_t col0,
-                                               const uint32_t (&q)[8]) {
+// The lane's 32 digits (0 past ncols) into the digit matrix (dcols columns,
+// 16-row blocks: digit_offset) as one 32-byte store.  Digit rows past nrows
+// and columns past the planes' padded width stay as allocated: zero.
+__device__ __forceinline__ void write_digits32(uint8_t *__restrict__ digits, int nbits, uint64_t ncols, uint64_t dcols,
+                                               uint4 tab, uint64_t r, uint64_t col0, const uint32_t (&q)[8]) {
   uint32_t d[8];
 #pragma unroll
-  for (int i = 0; i < 8; i++) {
-    d[i] = 0u;
-    if (r < nrows) {
-      d[i] = digits4(q[i], nbits, tab);
+  for (int i = 0; i < 8; i++) d[i] = digits4(q[i], nbits, tab);
+  if (col0 + 32 > ncols) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
       const uint64_t c = col0 + 4 * i;
       if (c + 4 > ncols) d[i] &= c >= ncols ? 0u : (0xFFFFFFFFu >> (8 * (4 - (ncols - c))));
     }
   }
-  uint4 *dst = reinterpret_cast<uint4 *>(digits + digit_offset(r, col0, dcols));
-  dst[0] = make_uint4(d[0], d[1], d[2], d[3]);
-  dst[1] = make_uint4(d[4], d[5], d[6], d[7]);
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(digits + digit_offset(r, col0, dcols)),
+               "r"(d[0]), "r"(d[1]), "r"(d[2]), "r"(d[3]), "r"(d[4]), "r"(d[5]), "r"(d[6]), "r"(d[7])
+               : "memory");
 }
 
-// The lane's 32 codes of row r < nrows into the nibble matrix (dcols columns,
-// blocks of nibble_offset): the low nbits bits of each code byte, two codes a
-// byte (even column low).  Codes past ncols are whatever the source gave:
-// the tensor-core kernel multiplies them by digits that are zero there.
+// The lane's 32 codes into the nibble matrix (dcols columns, blocks of
+// nibble_offset): the low nbits bits of each code byte, two codes a byte
+// (even column low).  Codes past ncols are whatever the source gave: the
+// tensor-core kernel multiplies them by digits that are zero there.
 __device__ __forceinline__ void write_nibbles32(uint8_t *__restrict__ nib, int nbits, uint64_t dcols, uint64_t r,
                                                 uint64_t col0, const uint32_t (&q)[8]) {
   const uint32_t msk = 0x01010101u * ((1u << nbits) - 1u);
@@ -157,229 +101,478 @@ __device__ __forceinline__ void write_nibbles32(uint8_t *__restrict__ nib, int n
   *reinterpret_cast<uint4 *>(nib + nibble_offset(r, col0, dcols)) = make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-// One 1024-column unit: codes, planes and (optionally) digits of the lane's 32 columns.
-__device__ __forceinline__ void pack_unit(const void *__restrict__ src, int dtype, int bipolar, int issigned,
-                                          int nbits,
-                                          uint64_t nrows, uint64_t ncols, uint64_t nrows_a, uint64_t wpr, int vec,
-                                          uint64_t *__restrict__ planes, uint8_t *__restrict__ digits,
-                                          uint64_t dcols, uint4 dtab, uint64_t r, uint64_t seg, int lane) {
-  const uint64_t col0 = seg * kSegCols + (uint64_t)lane * 32;
-  if (col0 >= wpr * 64) return;  // past the padded row
-  uint32_t q[8];
-  load_codes32(src, dtype, bipolar, issigned, nbits, nrows, ncols, vec, r, col0, q);
-  emit_planes32(nbits, nrows_a, wpr, planes, r, col0, q);
-  if (digits && r < nrows) write_digits32(digits, nbits, nrows, ncols, dcols, dtab, r, col0, q);
+// Everything a chunk (row r, chunk cc of the row) writes.
+__device__ __forceinline__ void emit_chunk(const PackJob &J, uint64_t r, uint32_t cc, const uint32_t (&q)[8]) {
+  emit_planes32(J.nbits, reinterpret_cast<uint32_t *>(J.planes), J.nrows_a * J.cpr, r * J.cpr + cc, q);
+  if (r >= J.nrows) return;
+  const uint64_t col0 = (uint64_t)cc * 32;
+  if (J.digits)
+    write_digits32(J.digits, J.nbits, J.ncols, J.dcols, make_uint4(J.dtab[0], J.dtab[1], J.dtab[2], J.dtab[3]), r,
+                   col0, q);
+  if (J.nibbles) write_nibbles32(J.nibbles, J.nbits, J.dcols, r, col0, q);
 }
 
-// Row-major pack of padded rows [row0, row0 + nrows_launch).  With digits
-// set, the lanes also write the rows' e4m3 digits (the tensor-core pipe's
-// operand), from the same loads.
-__global__ void __launch_bounds__(256) pack_rowmajor(const void *__restrict__ src, int dtype, int bipolar,
-                                                     int issigned, int nbits, uint64_t nrows, uint64_t ncols,
-                                                     uint64_t nrows_a, uint64_t wpr, int vec,
-                                                     uint64_t *__restrict__ planes, uint64_t row0,
-                                                     uint64_t nrows_launch, uint8_t *__restrict__ digits,
-                                                     uint64_t dcols, uint4 dtab) {
-  const uint64_t segs = segs_per_row(wpr);
-  const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (warp >= nrows_launch * segs) return;  // warp-uniform
-  pack_unit(src, dtype, bipolar, issigned, nbits, nrows, ncols, nrows_a, wpr, vec, planes, digits, dcols, dtab,
-            row0 + warp / segs,
-            warp % segs, threadIdx.x & 31);
+// ---------------------------------------------------------------- chunk numbering
+
+// A unit is 32 chunks, a lane each.  The unit's first chunk is located once;
+// the lanes then divide only small numbers: t = cc0 + i with i <= 31, and t /
+// cpr is a multiply-high by magic = 2^32 / cpr + 1 (exact while t * cpr <
+// 2^32, i < 32 (kMaxRun + 1)), or, for rows of 65000 chunks and more, 0 or 1.
+struct UnitBase {
+  uint64_t r;
+  uint32_t cc;
+};
+
+__device__ __forceinline__ UnitBase unit_base(uint32_t cpr, uint64_t row0, uint64_t unit) {
+  const uint64_t c = unit * 32;
+  UnitBase b;
+  if (c <= 0xFFFFFFFFull) {
+    const uint32_t q = (uint32_t)c / cpr;
+    b.r = row0 + q;
+    b.cc = (uint32_t)c - q * cpr;
+  } else {
+    const uint64_t q = c / cpr;
+    b.r = row0 + q;
+    b.cc = (uint32_t)(c - q * cpr);
+  }
+  return b;
 }
 
-// ---------------------------------------------------------------- threshold quantisation
+__device__ __forceinline__ void unit_chunk(const UnitBase &b, uint32_t i, uint32_t cpr, uint32_t magic, uint64_t &r,
+                                           uint32_t &cc) {
+  const uint32_t t = b.cc + i;
+  const uint32_t q = cpr < 65000u ? __umulhi(t, magic) : (t >= cpr ? 1u : 0u);
+  r = b.r + q;
+  cc = t - q * cpr;
+}
+
+// ---------------------------------------------------------------- 1-byte rows, 16-byte aligned
+
+// The lane's chunk straight from memory: one 32-byte load (VEC 2: rows and
+// source 32-byte aligned) or two of 16 bytes (VEC 1).  A warp's two strided
+// 16-byte loads touch each sector twice; the single load touches it once.
+template <int VEC>
+__device__ __forceinline__ void load_bytes32(const void *src, uint64_t nrows, uint64_t ncols, uint64_t r, uint32_t cc,
+                                             uint32_t (&q)[8]) {
+#pragma unroll
+  for (int i = 0; i < 8; i++) q[i] = 0u;
+  const uint64_t col0 = (uint64_t)cc * 32;
+  if (r >= nrows || col0 >= ncols) return;
+  const uint8_t *p = (const uint8_t *)src + r * ncols + col0;
+  if (VEC == 2) {  // ncols is a multiple of 32: the chunk is whole
+    asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7])
+                 : "l"(p));
+  } else {  // a multiple of 16: the chunk may be half
+    const uint4 v0 = reinterpret_cast<const uint4 *>(p)[0];
+    q[0] = v0.x; q[1] = v0.y; q[2] = v0.z; q[3] = v0.w;
+    if (col0 + 32 <= ncols) {
+      const uint4 v1 = reinterpret_cast<const uint4 *>(p)[1];
+      q[4] = v1.x; q[5] = v1.y; q[6] = v1.z; q[7] = v1.w;
+    }
+  }
+}
+
+__device__ __forceinline__ void codes_of_bytes(int dtype, int bipolar, uint32_t (&q)[8]) {
+  if (bipolar && dtype == GBS_I8) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) q[i] = __vcmpgts4(q[i], 0u) & 0x01010101u;
+  }
+}
+
+template <int VEC>
+__global__ void __launch_bounds__(256) pack_bytes(const __grid_constant__ PackJob J, uint64_t row0, uint64_t rend,
+                                                  uint64_t units) {
+  const uint64_t u = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (u >= units) return;  // warp-uniform
+  uint64_t r;
+  uint32_t cc, q[8];
+  unit_chunk(unit_base(J.cpr, row0, u), threadIdx.x & 31, J.cpr, J.magic, r, cc);
+  if (r >= rend) return;
+  load_bytes32<VEC>(J.src, J.nrows, J.ncols, r, cc, q);
+  codes_of_bytes(J.dtype, J.nbits == 1 && J.issigned, q);
+  emit_chunk(J, r, cc, q);
+}
+
+// ---------------------------------------------------------------- every other source
+
+// Four consecutive elements of a row (or, column-major, of a column) held raw.
+template <typename T>
+struct Raw4 {
+  uint32_t w[sizeof(T)];
+};
+
+// Elements [e, e + n) of the source, n <= 4 of them wanted (0 in the place of
+// the others).  ALIGNED: e and the source's address allow one vector load
+// whenever n = 4.  Otherwise 4-byte elements load one by one (the lanes' four
+// loads share their sectors), and 1- and 2-byte elements as the two aligned
+// words around them, shifted together, where those words lie inside the
+// source (total elements).
+template <typename T, bool ALIGNED>
+__device__ __forceinline__ Raw4<T> load4(const T *__restrict__ src, uint64_t e, uint32_t n, uint64_t total) {
+  Raw4<T> x;
+#pragma unroll
+  for (int i = 0; i < (int)sizeof(T); i++) x.w[i] = 0u;
+  if (n == 0) return x;
+  const T *p = src + e;
+  if (ALIGNED && n == 4) {
+    if constexpr (sizeof(T) == 1) {
+      x.w[0] = *reinterpret_cast<const uint32_t *>(p);
+    } else if constexpr (sizeof(T) == 2) {
+      const uint2 v = *reinterpret_cast<const uint2 *>(p);
+      x.w[0] = v.x; x.w[1] = v.y;
+    } else {
+      const uint4 v = *reinterpret_cast<const uint4 *>(p);
+      x.w[0] = v.x; x.w[1] = v.y; x.w[2] = v.z; x.w[3] = v.w;
+    }
+    return x;
+  }
+  if constexpr (sizeof(T) == 4) {
+    const uint32_t *p32 = reinterpret_cast<const uint32_t *>(p);
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      if ((uint32_t)i < n) x.w[i] = p32[i];
+  } else {
+    constexpr int W = (int)sizeof(T);  // words of four elements
+    const uintptr_t a = (uintptr_t)p, first = a & ~(uintptr_t)3;
+    const uint32_t off = (uint32_t)(a & 3);
+    if (n == 4 && first >= (uintptr_t)src && first + 4 * (W + 1) <= (uintptr_t)(src + total)) {
+      const uint32_t *p32 = reinterpret_cast<const uint32_t *>(first);
+      uint32_t v[W + 1];
+#pragma unroll
+      for (int i = 0; i <= W; i++) v[i] = p32[i];
+#pragma unroll
+      for (int i = 0; i < W; i++) x.w[i] = __funnelshift_r(v[i], v[i + 1], 8 * off);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if ((uint32_t)i < n) {
+          if constexpr (sizeof(T) == 1) x.w[0] |= (uint32_t)(uint8_t)p[i] << (8 * i);
+          else x.w[i >> 1] |= (uint32_t)(uint16_t)p[i] << (16 * (i & 1));
+        }
+    }
+  }
+  return x;
+}
+
+template <typename T>
+__device__ __forceinline__ T elem_of(const Raw4<T> &x, int i) {
+  if constexpr (sizeof(T) == 1) return (T)(x.w[0] >> (8 * i));
+  else if constexpr (sizeof(T) == 2) return (T)(x.w[i >> 1] >> (16 * (i & 1)));
+  else if constexpr (std::is_same<T, float>::value) return __uint_as_float(x.w[i]);
+  else return (T)x.w[i];
+}
+
+// The low byte of (int64)x.  The 32-bit conversion gives it, saturation
+// included, but for 2^31 <= x < 2^63, whose low byte is 0 (a float that large
+// is a multiple of 2^8) where the 32-bit conversion saturates to 0x7FFFFFFF.
+__device__ __forceinline__ uint32_t low_byte(float x) {
+  const uint32_t v = (uint32_t)__float2int_rz(x);
+  return (x >= 2147483648.f && x < 9223372036854775808.f) ? 0u : (v & 0xffu);
+}
+
+// quantize<float> (gemmbitserial.hpp:170-186): bipolar maps x > 0 to 1; a
+// negative x of a signed matrix becomes 2^(w-1) + (uint8_t)(x + 2^(w-1)), the
+// sum taken in float; otherwise (uint8_t)x.  Float -> integer casts truncate
+// toward zero, then keep the low byte.
+__device__ __forceinline__ uint32_t code_of_f32(float x, int bipolar, int issigned, int nbits) {
+  if (bipolar) return x > 0.f ? 1u : 0u;
+  if (issigned && x < 0.f) {
+    const int h = 1 << (nbits - 1);
+    return ((uint32_t)h + low_byte(x + (float)h)) & 0xffu;
+  }
+  return low_byte(x);
+}
+
+__device__ __forceinline__ uint32_t pack4(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  return __byte_perm(__byte_perm(a, b, 0x0040u), __byte_perm(c, d, 0x0040u), 0x5410u);
+}
+
+// Codes of importRegular<T> for four elements, one byte each.
+template <typename T>
+__device__ __forceinline__ uint32_t codes4(const Raw4<T> &x, int bipolar, int issigned, int nbits) {
+  if constexpr (std::is_same<T, uint8_t>::value) {
+    return x.w[0];  // the uint8_t overload keeps the raw byte, bipolar or not
+  } else if constexpr (std::is_same<T, float>::value) {
+    uint32_t c[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) c[i] = code_of_f32(__uint_as_float(x.w[i]), bipolar, issigned, nbits);
+    return pack4(c[0], c[1], c[2], c[3]);
+  } else if (bipolar) {
+    if constexpr (sizeof(T) == 1) return __vcmpgts4(x.w[0], 0u) & 0x01010101u;
+    return pack4(elem_of<T>(x, 0) > 0, elem_of<T>(x, 1) > 0, elem_of<T>(x, 2) > 0, elem_of<T>(x, 3) > 0);
+  } else {
+    if constexpr (sizeof(T) == 1) return x.w[0];
+    else if constexpr (sizeof(T) == 2) return __byte_perm(x.w[0], x.w[1], 0x6420u);
+    else return pack4(x.w[0], x.w[1], x.w[2], x.w[3]);
+  }
+}
+
 // importRegularAndQuantize<T> (gemmbitserial.hpp:282-305): element x of row r
 // becomes the index of the first threshold thr[t * nrows + r] with x <= thr
 // (compared in T), or nthres when x exceeds them all; with no thresholds the
-// element keeps its own value.  The low byte of that code is the code the
+// element keeps its own value.  The low byte of that index is the code the
 // planes store (the (uint8_t) cast of :298).  For float input without
-// thresholds the float is truncated toward zero to an integer first.
-template <typename T>
-__device__ __forceinline__ uint32_t own_code(T x) {
-  return (uint32_t)(int64_t)x & 0xFFu;
-}
-
-template <typename T>
-__device__ __forceinline__ uint32_t threshold_code(T x, const T *__restrict__ thr, int nthres, uint64_t r,
-                                                   uint64_t nrows) {
-  if (nthres == 0) return own_code(x);
-  int t = 0;
-  for (; t < nthres; t++)
-    if (x <= thr[(uint64_t)t * nrows + r]) break;
-  return (uint32_t)t & 0xFFu;
-}
-
-// Row-major: a warp per 1024-column segment of a padded row, lane = 32
-// columns.  Column-major (matrix[c * nrows + r]): a warp per 32 x 32 block,
-// lane = row, so the lanes' loads of one column are contiguous.  Either way a
-// lane ends up with 32 consecutive columns of one row and stores them like
-// the regular import (planes, and digits when requested).
-template <typename T>
-__global__ void __launch_bounds__(256) pack_quantize_kernel(const T *__restrict__ src, const T *__restrict__ thr,
-                                                            int nthres, int nbits, uint64_t nrows, uint64_t ncols,
-                                                            uint64_t nrows_a, uint64_t wpr, int col_major,
-                                                            uint64_t *__restrict__ planes,
-                                                            uint8_t *__restrict__ digits, uint64_t dcols, uint4 dtab) {
-  const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  uint64_t r, col0;
-  if (!col_major) {
-    const uint64_t segs = segs_per_row(wpr);
-    if (warp >= nrows_a * segs) return;
-    r = warp / segs;
-    col0 = (warp % segs) * kSegCols + (uint64_t)lane * 32;
-  } else {
-    const uint64_t cblocks = wpr * 2;
-    if (warp >= ((nrows_a + 31) / 32) * cblocks) return;
-    r = (warp / cblocks) * 32 + lane;
-    col0 = (warp % cblocks) * 32;
-    if (r >= nrows_a) return;  // lanes past the padded rows (no warp-wide step follows)
+// thresholds the float is truncated toward zero to an integer first.  The
+// four elements are scanned together, row r + i * RSTEP each (RSTEP 0: four
+// columns of a row; 1: four rows of a column; a row past nrows, whose code is
+// not wanted, reads the last row's thresholds).
+template <typename T, int RSTEP>
+__device__ __forceinline__ uint32_t threshold_codes4(const Raw4<T> &x, const T *__restrict__ thr, int nthres,
+                                                     uint64_t r, uint64_t nrows) {
+  uint32_t c[4];
+  if (nthres == 0) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      if constexpr (std::is_same<T, float>::value) c[i] = low_byte(elem_of<T>(x, i));
+      else c[i] = (uint32_t)elem_of<T>(x, i) & 0xffu;
+    }
+    return pack4(c[0], c[1], c[2], c[3]);
   }
-  if (col0 >= wpr * 64) return;
+  const T *p[RSTEP ? 4 : 1];
+#pragma unroll
+  for (int i = 0; i < (RSTEP ? 4 : 1); i++) p[i] = thr + (r + i < nrows ? r + i : nrows - 1);
+  T v[4];
+  bool over[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    v[i] = elem_of<T>(x, i);
+    over[i] = true;
+    c[i] = 0u;
+  }
+#pragma unroll 4
+  for (int t = 0; t < nthres; t++) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      over[i] = over[i] && !(v[i] <= p[RSTEP ? i : 0][(uint64_t)t * nrows]);
+      c[i] += over[i] ? 1u : 0u;
+    }
+    if ((t & 7) == 7 && !(over[0] || over[1] || over[2] || over[3])) break;
+  }
+  return pack4(c[0], c[1], c[2], c[3]);
+}
+
+// Row-major sources of any element type and alignment.  A warp loads the unit's
+// 1024 columns four elements a lane, 8 lanes to a chunk, so that its loads
+// are contiguous whatever the element size (a lane loading the 32 columns it
+// packs strides 32 elements from its neighbour, and every load then touches
+// 32 lines: 60 us for 2048 x 4096 floats); the codes, a word of four, change
+// hands through shared memory.  All eight loads are in flight before the first is converted.
+// Word j of chunk i lies at 8 i + (j ^ 4 (i / 4 & 1)): the 16-byte reads of
+// whole chunks then meet no bank conflict.
+template <typename T, bool QUANT, bool ALIGNED>
+__device__ __forceinline__ void pack_staged_unit(const PackJob &J, const T *__restrict__ thr, int nthres,
+                                                 uint64_t row0, uint64_t rend, uint64_t u, uint32_t *__restrict__ st) {
+  const uint32_t lane = threadIdx.x & 31, j = lane & 7;
+  const UnitBase b = unit_base(J.cpr, row0, u);
+  const uint64_t total = J.nrows * J.ncols;
+  const int bip = J.nbits == 1 && J.issigned;
+  Raw4<T> x[8];
+#pragma unroll
+  for (int s = 0; s < 8; s++) {
+    uint64_t r;
+    uint32_t cc;
+    unit_chunk(b, 4 * s + (lane >> 3), J.cpr, J.magic, r, cc);
+    const uint64_t col = (uint64_t)cc * 32 + 4 * j;
+    const uint32_t n = (r < J.nrows && col < J.ncols) ? (uint32_t)min((uint64_t)4, J.ncols - col) : 0u;
+    x[s] = load4<T, ALIGNED>((const T *)J.src, r * J.ncols + col, n, total);
+  }
+#pragma unroll
+  for (int s = 0; s < 8; s++) {
+    uint32_t w;
+    if (QUANT) {
+      uint64_t r;
+      uint32_t cc;
+      unit_chunk(b, 4 * s + (lane >> 3), J.cpr, J.magic, r, cc);
+      const uint64_t col = (uint64_t)cc * 32 + 4 * j;
+      const uint32_t n = (r < J.nrows && col < J.ncols) ? (uint32_t)min((uint64_t)4, J.ncols - col) : 0u;
+      w = n ? threshold_codes4<T, 0>(x[s], thr, nthres, r, J.nrows) : 0u;
+      if (n < 4) w &= (1u << (8 * n)) - 1u;  // the code of a 0 put past the row's end is no code
+    } else {
+      w = codes4<T>(x[s], bip, J.issigned, J.nbits);
+    }
+    st[(4 * s + (lane >> 3)) * 8 + (j ^ ((s & 1) << 2))] = w;
+  }
+  __syncwarp();
+  uint64_t r;
+  uint32_t cc, q[8];
+  unit_chunk(b, lane, J.cpr, J.magic, r, cc);
+  const uint32_t sw = ((lane >> 2) & 1u) << 2;
+  const uint4 v0 = *reinterpret_cast<const uint4 *>(st + lane * 8 + sw);
+  const uint4 v1 = *reinterpret_cast<const uint4 *>(st + lane * 8 + (sw ^ 4u));
+  q[0] = v0.x; q[1] = v0.y; q[2] = v0.z; q[3] = v0.w;
+  q[4] = v1.x; q[5] = v1.y; q[6] = v1.z; q[7] = v1.w;
+  if (r < rend) emit_chunk(J, r, cc, q);
+  __syncwarp();  // the next unit writes the staging words again
+}
+
+template <typename T, bool QUANT, bool ALIGNED>
+__global__ void __launch_bounds__(256) pack_staged(const __grid_constant__ PackJob J, const T *__restrict__ thr,
+                                                   int nthres, uint64_t row0, uint64_t rend, uint64_t units) {
+  __shared__ __align__(16) uint32_t st[8][256];
+  const uint64_t u = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (u >= units) return;  // warp-uniform; no block-wide barrier follows
+  pack_staged_unit<T, QUANT, ALIGNED>(J, thr, nthres, row0, rend, u, st[threadIdx.x >> 5]);
+}
+
+// ---------------------------------------------------------------- column-major sources
+
+// The reference's readColMajor: element (r, c) at c * nrows + r.  A block takes
+// 64 rows x 256 columns: threads load four consecutive rows of a column (a
+// vector load where ALIGNED allows), put the code word in shared memory, and
+// then each takes one chunk.  (Loading a column's rows one byte at a time by a
+// lane per column, each lane a whole column apart from the next, ran 15 us on
+// 169 x 2304.)  256 columns make the plane stores whole 32-byte sectors; 512
+// threads have the tile's loads in flight at once (128 threads in four
+// batches: 11.7 us on 169 x 2304, whose 27 tiles leave most SMs idle).  Word g
+// (rows 4g ..) of column c lies at 17 c + 4 (c / 32) + g: the warp's 8 chunks
+// read 8 different banks.
+constexpr int kCmRows = 64, kCmCols = 256, kCmThreads = 512;
+constexpr int kCmWords = kCmCols * 17 + 4 * (kCmCols / 32);
+
+template <typename T, bool QUANT, bool ALIGNED>
+__global__ void __launch_bounds__(kCmThreads) pack_colmajor(const __grid_constant__ PackJob J,
+                                                            const T *__restrict__ thr, int nthres) {
+  __shared__ uint32_t st[kCmWords];
+  // neighbouring blocks take neighbouring rows of the same columns: their reads are contiguous
+  const uint32_t rblocks = (uint32_t)((J.nrows_a + kCmRows - 1) / kCmRows);
+  const uint64_t r0 = (uint64_t)(blockIdx.x % rblocks) * kCmRows, c0 = (uint64_t)(blockIdx.x / rblocks) * kCmCols;
+  const uint32_t tid = threadIdx.x;
+  const uint64_t total = J.nrows * J.ncols;
+  const int bip = J.nbits == 1 && J.issigned;
+  constexpr int kLoads = kCmCols * (kCmRows / 4) / kCmThreads;  // a thread's row quadruples, all in flight at once
+  Raw4<T> x[kLoads];
+#pragma unroll
+  for (int i = 0; i < kLoads; i++) {
+    const uint32_t t = i * kCmThreads + tid;
+    const uint64_t c = c0 + (t >> 4), r = r0 + 4 * (t & 15);
+    const uint32_t n = (c < J.ncols && r < J.nrows) ? (uint32_t)min((uint64_t)4, J.nrows - r) : 0u;
+    x[i] = load4<T, ALIGNED>((const T *)J.src, c * J.nrows + r, n, total);
+  }
+#pragma unroll
+  for (int i = 0; i < kLoads; i++) {
+    const uint32_t t = i * kCmThreads + tid, col = t >> 4, g = t & 15;
+    uint32_t w;
+    if (QUANT) {
+      const uint64_t c = c0 + col, r = r0 + 4 * g;
+      const uint32_t n = (c < J.ncols && r < J.nrows) ? (uint32_t)min((uint64_t)4, J.nrows - r) : 0u;
+      w = n ? threshold_codes4<T, 1>(x[i], thr, nthres, r, J.nrows) : 0u;
+      if (n < 4) w &= (1u << (8 * n)) - 1u;
+    } else {
+      w = codes4<T>(x[i], bip, J.issigned, J.nbits);
+    }
+    st[col * 17 + 4 * (col >> 5) + g] = w;
+  }
+  __syncthreads();
+  // a thread per (row, chunk): lanes 0..7 of a row its 8 chunks, four rows of a quadruple a warp
+  const uint32_t k = tid & 7, i = (tid >> 3) & 3, g = tid >> 5;
+  const uint64_t cc = c0 / 32 + k, r = r0 + 4 * g + i;
+  if (cc >= J.cpr || r >= J.nrows_a) return;
+  const uint32_t *p = st + k * (32 * 17 + 4) + g;
+  const uint32_t sel = i | ((i + 4) << 4);  // byte i of two words
   uint32_t q[8];
 #pragma unroll
-  for (int i = 0; i < 8; i++) q[i] = 0u;
-  if (r < nrows) {
-#pragma unroll
-    for (int j = 0; j < 32; j++) {
-      const uint64_t c = col0 + j;
-      if (c < ncols) {
-        const T x = src[col_major ? c * nrows + r : r * ncols + c];
-        q[j >> 2] |= threshold_code(x, thr, nthres, r, nrows) << (8 * (j & 3));
-      }
-    }
-  }
-  emit_planes32(nbits, nrows_a, wpr, planes, r, col0, q);
-  if (digits && r < nrows) write_digits32(digits, nbits, nrows, ncols, dcols, dtab, r, col0, q);
+  for (int w = 0; w < 8; w++)
+    q[w] = __byte_perm(__byte_perm(p[(4 * w) * 17], p[(4 * w + 1) * 17], sel),
+                       __byte_perm(p[(4 * w + 2) * 17], p[(4 * w + 3) * 17], sel), 0x5410u);
+  emit_chunk(J, r, (uint32_t)cc, q);
 }
 
-// Index of the job owning global warp w: the last job with warp0 <= w.
-__device__ __forceinline__ int find_job(const PackJob *jobs, int njobs, uint64_t w) {
-  int lo = 0, hi = njobs - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (jobs[mid].warp0 <= w) lo = mid;
-    else hi = mid - 1;
+// ---------------------------------------------------------------- grouped import
+
+// The job owning run w (the last with warp0 <= w), found by the whole warp: 32
+// jobs probed a step, so 1024 jobs take two dependent loads, not ten.
+__device__ __forceinline__ int find_job(const PackJob *jobs, int njobs, uint64_t w, int lane) {
+  int lo = 0, n = njobs;  // the answer is in [lo, lo + n)
+  while (n > 1) {
+    const int step = (n + 31) / 32;
+    const int j = lo + lane * step;
+    const unsigned m = __ballot_sync(kFull, j < lo + n && jobs[j].warp0 <= w);  // lane 0 is always set
+    const int k = 31 - __clz(m);
+    n = min(step, n - k * step);
+    lo += k * step;
   }
   return lo;
 }
 
-// Grouped import: one launch packs every operand of a grouped GEMM
-// (row-major sources); units (1024-column segments of a row) are numbered
-// across the jobs.  A warp takes kRun consecutive units: one job lookup,
-// then the units in order.
-constexpr int kRun = 8;
+// One launch packs every operand of a grouped GEMM whose rows are 1-byte and
+// 16-byte aligned.  A run is `run` units of one job (pack_run_units: up to
+// kMaxRun, fewer when the group would leave warps without one); a warp takes
+// runs in a grid stride and keeps kDepth units' loads in flight.
+// HBM-bound on large groups: 7.7 GB of the 512-problem mix (1-byte sources in,
+// planes and nibble or digit matrices out) in 1.23 ms, 0.92 of the copy rate;
+// one strided pair of 16-byte loads per lane, a unit to a row segment and a
+// binary search per run took 2.17 ms.
+constexpr int kMaxRun = 8;
+constexpr int kDepth = 2;
 
-__global__ void __launch_bounds__(256) pack_grouped(const PackJob *__restrict__ jobs, int njobs, uint64_t total) {
+__device__ __forceinline__ void load_run_bytes(const PackJob &J, const UnitBase &b, uint32_t i, uint64_t &r,
+                                               uint32_t &cc, uint32_t (&q)[8]) {
+  unit_chunk(b, i, J.cpr, J.magic, r, cc);
+  if (J.vec == 2) load_bytes32<2>(J.src, J.nrows, J.ncols, r, cc, q);
+  else load_bytes32<1>(J.src, J.nrows, J.ncols, r, cc, q);
+}
+
+__global__ void __launch_bounds__(256, 4) pack_grouped(const PackJob *__restrict__ jobs, int njobs, uint64_t runs,
+                                                       uint32_t run) {
+  __shared__ PackJob sj[8];  // each warp's job: its fields stay out of the registers
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   const int lane = threadIdx.x & 31;
-  for (uint64_t base = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kRun; base < total;
-       base += nw * kRun) {
-    int j = find_job(jobs, njobs, base);
-    // unit w -> (job, row, segment), advancing the job index monotonically
-    auto locate = [&](uint64_t w, int &jj, uint64_t &r, uint64_t &sg) {
-      while (jj + 1 < njobs && jobs[jj + 1].warp0 <= w) jj++;
-      const PackJob &J = jobs[jj];
-      const uint64_t local = w - J.warp0;
-      if (local < 0xFFFFFFFFull) {  // 32-bit division in the common case
-        const uint32_t l32 = (uint32_t)local, r32 = l32 / J.segs;
-        r = r32;
-        sg = l32 - r32 * J.segs;
-      } else {
-        r = local / J.segs;
-        sg = local % J.segs;
-      }
-    };
-    auto load = [&](int jj, uint64_t r, uint64_t sg, uint32_t (&q)[8]) {
-      const PackJob &J = jobs[jj];
-      const uint64_t col0 = sg * kSegCols + (uint64_t)lane * 32;
-      if (col0 < J.wpr * 64)
-        load_codes32(J.src, J.dtype, J.nbits == 1 && J.issigned, J.issigned, J.nbits, J.nrows, J.ncols, J.vec, r,
-                     col0, q);
-    };
-    // the next unit's loads are in flight while the current unit is packed
-    const uint64_t last = min(base + (uint64_t)kRun, total);
-    int jc = j;
-    uint64_t rc, sc;
-    locate(base, jc, rc, sc);
-    uint32_t q[8];
-    load(jc, rc, sc, q);
+  PackJob &J = sj[threadIdx.x >> 5];
+  for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < runs; w += nw) {
+    const int j = find_job(jobs, njobs, w, lane);
+    static_assert(sizeof(PackJob) % 8 == 0 && sizeof(PackJob) / 8 <= 32, "one word a lane");
+    __syncwarp();
+    if (lane < (int)(sizeof(PackJob) / 8))
+      reinterpret_cast<uint64_t *>(&J)[lane] = reinterpret_cast<const uint64_t *>(jobs + j)[lane];
+    __syncwarp();
+    const UnitBase b = unit_base(J.cpr, 0, (w - J.warp0) * run);
+    const int bip = J.nbits == 1 && J.issigned;
 #pragma unroll 1
-    for (uint64_t w = base; w < last; w++) {
-      int jn = jc;
-      uint64_t rn = 0, sn = 0;
-      uint32_t qn[8];
-      if (w + 1 < last) {
-        locate(w + 1, jn, rn, sn);
-        load(jn, rn, sn, qn);
-      }
-      const PackJob &J = jobs[jc];
-      const uint64_t col0 = sc * kSegCols + (uint64_t)lane * 32;
-      if (col0 < J.wpr * 64) {
-        emit_planes32(J.nbits, J.nrows_a, J.wpr, J.planes, rc, col0, q);
-        if (J.digits && rc < J.nrows) {
-          const uint4 tab = make_uint4(J.dtab[0], J.dtab[1], J.dtab[2], J.dtab[3]);
-          write_digits32(J.digits, J.nbits, J.nrows, J.ncols, J.dcols, tab, rc, col0, q);
-        }
-        if (J.nibbles && rc < J.nrows) write_nibbles32(J.nibbles, J.nbits, J.dcols, rc, col0, q);
-      }
-      if (w + 1 < last) {
-        jc = jn;
-        rc = rn;
-        sc = sn;
+    for (uint32_t u = 0; u < run; u += kDepth) {
+      uint64_t r[kDepth];
+      uint32_t cc[kDepth], q[kDepth][8];
 #pragma unroll
-        for (int i = 0; i < 8; i++) q[i] = qn[i];
+      for (uint32_t d = 0; d < kDepth; d++)
+        if (u + d < run) load_run_bytes(J, b, 32 * (u + d) + lane, r[d], cc[d], q[d]);
+#pragma unroll
+      for (uint32_t d = 0; d < kDepth; d++) {
+        if (u + d >= run) break;
+        codes_of_bytes(J.dtype, bip, q[d]);
+        if (r[d] < J.nrows_a) emit_chunk(J, r[d], cc[d], q[d]);
       }
     }
   }
 }
 
-// Column-major pack (the reference's readColMajor: element (r, c) at c*nrows + r).
-// One warp covers 32 padded rows x 64 columns (one word per row and plane):
-// lane l reads column c0+l (then c0+32+l) down the 32 rows, and one ballot per
-// (row, plane) gathers 32 columns of that row.  Lane j keeps row j's word.
-__global__ void __launch_bounds__(256) pack_colmajor(const void *__restrict__ src, int dtype, int bipolar,
-                                                     int issigned, int nbits, uint64_t nrows, uint64_t ncols,
-                                                     uint64_t nrows_a, uint64_t wpr,
-                                                     uint64_t *__restrict__ planes) {
-  const uint64_t rgroups = (nrows_a + 31) / 32;
-  const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// The same for the other operands (wider elements, unaligned rows).
+template <typename T>
+__device__ __forceinline__ void pack_staged_run(const PackJob &J, uint64_t u0, uint32_t run, uint32_t *st) {
+  const uint64_t units = min((uint64_t)run, (J.nrows_a * J.cpr + 31) / 32 - u0);
+#pragma unroll 1
+  for (uint64_t u = u0; u < u0 + units; u++) {
+    if (J.vec) pack_staged_unit<T, false, true>(J, nullptr, 0, 0, J.nrows_a, u, st);
+    else pack_staged_unit<T, false, false>(J, nullptr, 0, 0, J.nrows_a, u, st);
+  }
+}
+
+__global__ void __launch_bounds__(256) pack_grouped_staged(const PackJob *__restrict__ jobs, int njobs,
+                                                           uint64_t runs, uint32_t run) {
+  __shared__ __align__(16) uint32_t st[8][256];
+  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (warp >= rgroups * wpr) return;  // warp-uniform
-  const uint64_t w = warp / rgroups, r0 = (warp % rgroups) * 32;
-  uint32_t lo[kMaxBits], hi[kMaxBits];
-#pragma unroll
-  for (int b = 0; b < kMaxBits; b++) lo[b] = hi[b] = 0u;
-#pragma unroll
-  for (int half = 0; half < 2; half++) {
-    const uint64_t c = w * 64 + half * 32 + lane;
-    uint32_t q[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};  // codes of rows r0..r0+31 of column c
-    if (c < ncols) {
-#pragma unroll
-      for (int j = 0; j < 32; j++) {
-        uint64_t r = r0 + j;
-        if (r < nrows) q[j >> 2] |= elem_code(src, dtype, c * nrows + r, bipolar, issigned, nbits) << (8 * (j & 3));
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 32; j++) {
-      uint32_t code = (q[j >> 2] >> (8 * (j & 3))) & 0xffu;
-#pragma unroll
-      for (int b = 0; b < kMaxBits; b++) {
-        if (b < nbits) {
-          uint32_t m = __ballot_sync(kFull, (code >> b) & 1u);
-          if (lane == j) { if (half) hi[b] = m; else lo[b] = m; }
-        }
-      }
+  uint32_t *my = st[threadIdx.x >> 5];
+  for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < runs; w += nw) {
+    const PackJob &J = jobs[find_job(jobs, njobs, w, lane)];
+    const uint64_t u0 = (w - J.warp0) * run;
+    switch (J.dtype) {
+      case GBS_I8: pack_staged_run<int8_t>(J, u0, run, my); break;
+      case GBS_U8: pack_staged_run<uint8_t>(J, u0, run, my); break;
+      case GBS_I16: pack_staged_run<int16_t>(J, u0, run, my); break;
+      case GBS_I32: pack_staged_run<int32_t>(J, u0, run, my); break;
+      default: pack_staged_run<float>(J, u0, run, my); break;
     }
   }
-  const uint64_t plane_words = nrows_a * wpr;
-  const uint64_t r = r0 + lane;
-  if (r >= nrows_a) return;  // the last group's lanes past the padded rows
-#pragma unroll
-  for (int b = 0; b < kMaxBits; b++)
-    if (b < nbits) planes[b * plane_words + r * wpr + w] = (uint64_t)lo[b] | ((uint64_t)hi[b] << 32);
 }
 
 // sumRows (arch-generic.hpp:6-37) of row r by one warp.  uint32 arithmetic
@@ -417,7 +610,7 @@ __global__ void __launch_bounds__(256) rowsum_grouped(const PackJob *__restrict_
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   const int lane = threadIdx.x & 31;
   for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < total; w += nw) {
-    const PackJob &J = jobs[find_job(jobs, njobs, w)];
+    const PackJob &J = jobs[find_job(jobs, njobs, w, lane)];
     const uint64_t r = w - J.warp0;
     const int32_t v = row_sum(J.planes, J.nbits, J.issigned, J.ncols, J.nrows_a, J.wpr, r, lane);
     if (lane == 0) J.rowsum[r] = v;
@@ -447,17 +640,116 @@ inline unsigned blocks_for(uint64_t threads, unsigned per_block) {
 
 }  // namespace
 
+PackJob make_pack_job(const Mat &m, const void *src, int dtype, uint8_t *digits, const uint32_t *dtab,
+                      uint8_t *nibbles) {
+  PackJob j;
+  memset(&j, 0, sizeof(j));
+  j.src = src;
+  j.planes = m.planes;
+  j.digits = digits;
+  j.nibbles = nibbles;
+  j.nrows = m.nrows;
+  j.ncols = m.ncols;
+  j.nrows_a = m.nrows_a;
+  j.wpr = m.wpr();
+  j.dcols = m.dcols;
+  j.nbits = (int)m.nbits;
+  j.issigned = m.issigned;
+  j.dtype = dtype;
+  j.cpr = (uint32_t)(m.ncols_a / 32);
+  j.magic = j.cpr ? (uint32_t)((1ull << 32) / j.cpr) + 1u : 0u;
+  if (dtab)
+    for (int i = 0; i < 4; i++) j.dtab[i] = dtab[i];
+  return j;
+}
+
+// 2 / 1: 1-byte rows, 32- / 16-byte aligned, packed by a load per lane; 0:
+// the staged kernels.
+static int bytes_vec(const Mat &m, const void *src, int dtype) {
+  if (dtype != GBS_I8 && dtype != GBS_U8) return 0;
+  const uintptr_t a = (uintptr_t)src | (uintptr_t)m.ncols;
+  return a % 32 == 0 ? 2 : (a % 16 == 0 ? 1 : 0);
+}
+
+// Four consecutive elements can be one vector load: `run` (columns, or rows
+// column-major) and the source's address allow it.
+static bool aligned4(const void *src, int dtype, uint64_t run) {
+  const uintptr_t size = (dtype == GBS_I16) ? 2 : (dtype == GBS_I32 || dtype == GBS_F32) ? 4 : 1;
+  return run % 4 == 0 && (uintptr_t)src % (4 * size) == 0;
+}
+
+bool pack_job_direct(PackJob &j, const Mat &m) {
+  j.vec = bytes_vec(m, j.src, j.dtype);
+  if (j.vec) return true;
+  j.vec = aligned4(j.src, j.dtype, m.ncols) ? 1 : 0;
+  return false;
+}
+
+uint64_t pack_job_units(const PackJob &j) { return (j.nrows_a * j.cpr + 31) / 32; }
+
+// Units per run of a grouped import of `units` units: enough runs for 32 warps
+// on each of 152 SMs before a run grows past one unit (CaffeNet's 1.2 M
+// unaligned bytes in runs of 8 were 147 warps and 48 us).
+uint32_t pack_run_units(uint64_t units) {
+  return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(kMaxRun, units / (152 * 32)));
+}
+
+namespace {
+
+// Calls f with the source's element type and whether four elements load as one vector.
+template <typename F>
+void with_source(int dtype, bool aligned, F f) {
+  auto go = [&](auto t) {
+    if (aligned) f(t, std::true_type{});
+    else f(t, std::false_type{});
+  };
+  switch (dtype) {
+    case GBS_I8: go(int8_t{}); break;
+    case GBS_U8: go(uint8_t{}); break;
+    case GBS_I16: go(int16_t{}); break;
+    case GBS_I32: go(int32_t{}); break;
+    default: go(float{}); break;
+  }
+}
+
+cudaError_t run_staged(const PackJob &j, const void *thr, int nthres, bool quant, bool aligned, uint64_t r0,
+                       uint64_t r1, cudaStream_t s) {
+  const uint64_t units = ((r1 - r0) * j.cpr + 31) / 32;
+  with_source(j.dtype, aligned, [&](auto t, auto al) {
+    using T = decltype(t);
+    constexpr bool A = decltype(al)::value;
+    if (quant)
+      pack_staged<T, true, A><<<blocks_for(units * 32, 256), 256, 0, s>>>(j, (const T *)thr, nthres, r0, r1, units);
+    else
+      pack_staged<T, false, A><<<blocks_for(units * 32, 256), 256, 0, s>>>(j, nullptr, 0, r0, r1, units);
+  });
+  count_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t run_colmajor(const PackJob &j, const void *thr, int nthres, bool quant, cudaStream_t s) {
+  const uint64_t blocks = ((j.nrows_a + kCmRows - 1) / kCmRows) * ((j.wpr * 64 + kCmCols - 1) / kCmCols);
+  if (blocks > 0x7FFFFFFFull) return cudaErrorInvalidConfiguration;
+  with_source(j.dtype, aligned4(j.src, j.dtype, j.nrows), [&](auto t, auto al) {
+    using T = decltype(t);
+    constexpr bool A = decltype(al)::value;
+    if (quant) pack_colmajor<T, true, A><<<(unsigned)blocks, kCmThreads, 0, s>>>(j, (const T *)thr, nthres);
+    else pack_colmajor<T, false, A><<<(unsigned)blocks, kCmThreads, 0, s>>>(j, nullptr, 0);
+  });
+  count_launch();
+  return cudaGetLastError();
+}
+
+}  // namespace
+
 cudaError_t launch_pack_rows(const Mat &m, const void *src, int dtype, uint64_t r0, uint64_t r1, uint8_t *digits,
                              const uint32_t *dtab, cudaStream_t s) {
   if (m.nrows_a == 0 || m.wpr() == 0 || r1 <= r0) return cudaSuccess;
-  const int bip = m.bipolar() ? 1 : 0;
-  const size_t esz = dtype == GBS_I16 ? 2 : (dtype == GBS_I32 || dtype == GBS_F32) ? 4 : 1;
-  const int vec = (esz == 1 && m.ncols % 16 == 0 && ((uintptr_t)src % 16) == 0) ? 1 : 0;
-  const uint64_t warps = (r1 - r0) * segs_per_row(m.wpr());
-  const uint4 tab = dtab ? make_uint4(dtab[0], dtab[1], dtab[2], dtab[3]) : make_uint4(0u, 0u, 0u, 0u);
-  pack_rowmajor<<<blocks_for(warps * 32, 256), 256, 0, s>>>(src, dtype, bip, m.issigned, (int)m.nbits, m.nrows, m.ncols,
-                                                          m.nrows_a, m.wpr(), vec, m.planes, r0, r1 - r0,
-                                                          digits, m.dcols, tab);
+  PackJob j = make_pack_job(m, src, dtype, digits, dtab, nullptr);
+  if (!pack_job_direct(j, m)) return run_staged(j, nullptr, 0, false, j.vec != 0, r0, r1, s);
+  const uint64_t units = ((r1 - r0) * j.cpr + 31) / 32;
+  if (j.vec == 2) pack_bytes<2><<<blocks_for(units * 32, 256), 256, 0, s>>>(j, r0, r1, units);
+  else pack_bytes<1><<<blocks_for(units * 32, 256), 256, 0, s>>>(j, r0, r1, units);
   count_launch();
   return cudaGetLastError();
 }
@@ -465,43 +757,24 @@ cudaError_t launch_pack_rows(const Mat &m, const void *src, int dtype, uint64_t 
 cudaError_t launch_pack_quantize(const Mat &m, const void *src, const void *thr, int nthres, int dtype,
                                  int col_major, uint8_t *digits, const uint32_t *dtab, cudaStream_t s) {
   if (m.nrows_a == 0 || m.wpr() == 0) return cudaSuccess;
-  const uint64_t warps = col_major ? ((m.nrows_a + 31) / 32) * m.wpr() * 2 : m.nrows_a * segs_per_row(m.wpr());
-  const unsigned blocks = blocks_for(warps * 32, 256);
-  const uint4 tab = dtab ? make_uint4(dtab[0], dtab[1], dtab[2], dtab[3]) : make_uint4(0u, 0u, 0u, 0u);
-#define GBS_QLAUNCH(T)                                                                                              \
-  pack_quantize_kernel<T><<<blocks, 256, 0, s>>>((const T *)src, (const T *)thr, nthres, (int)m.nbits, m.nrows,      \
-                                                 m.ncols, m.nrows_a, m.wpr(), col_major, m.planes, digits, m.dcols, \
-                                                 tab)
-  switch (dtype) {
-    case GBS_I8: GBS_QLAUNCH(int8_t); break;
-    case GBS_U8: GBS_QLAUNCH(uint8_t); break;
-    case GBS_I16: GBS_QLAUNCH(int16_t); break;
-    case GBS_I32: GBS_QLAUNCH(int32_t); break;
-    default: GBS_QLAUNCH(float); break;
-  }
-#undef GBS_QLAUNCH
-  count_launch();
-  return cudaGetLastError();
+  const PackJob j = make_pack_job(m, src, dtype, digits, dtab, nullptr);
+  if (col_major) return run_colmajor(j, thr, nthres, true, s);
+  return run_staged(j, thr, nthres, true, aligned4(src, dtype, m.ncols), 0, m.nrows_a, s);
 }
 
-cudaError_t launch_pack(const Mat &m, const void *src, int dtype, int col_major, cudaStream_t s) {
+cudaError_t launch_pack(const Mat &m, const void *src, int dtype, int col_major, uint8_t *digits,
+                        const uint32_t *dtab, cudaStream_t s) {
   if (m.nrows_a == 0 || m.wpr() == 0) return cudaSuccess;
-  const int bip = m.bipolar() ? 1 : 0;
-  if (!col_major) {
-    return launch_pack_rows(m, src, dtype, 0, m.nrows_a, nullptr, nullptr, s);
-  } else {
-    const uint64_t warps = ((m.nrows_a + 31) / 32) * m.wpr();
-    pack_colmajor<<<blocks_for(warps * 32, 256), 256, 0, s>>>(src, dtype, bip, m.issigned, (int)m.nbits, m.nrows, m.ncols,
-                                                            m.nrows_a, m.wpr(), m.planes);
-  }
-  count_launch();
-  return cudaGetLastError();
+  if (!col_major) return launch_pack_rows(m, src, dtype, 0, m.nrows_a, digits, dtab, s);
+  return run_colmajor(make_pack_job(m, src, dtype, digits, dtab, nullptr), nullptr, 0, false, s);
 }
 
-cudaError_t launch_pack_grouped(const PackJob *jobs, int njobs, uint64_t total_warps, cudaStream_t s) {
-  if (total_warps == 0 || njobs == 0) return cudaSuccess;
-  const uint64_t blocks = (total_warps + 8 * kRun - 1) / (8 * kRun);
-  pack_grouped<<<(unsigned)(blocks < 152 * 64 ? blocks : 152 * 64), 256, 0, s>>>(jobs, njobs, total_warps);
+cudaError_t launch_pack_grouped(const PackJob *jobs, int njobs, uint64_t runs, uint32_t run, bool direct,
+                                cudaStream_t s) {
+  if (runs == 0 || njobs == 0) return cudaSuccess;
+  const uint64_t blocks = std::min<uint64_t>((runs + 7) / 8, 152 * 64);
+  if (direct) pack_grouped<<<(unsigned)blocks, 256, 0, s>>>(jobs, njobs, runs, run);
+  else pack_grouped_staged<<<(unsigned)blocks, 256, 0, s>>>(jobs, njobs, runs, run);
   count_launch();
   return cudaGetLastError();
 }
