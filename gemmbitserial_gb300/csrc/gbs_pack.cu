@@ -66,15 +66,15 @@ __device__ __forceinline__ uint32_t digits4(uint32_t x, int nbits, uint4 tab) {
 // The lane's 32 digits (0 past ncols) into the digit matrix (dcols columns,
 // 16-row blocks: digit_offset) as one 32-byte store.  Digit rows past nrows
 // and columns past the planes' padded width stay as allocated: zero.
-__device__ __forceinline__ void write_digits32(uint8_t *__restrict__ digits, int nbits, uint64_t ncols, uint64_t dcols,
-                                               uint4 tab, uint64_t r, uint64_t col0, const uint32_t (&q)[8]) {
+__device__ __forceinline__ void write_digits32(uint8_t *__restrict__ digits, int nbits, uint32_t ncols, uint64_t dcols,
+                                               uint4 tab, uint32_t r, uint32_t col0, const uint32_t (&q)[8]) {
   uint32_t d[8];
 #pragma unroll
   for (int i = 0; i < 8; i++) d[i] = digits4(q[i], nbits, tab);
   if (col0 + 32 > ncols) {
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-      const uint64_t c = col0 + 4 * i;
+      const uint32_t c = col0 + 4 * i;
       if (c + 4 > ncols) d[i] &= c >= ncols ? 0u : (0xFFFFFFFFu >> (8 * (4 - (ncols - c))));
     }
   }
@@ -87,8 +87,8 @@ __device__ __forceinline__ void write_digits32(uint8_t *__restrict__ digits, int
 // nibble_offset): the low nbits bits of each code byte, two codes a byte
 // (even column low).  Codes past ncols are whatever the source gave: the
 // tensor-core kernel multiplies them by digits that are zero there.
-__device__ __forceinline__ void write_nibbles32(uint8_t *__restrict__ nib, int nbits, uint64_t dcols, uint64_t r,
-                                                uint64_t col0, const uint32_t (&q)[8]) {
+__device__ __forceinline__ void write_nibbles32(uint8_t *__restrict__ nib, int nbits, uint64_t dcols, uint32_t r,
+                                                uint32_t col0, const uint32_t (&q)[8]) {
   const uint32_t msk = 0x01010101u * ((1u << nbits) - 1u);
   uint32_t o[4];
 #pragma unroll
@@ -101,49 +101,60 @@ __device__ __forceinline__ void write_nibbles32(uint8_t *__restrict__ nib, int n
   *reinterpret_cast<uint4 *>(nib + nibble_offset(r, col0, dcols)) = make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-// Everything a chunk (row r, chunk cc of the row) writes.
-__device__ __forceinline__ void emit_chunk(const PackJob &J, uint64_t r, uint32_t cc, const uint32_t (&q)[8]) {
-  emit_planes32(J.nbits, reinterpret_cast<uint32_t *>(J.planes), J.nrows_a * J.cpr, r * J.cpr + cc, q);
-  if (r >= J.nrows) return;
-  const uint64_t col0 = (uint64_t)cc * 32;
+// Everything chunk cc of row r writes; idx is its number along the padded
+// rows, derived says whether the row is one of the matrix's own (padding rows
+// have no digits or nibbles).
+__device__ __forceinline__ void emit_chunk(const PackJob &J, uint64_t idx, uint32_t r, uint32_t cc, bool derived,
+                                           const uint32_t (&q)[8]) {
+  emit_planes32(J.nbits, reinterpret_cast<uint32_t *>(J.planes), J.nrows_a * J.cpr, idx, q);
+  if (!derived) return;
   if (J.digits)
-    write_digits32(J.digits, J.nbits, J.ncols, J.dcols, make_uint4(J.dtab[0], J.dtab[1], J.dtab[2], J.dtab[3]), r,
-                   col0, q);
-  if (J.nibbles) write_nibbles32(J.nibbles, J.nbits, J.dcols, r, col0, q);
+    write_digits32(J.digits, J.nbits, (uint32_t)J.ncols, J.dcols,
+                   make_uint4(J.dtab[0], J.dtab[1], J.dtab[2], J.dtab[3]), r, cc * 32, q);
+  if (J.nibbles) write_nibbles32(J.nibbles, J.nbits, J.dcols, r, cc * 32, q);
 }
 
 // ---------------------------------------------------------------- chunk numbering
 
-// A unit is 32 chunks, a lane each.  The unit's first chunk is located once;
-// the lanes then divide only small numbers: t = cc0 + i with i <= 31, and t /
-// cpr is a multiply-high by magic = 2^32 / cpr + 1 (exact while t * cpr <
-// 2^32, i < 32 (kMaxRun + 1)), or, for rows of 65000 chunks and more, 0 or 1.
+// A unit is 32 chunks, a lane each.  The unit's first chunk is located once, in
+// 64 bits: its row r, its chunk of the row cc, and how many rows from r on are
+// the matrix's own (rows) and to be written (rows_a).  The lanes then work in
+// 32 bits (integer arithmetic at half the rate of the other instructions is what
+// bounds these kernels once their loads are contiguous): chunk i is dr rows
+// further, t = cc + i divided by cpr through a multiply-high by magic = 2^32 /
+// cpr + 1 (exact while t * cpr < 2^32, i < 32 (kMaxRun + 1)), or, for rows of
+// 65000 chunks and more, 0 or 1.
 struct UnitBase {
   uint64_t r;
-  uint32_t cc;
+  uint32_t cc, rows, rows_a;
+};
+struct Chunk {
+  uint32_t dr, cc;
 };
 
-__device__ __forceinline__ UnitBase unit_base(uint32_t cpr, uint64_t row0, uint64_t unit) {
+__device__ __forceinline__ UnitBase unit_base(const PackJob &J, uint64_t row0, uint64_t rend, uint64_t unit) {
   const uint64_t c = unit * 32;
   UnitBase b;
   if (c <= 0xFFFFFFFFull) {
-    const uint32_t q = (uint32_t)c / cpr;
+    const uint32_t q = (uint32_t)c / J.cpr;
     b.r = row0 + q;
-    b.cc = (uint32_t)c - q * cpr;
+    b.cc = (uint32_t)c - q * J.cpr;
   } else {
-    const uint64_t q = c / cpr;
+    const uint64_t q = c / J.cpr;
     b.r = row0 + q;
-    b.cc = (uint32_t)(c - q * cpr);
+    b.cc = (uint32_t)(c - q * J.cpr);
   }
+  b.rows = J.nrows > b.r ? (uint32_t)min(J.nrows - b.r, (uint64_t)0x80000000u) : 0u;
+  b.rows_a = rend > b.r ? (uint32_t)min(rend - b.r, (uint64_t)0x80000000u) : 0u;
   return b;
 }
 
-__device__ __forceinline__ void unit_chunk(const UnitBase &b, uint32_t i, uint32_t cpr, uint32_t magic, uint64_t &r,
-                                           uint32_t &cc) {
+__device__ __forceinline__ Chunk unit_chunk(const UnitBase &b, uint32_t i, uint32_t cpr, uint32_t magic) {
   const uint32_t t = b.cc + i;
-  const uint32_t q = cpr < 65000u ? __umulhi(t, magic) : (t >= cpr ? 1u : 0u);
-  r = b.r + q;
-  cc = t - q * cpr;
+  Chunk c;
+  c.dr = cpr < 65000u ? __umulhi(t, magic) : (t >= cpr ? 1u : 0u);
+  c.cc = t - c.dr * cpr;
+  return c;
 }
 
 // ---------------------------------------------------------------- 1-byte rows, 16-byte aligned
@@ -152,13 +163,12 @@ __device__ __forceinline__ void unit_chunk(const UnitBase &b, uint32_t i, uint32
 // source 32-byte aligned) or two of 16 bytes (VEC 1).  A warp's two strided
 // 16-byte loads touch each sector twice; the single load touches it once.
 template <int VEC>
-__device__ __forceinline__ void load_bytes32(const void *src, uint64_t nrows, uint64_t ncols, uint64_t r, uint32_t cc,
-                                             uint32_t (&q)[8]) {
+__device__ __forceinline__ void load_bytes32(const PackJob &J, const UnitBase &b, const Chunk &c, uint32_t (&q)[8]) {
 #pragma unroll
   for (int i = 0; i < 8; i++) q[i] = 0u;
-  const uint64_t col0 = (uint64_t)cc * 32;
-  if (r >= nrows || col0 >= ncols) return;
-  const uint8_t *p = (const uint8_t *)src + r * ncols + col0;
+  const uint32_t col0 = c.cc * 32, ncols = (uint32_t)J.ncols;
+  if (c.dr >= b.rows || col0 >= ncols) return;
+  const uint8_t *p = (const uint8_t *)J.src + (b.r + c.dr) * J.ncols + col0;
   if (VEC == 2) {  // ncols is a multiple of 32: the chunk is whole
     asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7])
@@ -185,20 +195,21 @@ __global__ void __launch_bounds__(256) pack_bytes(const __grid_constant__ PackJo
                                                   uint64_t units) {
   const uint64_t u = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (u >= units) return;  // warp-uniform
-  uint64_t r;
-  uint32_t cc, q[8];
-  unit_chunk(unit_base(J.cpr, row0, u), threadIdx.x & 31, J.cpr, J.magic, r, cc);
-  if (r >= rend) return;
-  load_bytes32<VEC>(J.src, J.nrows, J.ncols, r, cc, q);
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t q[8];
+  const UnitBase b = unit_base(J, row0, rend, u);
+  const Chunk c = unit_chunk(b, lane, J.cpr, J.magic);
+  if (c.dr >= b.rows_a) return;
+  load_bytes32<VEC>(J, b, c, q);
   codes_of_bytes(J.dtype, J.nbits == 1 && J.issigned, q);
-  emit_chunk(J, r, cc, q);
+  emit_chunk(J, row0 * J.cpr + u * 32 + lane, (uint32_t)b.r + c.dr, c.cc, c.dr < b.rows, q);
 }
 
 // ---------------------------------------------------------------- every other source
 
 // Four consecutive elements of a row (or, column-major, of a column) held raw.
 template <typename T>
-struct Raw4 {
+struct alignas(4 * sizeof(T)) Raw4 {
   uint32_t w[sizeof(T)];
 };
 
@@ -313,29 +324,120 @@ __device__ __forceinline__ uint32_t codes4(const Raw4<T> &x, int bipolar, int is
 // (compared in T), or nthres when x exceeds them all; with no thresholds the
 // element keeps its own value.  The low byte of that index is the code the
 // planes store (the (uint8_t) cast of :298).  For float input without
-// thresholds the float is truncated toward zero to an integer first.  The
-// four elements are scanned together, row r + i * RSTEP each (RSTEP 0: four
-// columns of a row; 1: four rows of a column; a row past nrows, whose code is
-// not wanted, reads the last row's thresholds).
-template <typename T, int RSTEP>
-__device__ __forceinline__ uint32_t threshold_codes4(const Raw4<T> &x, const T *__restrict__ thr, int nthres,
-                                                     uint64_t r, uint64_t nrows) {
+// thresholds the float is truncated toward zero to an integer first.  Four
+// elements are scanned together; `over` says which have exceeded every
+// threshold so far.
+template <typename T>
+__device__ __forceinline__ uint32_t own_codes4(const Raw4<T> &x) {
   uint32_t c[4];
-  if (nthres == 0) {
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      if constexpr (std::is_same<T, float>::value) c[i] = low_byte(elem_of<T>(x, i));
-      else c[i] = (uint32_t)elem_of<T>(x, i) & 0xffu;
-    }
-    return pack4(c[0], c[1], c[2], c[3]);
-  }
-  const T *p[RSTEP ? 4 : 1];
-#pragma unroll
-  for (int i = 0; i < (RSTEP ? 4 : 1); i++) p[i] = thr + (r + i < nrows ? r + i : nrows - 1);
-  T v[4];
-  bool over[4];
 #pragma unroll
   for (int i = 0; i < 4; i++) {
+    if constexpr (std::is_same<T, float>::value) c[i] = low_byte(elem_of<T>(x, i));
+    else c[i] = (uint32_t)elem_of<T>(x, i) & 0xffu;
+  }
+  return pack4(c[0], c[1], c[2], c[3]);
+}
+
+// A value no x exceeds, in the place of thresholds past the last.
+template <typename T>
+__device__ __forceinline__ T no_threshold() {
+  if constexpr (std::is_same<T, float>::value) return __int_as_float(0x7f800000);
+  else if constexpr (sizeof(T) == 4) return (T)0x7fffffff;
+  else if constexpr (sizeof(T) == 2) return (T)0x7fff;
+  else return std::is_same<T, uint8_t>::value ? (T)0xff : (T)0x7f;
+}
+
+// Four columns of one row, the row's thresholds in the 8 lanes of its chunk
+// (lane j holds threshold 8 k + j of block k, block 0 in t0; past the last the
+// fill value): one load and shuffles, where a load per threshold (each a line
+// of its own, waited for in turn) took 31 us for 2048 x 4096 int32 against 7
+// thresholds.  A block that ascends, as the reference assumes, is searched:
+// LEVELS compares an element (3 for up to 7 thresholds), the threshold of
+// each picked by a shuffle of the element's own index (a scan of all 7 ran
+// 22 us, bound by integer instructions).  A block that does not is scanned for
+// its first crossing.  Elements past every threshold of a block of 8 go on to
+// the next.  2048 x 4096 int32 against 7 thresholds: 58 us loading a column
+// run per lane, 15 us now (33.5 MB in, 11.5 MB out: 6.6 us at the copy rate;
+// integer instructions bound it).  (A NaN exceeds the fill value too: counts are cut to the
+// thresholds there are.)  Every lane of the warp calls it.
+template <typename T, int LEVELS>
+__device__ __forceinline__ uint32_t row_threshold_codes4(const Raw4<T> &x, T t0, const T *__restrict__ thr, int nthres,
+                                                         uint64_t rthr, uint64_t nrows, bool row, bool wanted) {
+  using S = typename std::conditional<std::is_same<T, float>::value, float, int>::type;  // a type to shuffle
+  constexpr int kLast = LEVELS == 4 ? 8 : (1 << LEVELS) - 1;  // thresholds of a block
+  const int lane = threadIdx.x & 31, j = lane & 7;
+  S v[4], tv = (S)t0;
+  uint32_t c[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+  for (int i = 0; i < 4; i++) v[i] = (S)elem_of<T>(x, i);
+  bool over[4] = {wanted, wanted, wanted, wanted};
+  for (int k = 0;; k += 8) {
+    const S next = __shfl_down_sync(kFull, tv, 1, 8);  // lane j: threshold j + 1
+    uint32_t n[4];
+    if (__all_sync(kFull, j == 7 || tv <= next)) {
+#pragma unroll
+      for (int i = 0; i < 4; i++) n[i] = 0u;
+      if (LEVELS >= 3) {
+        const S mid = __shfl_sync(kFull, tv, 3, 8);
+#pragma unroll
+        for (int i = 0; i < 4; i++) n[i] = v[i] <= mid ? 0u : 4u;
+      }
+      if (LEVELS >= 2) {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          if (!(v[i] <= __shfl_sync(kFull, next, n[i], 8))) n[i] += 2u;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (!(v[i] <= __shfl_sync(kFull, tv, n[i], 8))) n[i] += 1u;
+      if (LEVELS == 4) {  // a block of 8: past 7 of them, the last is left (below 7 the answer stands)
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          if (!(v[i] <= __shfl_sync(kFull, tv, n[i], 8))) n[i] += 1u;
+      }
+    } else {
+      bool on[4] = {true, true, true, true};
+#pragma unroll
+      for (int i = 0; i < 4; i++) n[i] = 0u;
+#pragma unroll
+      for (int t = 0; t < kLast; t++) {
+        const S th = __shfl_sync(kFull, tv, t, 8);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          on[i] = on[i] && !(v[i] <= th);
+          if (on[i]) n[i] += 1u;
+        }
+      }
+    }
+    const uint32_t have = (uint32_t)min(kLast, nthres - k);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      if (std::is_same<T, float>::value) n[i] = min(n[i], have);
+      if (LEVELS == 4) {
+        if (over[i]) c[i] += n[i];
+        over[i] = over[i] && n[i] == have;
+      } else {
+        c[i] = n[i];
+      }
+    }
+    if (LEVELS < 4 || k + 8 >= nthres || !__any_sync(kFull, over[0] || over[1] || over[2] || over[3]))
+      return pack4(c[0], c[1], c[2], c[3]);
+    tv = (S)((k + 8 + j < nthres && row) ? thr[(uint64_t)(k + 8 + j) * nrows + rthr] : no_threshold<T>());
+  }
+}
+
+// Four rows r .. r + 3 of one column, each against its own thresholds (a row
+// past nrows, whose code is not wanted, reads the last row's).
+template <typename T>
+__device__ __forceinline__ uint32_t col_threshold_codes4(const Raw4<T> &x, const T *__restrict__ thr, int nthres,
+                                                         uint64_t r, uint64_t nrows) {
+  const T *p[4];
+  T v[4];
+  bool over[4];
+  uint32_t c[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    p[i] = thr + (r + i < nrows ? r + i : nrows - 1);
     v[i] = elem_of<T>(x, i);
     over[i] = true;
     c[i] = 0u;
@@ -344,7 +446,7 @@ __device__ __forceinline__ uint32_t threshold_codes4(const Raw4<T> &x, const T *
   for (int t = 0; t < nthres; t++) {
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-      over[i] = over[i] && !(v[i] <= p[RSTEP ? i : 0][(uint64_t)t * nrows]);
+      over[i] = over[i] && !(v[i] <= p[i][(uint64_t)t * nrows]);
       c[i] += over[i] ? 1u : 0u;
     }
     if ((t & 7) == 7 && !(over[0] || over[1] || over[2] || over[3])) break;
@@ -360,49 +462,82 @@ __device__ __forceinline__ uint32_t threshold_codes4(const Raw4<T> &x, const T *
 // hands through shared memory.  All eight loads are in flight before the first is converted.
 // Word j of chunk i lies at 8 i + (j ^ 4 (i / 4 & 1)): the 16-byte reads of
 // whole chunks then meet no bank conflict.
+template <typename T>
+struct QuantStage {  // a threshold import's raw elements and first thresholds, per warp and load
+  Raw4<T> raw[8][8][32];
+  T thr[8][8][32];
+};
+
 template <typename T, bool QUANT, bool ALIGNED>
 __device__ __forceinline__ void pack_staged_unit(const PackJob &J, const T *__restrict__ thr, int nthres,
-                                                 uint64_t row0, uint64_t rend, uint64_t u, uint32_t *__restrict__ st) {
-  const uint32_t lane = threadIdx.x & 31, j = lane & 7;
-  const UnitBase b = unit_base(J.cpr, row0, u);
-  const uint64_t total = J.nrows * J.ncols;
+                                                 uint64_t row0, uint64_t rend, uint64_t u, uint32_t *__restrict__ st,
+                                                 QuantStage<T> *__restrict__ qs) {
+  const uint32_t lane = threadIdx.x & 31, j = lane & 7, ncols = (uint32_t)J.ncols;
+  const UnitBase b = unit_base(J, row0, rend, u);
+  const uint64_t total = J.nrows * J.ncols, e0 = b.r * J.ncols;
   const int bip = J.nbits == 1 && J.issigned;
   Raw4<T> x[8];
+  T t0[8];
+  uint32_t part = 0u;  // nibble s: the elements of load s that exist
 #pragma unroll
   for (int s = 0; s < 8; s++) {
-    uint64_t r;
-    uint32_t cc;
-    unit_chunk(b, 4 * s + (lane >> 3), J.cpr, J.magic, r, cc);
-    const uint64_t col = (uint64_t)cc * 32 + 4 * j;
-    const uint32_t n = (r < J.nrows && col < J.ncols) ? (uint32_t)min((uint64_t)4, J.ncols - col) : 0u;
-    x[s] = load4<T, ALIGNED>((const T *)J.src, r * J.ncols + col, n, total);
-  }
-#pragma unroll
-  for (int s = 0; s < 8; s++) {
-    uint32_t w;
+    const Chunk c = unit_chunk(b, 4 * s + (lane >> 3), J.cpr, J.magic);
+    const uint32_t col = c.cc * 32 + 4 * j;
+    const bool row = c.dr < b.rows;
+    const uint32_t n = (row && col < ncols) ? min(4u, ncols - col) : 0u;
+    x[s] = load4<T, ALIGNED>((const T *)J.src, e0 + (uint64_t)c.dr * ncols + col, n, total);
     if (QUANT) {
-      uint64_t r;
-      uint32_t cc;
-      unit_chunk(b, 4 * s + (lane >> 3), J.cpr, J.magic, r, cc);
-      const uint64_t col = (uint64_t)cc * 32 + 4 * j;
-      const uint32_t n = (r < J.nrows && col < J.ncols) ? (uint32_t)min((uint64_t)4, J.ncols - col) : 0u;
-      w = n ? threshold_codes4<T, 0>(x[s], thr, nthres, r, J.nrows) : 0u;
-      if (n < 4) w &= (1u << (8 * n)) - 1u;  // the code of a 0 put past the row's end is no code
-    } else {
-      w = codes4<T>(x[s], bip, J.issigned, J.nbits);
+      t0[s] = (row && (int)j < nthres) ? thr[(uint64_t)j * J.nrows + (uint32_t)b.r + c.dr] : no_threshold<T>();
+      part |= n << (4 * s);
     }
-    st[(4 * s + (lane >> 3)) * 8 + (j ^ ((s & 1) << 2))] = w;
+  }
+  const uint32_t at = (lane >> 3) * 8;
+  if (QUANT) {
+    // the raw elements and first thresholds go through shared memory (the lane's own
+    // words), so that the search is a loop: unrolled over eight loads in registers
+    // it stalled on instruction fetch
+    Raw4<T> *rx = qs->raw[threadIdx.x >> 5][0] + lane;
+    T *rt = qs->thr[threadIdx.x >> 5][0] + lane;
+#pragma unroll
+    for (int s = 0; s < 8; s++) {
+      rx[32 * s] = x[s];
+      rt[32 * s] = t0[s];
+    }
+    auto codes = [&](auto scan) {
+#pragma unroll 1
+      for (int s = 0; s < 8; s++) {
+        const uint32_t n = (part >> (4 * s)) & 15u;
+        uint32_t w = scan(rx[32 * s], rt[32 * s], s, n != 0u);
+        if (n < 4) w &= (1u << (8 * n)) - 1u;  // the code of a 0 put past the row's end is no code
+        st[32 * s + at + (j ^ ((s & 1) << 2))] = w;
+      }
+    };
+    auto search = [&](auto levels) {
+      codes([&](const Raw4<T> &v, T t, int s, bool wanted) {
+        uint32_t dr = 0u;
+        if (decltype(levels)::value == 4) dr = unit_chunk(b, 4 * s + (lane >> 3), J.cpr, J.magic).dr;
+        return row_threshold_codes4<T, decltype(levels)::value>(v, t, thr, nthres, b.r + dr, J.nrows, dr < b.rows,
+                                                                wanted);
+      });
+    };
+    if (nthres == 0) codes([&](const Raw4<T> &v, T, int, bool) { return own_codes4<T>(v); });
+    else if (nthres == 1) search(std::integral_constant<int, 1>{});
+    else if (nthres <= 3) search(std::integral_constant<int, 2>{});
+    else if (nthres <= 7) search(std::integral_constant<int, 3>{});
+    else search(std::integral_constant<int, 4>{});
+  } else {
+#pragma unroll
+    for (int s = 0; s < 8; s++)
+      st[32 * s + at + (j ^ ((s & 1) << 2))] = codes4<T>(x[s], bip, J.issigned, J.nbits);
   }
   __syncwarp();
-  uint64_t r;
-  uint32_t cc, q[8];
-  unit_chunk(b, lane, J.cpr, J.magic, r, cc);
   const uint32_t sw = ((lane >> 2) & 1u) << 2;
   const uint4 v0 = *reinterpret_cast<const uint4 *>(st + lane * 8 + sw);
   const uint4 v1 = *reinterpret_cast<const uint4 *>(st + lane * 8 + (sw ^ 4u));
-  q[0] = v0.x; q[1] = v0.y; q[2] = v0.z; q[3] = v0.w;
-  q[4] = v1.x; q[5] = v1.y; q[6] = v1.z; q[7] = v1.w;
-  if (r < rend) emit_chunk(J, r, cc, q);
+  const uint32_t q[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+  const Chunk c = unit_chunk(b, lane, J.cpr, J.magic);
+  if (c.dr < b.rows_a)
+    emit_chunk(J, row0 * J.cpr + u * 32 + lane, (uint32_t)b.r + c.dr, c.cc, c.dr < b.rows, q);
   __syncwarp();  // the next unit writes the staging words again
 }
 
@@ -410,9 +545,11 @@ template <typename T, bool QUANT, bool ALIGNED>
 __global__ void __launch_bounds__(256) pack_staged(const __grid_constant__ PackJob J, const T *__restrict__ thr,
                                                    int nthres, uint64_t row0, uint64_t rend, uint64_t units) {
   __shared__ __align__(16) uint32_t st[8][256];
+  __shared__ typename std::conditional<QUANT, QuantStage<T>, char>::type qs;
   const uint64_t u = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (u >= units) return;  // warp-uniform; no block-wide barrier follows
-  pack_staged_unit<T, QUANT, ALIGNED>(J, thr, nthres, row0, rend, u, st[threadIdx.x >> 5]);
+  pack_staged_unit<T, QUANT, ALIGNED>(J, thr, nthres, row0, rend, u, st[threadIdx.x >> 5],
+                                      reinterpret_cast<QuantStage<T> *>(&qs));
 }
 
 // ---------------------------------------------------------------- column-major sources
@@ -456,7 +593,7 @@ __global__ void __launch_bounds__(kCmThreads) pack_colmajor(const __grid_constan
     if (QUANT) {
       const uint64_t c = c0 + col, r = r0 + 4 * g;
       const uint32_t n = (c < J.ncols && r < J.nrows) ? (uint32_t)min((uint64_t)4, J.nrows - r) : 0u;
-      w = n ? threshold_codes4<T, 1>(x[i], thr, nthres, r, J.nrows) : 0u;
+      w = n == 0 ? 0u : nthres == 0 ? own_codes4<T>(x[i]) : col_threshold_codes4<T>(x[i], thr, nthres, r, J.nrows);
       if (n < 4) w &= (1u << (8 * n)) - 1u;
     } else {
       w = codes4<T>(x[i], bip, J.issigned, J.nbits);
@@ -475,7 +612,7 @@ __global__ void __launch_bounds__(kCmThreads) pack_colmajor(const __grid_constan
   for (int w = 0; w < 8; w++)
     q[w] = __byte_perm(__byte_perm(p[(4 * w) * 17], p[(4 * w + 1) * 17], sel),
                        __byte_perm(p[(4 * w + 2) * 17], p[(4 * w + 3) * 17], sel), 0x5410u);
-  emit_chunk(J, r, (uint32_t)cc, q);
+  emit_chunk(J, r * J.cpr + cc, (uint32_t)r, (uint32_t)cc, r < J.nrows, q);
 }
 
 // ---------------------------------------------------------------- grouped import
@@ -506,13 +643,6 @@ __device__ __forceinline__ int find_job(const PackJob *jobs, int njobs, uint64_t
 constexpr int kMaxRun = 8;
 constexpr int kDepth = 2;
 
-__device__ __forceinline__ void load_run_bytes(const PackJob &J, const UnitBase &b, uint32_t i, uint64_t &r,
-                                               uint32_t &cc, uint32_t (&q)[8]) {
-  unit_chunk(b, i, J.cpr, J.magic, r, cc);
-  if (J.vec == 2) load_bytes32<2>(J.src, J.nrows, J.ncols, r, cc, q);
-  else load_bytes32<1>(J.src, J.nrows, J.ncols, r, cc, q);
-}
-
 __global__ void __launch_bounds__(256, 4) pack_grouped(const PackJob *__restrict__ jobs, int njobs, uint64_t runs,
                                                        uint32_t run) {
   __shared__ PackJob sj[8];  // each warp's job: its fields stay out of the registers
@@ -526,20 +656,26 @@ __global__ void __launch_bounds__(256, 4) pack_grouped(const PackJob *__restrict
     if (lane < (int)(sizeof(PackJob) / 8))
       reinterpret_cast<uint64_t *>(&J)[lane] = reinterpret_cast<const uint64_t *>(jobs + j)[lane];
     __syncwarp();
-    const UnitBase b = unit_base(J.cpr, 0, (w - J.warp0) * run);
+    const uint64_t u0 = (w - J.warp0) * run;
+    const UnitBase b = unit_base(J, 0, J.nrows_a, u0);
     const int bip = J.nbits == 1 && J.issigned;
 #pragma unroll 1
     for (uint32_t u = 0; u < run; u += kDepth) {
-      uint64_t r[kDepth];
-      uint32_t cc[kDepth], q[kDepth][8];
+      Chunk c[kDepth];
+      uint32_t q[kDepth][8];
 #pragma unroll
-      for (uint32_t d = 0; d < kDepth; d++)
-        if (u + d < run) load_run_bytes(J, b, 32 * (u + d) + lane, r[d], cc[d], q[d]);
+      for (uint32_t d = 0; d < kDepth; d++) {
+        if (u + d >= run) break;
+        c[d] = unit_chunk(b, 32 * (u + d) + lane, J.cpr, J.magic);
+        if (J.vec == 2) load_bytes32<2>(J, b, c[d], q[d]);
+        else load_bytes32<1>(J, b, c[d], q[d]);
+      }
 #pragma unroll
       for (uint32_t d = 0; d < kDepth; d++) {
         if (u + d >= run) break;
         codes_of_bytes(J.dtype, bip, q[d]);
-        if (r[d] < J.nrows_a) emit_chunk(J, r[d], cc[d], q[d]);
+        if (c[d].dr < b.rows_a)
+          emit_chunk(J, (u0 + u + d) * 32 + lane, (uint32_t)b.r + c[d].dr, c[d].cc, c[d].dr < b.rows, q[d]);
       }
     }
   }
@@ -551,8 +687,8 @@ __device__ __forceinline__ void pack_staged_run(const PackJob &J, uint64_t u0, u
   const uint64_t units = min((uint64_t)run, (J.nrows_a * J.cpr + 31) / 32 - u0);
 #pragma unroll 1
   for (uint64_t u = u0; u < u0 + units; u++) {
-    if (J.vec) pack_staged_unit<T, false, true>(J, nullptr, 0, 0, J.nrows_a, u, st);
-    else pack_staged_unit<T, false, false>(J, nullptr, 0, 0, J.nrows_a, u, st);
+    if (J.vec) pack_staged_unit<T, false, true>(J, nullptr, 0, 0, J.nrows_a, u, st, nullptr);
+    else pack_staged_unit<T, false, false>(J, nullptr, 0, 0, J.nrows_a, u, st, nullptr);
   }
 }
 
