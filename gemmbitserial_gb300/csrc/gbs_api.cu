@@ -432,9 +432,21 @@ int ensure_stage(gbs_ctx *c, int side, size_t bytes, cudaStream_t s) {
 }
 
 // The tensor-core digit pipe will run this context's GEMM: the import then
-// writes the digit matrix too, so the GEMM needs no expansion pass.
-bool import_writes_digits(const gbs_ctx *c) {
-  return effective_pipe(c) == GBS_PIPE_TC && c->lhs.nbits <= 4 && c->rhs.nbits <= 4;  // wide operands: per part, later
+// writes the digit matrices too (t), so the GEMM needs no expansion pass.
+// False when it does not, or when they cannot be allocated (the GEMM then
+// expands the digits itself).
+bool import_digit_target(gbs_ctx *c, int side, DigitTarget &t, cudaStream_t s) {
+  if (effective_pipe(c) != GBS_PIPE_TC) return false;
+  if (tc_wide(c)) return wide_digit_target(c, side, t, s);
+  if (ensure_digit_buffer(c, side) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  const Mat &m = side ? c->rhs : c->lhs;
+  t.lo = c->digits[side];
+  t.lo_bits = (int)m.nbits;
+  tc_digit_table(m, t.tab_lo);
+  return true;
 }
 
 }  // namespace
@@ -451,22 +463,14 @@ int gbs_import(gbs_ctx *c, int side, const void *src, int dtype, int col_major, 
   cudaStream_t s = as_stream(stream);
   c->digits_valid[side] = c->nibbles_valid[side] = false;
   c->vt_valid[side] = false;
-  uint8_t *digits = nullptr;
-  uint32_t dtab[4] = {0, 0, 0, 0};
-  if (import_writes_digits(c)) {
-    if (ensure_digit_buffer(c, side) == cudaSuccess) {
-      digits = c->digits[side];
-      tc_digit_table(m, dtab);
-    } else {
-      cudaGetLastError();  // the GEMM expands the digits itself
-    }
-  }
+  DigitTarget target;
+  const DigitTarget *digits = import_digit_target(c, side, target, s) ? &target : nullptr;
   cudaError_t e = cudaSuccess;
   const void *view = (n && !is_device_ptr(src) && c->host_import != GBS_HOST_IMPORT_STAGED)
                          ? device_view(src, c->device, true)
                          : nullptr;
   if (view) {  // host memory the device reads directly: the pack kernel is the copy
-    e = launch_pack(m, view, dtype, col_major, digits, dtab, s);
+    e = launch_pack(m, view, dtype, col_major, digits, s);
     if (e != cudaSuccess) return cuda_fail(e, "gbs_import: pack kernel");
     if (digits) c->digits_valid[side] = true;
     e = ensure_import_streams(c);
@@ -488,7 +492,7 @@ int gbs_import(gbs_ctx *c, int side, const void *src, int dtype, int col_major, 
       if (e == cudaSuccess) e = cudaEventRecord(c->ev_chunk[0], c->copy_stream);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(s, c->ev_chunk[0], 0);
       if (e != cudaSuccess) return cuda_fail(e, "gbs_import: host-to-device copy");
-      e = launch_pack(m, c->stage[side], dtype, 1, digits, dtab, s);
+      e = launch_pack(m, c->stage[side], dtype, 1, digits, s);
       if (e != cudaSuccess) return cuda_fail(e, "gbs_import: pack kernel");
     } else {  // row chunks: the pack of chunk i overlaps the copy of chunk i+1
       const size_t row_bytes = m.ncols * esz;
@@ -505,7 +509,7 @@ int gbs_import(gbs_ctx *c, int side, const void *src, int dtype, int col_major, 
         if (e == cudaSuccess) e = cudaStreamWaitEvent(s, c->ev_chunk[i], 0);
         if (e != cudaSuccess) return cuda_fail(e, "gbs_import: host-to-device copy");
         // the last chunk also writes the zero padding rows [nrows, nrows_a)
-        e = launch_pack_rows(m, c->stage[side], dtype, r0, r1 == m.nrows ? m.nrows_a : r1, digits, dtab, s);
+        e = launch_pack_rows(m, c->stage[side], dtype, r0, r1 == m.nrows ? m.nrows_a : r1, digits, s);
         if (e != cudaSuccess) return cuda_fail(e, "gbs_import: pack kernel");
         last = (int)i;
       }
@@ -521,7 +525,7 @@ int gbs_import(gbs_ctx *c, int side, const void *src, int dtype, int col_major, 
       if (e != cudaSuccess) return cuda_fail(e, "gbs_import: copy wait");
     }
   } else {
-    e = launch_pack(m, src, dtype, col_major, digits, dtab, s);
+    e = launch_pack(m, src, dtype, col_major, digits, s);
     if (e != cudaSuccess) return cuda_fail(e, "gbs_import: pack kernel");
     if (digits) c->digits_valid[side] = true;
   }
@@ -547,16 +551,8 @@ int gbs_import_quantize(gbs_ctx *c, int side, const void *src, const void *thres
   cudaStream_t s = as_stream(stream);
   c->digits_valid[side] = c->nibbles_valid[side] = false;
   c->vt_valid[side] = false;
-  uint8_t *digits = nullptr;
-  uint32_t dtab[4] = {0, 0, 0, 0};
-  if (import_writes_digits(c)) {
-    if (ensure_digit_buffer(c, side) == cudaSuccess) {
-      digits = c->digits[side];
-      tc_digit_table(m, dtab);
-    } else {
-      cudaGetLastError();  // the GEMM expands the digits itself
-    }
-  }
+  DigitTarget target;
+  const DigitTarget *digits = import_digit_target(c, side, target, s) ? &target : nullptr;
   bool host = false;
   const void *dsrc = src, *dthr = thresholds;
   cudaError_t e = cudaSuccess;
@@ -587,7 +583,7 @@ int gbs_import_quantize(gbs_ctx *c, int side, const void *src, const void *thres
     dthr = c->thr_stage[side];
     host = true;
   }
-  e = launch_pack_quantize(m, dsrc, dthr, nthres, dtype, col_major ? 1 : 0, digits, dtab, s);
+  e = launch_pack_quantize(m, dsrc, dthr, nthres, dtype, col_major ? 1 : 0, digits, s);
   if (e != cudaSuccess) return cuda_fail(e, "gbs_import_quantize: pack kernel");
   if (host && dsrc == c->stage[side]) {  // later host imports of this side wait before reusing the staging buffer
     e = ensure_import_streams(c);

@@ -105,14 +105,15 @@ int build_pack_jobs(gbs_group *g, const void *const *lhs, const void *const *rhs
       if (m.nrows_a == 0 || m.wpr() == 0) continue;
       if (m.nrows && m.ncols && (!src || !device_ptr(src)))
         return fail(GBS_EINVAL, "gbs_group: sources must be device pointers (problem " + std::to_string(p) + ")");
-      uint32_t dtab[4] = {0, 0, 0, 0};
-      uint8_t *digits = nullptr, *nibbles = nullptr;
+      DigitTarget digits;
+      uint8_t *nibbles = nullptr;
       if ((digit_sides >> side) & 1) {  // tensor-core problem: the import writes the digit matrices it reads
-        digits = g->ctxs[p]->digits[side];
-        tc_digit_table(m, dtab);
+        digits.lo = g->ctxs[p]->digits[side];
+        digits.lo_bits = (int)m.nbits;
+        tc_digit_table(m, digits.tab_lo);
       }
       if ((digit_sides >> (2 + side)) & 1) nibbles = g->ctxs[p]->nibbles[side];  // ... and nibble matrices
-      PackJob j = make_pack_job(m, src, dt, digits, dtab, nibbles);
+      PackJob j = make_pack_job(m, src, dt, &digits, nibbles);
       const int kind = pack_job_direct(j, m) ? 0 : 1;
       units[kind] += pack_job_units(j);
       jobs[kind].push_back(j);

@@ -94,15 +94,23 @@ struct GroupTile {
   uint32_t p, mt, nt, cls;
 };
 
+// The digit matrices an import writes beside the planes: one of the whole
+// codes (hi null, lo_bits the matrix's width), or, for 5-8-bit operands, one of
+// the low lo_bits planes and one of the rest.
+struct DigitTarget {
+  uint8_t *lo = nullptr, *hi = nullptr;
+  uint32_t tab_lo[4] = {0, 0, 0, 0}, tab_hi[4] = {0, 0, 0, 0};
+  int lo_bits = 0;
+};
+
 // One operand of an import or of a grouped row-sum pass; warp0 = its first
 // warp run (import) or row (row sums) of a grouped pass.  With digits set, the
-// import also writes the operand's e4m3 digit matrix (table dtab), the operand
-// of the tensor-core pipe.
+// import also writes the operand's e4m3 digit matrix (DigitTarget).
 struct PackJob {
   const void *src;
   uint64_t *planes;
   int32_t *rowsum;
-  uint8_t *digits;
+  uint8_t *digits, *digits_hi;
   uint8_t *nibbles;  // with nibbles set, the import also writes the nibble matrix (codes, 4 bits each)
   uint64_t nrows, ncols, nrows_a, wpr, warp0;
   uint64_t dcols;  // digit-matrix columns (a multiple of 256)
@@ -110,7 +118,8 @@ struct PackJob {
   // direct (1-byte, 16-byte-aligned rows): vec 2 when 32-byte aligned, else 1;
   // staged kernels of a grouped import: vec 1 when four elements load as one vector
   uint32_t cpr, magic;  // 32-column chunks per padded row, 2^32 / cpr + 1
-  uint32_t dtab[4];
+  uint32_t dtab[4], dtab_hi[4];
+  int lo_bits, pad;
 };
 
 // One problem of the persistent tensor-core kernels (device resident).  The
@@ -254,22 +263,21 @@ void count_launch(uint64_t n = 1);
 cudaError_t dev_alloc(void **p, size_t bytes);
 
 // kernels (gbs_pack.cu)
-// plain import (importRegular); with digits set also the e4m3 digit matrix (table dtab[4])
-cudaError_t launch_pack(const Mat &m, const void *src, int dtype, int col_major, uint8_t *digits,
-                        const uint32_t *dtab, cudaStream_t s);
+// plain import (importRegular); with a digit target also the e4m3 digit matrices
+cudaError_t launch_pack(const Mat &m, const void *src, int dtype, int col_major, const DigitTarget *digits,
+                        cudaStream_t s);
 // threshold-quantising import (importRegularAndQuantize); dtype GBS_I8..GBS_F32, thr [nthres][nrows]
 cudaError_t launch_pack_quantize(const Mat &m, const void *src, const void *thr, int nthres, int dtype,
-                                 int col_major, uint8_t *digits, const uint32_t *dtab, cudaStream_t s);
+                                 int col_major, const DigitTarget *digits, cudaStream_t s);
 // One operand as a pack job; digits / nibbles may be null.
-PackJob make_pack_job(const Mat &m, const void *src, int dtype, uint8_t *digits, const uint32_t *dtab,
-                      uint8_t *nibbles);
+PackJob make_pack_job(const Mat &m, const void *src, int dtype, const DigitTarget *digits, uint8_t *nibbles);
 // Sets j.vec; true when the direct kernels take the job, false for the staged ones.
 bool pack_job_direct(PackJob &j, const Mat &m);
 uint64_t pack_job_units(const PackJob &j);   // units (32 chunks, one warp) of the job
 uint32_t pack_run_units(uint64_t units);    // units per warp run of a grouped import of that many
-// row-major pack of padded rows [r0, r1); with digits set also the e4m3 digit rows (table dtab[4])
-cudaError_t launch_pack_rows(const Mat &m, const void *src, int dtype, uint64_t r0, uint64_t r1, uint8_t *digits,
-                             const uint32_t *dtab, cudaStream_t s);
+// row-major pack of padded rows [r0, r1)
+cudaError_t launch_pack_rows(const Mat &m, const void *src, int dtype, uint64_t r0, uint64_t r1,
+                             const DigitTarget *digits, cudaStream_t s);
 cudaError_t launch_rowsum(const Mat &m, int32_t *dst, cudaStream_t s);
 cudaError_t launch_export(const Mat &m, int32_t *dst, cudaStream_t s);
 
@@ -310,6 +318,7 @@ inline bool pair_split_variant(int v) {
   return (v == 1281 || v == 1282 || v == 1284 || v == 2561 || v == 2562 || v == 2564);
 }
 bool pdl_enabled();                          // programmatic dependent launch of the tensor-core kernels (GBS_PDL)
+bool pdl_for(cudaStream_t s);                // ... of a launch on this stream
 uint32_t tc_error_word();
 int tc_peaks(double *f8, double *bf16);
 
@@ -335,6 +344,8 @@ bool tc_map_nibbles(void *map, const uint8_t *base, uint64_t cols, uint64_t rows
 // tensor-core pipe for 5-8-bit operands (gbs_wide.cu): operands split into parts of <= 4 bits
 bool tc_wide(const gbs_ctx *c);
 cudaError_t launch_gemm_wide(gbs_ctx *c, cudaStream_t s, int variant);
+// The part digit matrices an import of `side` can write for the next GEMM; false when it expands them itself.
+bool wide_digit_target(gbs_ctx *c, int side, DigitTarget &t, cudaStream_t s);
 void wide_plan_free(WidePlan *p);
 // tensor-core adjoint (gbs_adjoint_tc.cu)
 int adjoint_tc(gbs_ctx *c, const float *dC, float *dA, float *dB, cudaStream_t s);

@@ -116,8 +116,8 @@ extern "C" int gbs_gemm_noalloc(const void *lhs, int lhs_dtype, const void *rhs,
   c.res = res;
   cudaStream_t s = (cudaStream_t)stream;
 
-  e = launch_pack(c.lhs, lhs, lhs_dtype, 0, nullptr, nullptr, s);
-  if (e == cudaSuccess) e = launch_pack(c.rhs, rhs, rhs_dtype, 0, nullptr, nullptr, s);
+  e = launch_pack(c.lhs, lhs, lhs_dtype, 0, nullptr, s);
+  if (e == cudaSuccess) e = launch_pack(c.rhs, rhs, rhs_dtype, 0, nullptr, s);
   if (e != cudaSuccess) return cuda_fail(e, "gbs_gemm_noalloc: pack kernel");
   Epilogue ep;
   make_epilogue(&c, ep, c.rowsum);

@@ -109,8 +109,15 @@ __device__ __forceinline__ void emit_chunk(const PackJob &J, uint64_t idx, uint3
   emit_planes32(J.nbits, reinterpret_cast<uint32_t *>(J.planes), J.nrows_a * J.cpr, idx, q);
   if (!derived) return;
   if (J.digits)
-    write_digits32(J.digits, J.nbits, (uint32_t)J.ncols, J.dcols,
+    write_digits32(J.digits, J.lo_bits, (uint32_t)J.ncols, J.dcols,
                    make_uint4(J.dtab[0], J.dtab[1], J.dtab[2], J.dtab[3]), r, cc * 32, q);
+  if (J.digits_hi) {  // the planes past lo_bits of a wide operand
+    uint32_t h[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) h[i] = q[i] >> J.lo_bits;  // bits of the next byte are masked off with the rest
+    write_digits32(J.digits_hi, J.nbits - J.lo_bits, (uint32_t)J.ncols, J.dcols,
+                   make_uint4(J.dtab_hi[0], J.dtab_hi[1], J.dtab_hi[2], J.dtab_hi[3]), r, cc * 32, h);
+  }
   if (J.nibbles) write_nibbles32(J.nibbles, J.nbits, J.dcols, r, cc * 32, q);
 }
 
@@ -776,13 +783,11 @@ inline unsigned blocks_for(uint64_t threads, unsigned per_block) {
 
 }  // namespace
 
-PackJob make_pack_job(const Mat &m, const void *src, int dtype, uint8_t *digits, const uint32_t *dtab,
-                      uint8_t *nibbles) {
+PackJob make_pack_job(const Mat &m, const void *src, int dtype, const DigitTarget *digits, uint8_t *nibbles) {
   PackJob j;
   memset(&j, 0, sizeof(j));
   j.src = src;
   j.planes = m.planes;
-  j.digits = digits;
   j.nibbles = nibbles;
   j.nrows = m.nrows;
   j.ncols = m.ncols;
@@ -794,8 +799,15 @@ PackJob make_pack_job(const Mat &m, const void *src, int dtype, uint8_t *digits,
   j.dtype = dtype;
   j.cpr = (uint32_t)(m.ncols_a / 32);
   j.magic = j.cpr ? (uint32_t)((1ull << 32) / j.cpr) + 1u : 0u;
-  if (dtab)
-    for (int i = 0; i < 4; i++) j.dtab[i] = dtab[i];
+  if (digits) {
+    j.digits = digits->lo;
+    j.digits_hi = digits->hi;
+    j.lo_bits = digits->lo_bits;
+    for (int i = 0; i < 4; i++) {
+      j.dtab[i] = digits->tab_lo[i];
+      j.dtab_hi[i] = digits->tab_hi[i];
+    }
+  }
   return j;
 }
 
@@ -878,10 +890,10 @@ cudaError_t run_colmajor(const PackJob &j, const void *thr, int nthres, bool qua
 
 }  // namespace
 
-cudaError_t launch_pack_rows(const Mat &m, const void *src, int dtype, uint64_t r0, uint64_t r1, uint8_t *digits,
-                             const uint32_t *dtab, cudaStream_t s) {
+cudaError_t launch_pack_rows(const Mat &m, const void *src, int dtype, uint64_t r0, uint64_t r1,
+                             const DigitTarget *digits, cudaStream_t s) {
   if (m.nrows_a == 0 || m.wpr() == 0 || r1 <= r0) return cudaSuccess;
-  PackJob j = make_pack_job(m, src, dtype, digits, dtab, nullptr);
+  PackJob j = make_pack_job(m, src, dtype, digits, nullptr);
   if (!pack_job_direct(j, m)) return run_staged(j, nullptr, 0, false, j.vec != 0, r0, r1, s);
   const uint64_t units = ((r1 - r0) * j.cpr + 31) / 32;
   if (j.vec == 2) pack_bytes<2><<<blocks_for(units * 32, 256), 256, 0, s>>>(j, r0, r1, units);
@@ -891,18 +903,18 @@ cudaError_t launch_pack_rows(const Mat &m, const void *src, int dtype, uint64_t 
 }
 
 cudaError_t launch_pack_quantize(const Mat &m, const void *src, const void *thr, int nthres, int dtype,
-                                 int col_major, uint8_t *digits, const uint32_t *dtab, cudaStream_t s) {
+                                 int col_major, const DigitTarget *digits, cudaStream_t s) {
   if (m.nrows_a == 0 || m.wpr() == 0) return cudaSuccess;
-  const PackJob j = make_pack_job(m, src, dtype, digits, dtab, nullptr);
+  const PackJob j = make_pack_job(m, src, dtype, digits, nullptr);
   if (col_major) return run_colmajor(j, thr, nthres, true, s);
   return run_staged(j, thr, nthres, true, aligned4(src, dtype, m.ncols), 0, m.nrows_a, s);
 }
 
-cudaError_t launch_pack(const Mat &m, const void *src, int dtype, int col_major, uint8_t *digits,
-                        const uint32_t *dtab, cudaStream_t s) {
+cudaError_t launch_pack(const Mat &m, const void *src, int dtype, int col_major, const DigitTarget *digits,
+                        cudaStream_t s) {
   if (m.nrows_a == 0 || m.wpr() == 0) return cudaSuccess;
-  if (!col_major) return launch_pack_rows(m, src, dtype, 0, m.nrows_a, digits, dtab, s);
-  return run_colmajor(make_pack_job(m, src, dtype, digits, dtab, nullptr), nullptr, 0, false, s);
+  if (!col_major) return launch_pack_rows(m, src, dtype, 0, m.nrows_a, digits, s);
+  return run_colmajor(make_pack_job(m, src, dtype, digits, nullptr), nullptr, 0, false, s);
 }
 
 cudaError_t launch_pack_grouped(const PackJob *jobs, int njobs, uint64_t runs, uint32_t run, bool direct,
