@@ -18,18 +18,26 @@
 // size, in a second; the epilogue adds the two.  So the only rounding is the
 // fp32 accumulation itself, done 16 products per MMA step.
 //
-// Both products are "Out[r, k] = sum_s X[r, s] * Vt[k, s]" with both operands
-// contraction-major in HBM: pre-passes write the three splits of dC as
-// [N][M] (dB: r = n, s = m) and transposed as [M][N] (dA: r = m, s = n), and
-// the operand values transposed as Vt[k][s] in bf16.
+// Both products are Out[r, k] = sum_s X[r, s] * V[s, k] with the operands left
+// as they lie in memory: the three bf16 terms of dC as [3][N][M] (dB: r = n, s
+// = m, a contraction-major X; dA: r = m, s = n, an X whose rows r are
+// contiguous, which tcgen05 reads as an MN-major operand) and the operand
+// values as [rows][K] (V, MN-major).  One pass over dC and the planes
+// (adjoint_prepare) makes all of them; transposing dC and the values for a
+// contraction-major form took two split passes and two transpositions, 30 us of
+// a 174 us adjoint at 4096 x 2048 x 2048.
 //
-// GEMM kernel: CTA tile 128 rows (r) x 256 columns (k), 32 values of s per
-// stage in a 5-stage ring: TMA loads the three 128 x 32 split tiles and the
-// 256 x 32 value tile (64-byte swizzle), warp 1 issues 6 tcgen05.mma.kind::f16
-// (M=128, N=256, K=16) per stage into the two accumulators (all 512 TMEM
-// columns), warps 2-5 add the accumulators and store through a padded
-// shared-memory tile so that each warp store covers 128 contiguous bytes of a
-// row of Out.  Every mbarrier wait is bounded.
+// GEMM kernel: one launch computes dA and dB.  Persistent SM pairs
+// (cta_group::2, M = 256, N = 256) walk 256 x 256 tiles of both, the gradient
+// with the longer contraction first, the other's tiles given out so that the
+// pairs finish together (deal_tiles).  32 values of s per stage in a 6-stage ring, 32 KB of
+// each SM; the leader's TMA loads a stage for both (the three terms in one
+// box), its MMA thread issues 6 tcgen05.mma.kind::f16 (K = 16) into the two
+// accumulators (all 512 TMEM columns).  Eight epilogue warps add the
+// accumulators into registers, release TMEM to the next tile's MMAs and store
+// while these run.  Tensor-bound: 6 pair MMAs of 68 ns a stage; a lone SM on
+// 128 x 256 tiles moved 112 KB of shared memory in that time and ran 0.49 us a
+// stage.  Every mbarrier wait is bounded.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -43,52 +51,128 @@
 namespace gbs {
 namespace {
 
-constexpr int kAdjThreads = 192;
-constexpr uint32_t kAdjScratchFloats = 32 * 33;          // per epilogue warp
-
-// Ring: 32 values of s per stage (64-byte rows, 64-byte swizzle), 5 stages of
-// 40 KB.  Two stages of 64 values (80 KB, 128-byte rows) hold the same bytes
-// but free them half as often; that ring ran the GEMMs latency-bound, 15 %
-// slower per adjoint.
+constexpr int kAdjEpiWarps = 8;
+constexpr int kAdjThreads = 64 + 32 * kAdjEpiWarps;
+constexpr uint32_t kAdjScratchFloats = 32 * 33;  // per epilogue warp
 constexpr int kAdjKs = 32;
-constexpr int kAdjStages = 5;
-constexpr uint32_t kAdjSplitBytes = 128 * kAdjKs * 2;  // 128 rows x 32 bf16
-constexpr uint32_t kAdjValBytes = 256 * kAdjKs * 2;    // 256 rows x 32 bf16
-constexpr uint32_t kAdjStageBytes = 3 * kAdjSplitBytes + kAdjValBytes;
+constexpr int kAdjStages = 6;
+constexpr uint32_t kAdjTermBytes = 128 * kAdjKs * 2;  // one term: 128 rows x 32 bf16
+constexpr uint32_t kAdjValBytes = 128 * kAdjKs * 2;   // this CTA's 128 of the tile's 256 value columns
+constexpr uint32_t kAdjStageBytes = 3 * kAdjTermBytes + kAdjValBytes;
 
 constexpr size_t adj_smem_bytes() {
-  return 1024 + kAdjStages * kAdjStageBytes + 4 * kAdjScratchFloats * 4 + 8 * (2 * kAdjStages + 2) + 16;
+  return 1024 + kAdjStages * kAdjStageBytes + kAdjEpiWarps * kAdjScratchFloats * 4 + 8 * (2 * kAdjStages + 3) + 16;
 }
 static_assert(adj_smem_bytes() <= 232448, "shared memory per CTA");
 
-struct AdjTcArgs {
-  float *out;  // R x K row-major
-  uint32_t R, K, nstages;
+// One gradient: R x K row-major, tiles row block t / ctiles, column block t % ctiles.
+struct AdjOut {
+  float *out;
+  uint32_t R, tiles, nstages;
   uint32_t idesc;
 };
 
-__device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t acc) {
+// Tiles of the two gradients dealt to P pairs (deal_tiles): gradient `first`
+// round robin (pairs below `a` get one more than the rest), then a contiguous
+// run of the other's, sa or sb tiles for a pair of either kind, one more for
+// the first `extra` pairs of kind `extra_kind`.
+struct AdjDeal {
+  uint32_t first, pairs, a, sa, sb, extra, extra_kind;
+};
+
+struct AdjTcArgs {
+  AdjOut o[2];  // 0: dB (contraction-major X), 1: dA (row-contiguous X)
+  uint32_t K, ctiles, vec;  // vec: K and both outputs allow 32-byte stores
+  AdjDeal deal;
+};
+
+// The i-th tile of pair p: its gradient and number, false when p has no i-th tile.
+__host__ __device__ inline bool dealt_tile(const AdjDeal &d, uint32_t nfirst, uint32_t p, uint32_t i, uint32_t &grad,
+                                           uint32_t &t) {
+  const uint32_t mine = nfirst > p ? (nfirst - p - 1) / d.pairs + 1 : 0;
+  if (i < mine) {
+    grad = d.first;
+    t = p + i * d.pairs;
+    return true;
+  }
+  i -= mine;
+  const bool b = p >= d.a;
+  const uint32_t r = b ? p - d.a : p, per = b ? d.sb : d.sa;
+  const uint32_t ex = d.extra_kind == (b ? 1u : 0u) ? d.extra : 0u;  // extra pairs of this kind
+  if (i >= per + (r < ex ? 1u : 0u)) return false;
+  const uint32_t before = b ? d.a * d.sa + (d.extra_kind == 0 ? d.extra : 0u) : 0u;  // the a pairs' tiles
+  grad = 1 - d.first;
+  t = before + r * per + (r < ex ? r : ex) + i;
+  return true;
+}
+
+__device__ __forceinline__ void mma_bf16_pair(uint32_t tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                              uint32_t acc) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+      " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc));
+}
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap *map, int x, int y, int z,
+                                                 uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, "
+      "%3, %4}], [%5];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const CUtensorMap *map, int x, int y, int z, int w,
+                                                 uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, "
+      "%3, %4, %5}], [%6];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar)
+      : "memory");
+}
+// MN-major operand, 128-byte swizzle: 64 values of the row (column) dimension
+// contiguous, the 32 contraction steps of a stage 128 bytes apart (groups of 8
+// 1024 bytes apart), the next 64 values 4096 bytes on.
+__device__ __forceinline__ uint64_t mn128_desc(uint32_t addr) {
+  return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(4096 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+         ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr));
+}
+// Waits for the thread's TMEM loads; the registers are operands, so no use of
+// them is scheduled ahead of the wait.
+__device__ __forceinline__ void tmem_wait_ld16(uint32_t (&v)[16], uint32_t (&w)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                 "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])
+               :
+               : "memory");
+  asm volatile(""
+               : "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3]), "+r"(w[4]), "+r"(w[5]), "+r"(w[6]), "+r"(w[7]),
+                 "+r"(w[8]), "+r"(w[9]), "+r"(w[10]), "+r"(w[11]), "+r"(w[12]), "+r"(w[13]), "+r"(w[14]), "+r"(w[15])
+               :
+               : "memory");
 }
 
 __global__ void __launch_bounds__(kAdjThreads, 1)
-    adjoint_tc_kernel(const __grid_constant__ CUtensorMap tmHi, const __grid_constant__ CUtensorMap tmMid,
-                      const __grid_constant__ CUtensorMap tmLo, const __grid_constant__ CUtensorMap tmV, AdjTcArgs a,
-                      uint32_t *err) {
+    adjoint_tc_kernel(const __grid_constant__ CUtensorMap tmXk, const __grid_constant__ CUtensorMap tmXmn,
+                      const __grid_constant__ CUtensorMap tmVa, const __grid_constant__ CUtensorMap tmVb,
+                      const __grid_constant__ AdjTcArgs a, uint32_t *err) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t peer = cluster_rank();  // rank 0 leads
   float *scratch = reinterpret_cast<float *>(smem + kAdjStages * kAdjStageBytes);
-  uint64_t *bars = reinterpret_cast<uint64_t *>(scratch + 4 * kAdjScratchFloats);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(scratch + kAdjEpiWarps * kAdjScratchFloats);
   const uint32_t full = smem_u32(bars), empty = full + 8 * kAdjStages, acc_full = empty + 8 * kAdjStages;
-  const uint32_t mma_done = acc_full + 8;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kAdjStages + 2);
+  const uint32_t acc_empty = acc_full + 8, mma_done = acc_empty + 8;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kAdjStages + 3);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-  const uint32_t r0 = blockIdx.x * 128, k0 = blockIdx.y * 256;
+  const uint32_t pid = blockIdx.x >> 1, nfirst = a.o[a.deal.first].tiles;
 
   if (tid == 0) {
     for (int i = 0; i < kAdjStages; i++) {
@@ -96,109 +180,161 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
       mbar_init(empty + 8 * i, 1);
     }
     mbar_init(acc_full, 1);
+    mbar_init(acc_empty, 2 * kAdjEpiWarps);  // the epilogue warps of both CTAs
     mbar_init(mma_done, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = *tmem_slot;  // columns [0, 256): hi accumulator; [256, 512): mid + lo
 
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t issued = 0;
-      for (uint32_t k = 0; k < a.nstages; k++) {
-        const uint32_t s = k % kAdjStages, use = k / kAdjStages;
-        if (use > 0 && !mbar_wait_err(empty + 8 * s, (use - 1) & 1, abort_flag, err)) break;
-        mbar_expect_tx(full + 8 * s, kAdjStageBytes);
-        const uint32_t dst = smem_u32(smem + s * kAdjStageBytes);
-        const int x = (int)(k * kAdjKs);
-        tma_load_2d(dst, &tmHi, x, (int)r0, full + 8 * s);
-        tma_load_2d(dst + kAdjSplitBytes, &tmMid, x, (int)r0, full + 8 * s);
-        tma_load_2d(dst + 2 * kAdjSplitBytes, &tmLo, x, (int)r0, full + 8 * s);
-        tma_load_2d(dst + 3 * kAdjSplitBytes, &tmV, x, (int)k0, full + 8 * s);
-        issued = k + 1;
+    if (lane == 0 && peer == 0) {
+      uint32_t g = 0, grad, t;
+      bool stop = false;
+      for (uint32_t i = 0; !stop && dealt_tile(a.deal, nfirst, pid, i, grad, t); i++) {
+        const uint32_t r0 = t / a.ctiles * 256u, k0 = t % a.ctiles * 256u, nk = a.o[grad].nstages;
+        for (uint32_t k = 0; k < nk; k++, g++) {
+          const uint32_t s = g % kAdjStages, use = g / kAdjStages;
+          if (use > 0 && !mbar_wait_err(empty + 8 * s, (use - 1) & 1, abort_flag, err)) {
+            stop = true;
+            break;
+          }
+          const uint32_t fb = map_to_rank(full + 8 * s, 0);
+          mbar_expect_tx(full + 8 * s, 2 * kAdjStageBytes);
+          const uint32_t dst = smem_u32(smem + s * kAdjStageBytes);
+          const int sk = (int)(k * kAdjKs);
+#pragma unroll
+          for (uint32_t h = 0; h < 2; h++) {  // the leader's halves, then the peer's
+            const uint32_t d = h ? map_to_rank(dst, 1) : dst;
+            if (grad == 0) tma_load_3d_pair(d, &tmXk, sk, (int)(r0 + 128 * h), 0, fb);
+            else tma_load_4d_pair(d, &tmXmn, 0, sk, (int)(r0 / 64 + 2 * h), 0, fb);
+            tma_load_3d_pair(d + 3 * kAdjTermBytes, grad == 0 ? &tmVa : &tmVb, 0, sk, (int)(k0 / 64 + 2 * h), fb);
+          }
+        }
       }
-      if (*abort_flag)
-        for (uint32_t k = (issued > (uint32_t)kAdjStages ? issued - kAdjStages : 0); k < issued; k++)
-          mbar_drain_err(full + 8 * (k % kAdjStages), (k / kAdjStages) & 1, err);
+      if (*abort_flag)  // wait (bounded) for the loads the barriers still expect
+        for (uint32_t q = (g > (uint32_t)kAdjStages ? g - kAdjStages : 0); q < g; q++)
+          mbar_drain_err(full + 8 * (q % kAdjStages), (q / kAdjStages) & 1, err);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (lane == 0 && peer == 0) {
       bool ok = true;
-      for (uint32_t k = 0; k < a.nstages && ok; k++) {
-        const uint32_t s = k % kAdjStages;
-        if (!mbar_wait_err(full + 8 * s, (k / kAdjStages) & 1, abort_flag, err)) {
+      uint32_t g = 0, grad, t;
+      for (uint32_t i = 0; ok && dealt_tile(a.deal, nfirst, pid, i, grad, t); i++) {
+        if (i > 0 && !mbar_wait_err(acc_empty, (i - 1) & 1, abort_flag, err)) {
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t base = smem_u32(smem + s * kAdjStageBytes), vb = base + 3 * kAdjSplitBytes;
+        const uint32_t nk = a.o[grad].nstages, idesc = a.o[grad].idesc;
+        for (uint32_t k = 0; k < nk; k++, g++) {
+          const uint32_t s = g % kAdjStages;
+          if (!mbar_wait_err(full + 8 * s, (g / kAdjStages) & 1, abort_flag, err)) {
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;");
+          const uint32_t base = smem_u32(smem + s * kAdjStageBytes), vb = base + 3 * kAdjTermBytes;
 #pragma unroll
-        for (int kk = 0; kk < kAdjKs / 16; kk++) {  // K = 16 per MMA: 32 bytes along the row
-          const uint64_t bd = sw64_desc(vb + kk * 32);
-          const uint32_t first = (k | kk) != 0;
-          mma_bf16(tmem, sw64_desc(base + kk * 32), bd, a.idesc, first);
-          mma_bf16(tmem + 256, sw64_desc(base + kAdjSplitBytes + kk * 32), bd, a.idesc, first);
-          mma_bf16(tmem + 256, sw64_desc(base + 2 * kAdjSplitBytes + kk * 32), bd, a.idesc, 1u);
+          for (int kk = 0; kk < kAdjKs / 16; kk++) {  // K = 16 per MMA
+            const uint64_t bd = mn128_desc(vb + kk * 2048);
+            const uint32_t more = (k | kk) != 0;
+            uint64_t x[3];
+#pragma unroll
+            for (int j = 0; j < 3; j++)
+              x[j] = grad == 0 ? sw64_desc(base + j * kAdjTermBytes + kk * 32)
+                               : mn128_desc(base + j * kAdjTermBytes + kk * 2048);
+            mma_bf16_pair(tmem, x[0], bd, idesc, more);
+            mma_bf16_pair(tmem + 256, x[1], bd, idesc, more);
+            mma_bf16_pair(tmem + 256, x[2], bd, idesc, 1u);
+          }
+          mma_commit_pair(empty + 8 * s, 3);
         }
-        mma_commit(empty + 8 * s);
+        if (ok) mma_commit_pair(acc_full, 3);
       }
-      if (ok) {
-        mma_commit(acc_full);
-      } else {  // issued MMAs finish before TMEM is freed
-        mma_commit(mma_done);
+      if (!ok) {  // issued MMAs finish before TMEM is freed
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mma_done)
+                     : "memory");
         mbar_drain_err(mma_done, 0, err);
       }
     }
   } else {
-    if (__all_sync(0xffffffffu, mbar_wait_err(acc_full, 0, abort_flag, err))) {
+    // a warp takes 32 rows (its TMEM lanes) x 128 columns of the tile
+    const int q = warp & 3;
+    const uint32_t half = (uint32_t)(warp - 2) >> 2;
+    float *sc = scratch + (warp - 2) * kAdjScratchFloats;  // [32 rows][33]
+    const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + 128 * half;
+    uint32_t grad, t;
+    for (uint32_t i = 0; dealt_tile(a.deal, nfirst, pid, i, grad, t); i++) {
+      if (!__all_sync(0xffffffffu, mbar_wait_err(acc_full, i & 1, abort_flag, err))) break;
       asm volatile("tcgen05.fence::after_thread_sync;");
-      const int q = warp & 3;
-      float *sc = scratch + (warp - 2) * kAdjScratchFloats;  // [32 rows][33]
-      const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16);
-#pragma unroll 1
-      for (uint32_t c = 0; c < 256; c += 32) {
-        uint32_t hi[32], lo[32];
-        tmem_ld32(taddr + c, hi);
-        tmem_ld32(taddr + 256 + c, lo);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      float o[128];
 #pragma unroll
-        for (int j = 0; j < 32; j++) sc[lane * 33 + j] = __uint_as_float(hi[j]) + __uint_as_float(lo[j]);
-        __syncwarp();
-        // rows r0 + 32q .. +31 of this column block: one base pointer, a fixed
-        // row stride, no per-element predicate when all 32 rows exist
-        const uint32_t col = k0 + c + lane, row0 = r0 + q * 32;
-        if (col < a.K) {
-          float *p = a.out + (uint64_t)row0 * a.K + col;
-          const uint64_t K = a.K;
-          if (row0 + 32 <= a.R) {
-#pragma unroll 8
-            for (int i = 0; i < 32; i++) p[(uint64_t)i * K] = sc[i * 33 + lane];
-          } else {
+      for (int c = 0; c < 128; c += 16) {
+        uint32_t hi[16], lo[16];
+        tmem_ld16(taddr + c, hi);
+        tmem_ld16(taddr + 256 + c, lo);
+        tmem_wait_ld16(hi, lo);
+#pragma unroll
+        for (int j = 0; j < 16; j++) o[c + j] = __uint_as_float(hi[j]) + __uint_as_float(lo[j]);
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;");
+      __syncwarp();
+      if (lane == 0) {  // the accumulators may take the next tile
+        if (peer == 0) {
+          mbar_arrive(acc_empty);
+        } else {
+          const uint32_t rb = map_to_rank(acc_empty, 0);
+          asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(rb) : "memory");
+        }
+      }
+      const uint32_t row0 = t / a.ctiles * 256u + 128u * peer + q * 32, col0 = t % a.ctiles * 256u + 128 * half;
+      const uint32_t R = a.o[grad].R;
+      if (a.vec) {  // K % 8 == 0: each lane writes its row, 32 bytes at a time
+        if (row0 + lane < R) {
+          float *p = a.o[grad].out + (uint64_t)(row0 + lane) * a.K + col0;
+#pragma unroll
+          for (int c = 0; c < 128; c += 8)
+            if (col0 + c < a.K)
+              asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p + c), "f"(o[c]), "f"(o[c + 1]),
+                           "f"(o[c + 2]), "f"(o[c + 3]), "f"(o[c + 4]), "f"(o[c + 5]), "f"(o[c + 6]), "f"(o[c + 7])
+                           : "memory");
+        }
+      } else {  // through shared memory: the lanes write 32 consecutive columns of a row
+#pragma unroll
+        for (int c = 0; c < 128; c += 32) {
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 32; j++) sc[lane * 33 + j] = o[c + j];
+          __syncwarp();
+          if (col0 + c + lane < a.K) {
+            float *p = a.o[grad].out + (uint64_t)row0 * a.K + col0 + c + lane;
 #pragma unroll 4
-            for (int i = 0; i < 32; i++)
-              if (row0 + i < a.R) p[(uint64_t)i * K] = sc[i * 33 + lane];
+            for (int r = 0; r < 32; r++)
+              if (row0 + r < R) p[(uint64_t)r * a.K] = sc[r * 33 + lane];
           }
         }
-        __syncwarp();
       }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem));
   }
 }
 
-// ------------------------------------------------------------ pre-passes
+// ------------------------------------------------------------ pre-pass
 __device__ __forceinline__ void split3(float x, __nv_bfloat16 &h, __nv_bfloat16 &m, __nv_bfloat16 &l) {
   h = __float2bfloat16_rn(x);
   const float r1 = x - __bfloat162float(h);
@@ -206,135 +342,100 @@ __device__ __forceinline__ void split3(float x, __nv_bfloat16 &h, __nv_bfloat16 
   l = __float2bfloat16_rn(r1 - __bfloat162float(m));
 }
 
-// dC [N][M] -> hi/mid/lo in both orientations: [N][pM] (rows n) and [M][pN]
-// (rows m).  A block takes 64 x 64 elements: 16 consecutive m per thread in,
-// 16 consecutive n per thread out of the transposed tile, 16-byte stores.
-// 16 bf16 values, packed two per word (element 2i in the low half of w[i]).
-__device__ __forceinline__ void store16(__nv_bfloat16 *dst, const uint32_t (&w)[8], uint32_t valid) {
-  if (valid >= 16) {
-    reinterpret_cast<uint4 *>(dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-    reinterpret_cast<uint4 *>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
-  } else {
-    unsigned short *d16 = reinterpret_cast<unsigned short *>(dst);
-#pragma unroll
-    for (int j = 0; j < 16; j++)
-      if ((uint32_t)j < valid) d16[j] = (unsigned short)(w[j >> 1] >> (16 * (j & 1)));
-  }
-}
-
 __device__ __forceinline__ uint32_t bf16_bits(__nv_bfloat16 x) { return (uint32_t)__bfloat16_as_ushort(x); }
 
-// The three split terms of 16 values, packed for store16.
-__device__ __forceinline__ void split16(const float (&x)[16], uint32_t (&h)[8], uint32_t (&m)[8], uint32_t (&l)[8]) {
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    __nv_bfloat16 h0, m0, l0, h1, m1, l1;
-    split3(x[2 * i], h0, m0, l0);
-    split3(x[2 * i + 1], h1, m1, l1);
-    h[i] = bf16_bits(h0) | (bf16_bits(h1) << 16);
-    m[i] = bf16_bits(m0) | (bf16_bits(m1) << 16);
-    l[i] = bf16_bits(l0) | (bf16_bits(l1) << 16);
+// One operand's values, [rows][pitch] bf16.
+struct AdjValues {
+  const uint64_t *planes;
+  __nv_bfloat16 *out;
+  uint64_t plane_words, wpr, pitch;
+  uint32_t rows, chunks;  // chunks: 16-column pieces per row
+  int nbits, neg_msb, bipolar;
+  uint32_t blocks;  // blocks of the launch that work on it (0: already valid)
+};
+
+struct AdjPrepare {
+  const float *dC;
+  __nv_bfloat16 *split;  // [3][N][pM]
+  uint64_t pM, term;     // row pitch, elements per term
+  uint32_t N, M, chunks, blocks;  // chunks: 8-value pieces per row
+  AdjValues v[2];
+};
+
+// idx -> (row, piece) of rows of `per` pieces.
+__device__ __forceinline__ void piece_of(uint64_t idx, uint32_t per, uint32_t &row, uint32_t &piece) {
+  if (idx <= 0xFFFFFFFFull) {
+    row = (uint32_t)idx / per;
+    piece = (uint32_t)idx - row * per;
+  } else {
+    row = (uint32_t)(idx / per);
+    piece = (uint32_t)(idx - (uint64_t)row * per);
   }
 }
 
-__global__ void __launch_bounds__(256) split_kernel(const float *__restrict__ dC, uint32_t N, uint32_t M, uint32_t pM,
-                                                    uint32_t pN, int want_d, int want_t,
-                                                    __nv_bfloat16 *__restrict__ dh, __nv_bfloat16 *__restrict__ dm,
-                                                    __nv_bfloat16 *__restrict__ dl, __nv_bfloat16 *__restrict__ th,
-                                                    __nv_bfloat16 *__restrict__ tm, __nv_bfloat16 *__restrict__ tl) {
-  __shared__ float t[64][65];
-  const uint32_t m0 = blockIdx.x * 64;
-  const int row = threadIdx.x >> 2, part = threadIdx.x & 3;
-  for (uint32_t n0 = blockIdx.y * 64; n0 < N; n0 += gridDim.y * 64) {
-    {
-      const uint32_t n = n0 + row, mb = m0 + 16 * part;
-      float x[16];
-      const uint32_t valid = (n < N && mb < M) ? min(16u, M - mb) : 0u;
-      if (valid == 16 && (M & 3) == 0) {
-        const float4 *src = reinterpret_cast<const float4 *>(dC + (uint64_t)n * M + mb);
+// dC into its three terms (8 values a thread, 16 bytes of each term) and both
+// operands' planes into bf16 values (16 a thread), in one launch: block ranges.
+// HBM-bound: 34 MB in, 50 + 25 MB out at 4096 x 2048 x 2048.
+__global__ void __launch_bounds__(256) adjoint_prepare(const __grid_constant__ AdjPrepare a) {
+  uint32_t b = blockIdx.x;
+  if (b < a.blocks) {
+    const uint64_t idx = (uint64_t)b * 256 + threadIdx.x;
+    uint32_t n, c;
+    piece_of(idx, a.chunks, n, c);
+    if (n >= a.N) return;
+    const uint32_t m0 = 8 * c;
+    const float *src = a.dC + (uint64_t)n * a.M + m0;
+    float x[8];
+    if ((a.M & 3) == 0 && m0 + 8 <= a.M) {
+      const float4 u = reinterpret_cast<const float4 *>(src)[0], v = reinterpret_cast<const float4 *>(src)[1];
+      x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
+      x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
+    } else {
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-          const float4 v = src[i];
-          x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 16; j++) x[j] = (uint32_t)j < valid ? dC[(uint64_t)n * M + mb + j] : 0.f;
-      }
-#pragma unroll
-      for (int j = 0; j < 16; j++) t[row][16 * part + j] = x[j];
-      if (want_d && valid) {
-        uint32_t h[8], m[8], l[8];
-        split16(x, h, m, l);
-        const uint64_t o = (uint64_t)n * pM + mb;
-        store16(dh + o, h, valid);
-        store16(dm + o, m, valid);
-        store16(dl + o, l, valid);
-      }
+      for (int j = 0; j < 8; j++) x[j] = m0 + j < a.M ? src[j] : 0.f;
     }
-    __syncthreads();
-    if (want_t) {
-      const uint32_t m = m0 + row, nb = n0 + 16 * part;
-      const uint32_t valid = (m < M && nb < N) ? min(16u, N - nb) : 0u;
-      if (valid) {
-        float x[16];
+    uint32_t w[3][4];
 #pragma unroll
-        for (int j = 0; j < 16; j++) x[j] = t[16 * part + j][row];
-        uint32_t h[8], md[8], l[8];
-        split16(x, h, md, l);
-        const uint64_t o = (uint64_t)m * pN + nb;
-        store16(th + o, h, valid);
-        store16(tm + o, md, valid);
-        store16(tl + o, l, valid);
-      }
+    for (int j = 0; j < 4; j++) {
+      __nv_bfloat16 h0, m0_, l0, h1, m1, l1;
+      split3(x[2 * j], h0, m0_, l0);
+      split3(x[2 * j + 1], h1, m1, l1);
+      w[0][j] = bf16_bits(h0) | (bf16_bits(h1) << 16);
+      w[1][j] = bf16_bits(m0_) | (bf16_bits(m1) << 16);
+      w[2][j] = bf16_bits(l0) | (bf16_bits(l1) << 16);
     }
-    __syncthreads();
+    __nv_bfloat16 *dst = a.split + (uint64_t)n * a.pM + m0;  // pM is a multiple of 64: whole pieces
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+      *reinterpret_cast<uint4 *>(dst + j * a.term) = make_uint4(w[j][0], w[j][1], w[j][2], w[j][3]);
+    return;
   }
-}
-
-// Operand values, transposed: planes (rows s < S, columns k < K) -> Vt[k][s]
-// in bf16 with row pitch pS.  A block decodes 64 rows x 64 columns (one plane
-// word per row) through shared memory; threads store 16 consecutive s.
-__global__ void __launch_bounds__(256) values_t_kernel(const uint64_t *__restrict__ planes, uint64_t plane_words,
-                                                       uint64_t wpr, int nbits, int neg_msb, int bipolar, uint32_t S,
-                                                       uint32_t K, uint32_t pS, __nv_bfloat16 *__restrict__ vt) {
-  __shared__ __align__(16) __nv_bfloat16 t[64][72];  // [k][s], 144-byte rows
-  const uint32_t kw = blockIdx.x;
-  const int hi = threadIdx.x >> 2, part = threadIdx.x & 3;
-  for (uint32_t s0 = blockIdx.y * 64; s0 < S; s0 += gridDim.y * 64) {
-    {
-      const uint32_t s = s0 + hi;  // this thread: row s, columns 16*part .. +16 of word kw
-      float v[16];
+  b -= a.blocks;
+  const bool second = b >= a.v[0].blocks;
+  const AdjValues &o = a.v[second ? 1 : 0];
+  if (second) b -= a.v[0].blocks;
+  const uint64_t idx = (uint64_t)b * 256 + threadIdx.x;
+  uint32_t r, c;
+  piece_of(idx, o.chunks, r, c);
+  if (r >= o.rows) return;
+  // the codes of 16 columns, then their values: bit j of plane i adds +-2^i (bipolar: 2 bit - 1)
+  float v[16];
 #pragma unroll
-      for (int j = 0; j < 16; j++) v[j] = 0.f;
-      if (s < S) {
-        for (int b = 0; b < nbits; b++) {
-          const uint32_t bits = (uint32_t)(planes[b * plane_words + (uint64_t)s * wpr + kw] >> (16 * part)) & 0xFFFFu;
-          const float w = bipolar ? 2.f : (b == neg_msb ? -(float)(1 << b) : (float)(1 << b));
+  for (int j = 0; j < 16; j++) v[j] = o.bipolar ? -1.f : 0.f;
+  const uint16_t *src = reinterpret_cast<const uint16_t *>(o.planes + (uint64_t)r * o.wpr) + c;
+  for (int i = 0; i < o.nbits; i++) {
+    const uint32_t bits = src[(uint64_t)i * o.plane_words * 4];
+    const float w = o.bipolar ? 2.f : (i == o.neg_msb ? -(float)(1 << i) : (float)(1 << i));
 #pragma unroll
-          for (int j = 0; j < 16; j++) v[j] += ((bits >> j) & 1u) ? w : 0.f;
-        }
-        if (bipolar) {
-#pragma unroll
-          for (int j = 0; j < 16; j++) v[j] -= 1.f;
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < 16; j++) t[16 * part + j][hi] = __float2bfloat16_rn(v[j]);
-    }
-    __syncthreads();
-    {
-      const uint32_t k = kw * 64 + hi, sb = s0 + 16 * part;  // this thread: row k, s = sb .. +16
-      const uint32_t valid = (k < K && sb < S) ? min(16u, S - sb) : 0u;
-      if (valid) {
-        const uint4 *src = reinterpret_cast<const uint4 *>(&t[hi][16 * part]);
-        const uint4 a0 = src[0], a1 = src[1];
-        const uint32_t o[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-        store16(vt + (uint64_t)k * pS + sb, o, valid);
-      }
-    }
-    __syncthreads();
+    for (int j = 0; j < 16; j++) v[j] += ((bits >> j) & 1u) ? w : 0.f;
   }
+  uint32_t w[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++)
+    w[j] = bf16_bits(__float2bfloat16_rn(v[2 * j])) | (bf16_bits(__float2bfloat16_rn(v[2 * j + 1])) << 16);
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(o.out + (uint64_t)r * o.pitch + 16 * c),
+               "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -358,45 +459,41 @@ EncodeTiledFn adj_encode_fn() {
   return f;
 }
 
-// 2-D bf16 map over [rows][cols] (row pitch `pitch` elements), box 32 x box_rows
-// (64-byte rows), 64-byte swizzle.
-bool bf16_map(CUtensorMap *map, const void *base, uint64_t cols, uint64_t rows, uint64_t pitch, uint32_t box_rows) {
+bool bf16_map(CUtensorMap *map, const void *base, int rank, const cuuint64_t *dims, const cuuint64_t *strides,
+              const cuuint32_t *box, CUtensorMapSwizzle swizzle) {
   EncodeTiledFn fn = adj_encode_fn();
   if (!fn) return false;
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {pitch * 2};
-  cuuint32_t box[2] = {(cuuint32_t)kAdjKs, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void *)base, dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, (void *)base, dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-uint64_t pitch8(uint64_t x) { return (x + 7) / 8 * 8; }
+// Operand values [rows][pitch] as [pitch / 64][rows][64]: a box is 32 rows of 128 columns, MN-major.
+bool values_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t pitch) {
+  const cuuint64_t dims[3] = {64, rows, pitch / 64}, strides[2] = {pitch * 2, 128};
+  const cuuint32_t box[3] = {64, (cuuint32_t)kAdjKs, 2};
+  return bf16_map(map, base, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+uint64_t pitch64(uint64_t x) { return (x + 63) / 64 * 64; }
 
 }  // namespace
 
-// Workspace of a context's tensor-core adjoint: the splits of dC in both
-// orientations and both operands' transposed values, with their tensor maps.
+// Workspace of a context's tensor-core adjoint: the three terms of dC and both
+// operands' values, with their tensor maps.  Row pitches are multiples of 64
+// values, so a box of an MN-major map never leaves its row's pitch; columns past
+// the matrix are unwritten there and reach only outputs that are not stored.
 struct AdjPlan {
   __nv_bfloat16 *ws = nullptr;
-  __nv_bfloat16 *split_d[3] = {};  // [N][pM]  (dB)
-  __nv_bfloat16 *split_t[3] = {};  // [M][pN]  (dA)
-  __nv_bfloat16 *vt_b = nullptr;   // B values [K][pN] (dA)
-  __nv_bfloat16 *vt_a = nullptr;   // A values [K][pM] (dB)
-  CUtensorMap map_d[3], map_t[3], map_vb, map_va;
-  // dB runs on a second, high-priority stream, forked from and joined back to
-  // the caller's, so that dA's kernels fill the SMs dB's leave idle
-  cudaStream_t side = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
+  __nv_bfloat16 *split = nullptr;  // [3][N][pM]
+  __nv_bfloat16 *val[2] = {};      // lhs values [M][pK], rhs values [N][pK]
+  CUtensorMap xk, xmn, va, vb;
 };
 
 void adj_plan_free(AdjPlan *p) {
   if (!p) return;
   if (p->ws) cudaFree(p->ws);
-  if (p->fork) cudaEventDestroy(p->fork);
-  if (p->join) cudaEventDestroy(p->join);
-  if (p->side) cudaStreamDestroy(p->side);
   delete p;
 }
 
@@ -406,83 +503,113 @@ namespace {
 
 int build_plan(gbs_ctx *c) {
   const uint64_t M = c->lhs.nrows, N = c->rhs.nrows, K = c->lhs.ncols;
-  const uint64_t pM = pitch8(M), pN = pitch8(N);
-  const uint64_t n_d = N * pM, n_t = M * pN, n_vb = K * pN, n_va = K * pM;
+  const uint64_t pM = pitch64(M), pK = pitch64(K), term = N * pM;
   AdjPlan *p = new AdjPlan();
-  const size_t bytes = (3 * n_d + 3 * n_t + n_vb + n_va + 64) * sizeof(__nv_bfloat16);
+  // every array starts on a 128-byte boundary: the pitches are multiples of 64 values
+  const size_t bytes = (3 * term + (M + N) * pK) * sizeof(__nv_bfloat16);
   if (dev_alloc((void **)&p->ws, bytes) != cudaSuccess) {
     cudaGetLastError();
     delete p;
     return fail(GBS_ENOMEM, "gbs_adjoint: workspace allocation failed");
   }
-  // every array starts on a 128-byte boundary
-  uint8_t *q = reinterpret_cast<uint8_t *>(p->ws);
-  auto take = [&](uint64_t elems) {
-    __nv_bfloat16 *r = reinterpret_cast<__nv_bfloat16 *>(q);
-    q += (elems * 2 + 127) / 128 * 128;
-    return r;
-  };
-  for (int i = 0; i < 3; i++) p->split_d[i] = take(n_d);
-  for (int i = 0; i < 3; i++) p->split_t[i] = take(n_t);
-  p->vt_b = take(n_vb);
-  p->vt_a = take(n_va);
-  bool ok = true;
-  for (int i = 0; i < 3; i++) {
-    ok = ok && bf16_map(&p->map_d[i], p->split_d[i], M, N, pM, 128);  // dB: rows n, contraction m
-    ok = ok && bf16_map(&p->map_t[i], p->split_t[i], N, M, pN, 128);  // dA: rows m, contraction n
-  }
-  ok = ok && bf16_map(&p->map_vb, p->vt_b, N, K, pN, 256);
-  ok = ok && bf16_map(&p->map_va, p->vt_a, M, K, pM, 256);
-  if (!ok) {
+  p->split = p->ws;
+  p->val[0] = p->ws + 3 * term;
+  p->val[1] = p->val[0] + M * pK;
+  // dB: rows n, contraction m (contiguous); the true M and N bound the boxes, past them reads are 0
+  const cuuint64_t dk[3] = {M, N, 3}, sk[2] = {pM * 2, term * 2};
+  const cuuint32_t bk[3] = {(cuuint32_t)kAdjKs, 128, 3};
+  // dA: rows m (contiguous, 64 at a time), contraction n
+  const cuuint64_t dmn[4] = {64, N, pM / 64, 3}, smn[3] = {pM * 2, 128, term * 2};
+  const cuuint32_t bmn[4] = {64, (cuuint32_t)kAdjKs, 2, 3};
+  if (!bf16_map(&p->xk, p->split, 3, dk, sk, bk, CU_TENSOR_MAP_SWIZZLE_64B) ||
+      !bf16_map(&p->xmn, p->split, 4, dmn, smn, bmn, CU_TENSOR_MAP_SWIZZLE_128B) ||
+      !values_map(&p->va, p->val[0], M, pK) || !values_map(&p->vb, p->val[1], N, pK)) {
     adj_plan_free(p);
     return fail(GBS_EUNSUPPORTED, "gbs_adjoint: tensor map encoding failed");
-  }
-  // the side stream runs dB, whose tiles contract over M (twice as many
-  // stages as dA's at the benchmark shape): at the highest priority its
-  // long tiles are placed first and dA's shorter ones fill around them
-  int least = 0, greatest = 0;
-  cudaError_t e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
-  if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&p->side, cudaStreamNonBlocking, greatest);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->join, cudaEventDisableTiming);
-  if (e != cudaSuccess) {
-    adj_plan_free(p);
-    return cuda_fail(e, "gbs_adjoint: stream/event creation");
   }
   c->adj = p;
   return GBS_OK;
 }
 
-cudaError_t launch_values_t(const Mat &op, __nv_bfloat16 *vt, uint64_t pS, cudaStream_t s) {
-  const int neg = (op.issigned && !op.bipolar()) ? (int)op.nbits - 1 : -1;
-  dim3 grid((unsigned)op.wpr(), (unsigned)std::min<uint64_t>((op.nrows + 63) / 64, 65535));
-  values_t_kernel<<<grid, 256, 0, s>>>(op.planes, op.nrows_a * op.wpr(), op.wpr(), (int)op.nbits, neg,
-                                       op.bipolar() ? 1 : 0, (uint32_t)op.nrows, (uint32_t)op.ncols, (uint32_t)pS, vt);
-  count_launch();
-  return cudaGetLastError();
+// SM pairs the adjoint kernel can hold at once, cached per device.
+int adj_max_pairs() {
+  static std::atomic<int> cache[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int v = cache[dev].load(std::memory_order_relaxed);
+  if (v == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(2);
+    cfg.blockDim = dim3(kAdjThreads);
+    cfg.dynamicSmemBytes = adj_smem_bytes();
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    cudaError_t e = cudaFuncSetAttribute(adjoint_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)adj_smem_bytes());
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, adjoint_tc_kernel, &cfg);
+    if (e != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      return 0;
+    }
+    v = n;
+    cache[dev].store(v, std::memory_order_relaxed);
+  }
+  return v;
 }
 
-cudaError_t launch_gemm(const CUtensorMap (&split)[3], const CUtensorMap &vmap, uint64_t R, uint64_t S, uint64_t K,
-                        float *out, cudaStream_t s) {
-  AdjTcArgs a;
-  a.out = out;
-  a.R = (uint32_t)R;
-  a.K = (uint32_t)K;
-  a.nstages = (uint32_t)((S + kAdjKs - 1) / kAdjKs);
-  // kind::f16: D fp32, A and B bf16, both K-major, M = 128, N = 256
-  a.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | ((128u >> 4) << 24);
-  uint32_t *err = tc_error_ptr();
-  if (!err) return cudaErrorInvalidSymbol;
-  cudaError_t e =
-      cudaFuncSetAttribute(adjoint_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adj_smem_bytes());
-  if (e != cudaSuccess) return e;
-  dim3 grid((unsigned)((R + 127) / 128), (unsigned)((K + 255) / 256));
-  adjoint_tc_kernel<<<grid, kAdjThreads, adj_smem_bytes(), s>>>(split[0], split[1], split[2], vmap, a, err);
-  count_launch();
-  return cudaGetLastError();
+AdjValues values_job(const Mat &op, __nv_bfloat16 *out, bool wanted) {
+  AdjValues v;
+  memset(&v, 0, sizeof(v));
+  v.planes = op.planes;
+  v.out = out;
+  v.plane_words = op.nrows_a * op.wpr();
+  v.wpr = op.wpr();
+  v.pitch = pitch64(op.ncols);
+  v.rows = (uint32_t)op.nrows;
+  v.chunks = (uint32_t)((op.ncols + 15) / 16);
+  v.nbits = (int)op.nbits;
+  v.neg_msb = (op.issigned && !op.bipolar()) ? (int)op.nbits - 1 : -1;
+  v.bipolar = op.bipolar() ? 1 : 0;
+  v.blocks = wanted ? (uint32_t)(((uint64_t)v.rows * v.chunks + 255) / 256) : 0;
+  return v;
 }
 
 }  // namespace
+
+// Deals nfirst tiles of cfirst stages round robin over P pairs, then nother
+// tiles of cother stages, each to the pairs with the least work so far: equal
+// finishing times to within one tile.
+static AdjDeal deal_tiles(uint32_t first, uint64_t nfirst, uint64_t cfirst, uint64_t nother, uint64_t cother,
+                          uint32_t pairs) {
+  AdjDeal d;
+  memset(&d, 0, sizeof(d));
+  d.first = first;
+  d.pairs = pairs;
+  d.a = (uint32_t)(nfirst % pairs);
+  const uint64_t size[2] = {d.a, pairs - d.a};
+  uint64_t load[2] = {(nfirst / pairs + 1) * cfirst, nfirst / pairs * cfirst}, s[2] = {0, 0};
+  while (nother) {
+    const int g = size[0] && load[0] < load[1] ? 0 : 1;
+    const uint64_t take = std::min(nother, size[g]);
+    if (take == size[g]) {
+      s[g]++;
+      load[g] += cother;
+    } else {
+      d.extra = (uint32_t)take;
+      d.extra_kind = (uint32_t)g;
+    }
+    nother -= take;
+  }
+  d.sa = (uint32_t)s[0];
+  d.sb = (uint32_t)s[1];
+  return d;
+}
 
 // dA = dC . B and dB = dC^T . A on the tensor cores (either output may be null).
 int adjoint_tc(gbs_ctx *c, const float *dC, float *dA, float *dB, cudaStream_t s) {
@@ -494,50 +621,71 @@ int adjoint_tc(gbs_ctx *c, const float *dC, float *dA, float *dB, cudaStream_t s
     if (e == cudaSuccess && dB && N && K) e = cudaMemsetAsync(dB, 0, N * K * 4, s);
     return e == cudaSuccess ? GBS_OK : cuda_fail(e, "gbs_adjoint: memset");
   }
+  if (!dA && !dB) return GBS_OK;
   if (!c->adj) {
     const int rc = build_plan(c);
     if (rc != GBS_OK) return rc;
   }
   AdjPlan &p = *c->adj;
-  const uint64_t pM = pitch8(M), pN = pitch8(N);
-  dim3 sg((unsigned)((M + 63) / 64), (unsigned)std::min<uint64_t>((N + 63) / 64, 65535));
-  cudaError_t e = cudaSuccess;
-  // dB on the high-priority side stream, enqueued first: its split of dC,
-  // A's values, the GEMM
-  if (dB) {
-    e = cudaEventRecord(p.fork, s);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(p.side, p.fork, 0);
-    if (e != cudaSuccess) return cuda_fail(e, "gbs_adjoint: stream fork");
-    split_kernel<<<sg, 256, 0, p.side>>>(dC, (uint32_t)N, (uint32_t)M, (uint32_t)pM, (uint32_t)pN, 1, 0, p.split_d[0],
-                                         p.split_d[1], p.split_d[2], p.split_t[0], p.split_t[1], p.split_t[2]);
-    count_launch();
-    e = cudaGetLastError();
-    if (e == cudaSuccess && !c->vt_valid[0]) {  // operand values: rebuilt only after an import
-      e = launch_values_t(c->lhs, p.vt_a, pM, p.side);
-      c->vt_valid[0] = e == cudaSuccess;
-    }
-    if (e == cudaSuccess) e = launch_gemm(p.map_d, p.map_va, N, M, K, dB, p.side);
-    if (e == cudaSuccess) e = cudaEventRecord(p.join, p.side);
-    if (e != cudaSuccess) return cuda_fail(e, "gbs_adjoint: dB kernels");
+  // dB contracts over m with A's values, dA over n with B's
+  const bool want[2] = {dB != nullptr, dA != nullptr};
+  AdjPrepare pr;
+  memset(&pr, 0, sizeof(pr));
+  pr.dC = dC;
+  pr.split = p.split;
+  pr.pM = pitch64(M);
+  pr.term = N * pr.pM;
+  pr.N = (uint32_t)N;
+  pr.M = (uint32_t)M;
+  pr.chunks = (uint32_t)((M + 7) / 8);
+  pr.blocks = (uint32_t)((N * pr.chunks + 255) / 256);
+  pr.v[0] = values_job(c->lhs, p.val[0], want[0] && !c->vt_valid[0]);
+  pr.v[1] = values_job(c->rhs, p.val[1], want[1] && !c->vt_valid[1]);
+  adjoint_prepare<<<pr.blocks + pr.v[0].blocks + pr.v[1].blocks, 256, 0, s>>>(pr);
+  count_launch();
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail(e, "gbs_adjoint: split kernel");
+  for (int side = 0; side < 2; side++)
+    if (want[side]) c->vt_valid[side] = true;
+
+  AdjTcArgs a;
+  memset(&a, 0, sizeof(a));
+  a.K = (uint32_t)K;
+  a.ctiles = (uint32_t)((K + 255) / 256);
+  a.vec = K % 8 == 0 && ((uintptr_t)dA | (uintptr_t)dB) % 32 == 0;
+  for (int g = 0; g < 2; g++) {
+    AdjOut &o = a.o[g];
+    const uint64_t R = g ? M : N, S = g ? N : M;
+    o.out = g ? dA : dB;
+    o.R = (uint32_t)R;
+    o.tiles = want[g] ? (uint32_t)((R + 255) / 256) * a.ctiles : 0;
+    o.nstages = (uint32_t)((S + kAdjKs - 1) / kAdjKs);
+    // kind::f16: D fp32, A and B bf16, M = 256, N = 256; B MN-major, A MN-major for dA
+    o.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)g << 15) | (1u << 16) | ((256u >> 3) << 17) |
+              ((256u >> 4) << 24);
   }
-  // dA on the caller's stream: its split of dC (transposed), B's values, the GEMM
-  if (dA) {
-    split_kernel<<<sg, 256, 0, s>>>(dC, (uint32_t)N, (uint32_t)M, (uint32_t)pM, (uint32_t)pN, 0, 1, p.split_d[0],
-                                    p.split_d[1], p.split_d[2], p.split_t[0], p.split_t[1], p.split_t[2]);
-    count_launch();
-    e = cudaGetLastError();
-    if (e == cudaSuccess && !c->vt_valid[1]) {
-      e = launch_values_t(c->rhs, p.vt_b, pN, s);
-      c->vt_valid[1] = e == cudaSuccess;
-    }
-    if (e == cudaSuccess) e = launch_gemm(p.map_t, p.map_vb, M, N, K, dA, s);
-    if (e != cudaSuccess) return cuda_fail(e, "gbs_adjoint: dA kernels");
-  }
-  if (dB) {
-    e = cudaStreamWaitEvent(s, p.join, 0);
-    if (e != cudaSuccess) return cuda_fail(e, "gbs_adjoint: stream join");
-  }
-  return GBS_OK;
+  const uint64_t tiles = (uint64_t)a.o[0].tiles + a.o[1].tiles;
+  const uint32_t pairs = (uint32_t)std::min<uint64_t>(tiles, (uint64_t)adj_max_pairs());
+  if (!pairs) return fail(GBS_ECUDA, "gbs_adjoint: the SM-pair kernel does not fit this device");
+  const uint32_t first = a.o[0].nstages >= a.o[1].nstages ? 0 : 1;  // the longer contraction
+  a.deal = deal_tiles(first, a.o[first].tiles, a.o[first].nstages, a.o[1 - first].tiles, a.o[1 - first].nstages, pairs);
+  uint32_t *err = tc_error_ptr();
+  if (!err) return fail(GBS_ECUDA, "gbs_adjoint: no error word");
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(2 * pairs);
+  cfg.blockDim = dim3(kAdjThreads);
+  cfg.dynamicSmemBytes = adj_smem_bytes();
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  e = cudaLaunchKernelEx(&cfg, adjoint_tc_kernel, p.xk, p.xmn, p.va, p.vb, a, err);
+  count_launch();
+  return e == cudaSuccess ? GBS_OK : cuda_fail(e, "gbs_adjoint: GEMM kernel");
 }
 
 }  // namespace gbs
