@@ -30,14 +30,17 @@
 // GEMM kernel: one launch computes dA and dB.  Persistent SM pairs
 // (cta_group::2, M = 256, N = 256) walk 256 x 256 tiles of both, the gradient
 // with the longer contraction first, the other's tiles given out so that the
-// pairs finish together (deal_tiles).  32 values of s per stage in a 6-stage ring, 32 KB of
-// each SM; the leader's TMA loads a stage for both (the three terms in one
-// box), its MMA thread issues 6 tcgen05.mma.kind::f16 (K = 16) into the two
-// accumulators (all 512 TMEM columns).  Eight epilogue warps add the
+// pairs finish together (deal_tiles).  64 values of s per stage in a 3-stage
+// ring, 64 KB of each SM; the leader's TMA loads a stage for both (the three
+// terms in one box), its MMA thread issues 12 tcgen05.mma.kind::f16 (K = 16) into
+// the two accumulators (all 512 TMEM columns).  Eight epilogue warps add the
 // accumulators into registers, release TMEM to the next tile's MMAs and store
-// while these run.  Tensor-bound: 6 pair MMAs of 68 ns a stage; a lone SM on
-// 128 x 256 tiles moved 112 KB of shared memory in that time and ran 0.49 us a
-// stage.  Every mbarrier wait is bounded.
+// while these run.  Tensor-bound: 0.80 us a stage, its MMAs' own time (12 pair
+// MMAs of 66-68 ns); a lone SM on 128 x 256 tiles moved 112 KB of shared memory per
+// half stage and ran 0.98 us.  Stages of 32 values hold the same bytes in
+// flight, but their 64-byte rows (64-byte swizzle) read slower than whole
+// 128-byte ones: 0.93 us per 64 values of the contraction-major gradient.
+// Every mbarrier wait is bounded.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -54,9 +57,9 @@ namespace {
 constexpr int kAdjEpiWarps = 8;
 constexpr int kAdjThreads = 64 + 32 * kAdjEpiWarps;
 constexpr uint32_t kAdjScratchFloats = 32 * 33;  // per epilogue warp
-constexpr int kAdjKs = 32;
-constexpr int kAdjStages = 6;
-constexpr uint32_t kAdjTermBytes = 128 * kAdjKs * 2;  // one term: 128 rows x 32 bf16
+constexpr int kAdjKs = 64;
+constexpr int kAdjStages = 3;
+constexpr uint32_t kAdjTermBytes = 128 * kAdjKs * 2;  // one term: 128 rows x kAdjKs bf16
 constexpr uint32_t kAdjValBytes = 128 * kAdjKs * 2;   // this CTA's 128 of the tile's 256 value columns
 constexpr uint32_t kAdjStageBytes = 3 * kAdjTermBytes + kAdjValBytes;
 
@@ -130,10 +133,10 @@ __device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const CUtensorMap
       : "memory");
 }
 // MN-major operand, 128-byte swizzle: 64 values of the row (column) dimension
-// contiguous, the 32 contraction steps of a stage 128 bytes apart (groups of 8
-// 1024 bytes apart), the next 64 values 4096 bytes on.
+// contiguous, the kAdjKs contraction steps of a stage 128 bytes apart (groups of
+// 8 1024 bytes apart), the next 64 values after all of them.
 __device__ __forceinline__ uint64_t mn128_desc(uint32_t addr) {
-  return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(4096 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+  return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(kAdjKs * 128 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
@@ -250,7 +253,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
             uint64_t x[3];
 #pragma unroll
             for (int j = 0; j < 3; j++)
-              x[j] = grad == 0 ? sw64_desc(base + j * kAdjTermBytes + kk * 32)
+              x[j] = grad == 0 ? sw128_desc(base + j * kAdjTermBytes + kk * 32)
                                : mn128_desc(base + j * kAdjTermBytes + kk * 2048);
             mma_bf16_pair(tmem, x[0], bd, idesc, more);
             mma_bf16_pair(tmem + 256, x[1], bd, idesc, more);
@@ -469,7 +472,7 @@ bool bf16_map(CUtensorMap *map, const void *base, int rank, const cuuint64_t *di
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Operand values [rows][pitch] as [pitch / 64][rows][64]: a box is 32 rows of 128 columns, MN-major.
+// Operand values [rows][pitch] as [pitch / 64][rows][64]: a box is kAdjKs rows of 128 columns, MN-major.
 bool values_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t pitch) {
   const cuuint64_t dims[3] = {64, rows, pitch / 64}, strides[2] = {pitch * 2, 128};
   const cuuint32_t box[3] = {64, (cuuint32_t)kAdjKs, 2};
@@ -521,7 +524,7 @@ int build_plan(gbs_ctx *c) {
   // dA: rows m (contiguous, 64 at a time), contraction n
   const cuuint64_t dmn[4] = {64, N, pM / 64, 3}, smn[3] = {pM * 2, 128, term * 2};
   const cuuint32_t bmn[4] = {64, (cuuint32_t)kAdjKs, 2, 3};
-  if (!bf16_map(&p->xk, p->split, 3, dk, sk, bk, CU_TENSOR_MAP_SWIZZLE_64B) ||
+  if (!bf16_map(&p->xk, p->split, 3, dk, sk, bk, CU_TENSOR_MAP_SWIZZLE_128B) ||
       !bf16_map(&p->xmn, p->split, 4, dmn, smn, bmn, CU_TENSOR_MAP_SWIZZLE_128B) ||
       !values_map(&p->va, p->val[0], M, pK) || !values_map(&p->vb, p->val[1], N, pK)) {
     adj_plan_free(p);
