@@ -29,8 +29,8 @@
 //
 // GEMM kernel: one launch computes dA and dB.  Persistent SM pairs
 // (cta_group::2, M = 256, N = 256) walk 256 x 256 tiles of both, the gradient
-// with the longer contraction first, the other's tiles given out so that the
-// pairs finish together (deal_tiles).  64 values of s per stage in a 3-stage
+// with the longer contraction first, the other's tiles and parts of tiles given
+// out so that the pairs finish together (deal_tiles).  64 values of s per stage in a 3-stage
 // ring, 64 KB of each SM; the leader's TMA loads a stage for both (the three
 // terms in one box), its MMA thread issues 12 tcgen05.mma.kind::f16 (K = 16) into
 // the two accumulators (all 512 TMEM columns).  Eight epilogue warps add the
@@ -75,38 +75,67 @@ struct AdjOut {
   uint32_t idesc;
 };
 
-// Tiles of the two gradients dealt to P pairs (deal_tiles): gradient `first`
-// round robin (pairs below `a` get one more than the rest), then a contiguous
-// run of the other's, sa or sb tiles for a pair of either kind, one more for
-// the first `extra` pairs of kind `extra_kind`.
+// Tiles of the two gradients dealt to the pairs (deal_tiles): gradient `first`
+// round robin (pairs below `a` get one more than the rest), or, with fpieces
+// above 1, in that many parts of its contraction, a part a pair; then a
+// contiguous run of the other's tiles, sa or sb for a pair below `a` or not;
+// the `rem` tiles left over go out in `pieces` parts, a part a pair from p0 on.
 struct AdjDeal {
-  uint32_t first, pairs, a, sa, sb, extra, extra_kind;
+  uint32_t first, pairs, a, sa, sb, rem, pieces, p0, fpieces;
+  uint32_t grid;  // pairs that have work
 };
 
 struct AdjTcArgs {
   AdjOut o[2];  // 0: dB (contraction-major X), 1: dA (row-contiguous X)
   uint32_t K, ctiles, vec;  // vec: K and both outputs allow 32-byte stores
   AdjDeal deal;
+  // split tiles: [first gradient or other][pair][CTA][epilogue warp][128 columns][32 rows] sums of a part,
+  // and whether they are there (zeroed by adjoint_prepare)
+  float *part;
+  uint32_t *flags;
 };
 
-// The i-th tile of pair p: its gradient and number, false when p has no i-th tile.
-__host__ __device__ inline bool dealt_tile(const AdjDeal &d, uint32_t nfirst, uint32_t p, uint32_t i, uint32_t &grad,
-                                           uint32_t &t) {
-  const uint32_t mine = nfirst > p ? (nfirst - p - 1) / d.pairs + 1 : 0;
-  if (i < mine) {
-    grad = d.first;
-    t = p + i * d.pairs;
-    return true;
+// A tile, or part `piece` of `pieces` of its contraction, that a pair works on.
+struct AdjTile {
+  uint32_t grad, t, piece, pieces;
+};
+
+// The i-th of pair p; false when it has no i-th.
+__host__ __device__ inline bool dealt_tile(const AdjDeal &d, uint32_t nfirst, uint32_t p, uint32_t i, AdjTile &w) {
+  w.piece = 0;
+  w.pieces = 1;
+  w.grad = d.first;
+  uint32_t mine;
+  if (d.fpieces > 1) {
+    mine = p < nfirst * d.fpieces ? 1 : 0;
+    w.t = p / d.fpieces;
+    if (i < mine) {
+      w.piece = p % d.fpieces;
+      w.pieces = d.fpieces;
+      return true;
+    }
+  } else {
+    mine = nfirst > p ? (nfirst - p - 1) / d.pairs + 1 : 0;
+    w.t = p + i * d.pairs;
+    if (i < mine) return true;
   }
   i -= mine;
-  const bool b = p >= d.a;
-  const uint32_t r = b ? p - d.a : p, per = b ? d.sb : d.sa;
-  const uint32_t ex = d.extra_kind == (b ? 1u : 0u) ? d.extra : 0u;  // extra pairs of this kind
-  if (i >= per + (r < ex ? 1u : 0u)) return false;
-  const uint32_t before = b ? d.a * d.sa + (d.extra_kind == 0 ? d.extra : 0u) : 0u;  // the a pairs' tiles
-  grad = 1 - d.first;
-  t = before + r * per + (r < ex ? r : ex) + i;
+  w.grad = 1 - d.first;
+  const uint32_t per = p < d.a ? d.sa : d.sb;
+  w.t = (p < d.a ? p * d.sa : d.a * d.sa + (p - d.a) * d.sb) + i;
+  if (i < per) return true;
+  const uint32_t x = p - d.p0;
+  if (i > per || p < d.p0 || x >= d.rem * d.pieces) return false;
+  w.t = d.a * d.sa + (d.pairs - d.a) * d.sb + x / d.pieces;
+  w.piece = x % d.pieces;
+  w.pieces = d.pieces;
   return true;
+}
+
+// Stages [lo, hi) of a tile's contraction that the piece covers.
+__host__ __device__ inline void piece_stages(const AdjTile &w, uint32_t nstages, uint32_t &lo, uint32_t &hi) {
+  lo = (uint32_t)((uint64_t)w.piece * nstages / w.pieces);
+  hi = (uint32_t)((uint64_t)(w.piece + 1) * nstages / w.pieces);
 }
 
 __device__ __forceinline__ void mma_bf16_pair(uint32_t tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
@@ -200,11 +229,13 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
 
   if (warp == 0) {
     if (lane == 0 && peer == 0) {
-      uint32_t g = 0, grad, t;
+      uint32_t g = 0, k_lo, k_hi;
+      AdjTile w;
       bool stop = false;
-      for (uint32_t i = 0; !stop && dealt_tile(a.deal, nfirst, pid, i, grad, t); i++) {
-        const uint32_t r0 = t / a.ctiles * 256u, k0 = t % a.ctiles * 256u, nk = a.o[grad].nstages;
-        for (uint32_t k = 0; k < nk; k++, g++) {
+      for (uint32_t i = 0; !stop && dealt_tile(a.deal, nfirst, pid, i, w); i++) {
+        const uint32_t r0 = w.t / a.ctiles * 256u, k0 = w.t % a.ctiles * 256u;
+        piece_stages(w, a.o[w.grad].nstages, k_lo, k_hi);
+        for (uint32_t k = k_lo; k < k_hi; k++, g++) {
           const uint32_t s = g % kAdjStages, use = g / kAdjStages;
           if (use > 0 && !mbar_wait_err(empty + 8 * s, (use - 1) & 1, abort_flag, err)) {
             stop = true;
@@ -217,9 +248,9 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
 #pragma unroll
           for (uint32_t h = 0; h < 2; h++) {  // the leader's halves, then the peer's
             const uint32_t d = h ? map_to_rank(dst, 1) : dst;
-            if (grad == 0) tma_load_3d_pair(d, &tmXk, sk, (int)(r0 + 128 * h), 0, fb);
+            if (w.grad == 0) tma_load_3d_pair(d, &tmXk, sk, (int)(r0 + 128 * h), 0, fb);
             else tma_load_4d_pair(d, &tmXmn, 0, sk, (int)(r0 / 64 + 2 * h), 0, fb);
-            tma_load_3d_pair(d + 3 * kAdjTermBytes, grad == 0 ? &tmVa : &tmVb, 0, sk, (int)(k0 / 64 + 2 * h), fb);
+            tma_load_3d_pair(d + 3 * kAdjTermBytes, w.grad == 0 ? &tmVa : &tmVb, 0, sk, (int)(k0 / 64 + 2 * h), fb);
           }
         }
       }
@@ -230,15 +261,17 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
   } else if (warp == 1) {
     if (lane == 0 && peer == 0) {
       bool ok = true;
-      uint32_t g = 0, grad, t;
-      for (uint32_t i = 0; ok && dealt_tile(a.deal, nfirst, pid, i, grad, t); i++) {
+      uint32_t g = 0, k_lo, k_hi;
+      AdjTile w;
+      for (uint32_t i = 0; ok && dealt_tile(a.deal, nfirst, pid, i, w); i++) {
         if (i > 0 && !mbar_wait_err(acc_empty, (i - 1) & 1, abort_flag, err)) {
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t nk = a.o[grad].nstages, idesc = a.o[grad].idesc;
-        for (uint32_t k = 0; k < nk; k++, g++) {
+        const uint32_t idesc = a.o[w.grad].idesc;
+        piece_stages(w, a.o[w.grad].nstages, k_lo, k_hi);
+        for (uint32_t k = k_lo; k < k_hi; k++, g++) {
           const uint32_t s = g % kAdjStages;
           if (!mbar_wait_err(full + 8 * s, (g / kAdjStages) & 1, abort_flag, err)) {
             ok = false;
@@ -249,11 +282,11 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
 #pragma unroll
           for (int kk = 0; kk < kAdjKs / 16; kk++) {  // K = 16 per MMA
             const uint64_t bd = mn128_desc(vb + kk * 2048);
-            const uint32_t more = (k | kk) != 0;
+            const uint32_t more = k != k_lo || kk != 0;
             uint64_t x[3];
 #pragma unroll
             for (int j = 0; j < 3; j++)
-              x[j] = grad == 0 ? sw128_desc(base + j * kAdjTermBytes + kk * 32)
+              x[j] = w.grad == 0 ? sw128_desc(base + j * kAdjTermBytes + kk * 32)
                                : mn128_desc(base + j * kAdjTermBytes + kk * 2048);
             mma_bf16_pair(tmem, x[0], bd, idesc, more);
             mma_bf16_pair(tmem + 256, x[1], bd, idesc, more);
@@ -275,8 +308,10 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
     const uint32_t half = (uint32_t)(warp - 2) >> 2;
     float *sc = scratch + (warp - 2) * kAdjScratchFloats;  // [32 rows][33]
     const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + 128 * half;
-    uint32_t grad, t;
-    for (uint32_t i = 0; dealt_tile(a.deal, nfirst, pid, i, grad, t); i++) {
+    // this warp's slot of the partial sums: pair p's of the same CTA and warp are 2 * kAdjEpiWarps slots apart
+    const uint32_t slot0 = (pid * 2 + peer) * kAdjEpiWarps + (warp - 2), kind_slots = a.deal.pairs * 2 * kAdjEpiWarps;
+    AdjTile w;
+    for (uint32_t i = 0; dealt_tile(a.deal, nfirst, pid, i, w); i++) {
       if (!__all_sync(0xffffffffu, mbar_wait_err(acc_full, i & 1, abort_flag, err))) break;
       asm volatile("tcgen05.fence::after_thread_sync;");
       float o[128];
@@ -299,11 +334,48 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
           asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(rb) : "memory");
         }
       }
-      const uint32_t row0 = t / a.ctiles * 256u + 128u * peer + q * 32, col0 = t % a.ctiles * 256u + 128 * half;
-      const uint32_t R = a.o[grad].R;
+      if (w.pieces > 1) {
+        // A split tile: the pairs of its first parts leave their sums, the last part's pair adds them in
+        // order.  It waits only for pairs before its own, each of which leaves its sums without waiting.
+        const uint32_t slot = slot0 + (w.grad == a.deal.first ? 0 : kind_slots);
+        if (w.piece + 1 < w.pieces) {
+          float *dst = a.part + (uint64_t)slot * 4096 + lane;
+#pragma unroll
+          for (int c = 0; c < 128; c++) dst[32 * c] = o[c];
+          __threadfence();
+          __syncwarp();
+          if (lane == 0)
+            asm volatile("st.release.gpu.global.u32 [%0], 1;" ::"l"(a.flags + slot) : "memory");
+          continue;
+        }
+        bool ok = true;
+        for (uint32_t h = w.pieces - 1; h > 0 && ok; h--) {
+          const uint32_t from = slot - h * 2 * kAdjEpiWarps;
+          uint32_t seen = 0;
+          for (uint32_t it = 0; it < kTcWaitLimit && !seen; it++) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.flags + from) : "memory");
+            if (!seen) {
+              if (*abort_flag) break;
+              __nanosleep(64);
+            }
+          }
+          ok = __all_sync(0xffffffffu, seen != 0);
+          if (!ok) break;
+          const float *src = a.part + (uint64_t)from * 4096 + lane;
+#pragma unroll
+          for (int c = 0; c < 128; c++) o[c] += __ldcg(src + 32 * c);
+        }
+        if (!ok) {
+          *abort_flag = 1;
+          if (lane == 0) atomicOr(err, 1u);
+          break;
+        }
+      }
+      const uint32_t row0 = w.t / a.ctiles * 256u + 128u * peer + q * 32, col0 = w.t % a.ctiles * 256u + 128 * half;
+      const uint32_t R = a.o[w.grad].R;
       if (a.vec) {  // K % 8 == 0: each lane writes its row, 32 bytes at a time
         if (row0 + lane < R) {
-          float *p = a.o[grad].out + (uint64_t)(row0 + lane) * a.K + col0;
+          float *p = a.o[w.grad].out + (uint64_t)(row0 + lane) * a.K + col0;
 #pragma unroll
           for (int c = 0; c < 128; c += 8)
             if (col0 + c < a.K)
@@ -319,7 +391,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
           for (int j = 0; j < 32; j++) sc[lane * 33 + j] = o[c + j];
           __syncwarp();
           if (col0 + c + lane < a.K) {
-            float *p = a.o[grad].out + (uint64_t)row0 * a.K + col0 + c + lane;
+            float *p = a.o[w.grad].out + (uint64_t)row0 * a.K + col0 + c + lane;
 #pragma unroll 4
             for (int r = 0; r < 32; r++)
               if (row0 + r < R) p[(uint64_t)r * a.K] = sc[r * 33 + lane];
@@ -355,6 +427,7 @@ struct AdjValues {
   uint32_t rows, chunks;  // chunks: 16-column pieces per row
   int nbits, neg_msb, bipolar;
   uint32_t blocks;  // blocks of the launch that work on it (0: already valid)
+  uint32_t lo[4], hi[4];  // at most 4 bits: low and high bytes of the bf16 value of every code, 4 per word
 };
 
 struct AdjPrepare {
@@ -363,6 +436,8 @@ struct AdjPrepare {
   uint64_t pM, term;     // row pitch, elements per term
   uint32_t N, M, chunks, blocks;  // chunks: 8-value pieces per row
   AdjValues v[2];
+  uint32_t *flags;  // the GEMM's split-tile flags, zeroed here
+  uint32_t nflags;
 };
 
 // idx -> (row, piece) of rows of `per` pieces.
@@ -381,6 +456,8 @@ __device__ __forceinline__ void piece_of(uint64_t idx, uint32_t per, uint32_t &r
 // HBM-bound: 34 MB in, 50 + 25 MB out at 4096 x 2048 x 2048.
 __global__ void __launch_bounds__(256) adjoint_prepare(const __grid_constant__ AdjPrepare a) {
   uint32_t b = blockIdx.x;
+  if (b == 0)
+    for (uint32_t i = threadIdx.x; i < a.nflags; i += 256) a.flags[i] = 0u;
   if (b < a.blocks) {
     const uint64_t idx = (uint64_t)b * 256 + threadIdx.x;
     uint32_t n, c;
@@ -421,21 +498,49 @@ __global__ void __launch_bounds__(256) adjoint_prepare(const __grid_constant__ A
   uint32_t r, c;
   piece_of(idx, o.chunks, r, c);
   if (r >= o.rows) return;
-  // the codes of 16 columns, then their values: bit j of plane i adds +-2^i (bipolar: 2 bit - 1)
-  float v[16];
-#pragma unroll
-  for (int j = 0; j < 16; j++) v[j] = o.bipolar ? -1.f : 0.f;
   const uint16_t *src = reinterpret_cast<const uint16_t *>(o.planes + (uint64_t)r * o.wpr) + c;
-  for (int i = 0; i < o.nbits; i++) {
-    const uint32_t bits = src[(uint64_t)i * o.plane_words * 4];
-    const float w = o.bipolar ? 2.f : (i == o.neg_msb ? -(float)(1 << i) : (float)(1 << i));
-#pragma unroll
-    for (int j = 0; j < 16; j++) v[j] += ((bits >> j) & 1u) ? w : 0.f;
-  }
   uint32_t w[8];
+  if (o.nbits <= 4) {
+    // the plane bits of 4 columns spread to the low bits of 4 nibbles, the planes or-ed into 4 codes, which
+    // select their bf16 bytes by byte permutes (adding 16 floats per plane bit by bit took 8 us of integer
+    // instructions at 4096 x 2048 and 2048 x 2048)
+    uint32_t p[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-  for (int j = 0; j < 8; j++)
-    w[j] = bf16_bits(__float2bfloat16_rn(v[2 * j])) | (bf16_bits(__float2bfloat16_rn(v[2 * j + 1])) << 16);
+    for (int i = 0; i < 4; i++)
+      if (i < o.nbits) p[i] = src[(uint64_t)i * o.plane_words * 4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      uint32_t sel = 0u;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        uint32_t x = (p[i] >> (4 * j)) & 15u;
+        x = (x | (x << 6)) & 0x0303u;
+        sel |= ((x | (x << 3)) & 0x1111u) << i;
+      }
+      uint32_t lo = __byte_perm(o.lo[0], o.lo[1], sel & 0x7777u), hi = __byte_perm(o.hi[0], o.hi[1], sel & 0x7777u);
+      if (o.nbits == 4) {  // codes of 8 and more take the tables' second half
+        uint32_t m;  // 0xFF in byte i when code i has bit 3: prmt replicating the sign bits
+        asm("prmt.b32 %0, %1, %2, 0xD9C8;" : "=r"(m) : "r"(sel << 4), "r"(sel));
+        lo = (lo & ~m) | (__byte_perm(o.lo[2], o.lo[3], sel & 0x7777u) & m);
+        hi = (hi & ~m) | (__byte_perm(o.hi[2], o.hi[3], sel & 0x7777u) & m);
+      }
+      w[2 * j] = __byte_perm(lo, hi, 0x5140u);
+      w[2 * j + 1] = __byte_perm(lo, hi, 0x7362u);
+    }
+  } else {  // bit j of plane i adds +-2^i
+    float v[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++) v[j] = 0.f;
+    for (int i = 0; i < o.nbits; i++) {
+      const uint32_t bits = src[(uint64_t)i * o.plane_words * 4];
+      const float f = i == o.neg_msb ? -(float)(1 << i) : (float)(1 << i);
+#pragma unroll
+      for (int j = 0; j < 16; j++) v[j] += ((bits >> j) & 1u) ? f : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+      w[j] = bf16_bits(__float2bfloat16_rn(v[2 * j])) | (bf16_bits(__float2bfloat16_rn(v[2 * j + 1])) << 16);
+  }
   asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(o.out + (uint64_t)r * o.pitch + 16 * c),
                "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
                : "memory");
@@ -492,47 +597,23 @@ struct AdjPlan {
   __nv_bfloat16 *split = nullptr;  // [3][N][pM]
   __nv_bfloat16 *val[2] = {};      // lhs values [M][pK], rhs values [N][pK]
   CUtensorMap xk, xmn, va, vb;
+  float *part = nullptr;      // split tiles' sums and flags (AdjTcArgs), when a deal splits
+  uint32_t *flags = nullptr;
+  uint32_t nflags = 0;
+  AdjDeal deal[4];            // by the wanted gradients: bit 0 dB, bit 1 dA
 };
 
 void adj_plan_free(AdjPlan *p) {
   if (!p) return;
   if (p->ws) cudaFree(p->ws);
+  if (p->part) cudaFree(p->part);
+  if (p->flags) cudaFree(p->flags);
   delete p;
 }
 
 bool adjoint_tc_available() { return adj_encode_fn() != nullptr; }
 
 namespace {
-
-int build_plan(gbs_ctx *c) {
-  const uint64_t M = c->lhs.nrows, N = c->rhs.nrows, K = c->lhs.ncols;
-  const uint64_t pM = pitch64(M), pK = pitch64(K), term = N * pM;
-  AdjPlan *p = new AdjPlan();
-  // every array starts on a 128-byte boundary: the pitches are multiples of 64 values
-  const size_t bytes = (3 * term + (M + N) * pK) * sizeof(__nv_bfloat16);
-  if (dev_alloc((void **)&p->ws, bytes) != cudaSuccess) {
-    cudaGetLastError();
-    delete p;
-    return fail(GBS_ENOMEM, "gbs_adjoint: workspace allocation failed");
-  }
-  p->split = p->ws;
-  p->val[0] = p->ws + 3 * term;
-  p->val[1] = p->val[0] + M * pK;
-  // dB: rows n, contraction m (contiguous); the true M and N bound the boxes, past them reads are 0
-  const cuuint64_t dk[3] = {M, N, 3}, sk[2] = {pM * 2, term * 2};
-  const cuuint32_t bk[3] = {(cuuint32_t)kAdjKs, 128, 3};
-  // dA: rows m (contiguous, 64 at a time), contraction n
-  const cuuint64_t dmn[4] = {64, N, pM / 64, 3}, smn[3] = {pM * 2, 128, term * 2};
-  const cuuint32_t bmn[4] = {64, (cuuint32_t)kAdjKs, 2, 3};
-  if (!bf16_map(&p->xk, p->split, 3, dk, sk, bk, CU_TENSOR_MAP_SWIZZLE_128B) ||
-      !bf16_map(&p->xmn, p->split, 4, dmn, smn, bmn, CU_TENSOR_MAP_SWIZZLE_128B) ||
-      !values_map(&p->va, p->val[0], M, pK) || !values_map(&p->vb, p->val[1], N, pK)) {
-    adj_plan_free(p);
-    return fail(GBS_EUNSUPPORTED, "gbs_adjoint: tensor map encoding failed");
-  }
-  c->adj = p;
-  return GBS_OK;
-}
 
 // SM pairs the adjoint kernel can hold at once, cached per device.
 int adj_max_pairs() {
@@ -566,6 +647,117 @@ int adj_max_pairs() {
   return v;
 }
 
+// Deals nfirst tiles of cfirst stages round robin over the pairs, then nother
+// tiles of cother stages in whole rounds over the pairs with the least work so
+// far; the tiles left over, fewer than those pairs, are split in parts of at
+// least kMinPiece stages.  4096 x 2048 x 2048: 64 tiles of 64 stages and 128 of
+// 32 over 76 pairs; whole tiles only would end with 28 pairs a tile (26 us)
+// behind the rest, halves of those 28 end half a tile behind.  Few long tiles (a
+// large batch against a small layer) are split too, down to an even share of
+// all the work.  A part costs its sums' way through L2, about 3 us: kMinPiece
+// stages of 0.8 us keep it worth while.
+constexpr uint32_t kMinPiece = 6, kMaxPieces = 8;
+
+AdjDeal deal_tiles(uint32_t first, uint64_t nfirst, uint64_t cfirst, uint64_t nother, uint64_t cother,
+                   uint32_t pairs) {
+  AdjDeal d;
+  memset(&d, 0, sizeof(d));
+  d.first = first;
+  d.pairs = pairs;
+  d.pieces = d.fpieces = 1;
+  const uint64_t share = std::max<uint64_t>((nfirst * cfirst + nother * cother) / pairs, kMinPiece);
+  if (nfirst && 2 * nfirst <= pairs && cfirst >= 2 * share)
+    d.fpieces = (uint32_t)std::min<uint64_t>(std::min<uint64_t>(kMaxPieces, pairs / nfirst), cfirst / share);
+  const bool split = d.fpieces > 1;
+  d.a = (uint32_t)(split ? nfirst * d.fpieces : nfirst % pairs);
+  const uint64_t size[2] = {d.a, pairs - d.a};
+  uint64_t load[2] = {split ? cfirst / d.fpieces : (nfirst / pairs + 1) * cfirst,
+                      split ? 0 : nfirst / pairs * cfirst};
+  uint64_t s[2] = {0, 0}, takers = pairs;
+  while (nother) {
+    const bool all = !size[0] || !size[1] || load[0] == load[1];
+    const int g = load[0] < load[1] ? 0 : 1;
+    takers = all ? pairs : size[g];
+    d.p0 = all || g == 0 ? 0 : d.a;
+    if (nother < takers) break;
+    for (int i = 0; i < 2; i++)
+      if (all || i == g) {
+        s[i]++;
+        load[i] += cother;
+      }
+    nother -= takers;
+  }
+  d.sa = (uint32_t)s[0];
+  d.sb = (uint32_t)s[1];
+  d.rem = (uint32_t)nother;
+  if (nother)
+    d.pieces = (uint32_t)std::max<uint64_t>(
+        1, std::min<uint64_t>(std::min<uint64_t>(kMaxPieces, takers / nother), cother / kMinPiece));
+  AdjTile w;
+  for (d.grid = pairs; d.grid > 1 && !dealt_tile(d, (uint32_t)(split || nfirst < pairs ? nfirst : pairs),
+                                                 d.grid - 1, 0, w);)
+    d.grid--;
+  return d;
+}
+
+uint32_t adj_stages(uint64_t S) { return (uint32_t)((S + kAdjKs - 1) / kAdjKs); }
+uint32_t adj_tiles(uint64_t R, uint64_t K) { return (uint32_t)(((R + 255) / 256) * ((K + 255) / 256)); }
+
+int build_plan(gbs_ctx *c) {
+  const uint64_t M = c->lhs.nrows, N = c->rhs.nrows, K = c->lhs.ncols;
+  const uint64_t pM = pitch64(M), pK = pitch64(K), term = N * pM;
+  AdjPlan *p = new AdjPlan();
+  // every array starts on a 128-byte boundary: the pitches are multiples of 64 values
+  const size_t bytes = (3 * term + (M + N) * pK) * sizeof(__nv_bfloat16);
+  if (dev_alloc((void **)&p->ws, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    delete p;
+    return fail(GBS_ENOMEM, "gbs_adjoint: workspace allocation failed");
+  }
+  p->split = p->ws;
+  p->val[0] = p->ws + 3 * term;
+  p->val[1] = p->val[0] + M * pK;
+  // dB: rows n, contraction m (contiguous); the true M and N bound the boxes, past them reads are 0
+  const cuuint64_t dk[3] = {M, N, 3}, sk[2] = {pM * 2, term * 2};
+  const cuuint32_t bk[3] = {(cuuint32_t)kAdjKs, 128, 3};
+  // dA: rows m (contiguous, 64 at a time), contraction n
+  const cuuint64_t dmn[4] = {64, N, pM / 64, 3}, smn[3] = {pM * 2, 128, term * 2};
+  const cuuint32_t bmn[4] = {64, (cuuint32_t)kAdjKs, 2, 3};
+  if (!bf16_map(&p->xk, p->split, 3, dk, sk, bk, CU_TENSOR_MAP_SWIZZLE_128B) ||
+      !bf16_map(&p->xmn, p->split, 4, dmn, smn, bmn, CU_TENSOR_MAP_SWIZZLE_128B) ||
+      !values_map(&p->va, p->val[0], M, pK) || !values_map(&p->vb, p->val[1], N, pK)) {
+    adj_plan_free(p);
+    return fail(GBS_EUNSUPPORTED, "gbs_adjoint: tensor map encoding failed");
+  }
+  const int max_pairs = adj_max_pairs();
+  if (!max_pairs) {
+    adj_plan_free(p);
+    return fail(GBS_ECUDA, "gbs_adjoint: the SM-pair kernel does not fit this device");
+  }
+  uint32_t split_pairs = 0;
+  for (uint32_t want = 1; want < 4; want++) {
+    const uint32_t n[2] = {(want & 1) ? adj_tiles(N, K) : 0, (want & 2) ? adj_tiles(M, K) : 0};
+    const uint32_t cost[2] = {adj_stages(M), adj_stages(N)};
+    const uint32_t pairs = (uint32_t)std::min<uint64_t>(
+        (uint64_t)max_pairs, std::max<uint64_t>((uint64_t)n[0] + n[1], 1) * kMaxPieces);
+    // the gradient with the longer contraction first; a lone one is dealt as the other, which may split
+    const uint32_t first = !n[0] ? 0 : !n[1] ? 1 : cost[0] >= cost[1] ? 0 : 1;
+    p->deal[want] = deal_tiles(first, n[first], cost[first], n[1 - first], cost[1 - first], pairs);
+    if (p->deal[want].pieces > 1 || p->deal[want].fpieces > 1) split_pairs = std::max(split_pairs, pairs);
+  }
+  if (split_pairs) {
+    p->nflags = 2 * split_pairs * 2 * kAdjEpiWarps;
+    if (dev_alloc((void **)&p->part, (size_t)p->nflags * 4096 * sizeof(float)) != cudaSuccess ||
+        dev_alloc((void **)&p->flags, (size_t)p->nflags * sizeof(uint32_t)) != cudaSuccess) {
+      cudaGetLastError();
+      adj_plan_free(p);
+      return fail(GBS_ENOMEM, "gbs_adjoint: workspace allocation failed");
+    }
+  }
+  c->adj = p;
+  return GBS_OK;
+}
+
 AdjValues values_job(const Mat &op, __nv_bfloat16 *out, bool wanted) {
   AdjValues v;
   memset(&v, 0, sizeof(v));
@@ -579,40 +771,21 @@ AdjValues values_job(const Mat &op, __nv_bfloat16 *out, bool wanted) {
   v.nbits = (int)op.nbits;
   v.neg_msb = (op.issigned && !op.bipolar()) ? (int)op.nbits - 1 : -1;
   v.bipolar = op.bipolar() ? 1 : 0;
+  for (int code = 0; code < 16 && op.nbits <= 4; code++) {  // bf16 of small integers: the high half of the float
+    int x = op.bipolar() ? ((code & 1) ? 1 : -1) : 0;
+    for (int i = 0; i < v.nbits && !op.bipolar(); i++)
+      if ((code >> i) & 1) x += i == v.neg_msb ? -(1 << i) : 1 << i;
+    const float f = (float)x;
+    uint32_t bits;
+    memcpy(&bits, &f, 4);
+    v.lo[code >> 2] |= ((bits >> 16) & 0xFFu) << (8 * (code & 3));
+    v.hi[code >> 2] |= (bits >> 24) << (8 * (code & 3));
+  }
   v.blocks = wanted ? (uint32_t)(((uint64_t)v.rows * v.chunks + 255) / 256) : 0;
   return v;
 }
 
 }  // namespace
-
-// Deals nfirst tiles of cfirst stages round robin over P pairs, then nother
-// tiles of cother stages, each to the pairs with the least work so far: equal
-// finishing times to within one tile.
-static AdjDeal deal_tiles(uint32_t first, uint64_t nfirst, uint64_t cfirst, uint64_t nother, uint64_t cother,
-                          uint32_t pairs) {
-  AdjDeal d;
-  memset(&d, 0, sizeof(d));
-  d.first = first;
-  d.pairs = pairs;
-  d.a = (uint32_t)(nfirst % pairs);
-  const uint64_t size[2] = {d.a, pairs - d.a};
-  uint64_t load[2] = {(nfirst / pairs + 1) * cfirst, nfirst / pairs * cfirst}, s[2] = {0, 0};
-  while (nother) {
-    const int g = size[0] && load[0] < load[1] ? 0 : 1;
-    const uint64_t take = std::min(nother, size[g]);
-    if (take == size[g]) {
-      s[g]++;
-      load[g] += cother;
-    } else {
-      d.extra = (uint32_t)take;
-      d.extra_kind = (uint32_t)g;
-    }
-    nother -= take;
-  }
-  d.sa = (uint32_t)s[0];
-  d.sb = (uint32_t)s[1];
-  return d;
-}
 
 // dA = dC . B and dB = dC^T . A on the tensor cores (either output may be null).
 int adjoint_tc(gbs_ctx *c, const float *dC, float *dA, float *dB, cudaStream_t s) {
@@ -644,6 +817,8 @@ int adjoint_tc(gbs_ctx *c, const float *dC, float *dA, float *dB, cudaStream_t s
   pr.blocks = (uint32_t)((N * pr.chunks + 255) / 256);
   pr.v[0] = values_job(c->lhs, p.val[0], want[0] && !c->vt_valid[0]);
   pr.v[1] = values_job(c->rhs, p.val[1], want[1] && !c->vt_valid[1]);
+  pr.flags = p.flags;
+  pr.nflags = p.nflags;
   adjoint_prepare<<<pr.blocks + pr.v[0].blocks + pr.v[1].blocks, 256, 0, s>>>(pr);
   count_launch();
   cudaError_t e = cudaGetLastError();
@@ -661,17 +836,15 @@ int adjoint_tc(gbs_ctx *c, const float *dC, float *dA, float *dB, cudaStream_t s
     const uint64_t R = g ? M : N, S = g ? N : M;
     o.out = g ? dA : dB;
     o.R = (uint32_t)R;
-    o.tiles = want[g] ? (uint32_t)((R + 255) / 256) * a.ctiles : 0;
-    o.nstages = (uint32_t)((S + kAdjKs - 1) / kAdjKs);
+    o.tiles = want[g] ? adj_tiles(R, K) : 0;
+    o.nstages = adj_stages(S);
     // kind::f16: D fp32, A and B bf16, M = 256, N = 256; B MN-major, A MN-major for dA
     o.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)g << 15) | (1u << 16) | ((256u >> 3) << 17) |
               ((256u >> 4) << 24);
   }
-  const uint64_t tiles = (uint64_t)a.o[0].tiles + a.o[1].tiles;
-  const uint32_t pairs = (uint32_t)std::min<uint64_t>(tiles, (uint64_t)adj_max_pairs());
-  if (!pairs) return fail(GBS_ECUDA, "gbs_adjoint: the SM-pair kernel does not fit this device");
-  const uint32_t first = a.o[0].nstages >= a.o[1].nstages ? 0 : 1;  // the longer contraction
-  a.deal = deal_tiles(first, a.o[first].tiles, a.o[first].nstages, a.o[1 - first].tiles, a.o[1 - first].nstages, pairs);
+  a.deal = p.deal[(dB ? 1 : 0) | (dA ? 2 : 0)];
+  a.part = p.part;
+  a.flags = p.flags;
   uint32_t *err = tc_error_ptr();
   if (!err) return fail(GBS_ECUDA, "gbs_adjoint: no error word");
   cudaLaunchConfig_t cfg = {};
@@ -680,7 +853,7 @@ int adjoint_tc(gbs_ctx *c, const float *dC, float *dA, float *dB, cudaStream_t s
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3(2 * pairs);
+  cfg.gridDim = dim3(2 * a.deal.grid);
   cfg.blockDim = dim3(kAdjThreads);
   cfg.dynamicSmemBytes = adj_smem_bytes();
   cfg.stream = s;

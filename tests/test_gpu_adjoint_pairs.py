@@ -1,6 +1,7 @@
 """The persistent adjoint kernel: tiles of both gradients dealt over the SM pairs (more tiles than pairs, one
-gradient only, either contraction the longer), row and column remainders, and outputs that do not start on 32 bytes.
-dC holds small integers, so every sum is exact in fp32 and the gradients must equal the int64 products."""
+gradient only, either contraction the longer, long tiles and left-over ones split over pairs), row and column
+remainders, and outputs that do not start on 32 bytes.  dC holds small integers, so every sum is exact in fp32 and
+the gradients must equal the int64 products."""
 import ctypes as C
 
 import numpy as np
@@ -20,7 +21,8 @@ def lib(gbs_lib):
 
 
 @pytest.mark.parametrize("shape", [(1, 1, 1), (33, 8, 31), (256, 256, 256), (257, 264, 65), (64, 1000, 700),
-                                   (2600, 1300, 2100), (900, 2300, 3100), (5000, 777, 40)])
+                                   (2600, 1300, 2100), (900, 2300, 3100), (5000, 777, 40),
+                                   (6000, 300, 200), (200, 520, 9000), (4096, 2048, 2048)])
 @pytest.mark.parametrize("want", ["both", "dA", "dB"])
 def test_exact_gradients(shape, want):
     import torch
