@@ -205,6 +205,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kAdjStages + 3);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   const uint32_t pid = blockIdx.x >> 1, nfirst = a.o[a.deal.first].tiles;
+  griddep_launch_dependents();
 
   if (tid == 0) {
     for (int i = 0; i < kAdjStages; i++) {
@@ -226,6 +227,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = *tmem_slot;  // columns [0, 256): hi accumulator; [256, 512): mid + lo
+  griddep_wait();  // operands and gradients belong to earlier kernels until here
 
   if (warp == 0) {
     if (lane == 0 && peer == 0) {
@@ -455,6 +457,8 @@ __device__ __forceinline__ void piece_of(uint64_t idx, uint32_t per, uint32_t &r
 // operands' planes into bf16 values (16 a thread), in one launch: block ranges.
 // HBM-bound: 34 MB in, 50 + 25 MB out at 4096 x 2048 x 2048.
 __global__ void __launch_bounds__(256) adjoint_prepare(const __grid_constant__ AdjPrepare a) {
+  griddep_launch_dependents();
+  griddep_wait();  // dC, the planes and the workspace belong to earlier kernels until here
   uint32_t b = blockIdx.x;
   if (b == 0)
     for (uint32_t i = threadIdx.x; i < a.nflags; i += 256) a.flags[i] = 0u;
@@ -819,9 +823,8 @@ int adjoint_tc(gbs_ctx *c, const float *dC, float *dA, float *dB, cudaStream_t s
   pr.v[1] = values_job(c->rhs, p.val[1], want[1] && !c->vt_valid[1]);
   pr.flags = p.flags;
   pr.nflags = p.nflags;
-  adjoint_prepare<<<pr.blocks + pr.v[0].blocks + pr.v[1].blocks, 256, 0, s>>>(pr);
+  cudaError_t e = launch_pdl(adjoint_prepare, pr.blocks + pr.v[0].blocks + pr.v[1].blocks, 256, 0, s, pr);
   count_launch();
-  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "gbs_adjoint: split kernel");
   for (int side = 0; side < 2; side++)
     if (want[side]) c->vt_valid[side] = true;
@@ -848,17 +851,19 @@ int adjoint_tc(gbs_ctx *c, const float *dC, float *dA, float *dB, cudaStream_t s
   uint32_t *err = tc_error_ptr();
   if (!err) return fail(GBS_ECUDA, "gbs_adjoint: no error word");
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.gridDim = dim3(2 * a.deal.grid);
   cfg.blockDim = dim3(kAdjThreads);
   cfg.dynamicSmemBytes = adj_smem_bytes();
   cfg.stream = s;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = pdl_for(s) ? 2 : 1;
   e = cudaLaunchKernelEx(&cfg, adjoint_tc_kernel, p.xk, p.xmn, p.va, p.vb, a, err);
   count_launch();
   return e == cudaSuccess ? GBS_OK : cuda_fail(e, "gbs_adjoint: GEMM kernel");

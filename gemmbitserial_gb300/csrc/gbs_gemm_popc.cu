@@ -24,6 +24,7 @@
 //  * gemm_popc_skinny: one warp per output element, lanes stride over the K
 //    words; for matrix-vector and other small-output shapes.
 #include "gbs_internal.h"
+#include "gbs_tc_common.cuh"
 
 namespace gbs {
 namespace {
@@ -301,12 +302,16 @@ __device__ __forceinline__ void popc_rows_dispatch(const TileArgs &g, uint64_t n
 template <bool XOR>
 __global__ void __launch_bounds__(NT, 2) gemm_popc_rows(TileArgs g) {
   extern __shared__ __align__(16) uint64_t smem[];
+  griddep_launch_dependents();
+  griddep_wait();  // operands and result belong to earlier kernels until here
   popc_rows_dispatch<kRowsKC, XOR>(g, (uint64_t)blockIdx.x * rows_tile_n(g.M), smem);
 }
 
 template <int BM, int BN, int KC, bool XOR>
 __global__ void __launch_bounds__(NT, 2) gemm_popc_tiled(TileArgs g) {
   extern __shared__ __align__(16) uint64_t smem[];
+  griddep_launch_dependents();
+  griddep_wait();  // operands and result belong to earlier kernels until here
   popc_tile<BM, BN, KC, XOR>(g, (uint64_t)blockIdx.x * BM, (uint64_t)blockIdx.y * BN, smem);
 }
 
@@ -435,6 +440,8 @@ __global__ void __launch_bounds__(NT, 2) gemm_popc_grouped(const GroupProblem *_
 
 // One warp per output (m, n); lanes stride over the K words.
 __global__ void __launch_bounds__(256) gemm_popc_skinny(GemmShape g, Epilogue e) {
+  griddep_launch_dependents();
+  griddep_wait();  // operands and result belong to earlier kernels until here
   const uint64_t o = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (o >= g.M * g.N) return;  // warp-uniform
@@ -456,9 +463,9 @@ cudaError_t run_tiled(const TileArgs &t, cudaStream_t s) {
   cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess) return err;
   dim3 grid((unsigned)((t.M + BM - 1) / BM), (unsigned)((t.N + BN - 1) / BN));
-  kern<<<grid, NT, smem, s>>>(t);
+  err = launch_pdl(kern, grid, NT, smem, s, t);
   count_launch();
-  return cudaGetLastError();
+  return err != cudaSuccess ? err : cudaGetLastError();
 }
 
 template <int BM, int BN, bool XOR>
@@ -483,9 +490,9 @@ cudaError_t run_rows(const TileArgs &t, cudaStream_t s) {
   cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess) return err;
   const uint64_t bnr = rows_tile_n(t.M);
-  kern<<<(unsigned)((t.N + bnr - 1) / bnr), NT, smem, s>>>(t);
+  err = launch_pdl(kern, (unsigned)((t.N + bnr - 1) / bnr), NT, smem, s, t);
   count_launch();
-  return cudaGetLastError();
+  return err != cudaSuccess ? err : cudaGetLastError();
 }
 
 }  // namespace
@@ -511,9 +518,9 @@ cudaError_t launch_gemm_popc(const GemmShape &g, const Epilogue &e, cudaStream_t
   const bool skinny = g.tile_cls < 0 && popc_skinny(g.M, g.N);
   if (skinny) {
     const uint64_t threads = g.M * g.N * 32;
-    gemm_popc_skinny<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(g, e);
+    const cudaError_t err = launch_pdl(gemm_popc_skinny, (unsigned)((threads + 255) / 256), 256, 0, s, g, e);
     count_launch();
-    return cudaGetLastError();
+    return err != cudaSuccess ? err : cudaGetLastError();
   }
   TileArgs t;
   t.A = g.A; t.B = g.B; t.C = g.C; t.ra = e.ra; t.rb = e.rb;

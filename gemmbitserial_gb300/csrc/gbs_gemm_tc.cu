@@ -1564,11 +1564,14 @@ bool pdl_enabled() {
   return on;
 }
 
-// Programmatic stream serialization for a launch on `s`: on unless GBS_PDL=0,
-// the stream is the legacy default stream (which synchronises with others) or
-// the stream is being captured (graph launches keep plain edges).
+// Programmatic stream serialization for a launch on `s`: on unless GBS_PDL=0
+// or the stream is being captured (graph launches keep plain edges).  The
+// legacy default stream cannot be captured.  (It synchronises with other
+// streams; those dependencies stay full ones, only the one on the kernel before in the
+// same stream becomes programmatic.)
 bool pdl_for(cudaStream_t s) {
-  if (!pdl_enabled() || s == nullptr) return false;
+  if (!pdl_enabled()) return false;
+  if (s == nullptr || s == cudaStreamLegacy) return true;
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
     cudaGetLastError();

@@ -72,6 +72,7 @@ __global__ void __launch_bounds__(kTgThreads, 1)
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kTgStages + 5);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   const uint32_t G = gridDim.x, b = blockIdx.x;
+  griddep_launch_dependents();
 
   if (tid == 0) {
     for (int i = 0; i < kTgStages; i++) {
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(kTgThreads, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = *tmem_slot;
+  griddep_wait();  // operands and results belong to earlier kernels until here
 
   if (warp == 0) {
     if (lane == 0) {
@@ -312,6 +314,8 @@ __device__ __forceinline__ void expand_thread(const ExpandJob &j, uint64_t local
 }
 
 __global__ void __launch_bounds__(256) expand_one_kernel(const ExpandJob job) {
+  griddep_launch_dependents();
+  griddep_wait();
   expand_thread(job, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -375,9 +379,9 @@ ExpandJob make_nibble_job(const Mat &m, uint8_t *nibbles) {
 cudaError_t launch_expand(const ExpandJob &job, cudaStream_t s) {
   const uint64_t threads = (uint64_t)job.nrows * job.chunks;
   if (threads == 0) return cudaSuccess;
-  expand_one_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(job);
+  const cudaError_t e = launch_pdl(expand_one_kernel, (unsigned)((threads + 255) / 256), 256, 0, s, job);
   count_launch();
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 // Digit matrix [drows][dcols] of one side, allocated zeroed on first use
@@ -613,11 +617,11 @@ cudaError_t tcg_expand(TcgPlan &plan, cudaStream_t s) {
 cudaError_t tcg_gemm(const TcgPlan &plan, uint32_t *err, cudaStream_t s, int32_t *out0) {
   if (!plan.ntiles) return cudaSuccess;
   if (plan.nibbles) return tcgn_gemm(plan, err, s, out0);
-  gemm_tcg_kernel<<<plan.grid, kTgThreads, tcg_smem_bytes(), s>>>(
-      plan.d_probs, reinterpret_cast<const CUtensorMap *>(plan.d_maps), plan.d_tiles, plan.ntiles, plan.nprob, err,
-      out0);
+  const cudaError_t e = launch_pdl(gemm_tcg_kernel, plan.grid, kTgThreads, tcg_smem_bytes(), s, plan.d_probs,
+                                   reinterpret_cast<const CUtensorMap *>(plan.d_maps), plan.d_tiles, plan.ntiles,
+                                   plan.nprob, err, out0);
   count_launch();
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 }  // namespace gbs

@@ -319,6 +319,24 @@ inline bool pair_split_variant(int v) {
 }
 bool pdl_enabled();                          // programmatic dependent launch of the tensor-core kernels (GBS_PDL)
 bool pdl_for(cudaStream_t s);                // ... of a launch on this stream
+
+// kern<<<grid, block, smem, s>>>(args...) with programmatic stream
+// serialization where pdl_for allows it: for kernels that call griddep_wait()
+// before their first global access.
+template <typename... P, typename... A>
+cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_for(s) ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
 uint32_t tc_error_word();
 int tc_peaks(double *f8, double *bf16);
 

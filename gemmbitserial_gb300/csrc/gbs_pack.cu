@@ -21,6 +21,7 @@
 #include <type_traits>
 
 #include "gbs_internal.h"
+#include "gbs_tc_common.cuh"
 
 namespace gbs {
 namespace {
@@ -200,6 +201,8 @@ __device__ __forceinline__ void codes_of_bytes(int dtype, int bipolar, uint32_t 
 template <int VEC>
 __global__ void __launch_bounds__(256) pack_bytes(const __grid_constant__ PackJob J, uint64_t row0, uint64_t rend,
                                                   uint64_t units) {
+  griddep_launch_dependents();
+  griddep_wait();  // source, planes and digits belong to earlier kernels until here
   const uint64_t u = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (u >= units) return;  // warp-uniform
   const uint32_t lane = threadIdx.x & 31;
@@ -553,6 +556,8 @@ __global__ void __launch_bounds__(256) pack_staged(const __grid_constant__ PackJ
                                                    int nthres, uint64_t row0, uint64_t rend, uint64_t units) {
   __shared__ __align__(16) uint32_t st[8][256];
   __shared__ typename std::conditional<QUANT, QuantStage<T>, char>::type qs;
+  griddep_launch_dependents();
+  griddep_wait();  // source, planes and digits belong to earlier kernels until here
   const uint64_t u = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (u >= units) return;  // warp-uniform; no block-wide barrier follows
   pack_staged_unit<T, QUANT, ALIGNED>(J, thr, nthres, row0, rend, u, st[threadIdx.x >> 5],
@@ -578,6 +583,8 @@ template <typename T, bool QUANT, bool ALIGNED>
 __global__ void __launch_bounds__(kCmThreads) pack_colmajor(const __grid_constant__ PackJob J,
                                                             const T *__restrict__ thr, int nthres) {
   __shared__ uint32_t st[kCmWords];
+  griddep_launch_dependents();
+  griddep_wait();  // source, planes and digits belong to earlier kernels until here
   // neighbouring blocks take neighbouring rows of the same columns: their reads are contiguous
   const uint32_t rblocks = (uint32_t)((J.nrows_a + kCmRows - 1) / kCmRows);
   const uint64_t r0 = (uint64_t)(blockIdx.x % rblocks) * kCmRows, c0 = (uint64_t)(blockIdx.x / rblocks) * kCmCols;
@@ -653,6 +660,8 @@ constexpr int kDepth = 2;
 __global__ void __launch_bounds__(256, 4) pack_grouped(const PackJob *__restrict__ jobs, int njobs, uint64_t runs,
                                                        uint32_t run) {
   __shared__ PackJob sj[8];  // each warp's job: its fields stay out of the registers
+  griddep_launch_dependents();
+  griddep_wait();  // source, planes and digits belong to earlier kernels until here
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   const int lane = threadIdx.x & 31;
   PackJob &J = sj[threadIdx.x >> 5];
@@ -702,6 +711,8 @@ __device__ __forceinline__ void pack_staged_run(const PackJob &J, uint64_t u0, u
 __global__ void __launch_bounds__(256) pack_grouped_staged(const PackJob *__restrict__ jobs, int njobs,
                                                            uint64_t runs, uint32_t run) {
   __shared__ __align__(16) uint32_t st[8][256];
+  griddep_launch_dependents();
+  griddep_wait();  // source, planes and digits belong to earlier kernels until here
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   const int lane = threadIdx.x & 31;
   uint32_t *my = st[threadIdx.x >> 5];
@@ -741,6 +752,8 @@ __device__ __forceinline__ int32_t row_sum(const uint64_t *__restrict__ planes, 
 __global__ void __launch_bounds__(256) rowsum_kernel(const uint64_t *__restrict__ planes, int nbits, int issigned,
                                                      uint64_t nrows, uint64_t ncols, uint64_t nrows_a,
                                                      uint64_t wpr, int32_t *__restrict__ dst) {
+  griddep_launch_dependents();
+  griddep_wait();  // source, planes and digits belong to earlier kernels until here
   const uint64_t r = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (r >= nrows) return;
@@ -750,6 +763,8 @@ __global__ void __launch_bounds__(256) rowsum_kernel(const uint64_t *__restrict_
 
 // Grouped row sums: one warp per row over every job (warp0 counts rows).
 __global__ void __launch_bounds__(256) rowsum_grouped(const PackJob *__restrict__ jobs, int njobs, uint64_t total) {
+  griddep_launch_dependents();
+  griddep_wait();  // source, planes and digits belong to earlier kernels until here
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   const int lane = threadIdx.x & 31;
   for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < total; w += nw) {
@@ -863,29 +878,29 @@ void with_source(int dtype, bool aligned, F f) {
 cudaError_t run_staged(const PackJob &j, const void *thr, int nthres, bool quant, bool aligned, uint64_t r0,
                        uint64_t r1, cudaStream_t s) {
   const uint64_t units = ((r1 - r0) * j.cpr + 31) / 32;
+  cudaError_t e = cudaSuccess;
   with_source(j.dtype, aligned, [&](auto t, auto al) {
     using T = decltype(t);
     constexpr bool A = decltype(al)::value;
-    if (quant)
-      pack_staged<T, true, A><<<blocks_for(units * 32, 256), 256, 0, s>>>(j, (const T *)thr, nthres, r0, r1, units);
-    else
-      pack_staged<T, false, A><<<blocks_for(units * 32, 256), 256, 0, s>>>(j, nullptr, 0, r0, r1, units);
+    e = launch_pdl(quant ? pack_staged<T, true, A> : pack_staged<T, false, A>, blocks_for(units * 32, 256), 256, 0, s, j,
+                   (const T *)thr, nthres, r0, r1, units);
   });
   count_launch();
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t run_colmajor(const PackJob &j, const void *thr, int nthres, bool quant, cudaStream_t s) {
   const uint64_t blocks = ((j.nrows_a + kCmRows - 1) / kCmRows) * ((j.wpr * 64 + kCmCols - 1) / kCmCols);
   if (blocks > 0x7FFFFFFFull) return cudaErrorInvalidConfiguration;
+  cudaError_t e = cudaSuccess;
   with_source(j.dtype, aligned4(j.src, j.dtype, j.nrows), [&](auto t, auto al) {
     using T = decltype(t);
     constexpr bool A = decltype(al)::value;
-    if (quant) pack_colmajor<T, true, A><<<(unsigned)blocks, kCmThreads, 0, s>>>(j, (const T *)thr, nthres);
-    else pack_colmajor<T, false, A><<<(unsigned)blocks, kCmThreads, 0, s>>>(j, nullptr, 0);
+    e = launch_pdl(quant ? pack_colmajor<T, true, A> : pack_colmajor<T, false, A>, (unsigned)blocks, kCmThreads, 0, s, j,
+                   (const T *)thr, nthres);
   });
   count_launch();
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 }  // namespace
@@ -896,10 +911,10 @@ cudaError_t launch_pack_rows(const Mat &m, const void *src, int dtype, uint64_t 
   PackJob j = make_pack_job(m, src, dtype, digits, nullptr);
   if (!pack_job_direct(j, m)) return run_staged(j, nullptr, 0, false, j.vec != 0, r0, r1, s);
   const uint64_t units = ((r1 - r0) * j.cpr + 31) / 32;
-  if (j.vec == 2) pack_bytes<2><<<blocks_for(units * 32, 256), 256, 0, s>>>(j, r0, r1, units);
-  else pack_bytes<1><<<blocks_for(units * 32, 256), 256, 0, s>>>(j, r0, r1, units);
+  const cudaError_t e =
+      launch_pdl(j.vec == 2 ? pack_bytes<2> : pack_bytes<1>, blocks_for(units * 32, 256), 256, 0, s, j, r0, r1, units);
   count_launch();
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_pack_quantize(const Mat &m, const void *src, const void *thr, int nthres, int dtype,
@@ -921,26 +936,27 @@ cudaError_t launch_pack_grouped(const PackJob *jobs, int njobs, uint64_t runs, u
                                 cudaStream_t s) {
   if (runs == 0 || njobs == 0) return cudaSuccess;
   const uint64_t blocks = std::min<uint64_t>((runs + 7) / 8, 152 * 64);
-  if (direct) pack_grouped<<<(unsigned)blocks, 256, 0, s>>>(jobs, njobs, runs, run);
-  else pack_grouped_staged<<<(unsigned)blocks, 256, 0, s>>>(jobs, njobs, runs, run);
+  const cudaError_t e =
+      launch_pdl(direct ? pack_grouped : pack_grouped_staged, (unsigned)blocks, 256, 0, s, jobs, njobs, runs, run);
   count_launch();
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_rowsum_grouped(const PackJob *jobs, int njobs, uint64_t total_warps, cudaStream_t s) {
   if (total_warps == 0 || njobs == 0) return cudaSuccess;
   const uint64_t blocks = (total_warps + 7) / 8;
-  rowsum_grouped<<<(unsigned)(blocks < 152 * 64 ? blocks : 152 * 64), 256, 0, s>>>(jobs, njobs, total_warps);
+  const cudaError_t e =
+      launch_pdl(rowsum_grouped, (unsigned)(blocks < 152 * 64 ? blocks : 152 * 64), 256, 0, s, jobs, njobs, total_warps);
   count_launch();
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_rowsum(const Mat &m, int32_t *dst, cudaStream_t s) {
   if (m.nrows == 0) return cudaSuccess;
-  rowsum_kernel<<<blocks_for(m.nrows * 32, 256), 256, 0, s>>>(m.planes, (int)m.nbits, m.issigned, m.nrows,
-                                                              m.ncols, m.nrows_a, m.wpr(), dst);
+  const cudaError_t e = launch_pdl(rowsum_kernel, blocks_for(m.nrows * 32, 256), 256, 0, s, m.planes, (int)m.nbits,
+                                   m.issigned, m.nrows, m.ncols, m.nrows_a, m.wpr(), dst);
   count_launch();
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_export(const Mat &m, int32_t *dst, cudaStream_t s) {

@@ -85,6 +85,8 @@ __global__ void __launch_bounds__(256) combine_kernel(int32_t *__restrict__ out,
                                                       const int32_t *__restrict__ in1, const int32_t *__restrict__ in2,
                                                       const int32_t *__restrict__ in3, int nin, uint32_t sh1,
                                                       uint32_t sh2, uint32_t sh3, uint64_t n) {
+  griddep_launch_dependents();
+  griddep_wait();
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; q < (n + 3) / 4; q += stride) {
     const uint64_t i0 = 4 * q;
@@ -343,6 +345,7 @@ cudaError_t alloc_parts(const gbs_ctx *c, const WidePlan &p, uint8_t *(&digits)[
       if (digits[side][k]) continue;
       cudaError_t e = dev_alloc((void **)&digits[side][k], bytes);
       if (e == cudaSuccess) e = cudaMemset(digits[side][k], 0, bytes);
+      if (e == cudaSuccess) e = cudaDeviceSynchronize();  // kernels on any stream may write it right after
       if (e != cudaSuccess) {
         cudaGetLastError();
         return cudaErrorMemoryAllocation;
@@ -458,10 +461,10 @@ cudaError_t launch_combine(gbs_ctx *c, const int32_t *const (&parts)[4], int n, 
   const uint64_t total = c->lhs.nrows * c->rhs.nrows;
   const uint64_t threads = (total + 3) / 4;
   const unsigned blocks = (unsigned)std::min<uint64_t>((threads + 255) / 256, 152 * 32);
-  combine_kernel<<<blocks, 256, 0, s>>>(result_ptr(c), parts[0], parts[1], parts[2], parts[3], n, shift[1], shift[2],
-                                        shift[3], total);
+  const cudaError_t e = launch_pdl(combine_kernel, blocks, 256, 0, s, result_ptr(c), parts[0], parts[1], parts[2],
+                                   parts[3], n, shift[1], shift[2], shift[3], total);
   count_launch();
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 }  // namespace
