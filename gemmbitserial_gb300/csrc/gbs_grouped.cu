@@ -23,6 +23,15 @@
 
 #include "gbs_internal.h"
 
+// Pack jobs of a grouped import on the device: those of the direct kernel, then those of the staged one.
+struct PackTable {
+  gbs::PackJob *jobs = nullptr;
+  size_t capacity = 0;
+  int n[2] = {0, 0};
+  uint64_t runs[2] = {0, 0};
+  uint32_t run[2] = {1, 1};  // units per run
+};
+
 struct gbs_group {
   int device = 0;
   std::vector<gbs_ctx *> ctxs;
@@ -33,15 +42,13 @@ struct gbs_group {
   gbs::PackJob *d_rs_jobs = nullptr;
   int nrs = 0;
   uint64_t rs_warps = 0;
-  // pack jobs of the grouped import: those of the direct kernel, then those of the staged one
-  gbs::PackJob *d_pack_jobs = nullptr;
-  int npack[2] = {0, 0};
-  uint64_t pack_runs[2] = {0, 0};
-  uint32_t pack_run[2] = {1, 1};  // units per run
+  PackTable imports, captured;  // of gbs_group_import, and of the captured graph (which keeps reading it)
+  cudaEvent_t packed = nullptr;  // the last import's pack: its table may be written again
   size_t smem = 0;
   int grid = 0;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
+  bool graph_packs = false;  // the captured graph imports
   gbs::TcgPlan tc;  // problems on the tensor-core kernel
   std::vector<char> is_tc;  // per problem: on the tensor-core kernel
   // with both kernel types, the tensor-core kernel runs on a stream forked
@@ -78,7 +85,9 @@ void free_group(gbs_group *g) {
   if (g->d_tiles) cudaFree(g->d_tiles);
   if (g->d_scratch) cudaFree(g->d_scratch);
   if (g->d_rs_jobs) cudaFree(g->d_rs_jobs);
-  if (g->d_pack_jobs) cudaFree(g->d_pack_jobs);
+  if (g->imports.jobs) cudaFree(g->imports.jobs);
+  if (g->captured.jobs) cudaFree(g->captured.jobs);
+  if (g->packed) cudaEventDestroy(g->packed);
   delete g;
 }
 
@@ -90,8 +99,13 @@ cudaError_t upload(T **dst, const std::vector<T> &v) {
   return cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
 }
 
-// Builds the pack-job table for (lhs_srcs[p], rhs_srcs[p]) of every problem.
-int build_pack_jobs(gbs_group *g, const void *const *lhs, const void *const *rhs, const int *dtypes) {
+// Builds the pack-job table for (lhs_srcs[p], rhs_srcs[p]) of every problem and
+// copies it to the device in the order of stream s: after the last pack that
+// read it, before the next.  (Allocating and copying it anew on each import
+// freed the old one, which waited for the whole device: 25 us of a CaffeNet
+// import.)
+int build_pack_jobs(gbs_group *g, PackTable &tab, const void *const *lhs, const void *const *rhs, const int *dtypes,
+                    cudaStream_t s) {
   std::vector<PackJob> jobs[2];  // direct, staged
   uint64_t units[2] = {0, 0};
   size_t ti = 0;  // index among the tensor-core problems
@@ -126,26 +140,36 @@ int build_pack_jobs(gbs_group *g, const void *const *lhs, const void *const *rhs
       j.warp0 = runs;
       runs += (pack_job_units(j) + run - 1) / run;
     }
-    g->npack[k] = (int)jobs[k].size();
-    g->pack_runs[k] = runs;
-    g->pack_run[k] = run;
+    tab.n[k] = (int)jobs[k].size();
+    tab.runs[k] = runs;
+    tab.run[k] = run;
   }
   jobs[0].insert(jobs[0].end(), jobs[1].begin(), jobs[1].end());
-  if (g->d_pack_jobs) cudaFree(g->d_pack_jobs);
-  g->d_pack_jobs = nullptr;
-  if (upload(&g->d_pack_jobs, jobs[0]) != cudaSuccess) {
+  const size_t bytes = jobs[0].size() * sizeof(PackJob);
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(s, &st);
+  if (e == cudaSuccess && st != cudaStreamCaptureStatusNone) e = cudaErrorStreamCaptureUnsupported;
+  if (e == cudaSuccess && tab.capacity < bytes) {
+    if (tab.jobs) cudaFree(tab.jobs);  // waits for the device: nothing reads the old table any more
+    tab.jobs = nullptr;
+    tab.capacity = 0;
+    e = dev_alloc((void **)&tab.jobs, bytes);
+    if (e == cudaSuccess) tab.capacity = bytes;
+  } else if (e == cudaSuccess) {
+    e = cudaStreamWaitEvent(s, g->packed, 0);
+  }
+  if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(tab.jobs, jobs[0].data(), bytes, cudaMemcpyHostToDevice, s);
+  if (e != cudaSuccess) {
     cudaGetLastError();
-    g->npack[0] = g->npack[1] = 0;
+    tab.n[0] = tab.n[1] = 0;
     return fail(GBS_ENOMEM, "gbs_group: pack table upload failed");
   }
   return GBS_OK;
 }
 
-cudaError_t enqueue_pack(const gbs_group *g, cudaStream_t s) {
-  cudaError_t e = launch_pack_grouped(g->d_pack_jobs, g->npack[0], g->pack_runs[0], g->pack_run[0], true, s);
-  if (e == cudaSuccess)
-    e = launch_pack_grouped(g->d_pack_jobs + g->npack[0], g->npack[1], g->pack_runs[1], g->pack_run[1],
-                            false, s);
+cudaError_t enqueue_pack(const PackTable &tab, cudaStream_t s) {
+  cudaError_t e = launch_pack_grouped(tab.jobs, tab.n[0], tab.runs[0], tab.run[0], true, s);
+  if (e == cudaSuccess) e = launch_pack_grouped(tab.jobs + tab.n[0], tab.n[1], tab.runs[1], tab.run[1], false, s);
   return e;
 }
 
@@ -347,6 +371,7 @@ int gbs_group_create(gbs_ctx *const *ctxs, int count, gbs_group **out) {
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&g->side, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&g->fork, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&g->join, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&g->packed, cudaEventDisableTiming);
   if (e != cudaSuccess) {
     cudaGetLastError();
     free_group(g);
@@ -374,9 +399,10 @@ int gbs_group_free(gbs_group *g) {
 int gbs_group_import(gbs_group *g, const void *const *lhs_srcs, const void *const *rhs_srcs, const int *dtypes,
                      void *stream) {
   if (!g || !lhs_srcs || !rhs_srcs) return fail(GBS_EINVAL, "gbs_group_import: NULL argument");
-  int rc = build_pack_jobs(g, lhs_srcs, rhs_srcs, dtypes);
+  int rc = build_pack_jobs(g, g->imports, lhs_srcs, rhs_srcs, dtypes, (cudaStream_t)stream);
   if (rc != GBS_OK) return rc;
-  cudaError_t e = enqueue_pack(g, (cudaStream_t)stream);
+  cudaError_t e = enqueue_pack(g->imports, (cudaStream_t)stream);
+  if (e == cudaSuccess) e = cudaEventRecord(g->packed, (cudaStream_t)stream);
   if (e != cudaSuccess) return cuda_fail(e, "gbs_group_import: pack kernel");
   for (gbs_ctx *c : g->ctxs) {
     c->lhs.imported = c->rhs.imported = true;
@@ -405,8 +431,13 @@ int gbs_group_capture(gbs_group *g, const void *const *lhs_srcs, const void *con
     return fail(GBS_EINVAL, "gbs_group_capture: capture needs a created stream, not the legacy default stream");
   const bool with_pack = lhs_srcs && rhs_srcs;
   if (with_pack) {
-    int rc = build_pack_jobs(g, lhs_srcs, rhs_srcs, dtypes);
+    // a graph captured before may still run and read its table; the new table is there before any replay
+    cudaError_t se = g->captured.jobs ? cudaDeviceSynchronize() : cudaSuccess;
+    if (se != cudaSuccess) return cuda_fail(se, "gbs_group_capture: device sync");
+    int rc = build_pack_jobs(g, g->captured, lhs_srcs, rhs_srcs, dtypes, (cudaStream_t)stream);
     if (rc != GBS_OK) return rc;
+    se = cudaStreamSynchronize((cudaStream_t)stream);
+    if (se != cudaSuccess) return cuda_fail(se, "gbs_group_capture: pack table upload");
   } else {
     for (gbs_ctx *c : g->ctxs)
       if (!c->lhs.imported || !c->rhs.imported)
@@ -424,15 +455,16 @@ int gbs_group_capture(gbs_group *g, const void *const *lhs_srcs, const void *con
   cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return cuda_fail(e, "gbs_group_capture: begin capture");
   cudaError_t ke = cudaSuccess;
-  if (with_pack) ke = enqueue_pack(g, s);
+  if (with_pack) ke = enqueue_pack(g->captured, s);
   if (ke == cudaSuccess) ke = enqueue_gemm(g, s);
   e = cudaStreamEndCapture(s, &g->graph);
   if (ke != cudaSuccess) return cuda_fail(ke, "gbs_group_capture: enqueue");
   if (e != cudaSuccess) return cuda_fail(e, "gbs_group_capture: end capture");
   e = cudaGraphInstantiate(&g->exec, g->graph, 0);
   if (e != cudaSuccess) return cuda_fail(e, "gbs_group_capture: instantiate");
-  g->launches_per_replay = (with_pack ? (g->npack[0] ? 1 : 0) + (g->npack[1] ? 1 : 0) : 0) + (g->popc_tiles ? 1 + (g->nrs ? 1 : 0) : 0) +
-                           (g->tc.ntiles ? 1 : 0);
+  g->launches_per_replay = (with_pack ? (g->captured.n[0] ? 1 : 0) + (g->captured.n[1] ? 1 : 0) : 0) +
+                           (g->popc_tiles ? 1 + (g->nrs ? 1 : 0) : 0) + (g->tc.ntiles ? 1 : 0);
+  g->graph_packs = with_pack;
   if (with_pack) {
     for (gbs_ctx *c : g->ctxs) c->lhs.imported = c->rhs.imported = true;
     mark_packed_digits(g);  // each replay packs them
@@ -444,7 +476,7 @@ int gbs_group_replay(gbs_group *g, void *stream) {
   if (!g || !g->exec) return fail(GBS_ESTATE, "gbs_group_replay: capture the group first");
   cudaError_t e = cudaGraphLaunch(g->exec, (cudaStream_t)stream);
   if (e != cudaSuccess) return cuda_fail(e, "gbs_group_replay");
-  if (g->npack[0] || g->npack[1]) {  // the replay packs new planes: cached adjoint operands and other derived copies are stale
+  if (g->graph_packs) {  // the replay packs new planes: cached adjoint operands and other derived copies are stale
     for (gbs_ctx *c : g->ctxs) c->vt_valid[0] = c->vt_valid[1] = false;
     mark_packed_digits(g);
   }

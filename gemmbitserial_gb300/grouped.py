@@ -12,11 +12,15 @@ import ctypes as C
 from . import _capi
 from .api import _stream_handle
 
+_DTYPES: dict = {}
+
 
 def _dtype_code(t):
-    import torch
-    return {torch.int8: _capi.GBS_I8, torch.uint8: _capi.GBS_U8,
-            torch.int16: _capi.GBS_I16, torch.int32: _capi.GBS_I32}[t.dtype]
+    if not _DTYPES:
+        import torch
+        _DTYPES.update({torch.int8: _capi.GBS_I8, torch.uint8: _capi.GBS_U8,
+                        torch.int16: _capi.GBS_I16, torch.int32: _capi.GBS_I32})
+    return _DTYPES[t.dtype]
 
 
 class Group:
