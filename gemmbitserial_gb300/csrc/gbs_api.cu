@@ -127,6 +127,7 @@ void free_ctx_buffers(gbs_ctx *c) {
     delete c->plan1;
   }
   adj_plan_free(c->adj);
+  small_plan_free(c->small);
   wide_plan_free(c->wide);
   if (c->sk_ws) cudaFree(c->sk_ws);
   if (c->sk_flags) cudaFree(c->sk_flags);

@@ -1581,9 +1581,9 @@ bool pdl_for(cudaStream_t s) {
 }
 
 cudaError_t launch_gemm_tc_hbm(gbs_ctx *c, cudaStream_t s, int bn_req) {
-  if (bn_req < 0 && (c->lhs.nrows < 256 || c->rhs.nrows < 256)) {
-    // a side of fewer than 256 rows: the persistent kernel over a one-problem
-    // plan (larger side as the MMA's 128-row operand, MMA N down to 16)
+  const bool small = bn_req < 0 && (c->lhs.nrows < 256 || c->rhs.nrows < 256);
+  if (small && (c->plan1_ready || tcg_nibbles_mode() == 1)) {
+    // the nibble kernel forced on a side of fewer than 256 rows: a one-problem plan
     if (!c->plan1_ready) {
       if (!c->plan1) c->plan1 = new TcgPlan();
       gbs_ctx *one[1] = {c};
@@ -1606,6 +1606,7 @@ cudaError_t launch_gemm_tc_hbm(gbs_ctx *c, cudaStream_t s, int bn_req) {
       cudaError_t e = expand_side(c, side, s);
       if (e != cudaSuccess) return e;
     }
+  if (small) return launch_gemm_tcs(c, s);
   if (!c->digit_maps_ready) {
     if (!make_digit_map(reinterpret_cast<CUtensorMap *>(c->tc_map_da), c->digits[0], c->lhs) ||
         !make_digit_map(reinterpret_cast<CUtensorMap *>(c->tc_map_db), c->digits[1], c->rhs))

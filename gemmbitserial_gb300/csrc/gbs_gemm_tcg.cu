@@ -433,17 +433,18 @@ void tcg_plan_free(TcgPlan *p) {
   *p = TcgPlan();
 }
 
-namespace {
-
 // GBS_TCG_NIBBLES in the environment when a plan is built: 0 keeps it on the
 // digit kernel, 1 puts it on the nibble kernel; unset, the estimate below
-// chooses.  Returns 0, 1 or -1 (choose).
-int nibbles_mode() {
+// chooses for groups, and single contexts run on the digits their imports
+// write.  Returns 0, 1 or -1 (choose).
+int tcg_nibbles_mode() {
   const char *v = getenv("GBS_TCG_NIBBLES");
   if (v && v[0] == '0') return 0;
   if (v && v[0] == '1') return 1;
   return -1;
 }
+
+namespace {
 
 // Which persistent kernel serves a plan faster, by an estimate of its
 // critical path.  The nibble kernel reads half a byte per element of each
@@ -490,7 +491,7 @@ bool plan_prefers_nibbles(gbs_ctx *const *ctxs, int n) {
 
 int tcg_plan_build(TcgPlan *plan, gbs_ctx *const *ctxs, int n) {
   tcg_plan_free(plan);
-  const int mode = nibbles_mode();
+  const int mode = tcg_nibbles_mode();
   const bool nib = mode < 0 ? plan_prefers_nibbles(ctxs, n) : mode == 1;
   plan->nibbles = nib;
   std::vector<TcgProblem> probs;

@@ -12,6 +12,7 @@ namespace gbs {
 
 struct AdjPlan;   // workspace of the tensor-core adjoint (gbs_adjoint_tc.cu)
 struct WidePlan;  // part sub-contexts of a context with 5-8-bit operands (gbs_wide.cu)
+struct SmallPlan;  // tiles and maps of a context with a side under 256 rows (gbs_gemm_tcs.cu)
 
 // Padding of the e4m3 digit matrices (the tensor-core operands): rows to a
 // multiple of every tile's row count, columns to whole 256-digit stages.  The
@@ -240,7 +241,8 @@ struct gbs_ctx {
   float *sk_ws = nullptr;
   uint32_t *sk_flags = nullptr;
   uint32_t sk_pairs = 0, sk_epoch = 0;
-  // one-problem plan of the persistent tensor-core kernel (shapes with a side under 256 rows)
+  gbs::SmallPlan *small = nullptr;  // a side under 256 rows: built on first use
+  // one-problem plan of the persistent nibble kernel, where that is forced on such a context
   gbs::TcgPlan *plan1 = nullptr;
   bool plan1_ready = false;
   gbs::AdjPlan *adj = nullptr;  // tensor-core adjoint workspace, built on first use
@@ -359,6 +361,11 @@ cudaError_t ensure_nibble_buffer(gbs_ctx *c, int side);
 cudaError_t tcgn_gemm(const TcgPlan &plan, uint32_t *err, cudaStream_t s, int32_t *out0);
 cudaError_t tcgn_prepare();  // kernel attributes, once per plan build
 bool tc_map_nibbles(void *map, const uint8_t *base, uint64_t cols, uint64_t rows);
+// GBS_TCG_NIBBLES in the environment: 0 the digit kernels, 1 the nibble kernel, -1 unset
+int tcg_nibbles_mode();
+// one context with a side under 256 rows on its digit matrices (gbs_gemm_tcs.cu)
+cudaError_t launch_gemm_tcs(gbs_ctx *c, cudaStream_t s);
+void small_plan_free(SmallPlan *p);
 // tensor-core pipe for 5-8-bit operands (gbs_wide.cu): operands split into parts of <= 4 bits
 bool tc_wide(const gbs_ctx *c);
 cudaError_t launch_gemm_wide(gbs_ctx *c, cudaStream_t s, int variant);

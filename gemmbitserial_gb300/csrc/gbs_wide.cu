@@ -491,6 +491,7 @@ void wide_plan_free(WidePlan *p) {
         tcg_plan_free(s->plan1);
         delete s->plan1;
       }
+      small_plan_free(s->small);
       if (s->sk_ws) cudaFree(s->sk_ws);
       if (s->sk_flags) cudaFree(s->sk_flags);
       for (uint8_t *nb : s->nibbles)
