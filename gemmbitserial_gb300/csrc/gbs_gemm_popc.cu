@@ -381,11 +381,12 @@ __device__ __forceinline__ void grouped_skinny_output(const GroupProblem &P, uin
 
 // Persistent grouped GEMM: each CTA takes the next tile from the queue until
 // the queue is drained.  Tile classes 0-2 are BM x BN output tiles; class 3
-// is kSkinnyTile outputs, one per warp.  A descriptor that fails validation
+// is 8 * skinny outputs, `skinny` per warp.  A descriptor that fails validation
 // sets a bit in *err and is skipped (no device fault, no wait).
 __global__ void __launch_bounds__(NT, 2) gemm_popc_grouped(const GroupProblem *__restrict__ probs, int nprob,
                                                            const GroupTile *__restrict__ tiles, uint32_t ntiles,
-                                                           uint32_t *counter, uint32_t *err) {
+                                                           uint32_t *counter, uint32_t *done, uint32_t *err,
+                                                           uint32_t skinny) {
   extern __shared__ __align__(16) uint64_t smem[];
   __shared__ uint32_t s_tile;
   for (;;) {
@@ -401,13 +402,15 @@ __global__ void __launch_bounds__(NT, 2) gemm_popc_grouped(const GroupProblem *_
     }
     const GroupProblem &P = probs[tl.p];
     if (tl.cls == kSkinnyCls) {
-      const uint64_t o0 = (uint64_t)tl.mt * kSkinnyTile;
+      const uint64_t o0 = (uint64_t)tl.mt * (8 * skinny);
       if (o0 >= P.M * P.N || P.wa < 1 || P.wa > kMaxBits || P.wb < 1 || P.wb > kMaxBits) {
         if (threadIdx.x == 0) atomicOr(err, 2u);
         continue;
       }
-      const uint64_t o = o0 + (threadIdx.x >> 5);
-      if (o < P.M * P.N) grouped_skinny_output(P, o, threadIdx.x & 31);
+      for (uint32_t i = 0; i < skinny; i++) {
+        const uint64_t o = o0 + 8 * i + (threadIdx.x >> 5);
+        if (o < P.M * P.N) grouped_skinny_output(P, o, threadIdx.x & 31);
+      }
       continue;
     }
     const bool rows = tl.cls == kRowsCls;
@@ -434,6 +437,14 @@ __global__ void __launch_bounds__(NT, 2) gemm_popc_grouped(const GroupProblem *_
       if (tl.cls == 0) popc_tile<64, 64, kGroupKC, false>(g, m0, n0, smem);
       else if (tl.cls == 1) popc_tile<32, 128, kGroupKC, false>(g, m0, n0, smem);
       else popc_tile<16, 256, kGroupKC, false>(g, m0, n0, smem);
+    }
+  }
+  // the CTA that finishes last readies the queue for the next launch
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(done, 1u) == gridDim.x - 1) {
+      *counter = 0u;
+      *done = 0u;
     }
   }
 }
@@ -549,8 +560,9 @@ int grouped_blocks_per_sm(size_t smem) {
 }
 
 cudaError_t launch_gemm_popc_grouped(const GroupProblem *probs, int nprob, const GroupTile *tiles, uint32_t ntiles,
-                                     uint32_t *counter, uint32_t *err, size_t smem, int grid, cudaStream_t s) {
-  gemm_popc_grouped<<<grid, NT, smem, s>>>(probs, nprob, tiles, ntiles, counter, err);
+                                     uint32_t *counter, uint32_t *done, uint32_t *err, uint32_t skinny, size_t smem,
+                                     int grid, cudaStream_t s) {
+  gemm_popc_grouped<<<grid, NT, smem, s>>>(probs, nprob, tiles, ntiles, counter, done, err, skinny);
   count_launch();
   return cudaGetLastError();
 }

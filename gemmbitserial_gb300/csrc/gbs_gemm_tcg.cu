@@ -489,6 +489,41 @@ bool plan_prefers_nibbles(gbs_ctx *const *ctxs, int n) {
 
 }  // namespace
 
+// MMA N (tile width over the smaller side) of every problem of a digit plan:
+// the whole smaller side up to 256 rows; while the plan's tiles leave SMs idle,
+// the problem with the longest tiles gets narrower ones (a power of two: the
+// padded rows are whole multiples).  CaffeNet's five GEMMs had 38 tiles, the
+// longest 27 stages of 38 KB.
+static std::vector<uint32_t> tile_widths(gbs_ctx *const *ctxs, int n) {
+  const uint64_t sms = (uint64_t)std::max(1, sm_count());
+  std::vector<uint32_t> bn(n);
+  auto stage_ns = [](double w) {
+    return std::max((16384.0 + 128.0 * w) / 105.0, 4 * (w <= 128 ? 37.0 : 37.0 + (w - 128) * (31.0 / 128)));
+  };
+  auto rows = [&](int i, bool large) {
+    const uint64_t a = ctxs[i]->lhs.nrows, b = ctxs[i]->rhs.nrows;
+    return large ? std::max(a, b) : std::min(a, b);
+  };
+  auto ntiles = [&](int i, uint32_t w) { return (rows(i, true) + 127) / 128 * ((rows(i, false) + w - 1) / w); };
+  auto tile_ns = [&](int i) { return (double)((ctxs[i]->lhs.ncols + 127) / 128) * stage_ns(bn[i]); };
+  uint64_t total = 0;
+  for (int i = 0; i < n; i++) {
+    bn[i] = (uint32_t)std::min<uint64_t>(256, std::max<uint64_t>(16, (rows(i, false) + 15) / 16 * 16));
+    total += ntiles(i, bn[i]);
+  }
+  while (total < sms) {
+    int worst = 0;
+    for (int i = 1; i < n; i++)
+      if (tile_ns(i) > tile_ns(worst)) worst = i;
+    uint32_t next = 128;
+    while (next >= bn[worst]) next /= 2;
+    if (next < 16 || total - ntiles(worst, bn[worst]) + ntiles(worst, next) > sms) break;
+    total += ntiles(worst, next) - ntiles(worst, bn[worst]);
+    bn[worst] = next;
+  }
+  return bn;
+}
+
 int tcg_plan_build(TcgPlan *plan, gbs_ctx *const *ctxs, int n) {
   tcg_plan_free(plan);
   const int mode = tcg_nibbles_mode();
@@ -500,6 +535,7 @@ int tcg_plan_build(TcgPlan *plan, gbs_ctx *const *ctxs, int n) {
   std::vector<uint64_t> cost;
   std::vector<ExpandJob> jobs;
   uint64_t threads = 0;
+  const std::vector<uint32_t> widths = nib ? std::vector<uint32_t>() : tile_widths(ctxs, n);
   for (int i = 0; i < n; i++) {
     gbs_ctx *c = ctxs[i];
     const Mat &L = c->lhs, &R = c->rhs;
@@ -530,7 +566,7 @@ int tcg_plan_build(TcgPlan *plan, gbs_ctx *const *ctxs, int n) {
     CUtensorMap m2[2];
     uint32_t rt, ct;
     if (!nib) {
-      P.bn = (uint32_t)std::min<uint64_t>(256, (MB.nrows + 15) / 16 * 16);
+      P.bn = widths[i];
       P.idesc = (1u << 4) | ((P.bn >> 3) << 17) | ((128u >> 4) << 24);
       if (!tc_map_u8(&m2[0], c->digits[sa], MA.dcols, MA.drows, 128) ||
           !tc_map_u8(&m2[1], c->digits[sb], MB.dcols, MB.drows, P.bn))

@@ -25,8 +25,11 @@
 
 // Pack jobs of a grouped import on the device: those of the direct kernel, then those of the staged one.
 struct PackTable {
-  gbs::PackJob *jobs = nullptr;
+  std::vector<gbs::PackJob> host;  // at most kInlinePackJobs of them go with the launch
+  bool with_launch = false;
+  gbs::PackJob *jobs = nullptr;    // the others' device table
   size_t capacity = 0;
+  gbs::PackJob *recorded = nullptr;  // the table of an import recorded into a caller's capture
   int n[2] = {0, 0};
   uint64_t runs[2] = {0, 0};
   uint32_t run[2] = {1, 1};  // units per run
@@ -38,11 +41,15 @@ struct gbs_group {
   gbs::GroupProblem *d_probs = nullptr;
   gbs::GroupTile *d_tiles = nullptr;
   uint32_t ntiles = 0;
-  uint32_t *d_scratch = nullptr;  // [0] tile counter, [1] popcount-kernel error bits, [2] tensor-core error bits
+  // [0] tile counter, [1] popcount-kernel error bits, [2] tensor-core error bits, [3] finished CTAs of the
+  // popcount kernel, whose last one zeroes [0] and [3] for the next launch
+  uint32_t *d_scratch = nullptr;
+  uint32_t skinny = 1;  // outputs per warp of a skinny tile
   gbs::PackJob *d_rs_jobs = nullptr;
   int nrs = 0;
   uint64_t rs_warps = 0;
   PackTable imports, captured;  // of gbs_group_import, and of the captured graph (which keeps reading it)
+  std::vector<gbs::PackJob *> foreign;  // tables of imports recorded into a caller's own capture
   cudaEvent_t packed = nullptr;  // the last import's pack: its table may be written again
   size_t smem = 0;
   int grid = 0;
@@ -51,8 +58,8 @@ struct gbs_group {
   bool graph_packs = false;  // the captured graph imports
   gbs::TcgPlan tc;  // problems on the tensor-core kernel
   std::vector<char> is_tc;  // per problem: on the tensor-core kernel
-  // with both kernel types, the tensor-core kernel runs on a stream forked
-  // from the caller's (and joined back), so the two share the SMs
+  // with both kernel types, the popcount kernel runs on a stream forked from
+  // the caller's (and joined back), so the two share the SMs
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
   uint64_t launches_per_replay = 0;
@@ -87,6 +94,7 @@ void free_group(gbs_group *g) {
   if (g->d_rs_jobs) cudaFree(g->d_rs_jobs);
   if (g->imports.jobs) cudaFree(g->imports.jobs);
   if (g->captured.jobs) cudaFree(g->captured.jobs);
+  for (gbs::PackJob *t : g->foreign) cudaFree(t);
   if (g->packed) cudaEventDestroy(g->packed);
   delete g;
 }
@@ -145,56 +153,69 @@ int build_pack_jobs(gbs_group *g, PackTable &tab, const void *const *lhs, const 
     tab.run[k] = run;
   }
   jobs[0].insert(jobs[0].end(), jobs[1].begin(), jobs[1].end());
-  const size_t bytes = jobs[0].size() * sizeof(PackJob);
+  tab.host.swap(jobs[0]);
+  tab.with_launch = false;
+  const size_t bytes = tab.host.size() * sizeof(PackJob);
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   cudaError_t e = cudaStreamIsCapturing(s, &st);
-  if (e == cudaSuccess && st != cudaStreamCaptureStatusNone) e = cudaErrorStreamCaptureUnsupported;
-  if (e == cudaSuccess && tab.capacity < bytes) {
-    if (tab.jobs) cudaFree(tab.jobs);  // waits for the device: nothing reads the old table any more
-    tab.jobs = nullptr;
-    tab.capacity = 0;
-    e = dev_alloc((void **)&tab.jobs, bytes);
-    if (e == cudaSuccess) tab.capacity = bytes;
+  if (e == cudaSuccess && st != cudaStreamCaptureStatusNone) {
+    // recorded into the caller's capture, where its mode allows allocating: a table that stays as it is
+    gbs::PackJob *t = nullptr;
+    e = upload(&t, tab.host);
+    if (e == cudaSuccess) {
+      g->foreign.push_back(t);
+      tab.recorded = t;
+    }
+  } else if (e == cudaSuccess && tab.host.size() <= (size_t)kInlinePackJobs) {
+    tab.with_launch = true;
   } else if (e == cudaSuccess) {
-    e = cudaStreamWaitEvent(s, g->packed, 0);
+    if (tab.capacity < bytes) {
+      if (tab.jobs) cudaFree(tab.jobs);  // waits for the device: nothing reads the old table any more
+      tab.jobs = nullptr;
+      tab.capacity = 0;
+      e = dev_alloc((void **)&tab.jobs, bytes);
+      if (e == cudaSuccess) tab.capacity = bytes;
+    } else {
+      e = cudaStreamWaitEvent(s, g->packed, 0);
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(tab.jobs, tab.host.data(), bytes, cudaMemcpyHostToDevice, s);
+    tab.recorded = nullptr;
   }
-  if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(tab.jobs, jobs[0].data(), bytes, cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) {
     cudaGetLastError();
-    tab.n[0] = tab.n[1] = 0;
+    tab.runs[0] = tab.runs[1] = 0;
     return fail(GBS_ENOMEM, "gbs_group: pack table upload failed");
   }
   return GBS_OK;
 }
 
 cudaError_t enqueue_pack(const PackTable &tab, cudaStream_t s) {
-  cudaError_t e = launch_pack_grouped(tab.jobs, tab.n[0], tab.runs[0], tab.run[0], true, s);
-  if (e == cudaSuccess) e = launch_pack_grouped(tab.jobs + tab.n[0], tab.n[1], tab.runs[1], tab.run[1], false, s);
+  return launch_pack_grouped(tab.with_launch ? tab.host.data() : nullptr, tab.recorded ? tab.recorded : tab.jobs, tab.n,
+                             tab.runs, tab.run, s);
+}
+
+cudaError_t enqueue_popc(gbs_group *g, cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
+  if (g->nrs) e = launch_rowsum_grouped(g->d_rs_jobs, g->nrs, g->rs_warps, s);
+  if (e == cudaSuccess)
+    e = launch_gemm_popc_grouped(g->d_probs, (int)g->ctxs.size(), g->d_tiles, g->popc_tiles, g->d_scratch,
+                                 g->d_scratch + 3, g->d_scratch + 1, g->skinny, g->smem, g->grid, s);
   return e;
 }
 
+// With both kernel types, the tensor-core kernel follows on the caller's stream
+// and the popcount kernel forks off: it starts a few us later, once the
+// tensor-core CTAs have their SMs, and its CTAs take the room they leave (placed
+// first, two of its CTAs fill an SM's registers).
 cudaError_t enqueue_gemm(gbs_group *g, cudaStream_t s) {
-  cudaError_t e = cudaSuccess;
-  const bool both = g->popc_tiles && g->tc.ntiles;
-  if (both) {  // the tensor-core kernel on the side stream
-    e = cudaEventRecord(g->fork, s);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(g->side, g->fork, 0);
-    if (e == cudaSuccess) e = tcg_gemm(g->tc, g->d_scratch + 2, g->side);
-    if (e == cudaSuccess) e = cudaEventRecord(g->join, g->side);
-    if (e != cudaSuccess) return e;
-  }
-  if (g->popc_tiles) {
-    e = cudaMemsetAsync(g->d_scratch, 0, sizeof(uint32_t), s);  // tile counter only
-    if (e == cudaSuccess && g->nrs) e = launch_rowsum_grouped(g->d_rs_jobs, g->nrs, g->rs_warps, s);
-    if (e == cudaSuccess)
-      e = launch_gemm_popc_grouped(g->d_probs, (int)g->ctxs.size(), g->d_tiles, g->popc_tiles, g->d_scratch,
-                                   g->d_scratch + 1, g->smem, g->grid, s);
-  }
-  if (both) {
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, g->join, 0);
-  } else if (e == cudaSuccess) {
-    e = tcg_gemm(g->tc, g->d_scratch + 2, s);
-  }
+  if (!g->popc_tiles) return tcg_gemm(g->tc, g->d_scratch + 2, s);
+  if (!g->tc.ntiles) return enqueue_popc(g, s);
+  cudaError_t e = cudaEventRecord(g->fork, s);
+  if (e == cudaSuccess) e = tcg_gemm(g->tc, g->d_scratch + 2, s);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(g->side, g->fork, 0);
+  if (e == cudaSuccess) e = enqueue_popc(g, g->side);
+  if (e == cudaSuccess) e = cudaEventRecord(g->join, g->side);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(s, g->join, 0);
   return e;
 }
 
@@ -253,6 +274,8 @@ int gbs_group_create(gbs_ctx *const *ctxs, int count, gbs_group **out) {
   size_t smem = 16;
   const int mode = group_pipe_mode();
   std::vector<gbs_ctx *> tc_ctxs;
+  std::vector<uint32_t> skinny_probs;
+  uint64_t skinny_outputs = 0;
   for (int p = 0; p < count; p++) {
     gbs_ctx *c = ctxs[p];
     if (!c) {
@@ -295,7 +318,7 @@ int gbs_group_create(gbs_ctx *const *ctxs, int count, gbs_group **out) {
     P.neg_j = e.neg_j;
     P.shift = e.shift;
     P.c0 = e.c0;
-    // kSkinnyTile outputs per tile, a warp each, where every BM x BN class would
+    // the skinny class, outputs of a warp each, where every BM x BN class would
     // leave most of its tile empty: fewer than 16 rhs rows (the classes' BN is
     // 64 or more), or a tiny output of more than 16 lhs rows; at most 16 lhs
     // rows take the rows class below (a warp per output waits on memory once
@@ -304,11 +327,8 @@ int gbs_group_create(gbs_ctx *const *ctxs, int count, gbs_group **out) {
     if (P.N < 16 || (P.M * P.N <= 4096 && !rows_fit)) {
       P.cls = kSkinnyCls;
       probs.push_back(P);
-      const uint64_t nt = (P.M * P.N + kSkinnyTile - 1) / kSkinnyTile;
-      for (uint64_t i = 0; i < nt; i++) {
-        tiles.push_back(GroupTile{(uint32_t)p, (uint32_t)i, 0u, (uint32_t)kSkinnyCls});
-        cost.push_back(std::max<uint64_t>(1, (uint64_t)P.wa * P.wb * P.wpr / 512));
-      }
+      skinny_probs.push_back((uint32_t)p);
+      skinny_outputs += P.M * P.N;
     } else if (rows_fit) {
       // at most 16 lhs rows: the rows class, one rhs row per thread (no popcounts on padding rows)
       P.cls = kRowsCls;
@@ -348,6 +368,17 @@ int gbs_group_create(gbs_ctx *const *ctxs, int count, gbs_group **out) {
       if (reg.nrows) rs.push_back(j);
     }
   }
+  // Skinny tiles: one output per warp until they fill the GPU (8 warps a CTA, 2
+  // CTAs on each of 152 SMs), then up to 4: a warp's outputs share a trip to the queue
+  g->skinny = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(4, skinny_outputs / (8 * 2 * 152)));
+  for (uint32_t p : skinny_probs) {
+    const GroupProblem &P = probs[p];
+    const uint64_t per = 8 * g->skinny, nt = (P.M * P.N + per - 1) / per;
+    for (uint64_t i = 0; i < nt; i++) {
+      tiles.push_back(GroupTile{p, (uint32_t)i, 0u, (uint32_t)kSkinnyCls});
+      cost.push_back(std::max<uint64_t>(1, (uint64_t)g->skinny * P.wa * P.wb * P.wpr / 512));
+    }
+  }
   // Longest tiles first: the queue then balances like LPT scheduling.
   std::vector<size_t> order(tiles.size());
   for (size_t i = 0; i < order.size(); i++) order[i] = i;
@@ -365,8 +396,8 @@ int gbs_group_create(gbs_ctx *const *ctxs, int count, gbs_group **out) {
   cudaError_t e = upload(&g->d_probs, probs);
   if (e == cudaSuccess) e = upload(&g->d_tiles, sorted);
   if (e == cudaSuccess) e = upload(&g->d_rs_jobs, rs);
-  if (e == cudaSuccess) e = dev_alloc((void **)&g->d_scratch, 3 * sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMemset(g->d_scratch, 0, 3 * sizeof(uint32_t));
+  if (e == cudaSuccess) e = dev_alloc((void **)&g->d_scratch, 4 * sizeof(uint32_t));
+  if (e == cudaSuccess) e = cudaMemset(g->d_scratch, 0, 4 * sizeof(uint32_t));
   if (e == cudaSuccess) e = prepare_gemm_popc_grouped(smem);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&g->side, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&g->fork, cudaEventDisableTiming);
@@ -462,7 +493,7 @@ int gbs_group_capture(gbs_group *g, const void *const *lhs_srcs, const void *con
   if (e != cudaSuccess) return cuda_fail(e, "gbs_group_capture: end capture");
   e = cudaGraphInstantiate(&g->exec, g->graph, 0);
   if (e != cudaSuccess) return cuda_fail(e, "gbs_group_capture: instantiate");
-  g->launches_per_replay = (with_pack ? (g->captured.n[0] ? 1 : 0) + (g->captured.n[1] ? 1 : 0) : 0) +
+  g->launches_per_replay = (with_pack && !g->captured.host.empty() ? 1 : 0) +
                            (g->popc_tiles ? 1 + (g->nrs ? 1 : 0) : 0) + (g->tc.ntiles ? 1 : 0);
   g->graph_packs = with_pack;
   if (with_pack) {

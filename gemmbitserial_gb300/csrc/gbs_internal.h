@@ -288,8 +288,7 @@ cudaError_t launch_gemm_popc(const GemmShape &g, const Epilogue &e, cudaStream_t
 int popc_tile_class(uint64_t M, int wa, int wb, size_t smem_cap);
 // small-output shapes (matrix-vector and the like): one warp per output
 bool popc_skinny(uint64_t M, uint64_t N);
-constexpr int kSkinnyCls = 3;    // grouped tile class of kSkinnyTile outputs, one per warp
-constexpr int kSkinnyTile = 8;
+constexpr int kSkinnyCls = 3;    // grouped tile class of 8 * skinny outputs (a launch's skinny), `skinny` per warp
 constexpr int kRowsCls = 4;      // grouped tile class of all <= kRowsMaxM lhs rows x 256 rhs rows
 constexpr int kRowsMaxM = 16;
 constexpr int kRowsKC = 16;      // K words per pipeline step of the rows tile (128 bytes of each row)
@@ -300,10 +299,14 @@ size_t popc_stage_smem(int cls, int wa, int wb, int kc);
 constexpr int kGroupKC = 8;
 cudaError_t prepare_gemm_popc_grouped(size_t smem);
 cudaError_t launch_gemm_popc_grouped(const GroupProblem *probs, int nprob, const GroupTile *tiles, uint32_t ntiles,
-                                     uint32_t *counter, uint32_t *err, size_t smem, int grid, cudaStream_t s);
+                                     uint32_t *counter, uint32_t *done, uint32_t *err, uint32_t skinny, size_t smem,
+                                     int grid, cudaStream_t s);
 int grouped_blocks_per_sm(size_t smem);
-cudaError_t launch_pack_grouped(const PackJob *jobs, int njobs, uint64_t runs, uint32_t run, bool direct,
-                                cudaStream_t s);
+// Grouped import: n[0] direct jobs, then n[1] staged ones, each kind runs[k] runs of run[k] units; from `host` (at
+// most kInlinePackJobs jobs, passed with the launch) or, host null, from the device table `jobs`.
+constexpr int kInlinePackJobs = 24;
+cudaError_t launch_pack_grouped(const PackJob *host, const PackJob *jobs, const int (&n)[2], const uint64_t (&runs)[2],
+                                const uint32_t (&run)[2], cudaStream_t s);
 cudaError_t launch_rowsum_grouped(const PackJob *jobs, int njobs, uint64_t total_warps, cudaStream_t s);
 cudaError_t launch_gemm_bmma(const GemmShape &g, const Epilogue &e, cudaStream_t s);
 bool bmma_supported(int wa, int wb, int use_xor);

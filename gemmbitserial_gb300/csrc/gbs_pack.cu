@@ -657,15 +657,17 @@ __device__ __forceinline__ int find_job(const PackJob *jobs, int njobs, uint64_t
 constexpr int kMaxRun = 8;
 constexpr int kDepth = 2;
 
-__global__ void __launch_bounds__(256, 4) pack_grouped(const PackJob *__restrict__ jobs, int njobs, uint64_t runs,
-                                                       uint32_t run) {
-  __shared__ PackJob sj[8];  // each warp's job: its fields stay out of the registers
-  griddep_launch_dependents();
-  griddep_wait();  // source, planes and digits belong to earlier kernels until here
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+// Jobs of a small group as a kernel parameter: no table to copy before the launch.
+struct InlineJobs {
+  PackJob jobs[kInlinePackJobs];
+};
+static_assert(sizeof(InlineJobs) <= 4000, "kernel parameters");
+
+// Packs direct runs w0, w0 + nw, ... of the warp; sj is the warp's shared-memory copy of its job.
+__device__ __forceinline__ void pack_direct_runs(const PackJob *jobs, int njobs, uint64_t w0, uint64_t nw,
+                                                 uint64_t runs, uint32_t run, PackJob &J) {
   const int lane = threadIdx.x & 31;
-  PackJob &J = sj[threadIdx.x >> 5];
-  for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < runs; w += nw) {
+  for (uint64_t w = w0; w < runs; w += nw) {
     const int j = find_job(jobs, njobs, w, lane);
     static_assert(sizeof(PackJob) % 8 == 0 && sizeof(PackJob) / 8 <= 32, "one word a lane");
     __syncwarp();
@@ -697,6 +699,15 @@ __global__ void __launch_bounds__(256, 4) pack_grouped(const PackJob *__restrict
   }
 }
 
+__global__ void __launch_bounds__(256, 4) pack_grouped(const PackJob *__restrict__ jobs, int njobs, uint64_t runs,
+                                                       uint32_t run) {
+  __shared__ PackJob sj[8];  // each warp's job: its fields stay out of the registers
+  griddep_launch_dependents();
+  griddep_wait();  // sources, planes and digits belong to earlier kernels until here
+  pack_direct_runs(jobs, njobs, ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+                   ((uint64_t)gridDim.x * blockDim.x) >> 5, runs, run, sj[threadIdx.x >> 5]);
+}
+
 // The same for the other operands (wider elements, unaligned rows).
 template <typename T>
 __device__ __forceinline__ void pack_staged_run(const PackJob &J, uint64_t u0, uint32_t run, uint32_t *st) {
@@ -708,15 +719,10 @@ __device__ __forceinline__ void pack_staged_run(const PackJob &J, uint64_t u0, u
   }
 }
 
-__global__ void __launch_bounds__(256) pack_grouped_staged(const PackJob *__restrict__ jobs, int njobs,
-                                                           uint64_t runs, uint32_t run) {
-  __shared__ __align__(16) uint32_t st[8][256];
-  griddep_launch_dependents();
-  griddep_wait();  // source, planes and digits belong to earlier kernels until here
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+__device__ __forceinline__ void pack_staged_runs(const PackJob *jobs, int njobs, uint64_t w0, uint64_t nw,
+                                                 uint64_t runs, uint32_t run, uint32_t *my) {
   const int lane = threadIdx.x & 31;
-  uint32_t *my = st[threadIdx.x >> 5];
-  for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < runs; w += nw) {
+  for (uint64_t w = w0; w < runs; w += nw) {
     const PackJob &J = jobs[find_job(jobs, njobs, w, lane)];
     const uint64_t u0 = (w - J.warp0) * run;
     switch (J.dtype) {
@@ -727,6 +733,42 @@ __global__ void __launch_bounds__(256) pack_grouped_staged(const PackJob *__rest
       default: pack_staged_run<float>(J, u0, run, my); break;
     }
   }
+}
+
+// Both kinds of jobs in one launch: the first `sblocks` blocks take the staged
+// ones, which wait longer per unit, the others the direct ones.  CaffeNet's
+// two kinds one after the other took 20 + 17 us.
+struct PackRuns {
+  int n;  // jobs of the kind
+  uint32_t run;
+  uint64_t runs;
+};
+
+__device__ __forceinline__ void pack_both(const PackJob *jobs, PackRuns direct, PackRuns staged, uint32_t sblocks) {
+  union Shared {
+    PackJob sj[8];
+    uint32_t st[8][256];
+  };
+  __shared__ __align__(16) unsigned char raw[sizeof(Shared)];
+  Shared &sh = *reinterpret_cast<Shared *>(raw);
+  griddep_launch_dependents();
+  griddep_wait();  // sources, planes and digits belong to earlier kernels until here
+  const uint32_t warp = threadIdx.x >> 5;
+  if (blockIdx.x < sblocks)
+    pack_staged_runs(jobs + direct.n, staged.n, (uint64_t)blockIdx.x * 8 + warp, (uint64_t)sblocks * 8, staged.runs,
+                     staged.run, sh.st[warp]);
+  else
+    pack_direct_runs(jobs, direct.n, (uint64_t)(blockIdx.x - sblocks) * 8 + warp,
+                     (uint64_t)(gridDim.x - sblocks) * 8, direct.runs, direct.run, sh.sj[warp]);
+}
+
+__global__ void __launch_bounds__(256, 4) pack_grouped_both(const PackJob *__restrict__ jobs, PackRuns direct,
+                                                            PackRuns staged, uint32_t sblocks) {
+  pack_both(jobs, direct, staged, sblocks);
+}
+__global__ void __launch_bounds__(256, 4) pack_grouped_inline(const __grid_constant__ InlineJobs t, PackRuns direct,
+                                                              PackRuns staged, uint32_t sblocks) {
+  pack_both(t.jobs, direct, staged, sblocks);
 }
 
 // sumRows (arch-generic.hpp:6-37) of row r by one warp.  uint32 arithmetic
@@ -850,11 +892,11 @@ bool pack_job_direct(PackJob &j, const Mat &m) {
 
 uint64_t pack_job_units(const PackJob &j) { return (j.nrows_a * j.cpr + 31) / 32; }
 
-// Units per run of a grouped import of `units` units: enough runs for 32 warps
-// on each of 152 SMs before a run grows past one unit (CaffeNet's 1.2 M
-// unaligned bytes in runs of 8 were 147 warps and 48 us).
+// Units per run of a grouped import of `units` units: four runs for each of 32
+// warps on 152 SMs before a run grows past one unit (CaffeNet's 1.2 M unaligned
+// bytes in runs of 8 were 147 warps and 48 us).
 uint32_t pack_run_units(uint64_t units) {
-  return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(kMaxRun, units / (152 * 32)));
+  return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(kMaxRun, units / (4 * 152 * 32)));
 }
 
 namespace {
@@ -932,12 +974,23 @@ cudaError_t launch_pack(const Mat &m, const void *src, int dtype, int col_major,
   return run_colmajor(make_pack_job(m, src, dtype, digits, nullptr), nullptr, 0, false, s);
 }
 
-cudaError_t launch_pack_grouped(const PackJob *jobs, int njobs, uint64_t runs, uint32_t run, bool direct,
-                                cudaStream_t s) {
-  if (runs == 0 || njobs == 0) return cudaSuccess;
-  const uint64_t blocks = std::min<uint64_t>((runs + 7) / 8, 152 * 64);
-  const cudaError_t e =
-      launch_pdl(direct ? pack_grouped : pack_grouped_staged, (unsigned)blocks, 256, 0, s, jobs, njobs, runs, run);
+cudaError_t launch_pack_grouped(const PackJob *host, const PackJob *jobs, const int (&n)[2], const uint64_t (&runs)[2],
+                                const uint32_t (&run)[2], cudaStream_t s) {
+  if (runs[0] + runs[1] == 0) return cudaSuccess;
+  const PackRuns direct{n[0], run[0], runs[0]}, staged{n[1], run[1], runs[1]};
+  const unsigned db = (unsigned)std::min<uint64_t>((runs[0] + 7) / 8, 152 * 64);
+  const unsigned sb = (unsigned)std::min<uint64_t>((runs[1] + 7) / 8, 152 * 16);
+  cudaError_t e;
+  if (host) {
+    InlineJobs t;
+    memset(&t, 0, sizeof(t));
+    memcpy(t.jobs, host, (size_t)(n[0] + n[1]) * sizeof(PackJob));
+    e = launch_pdl(pack_grouped_inline, sb + db, 256, 0, s, t, direct, staged, sb);
+  } else if (runs[1]) {
+    e = launch_pdl(pack_grouped_both, sb + db, 256, 0, s, jobs, direct, staged, sb);
+  } else {
+    e = launch_pdl(pack_grouped, db, 256, 0, s, jobs, n[0], runs[0], run[0]);
+  }
   count_launch();
   return e != cudaSuccess ? e : cudaGetLastError();
 }
