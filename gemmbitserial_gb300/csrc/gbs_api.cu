@@ -130,6 +130,7 @@ void free_ctx_buffers(gbs_ctx *c) {
   small_plan_free(c->small);
   wide_plan_free(c->wide);
   if (c->sk_ws) cudaFree(c->sk_ws);
+  if (c->split_ws) cudaFree(c->split_ws);
   if (c->sk_flags) cudaFree(c->sk_flags);
   if (c->digits[0]) cudaFree(c->digits[0]);
   if (c->digits[1]) cudaFree(c->digits[1]);
@@ -439,7 +440,7 @@ int ensure_stage(gbs_ctx *c, int side, size_t bytes, cudaStream_t s) {
 bool import_digit_target(gbs_ctx *c, int side, DigitTarget &t, cudaStream_t s) {
   if (effective_pipe(c) != GBS_PIPE_TC) return false;
   if (tc_wide(c)) return wide_digit_target(c, side, t, s);
-  if (ensure_digit_buffer(c, side) != cudaSuccess) {
+  if (ensure_digit_buffer(c, side, &s) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }

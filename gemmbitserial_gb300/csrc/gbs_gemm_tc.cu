@@ -1330,7 +1330,7 @@ bool make_digit_map(CUtensorMap *map, const uint8_t *digits, const Mat &m, uint3
 }
 
 cudaError_t expand_side(gbs_ctx *c, int side, cudaStream_t s) {
-  cudaError_t e = ensure_digit_buffer(c, side);
+  cudaError_t e = ensure_digit_buffer(c, side, &s);
   if (e != cudaSuccess) return e;
   e = launch_expand(make_expand_job(side ? c->rhs : c->lhs, c->digits[side]), s);
   if (e == cudaSuccess) c->digits_valid[side] = true;
@@ -1338,7 +1338,7 @@ cudaError_t expand_side(gbs_ctx *c, int side, cudaStream_t s) {
 }
 
 cudaError_t expand_nibble_side(gbs_ctx *c, int side, cudaStream_t s) {
-  cudaError_t e = ensure_nibble_buffer(c, side);
+  cudaError_t e = ensure_nibble_buffer(c, side, &s);
   if (e != cudaSuccess) return e;
   e = launch_expand(make_nibble_job(side ? c->rhs : c->lhs, c->nibbles[side]), s);
   if (e == cudaSuccess) c->nibbles_valid[side] = true;
@@ -1654,6 +1654,22 @@ cudaError_t launch_gemm_tc_hbm(gbs_ctx *c, cudaStream_t s, int bn_req) {
           splits = cs;
         }
         if (2 * used >= pairs) break;
+      }
+    }
+    if (bn_req < 0) {
+      // Few tiles and a long K: 256 x 256 tiles split over independent pairs, where
+      // that is estimated faster than the choice above (measured: 0.35 us a stage,
+      // whatever the width, and 6 us a launch, split in a cluster or not)
+      const uint64_t pairs = (uint64_t)sm_count_cached() / 2, tiles = mt * ((a.N + 255) / 256);
+      const uint64_t chosen = mt * ((a.N + bn - 1) / bn) * splits;
+      const double us = (double)((chosen + pairs - 1) / pairs) * 0.35 * (a.nstages / splits) + 6.0;
+      const uint32_t gather = pair_gather_splits(tiles, a.nstages, pairs, us);
+      if (gather > 1 && ensure_split_workspace(c, tiles, gather, s)) {
+        c->last_pair_bn = 256;
+        c->last_pair_splits = (int)gather;
+        c->last_pair_persistent = false;
+        c->last_pair_streamk = 0;
+        return launch_pair_gather(c, c->tc_map_da, c->tc_map_db, gather, s);
       }
     }
     if (bn == 128 && !c->digit_map_b64_ready) {

@@ -384,15 +384,34 @@ cudaError_t launch_expand(const ExpandJob &job, cudaStream_t s) {
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
+// Allocates a zeroed buffer.  With a stream (order) the zeroing is queued there,
+// before whatever that stream does with the buffer next; into a capture, where it
+// would be recorded instead, and without a stream it is done before returning.
+// (Waiting for the device on each buffer was most of a new context's first call.)
+cudaError_t alloc_zeroed(void **p, size_t bytes, const cudaStream_t *order) {
+  cudaError_t e = dev_alloc(p, bytes);
+  if (e != cudaSuccess) return e;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusActive;
+  if (order && cudaStreamIsCapturing(*order, &st) != cudaSuccess) cudaGetLastError();
+  if (order && st == cudaStreamCaptureStatusNone) {
+    e = cudaMemsetAsync(*p, 0, bytes, *order);
+  } else {
+    e = cudaMemset(*p, 0, bytes);
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  }
+  if (e != cudaSuccess) {
+    cudaFree(*p);
+    *p = nullptr;
+  }
+  return e;
+}
+
 // Digit matrix [drows][dcols] of one side, allocated zeroed on first use
-// (synchronously: kernels on any stream may write it right after).
-cudaError_t ensure_digit_buffer(gbs_ctx *c, int side) {
+// (order: alloc_zeroed).
+cudaError_t ensure_digit_buffer(gbs_ctx *c, int side, const cudaStream_t *order) {
   if (c->digits[side]) return cudaSuccess;
   const Mat &m = side ? c->rhs : c->lhs;
-  const size_t bytes = std::max<size_t>(m.drows * m.dcols, 16);
-  cudaError_t e = dev_alloc((void **)&c->digits[side], bytes);
-  if (e == cudaSuccess) e = cudaMemset(c->digits[side], 0, bytes);
-  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  cudaError_t e = alloc_zeroed((void **)&c->digits[side], std::max<size_t>(m.drows * m.dcols, 16), order);
   c->digit_maps_ready = false;
   c->digit_map_b64_ready = false;
   c->plan1_ready = false;
@@ -401,13 +420,10 @@ cudaError_t ensure_digit_buffer(gbs_ctx *c, int side) {
 }
 
 // Nibble matrix [drows][dcols / 2] of one side, allocated zeroed on first use.
-cudaError_t ensure_nibble_buffer(gbs_ctx *c, int side) {
+cudaError_t ensure_nibble_buffer(gbs_ctx *c, int side, const cudaStream_t *order) {
   if (c->nibbles[side]) return cudaSuccess;
   const Mat &m = side ? c->rhs : c->lhs;
-  const size_t bytes = std::max<size_t>(m.drows * m.dcols / 2, 16);
-  cudaError_t e = dev_alloc((void **)&c->nibbles[side], bytes);
-  if (e == cudaSuccess) e = cudaMemset(c->nibbles[side], 0, bytes);
-  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  cudaError_t e = alloc_zeroed((void **)&c->nibbles[side], std::max<size_t>(m.drows * m.dcols / 2, 16), order);
   c->plan1_ready = false;
   c->nibbles_valid[side] = false;
   return e;

@@ -241,6 +241,9 @@ struct gbs_ctx {
   float *sk_ws = nullptr;
   uint32_t *sk_flags = nullptr;
   uint32_t sk_pairs = 0, sk_epoch = 0;
+  // K-split SM pairs (gbs_gemm_tcp.cu): partial columns, and the arrival counters after them
+  void *split_ws = nullptr;
+  uint32_t *split_counters = nullptr;
   gbs::SmallPlan *small = nullptr;  // a side under 256 rows: built on first use
   // one-problem plan of the persistent nibble kernel, where that is forced on such a context
   gbs::TcgPlan *plan1 = nullptr;
@@ -358,14 +361,19 @@ int tcg_plan_build(TcgPlan *plan, gbs_ctx *const *ctxs, int n);
 void tcg_plan_free(TcgPlan *plan);
 cudaError_t tcg_expand(TcgPlan &plan, cudaStream_t s);
 cudaError_t tcg_gemm(const TcgPlan &plan, uint32_t *err, cudaStream_t s, int32_t *out0 = nullptr);
-cudaError_t ensure_digit_buffer(gbs_ctx *c, int side);
-cudaError_t ensure_nibble_buffer(gbs_ctx *c, int side);
+cudaError_t alloc_zeroed(void **p, size_t bytes, const cudaStream_t *order);
+cudaError_t ensure_digit_buffer(gbs_ctx *c, int side, const cudaStream_t *order = nullptr);
+cudaError_t ensure_nibble_buffer(gbs_ctx *c, int side, const cudaStream_t *order = nullptr);
 // the nibble kernel over a plan built with nibbles set (gbs_gemm_tcgn.cu)
 cudaError_t tcgn_gemm(const TcgPlan &plan, uint32_t *err, cudaStream_t s, int32_t *out0);
 cudaError_t tcgn_prepare();  // kernel attributes, once per plan build
 bool tc_map_nibbles(void *map, const uint8_t *base, uint64_t cols, uint64_t rows);
 // GBS_TCG_NIBBLES in the environment: 0 the digit kernels, 1 the nibble kernel, -1 unset
 int tcg_nibbles_mode();
+// SM-pair tiles with K split, partial tiles summed through L2 (gbs_gemm_tcp.cu)
+uint32_t pair_gather_splits(uint64_t tiles, uint32_t nstages, uint64_t pairs, double other_us);
+bool ensure_split_workspace(gbs_ctx *c, uint64_t tiles, uint32_t splits, cudaStream_t s);
+cudaError_t launch_pair_gather(gbs_ctx *c, const void *map_a, const void *map_b, uint32_t splits, cudaStream_t s);
 // one context with a side under 256 rows on its digit matrices (gbs_gemm_tcs.cu)
 cudaError_t launch_gemm_tcs(gbs_ctx *c, cudaStream_t s);
 void small_plan_free(SmallPlan *p);

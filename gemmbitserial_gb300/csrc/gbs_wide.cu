@@ -338,15 +338,13 @@ void scale_table(uint32_t (&tab)[4], int power) {
 }
 
 cudaError_t alloc_parts(const gbs_ctx *c, const WidePlan &p, uint8_t *(&digits)[2][2]) {
+  // (both sides' buffers at once, which the two imports may write on different streams: zeroed before returning)
   for (int side = 0; side < 2; side++) {
     const Mat &m = side ? c->rhs : c->lhs;
     const size_t bytes = std::max<size_t>(m.drows * m.dcols, 16);
     for (int k = 0; k < p.parts[side]; k++) {
       if (digits[side][k]) continue;
-      cudaError_t e = dev_alloc((void **)&digits[side][k], bytes);
-      if (e == cudaSuccess) e = cudaMemset(digits[side][k], 0, bytes);
-      if (e == cudaSuccess) e = cudaDeviceSynchronize();  // kernels on any stream may write it right after
-      if (e != cudaSuccess) {
+      if (alloc_zeroed((void **)&digits[side][k], bytes, nullptr) != cudaSuccess) {
         cudaGetLastError();
         return cudaErrorMemoryAllocation;
       }
@@ -493,6 +491,7 @@ void wide_plan_free(WidePlan *p) {
       }
       small_plan_free(s->small);
       if (s->sk_ws) cudaFree(s->sk_ws);
+      if (s->split_ws) cudaFree(s->split_ws);
       if (s->sk_flags) cudaFree(s->sk_flags);
       for (uint8_t *nb : s->nibbles)
         if (nb) cudaFree(nb);
