@@ -357,6 +357,50 @@ __device__ __forceinline__ T no_threshold() {
   else return std::is_same<T, uint8_t>::value ? (T)0xff : (T)0x7f;
 }
 
+template <typename T>
+using Shuffled = typename std::conditional<std::is_same<T, float>::value, float, int>::type;  // a type to shuffle
+
+// At most 7 thresholds of a row, lane j of each 8 holding the j-th (past the
+// last the fill value), and what a search of them reads: every code of the row
+// costs LEVELS compares, the threshold of each picked by a shuffle of the
+// element's own index.
+template <typename T>
+struct RowThresholds {
+  Shuffled<T> tv, next, mid;
+  bool sorted;
+  __device__ __forceinline__ explicit RowThresholds(T t) {
+    tv = (Shuffled<T>)t;
+    next = __shfl_down_sync(kFull, tv, 1, 8);  // lane j: threshold j + 1
+    mid = __shfl_sync(kFull, tv, 3, 8);
+    sorted = __all_sync(kFull, (threadIdx.x & 7) == 7 || tv <= next);
+  }
+  template <int LEVELS>
+  __device__ __forceinline__ void search(const Shuffled<T> (&v)[4], uint32_t (&n)[4]) const {
+#pragma unroll
+    for (int i = 0; i < 4; i++) n[i] = LEVELS >= 3 && !(v[i] <= mid) ? 4u : 0u;
+    if (LEVELS >= 2) {
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (!(v[i] <= __shfl_sync(kFull, next, n[i], 8))) n[i] += 2u;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      if (!(v[i] <= __shfl_sync(kFull, tv, n[i], 8))) n[i] += 1u;
+  }
+  template <int LEVELS>
+  __device__ __forceinline__ uint32_t codes4(const Raw4<T> &x, int nthres) const {
+    Shuffled<T> v[4];
+    uint32_t n[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[i] = (Shuffled<T>)elem_of<T>(x, i);
+    search<LEVELS>(v, n);
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      if (std::is_same<T, float>::value) n[i] = min(n[i], (uint32_t)nthres);  // a NaN exceeds the fill value too
+    return pack4(n[0], n[1], n[2], n[3]);
+  }
+};
+
 // Four columns of one row, the row's thresholds in the 8 lanes of its chunk
 // (lane j holds threshold 8 k + j of block k, block 0 in t0; past the last the
 // fill value): one load and shuffles, where a load per threshold (each a line
@@ -373,7 +417,7 @@ __device__ __forceinline__ T no_threshold() {
 template <typename T, int LEVELS>
 __device__ __forceinline__ uint32_t row_threshold_codes4(const Raw4<T> &x, T t0, const T *__restrict__ thr, int nthres,
                                                          uint64_t rthr, uint64_t nrows, bool row, bool wanted) {
-  using S = typename std::conditional<std::is_same<T, float>::value, float, int>::type;  // a type to shuffle
+  using S = Shuffled<T>;
   constexpr int kLast = LEVELS == 4 ? 8 : (1 << LEVELS) - 1;  // thresholds of a block
   const int lane = threadIdx.x & 31, j = lane & 7;
   S v[4], tv = (S)t0;
@@ -382,24 +426,10 @@ __device__ __forceinline__ uint32_t row_threshold_codes4(const Raw4<T> &x, T t0,
   for (int i = 0; i < 4; i++) v[i] = (S)elem_of<T>(x, i);
   bool over[4] = {wanted, wanted, wanted, wanted};
   for (int k = 0;; k += 8) {
-    const S next = __shfl_down_sync(kFull, tv, 1, 8);  // lane j: threshold j + 1
+    const RowThresholds<T> block((T)tv);
     uint32_t n[4];
-    if (__all_sync(kFull, j == 7 || tv <= next)) {
-#pragma unroll
-      for (int i = 0; i < 4; i++) n[i] = 0u;
-      if (LEVELS >= 3) {
-        const S mid = __shfl_sync(kFull, tv, 3, 8);
-#pragma unroll
-        for (int i = 0; i < 4; i++) n[i] = v[i] <= mid ? 0u : 4u;
-      }
-      if (LEVELS >= 2) {
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-          if (!(v[i] <= __shfl_sync(kFull, next, n[i], 8))) n[i] += 2u;
-      }
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-        if (!(v[i] <= __shfl_sync(kFull, tv, n[i], 8))) n[i] += 1u;
+    if (block.sorted) {
+      block.template search<(LEVELS < 3 ? LEVELS : 3)>(v, n);
       if (LEVELS == 4) {  // a block of 8: past 7 of them, the last is left (below 7 the answer stands)
 #pragma unroll
         for (int i = 0; i < 4; i++)
@@ -487,58 +517,91 @@ __device__ __forceinline__ void pack_staged_unit(const PackJob &J, const T *__re
   const uint64_t total = J.nrows * J.ncols, e0 = b.r * J.ncols;
   const int bip = J.nbits == 1 && J.issigned;
   Raw4<T> x[8];
-  T t0[8];
-  uint32_t part = 0u;  // nibble s: the elements of load s that exist
-#pragma unroll
-  for (int s = 0; s < 8; s++) {
-    const Chunk c = unit_chunk(b, 4 * s + (lane >> 3), J.cpr, J.magic);
-    const uint32_t col = c.cc * 32 + 4 * j;
-    const bool row = c.dr < b.rows;
-    const uint32_t n = (row && col < ncols) ? min(4u, ncols - col) : 0u;
-    x[s] = load4<T, ALIGNED>((const T *)J.src, e0 + (uint64_t)c.dr * ncols + col, n, total);
-    if (QUANT) {
-      t0[s] = (row && (int)j < nthres) ? thr[(uint64_t)j * J.nrows + (uint32_t)b.r + c.dr] : no_threshold<T>();
-      part |= n << (4 * s);
-    }
-  }
   const uint32_t at = (lane >> 3) * 8;
-  if (QUANT) {
-    // the raw elements and first thresholds go through shared memory (the lane's own
-    // words), so that the search is a loop: unrolled over eight loads in registers
-    // it stalled on instruction fetch
-    Raw4<T> *rx = qs->raw[threadIdx.x >> 5][0] + lane;
-    T *rt = qs->thr[threadIdx.x >> 5][0] + lane;
+  const auto put = [&](int s, uint32_t w) { st[32 * s + at + (j ^ ((s & 1) << 2))] = w; };
+  if (ALIGNED && (!QUANT || (nthres > 0 && nthres < 8)) && b.rows && b.cc + 32 <= J.cpr &&
+      (b.cc + 32) * 32 <= ncols) {
+    // The whole unit lies in one row: element 128 s + 4 lane of it, one set of thresholds
+    const Raw4<T> *p = reinterpret_cast<const Raw4<T> *>((const T *)J.src + e0 + b.cc * 32 + 4 * lane);
+#pragma unroll
+    for (int s = 0; s < 8; s++) x[s] = p[32 * s];
+    if (QUANT) {
+      const T t = (int)j < nthres ? thr[(uint64_t)j * J.nrows + b.r] : no_threshold<T>();
+      auto search = [&](auto levels) {
+        const RowThresholds<T> r(t);
+        if (r.sorted) {
+#pragma unroll
+          for (int s = 0; s < 8; s++) put(s, r.template codes4<decltype(levels)::value>(x[s], nthres));
+        } else {
+#pragma unroll 1
+          for (int s = 0; s < 8; s++) {
+            Raw4<T> v = x[0];
+#pragma unroll
+            for (int i = 1; i < 8; i++) v = s == i ? x[i] : v;
+            put(s, row_threshold_codes4<T, decltype(levels)::value>(v, t, thr, nthres, b.r, J.nrows, true, true));
+          }
+        }
+      };
+      if (nthres == 1) search(std::integral_constant<int, 1>{});
+      else if (nthres <= 3) search(std::integral_constant<int, 2>{});
+      else search(std::integral_constant<int, 3>{});
+    } else {
+#pragma unroll
+      for (int s = 0; s < 8; s++) put(s, codes4<T>(x[s], bip, J.issigned, J.nbits));
+    }
+  } else {
+    T t0[8];
+    uint32_t part = 0u;  // nibble s: the elements of load s that exist
 #pragma unroll
     for (int s = 0; s < 8; s++) {
-      rx[32 * s] = x[s];
-      rt[32 * s] = t0[s];
-    }
-    auto codes = [&](auto scan) {
-#pragma unroll 1
-      for (int s = 0; s < 8; s++) {
-        const uint32_t n = (part >> (4 * s)) & 15u;
-        uint32_t w = scan(rx[32 * s], rt[32 * s], s, n != 0u);
-        if (n < 4) w &= (1u << (8 * n)) - 1u;  // the code of a 0 put past the row's end is no code
-        st[32 * s + at + (j ^ ((s & 1) << 2))] = w;
+      const Chunk c = unit_chunk(b, 4 * s + (lane >> 3), J.cpr, J.magic);
+      const uint32_t col = c.cc * 32 + 4 * j;
+      const bool row = c.dr < b.rows;
+      const uint32_t n = (row && col < ncols) ? min(4u, ncols - col) : 0u;
+      x[s] = load4<T, ALIGNED>((const T *)J.src, e0 + (uint64_t)c.dr * ncols + col, n, total);
+      if (QUANT) {
+        t0[s] = (row && (int)j < nthres) ? thr[(uint64_t)j * J.nrows + (uint32_t)b.r + c.dr] : no_threshold<T>();
+        part |= n << (4 * s);
       }
-    };
-    auto search = [&](auto levels) {
-      codes([&](const Raw4<T> &v, T t, int s, bool wanted) {
-        uint32_t dr = 0u;
-        if (decltype(levels)::value == 4) dr = unit_chunk(b, 4 * s + (lane >> 3), J.cpr, J.magic).dr;
-        return row_threshold_codes4<T, decltype(levels)::value>(v, t, thr, nthres, b.r + dr, J.nrows, dr < b.rows,
-                                                                wanted);
-      });
-    };
-    if (nthres == 0) codes([&](const Raw4<T> &v, T, int, bool) { return own_codes4<T>(v); });
-    else if (nthres == 1) search(std::integral_constant<int, 1>{});
-    else if (nthres <= 3) search(std::integral_constant<int, 2>{});
-    else if (nthres <= 7) search(std::integral_constant<int, 3>{});
-    else search(std::integral_constant<int, 4>{});
-  } else {
+    }
+    if (QUANT) {
+      // the raw elements and first thresholds go through shared memory (the lane's own
+      // words), so that the search is a loop: unrolled over eight loads in registers
+      // it stalled on instruction fetch
+      Raw4<T> *rx = qs->raw[threadIdx.x >> 5][0] + lane;
+      T *rt = qs->thr[threadIdx.x >> 5][0] + lane;
 #pragma unroll
-    for (int s = 0; s < 8; s++)
-      st[32 * s + at + (j ^ ((s & 1) << 2))] = codes4<T>(x[s], bip, J.issigned, J.nbits);
+      for (int s = 0; s < 8; s++) {
+        rx[32 * s] = x[s];
+        rt[32 * s] = t0[s];
+      }
+      auto codes = [&](auto scan) {
+#pragma unroll 1
+        for (int s = 0; s < 8; s++) {
+          const uint32_t n = (part >> (4 * s)) & 15u;
+          uint32_t w = scan(rx[32 * s], rt[32 * s], s, n != 0u);
+          if (n < 4) w &= (1u << (8 * n)) - 1u;  // the code of a 0 put past the row's end is no code
+          put(s, w);
+        }
+      };
+      auto search = [&](auto levels) {
+        codes([&](const Raw4<T> &v, T t, int s, bool wanted) {
+          uint32_t dr = 0u;
+          if (decltype(levels)::value == 4) dr = unit_chunk(b, 4 * s + (lane >> 3), J.cpr, J.magic).dr;
+          return row_threshold_codes4<T, decltype(levels)::value>(v, t, thr, nthres, b.r + dr, J.nrows, dr < b.rows,
+                                                                  wanted);
+        });
+      };
+      if (nthres == 0) codes([&](const Raw4<T> &v, T, int, bool) { return own_codes4<T>(v); });
+      else if (nthres == 1) search(std::integral_constant<int, 1>{});
+      else if (nthres <= 3) search(std::integral_constant<int, 2>{});
+      else if (nthres <= 7) search(std::integral_constant<int, 3>{});
+      else search(std::integral_constant<int, 4>{});
+    } else {
+#pragma unroll
+      for (int s = 0; s < 8; s++)
+        put(s, codes4<T>(x[s], bip, J.issigned, J.nbits));
+    }
   }
   __syncwarp();
   const uint32_t sw = ((lane >> 2) & 1u) << 2;

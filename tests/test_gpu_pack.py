@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 DTYPES = {"int8": np.int8, "uint8": np.uint8, "int16": np.int16, "int32": np.int32, "float32": np.float32}
 # row lengths: below, at and above a 4-element group, a 32-column chunk and a 1024-column unit
 SHAPES = [(1, 1), (3, 31), (5, 32), (2, 48), (67, 33), (64, 100), (9, 363), (130, 257), (33, 1024), (17, 1056),
-          (31, 2051), (259, 64)]
+          (31, 2051), (259, 64), (40, 2048), (5, 1028), (6, 1100), (24, 3072)]
 
 
 @pytest.fixture(scope="module", autouse=True)
