@@ -1234,19 +1234,20 @@ bool tc_map_u8(void *map, const uint8_t *base, uint64_t cols, uint64_t rows, uin
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Map of a nibble matrix (rows x cols codes, blocks of nibble_offset) as the
-// 4-D tensor [rows/16][cols/128][16][64] bytes; a box is 256 rows of one
-// 128-column chunk, 64-byte swizzled.
-bool tc_map_nibbles(void *map, const uint8_t *base, uint64_t cols, uint64_t rows) {
+// Map of a packed matrix (rows x cols 4-bit values, blocks of packed_offset) as
+// the 4-D tensor [rows/16][cols/128][16][128]; a box is 128 rows of one 128-column
+// chunk, which lands as the digits' boxes do, 128-byte swizzled, with each 16
+// values at the start of 16 bytes.
+bool tc_map_packed(void *map, const uint8_t *base, uint64_t cols, uint64_t rows) {
   EncodeTiledFn fn = encode_fn();
-  if (!fn || cols % 128 || rows % 256 || rows == 0) return false;
-  cuuint64_t dims[4] = {64, 16, cols / 128, rows / 16};
+  if (!fn || cols % 128 || rows % 128 || rows == 0) return false;
+  cuuint64_t dims[4] = {128, 16, cols / 128, rows / 16};
   cuuint64_t strides[3] = {64, 1024, (cols / 128) * 1024};
-  cuuint32_t box[4] = {64, 16, 1, 16};
+  cuuint32_t box[4] = {128, 16, 1, 8};
   cuuint32_t estr[4] = {1, 1, 1, 1};
-  return fn(reinterpret_cast<CUtensorMap *>(map), CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void *)base, dims, strides, box,
-            estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return fn(reinterpret_cast<CUtensorMap *>(map), CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 4, (void *)base, dims,
+            strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 void tc_digit_table(const Mat &m, uint32_t tab[4]) {
@@ -1337,11 +1338,11 @@ cudaError_t expand_side(gbs_ctx *c, int side, cudaStream_t s) {
   return e;
 }
 
-cudaError_t expand_nibble_side(gbs_ctx *c, int side, cudaStream_t s) {
-  cudaError_t e = ensure_nibble_buffer(c, side, &s);
+cudaError_t expand_packed_side(gbs_ctx *c, int side, cudaStream_t s) {
+  cudaError_t e = ensure_packed_buffer(c, side, &s);
   if (e != cudaSuccess) return e;
-  e = launch_expand(make_nibble_job(side ? c->rhs : c->lhs, c->nibbles[side]), s);
-  if (e == cudaSuccess) c->nibbles_valid[side] = true;
+  e = launch_expand(make_packed_job(side ? c->rhs : c->lhs, c->packed[side]), s);
+  if (e == cudaSuccess) c->packed_valid[side] = true;
   return e;
 }
 
@@ -1582,19 +1583,19 @@ bool pdl_for(cudaStream_t s) {
 
 cudaError_t launch_gemm_tc_hbm(gbs_ctx *c, cudaStream_t s, int bn_req) {
   const bool small = bn_req < 0 && (c->lhs.nrows < 256 || c->rhs.nrows < 256);
-  if (small && (c->plan1_ready || tcg_nibbles_mode() == 1)) {
-    // the nibble kernel forced on a side of fewer than 256 rows: a one-problem plan
+  if (small && (c->plan1_ready || tcg_packed_mode() == 1)) {
+    // packed plans forced on a side of fewer than 256 rows: a one-problem plan
     if (!c->plan1_ready) {
       if (!c->plan1) c->plan1 = new TcgPlan();
       gbs_ctx *one[1] = {c};
       if (tcg_plan_build(c->plan1, one, 1) != GBS_OK) return cudaErrorInvalidValue;
       c->plan1_ready = true;
     }
-    for (int side = 0; side < 2; side++) {  // the digit and nibble matrices the plan reads
+    for (int side = 0; side < 2; side++) {  // the digit and packed matrices the plan reads
       cudaError_t e = cudaSuccess;
       if (((c->plan1->sides[0] >> side) & 1) && !c->digits_valid[side]) e = expand_side(c, side, s);
-      if (e == cudaSuccess && ((c->plan1->sides[0] >> (2 + side)) & 1) && !c->nibbles_valid[side])
-        e = expand_nibble_side(c, side, s);
+      if (e == cudaSuccess && ((c->plan1->sides[0] >> (2 + side)) & 1) && !c->packed_valid[side])
+        e = expand_packed_side(c, side, s);
       if (e != cudaSuccess) return e;
     }
     uint32_t *err = tc_error_ptr();

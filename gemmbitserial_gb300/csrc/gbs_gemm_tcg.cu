@@ -17,14 +17,27 @@
 // the MMA-B operand; per problem the larger side is MMA-A ("swap" when that
 // is the rhs), so a problem with few lhs rows uses an MMA N as small as 16
 // instead of padding M to 128.
-//   warp 0     lane 0: TMA producer -- A box 128 x 128 bytes and B box
-//              bn x 128 bytes per stage, 128-byte swizzle, into a 4-slot ring
-//              that runs across tile boundaries
+//
+// Large groups read HBM once per element of the larger sides, so a "packed" plan
+// holds those that allow it as 4-bit floats (packed_offset): the TMA unpacks them
+// on the way into shared memory and the MMA takes them as they land there (e2m1
+// against the other side's e4m3), so nothing is decoded by threads.
+//
+//   warp 0     lane 0: TMA producer -- A box 128 x 128 values and B box
+//              bn x 128 bytes, 128-byte swizzle, one or two of each a stage,
+//              into a 4-slot ring that runs across tile boundaries
 //   warp 1     allocates all 512 TMEM columns (two 256-column accumulators);
-//              lane 0 issues 4 tcgen05.mma (K = 32) per stage and commits the
+//              lane 0 issues 4 or 8 tcgen05.mma (K = 32) per stage and commits the
 //              accumulator of each tile
 //   warps 2-5  epilogue of tile j while the MMAs of tile j+1 run: tcgen05.ld
-//              32 lanes x 16 columns, fp32 -> int32, stores into res[n*M + m]
+//              32 lanes x 32 columns, fp32 -> int32, stores into res[n*M + m]
+//
+// Warps 0 and 1 walk the stages whole and issue from an elected lane: from lane 0
+// of a diverged warp an MMA took 47-76 ns to issue, so even the narrowest stage
+// took 0.27 us; elected, eight MMAs of N = 16 take 34 ns each, of 256 66 (the
+// rate of the tensor cores).  The 397 tensor-core problems of the 512-problem mix:
+// 589 us on digits, 448 packed (2.3 GB of operands, 350 us at the copy rate); a
+// kernel whose warps decoded 4-bit codes into digits took 579.
 // Every mbarrier wait is bounded; on timeout the CTA sets a bit in the
 // caller's error word, stops issuing, drains what it issued and frees TMEM.
 #include <algorithm>
@@ -39,13 +52,19 @@
 namespace gbs {
 namespace {
 
-constexpr int kTgStages = 4;
-constexpr uint32_t kTgABytes = 128 * 128;           // MMA-A box: 128 rows x 128 digits
-constexpr uint32_t kTgSlotBytes = kTgABytes + 256 * 128;  // + MMA-B box of up to 256 rows
+constexpr uint32_t kTgStages = 4;
+constexpr uint32_t kTgABytes = 128 * 128;  // MMA-A chunk: 128 rows x 128 digits (packed values in 16-byte groups)
+// A stage is one 128-column chunk of MMA-A and up to 256 rows of MMA-B, or two
+// chunks of each where MMA-B has at most kTgTwoRows rows: as many bytes, and half
+// as many barriers for the MMAs of narrow tiles to wait on.
+constexpr uint32_t kTgSlotBytes = kTgABytes + 256 * 128;
+constexpr uint32_t kTgTwoRows = 64;
+static_assert(2 * (kTgABytes + kTgTwoRows * 128) <= kTgSlotBytes, "two chunks must fit a slot");
 constexpr int kTgThreads = 192;
 constexpr uint32_t kTgAccCols = 256;
-
-constexpr size_t tcg_smem_bytes() { return 1024 + kTgStages * kTgSlotBytes + 8 * (2 * kTgStages + 5) + 16; }
+constexpr uint32_t kTgBarBytes = 128;
+static_assert(8 * (2 * kTgStages + 5) + 8 <= kTgBarBytes, "barriers, TMEM address, abort flag");
+constexpr size_t tcg_smem_bytes() { return 1024 + kTgStages * kTgSlotBytes + kTgBarBytes + 4 * 32 * 33 * 4; }
 
 // Tile j of CTA b among G CTAs: rounds of G consecutive table entries, every
 // other round walked backwards, so each CTA's share of a cost-sorted table
@@ -56,8 +75,66 @@ __device__ __forceinline__ uint32_t snake_tile(uint32_t j, uint32_t b, uint32_t 
 
 __device__ __forceinline__ bool tile_ok(const TcgTile &t, const TcgProblem &P, uint32_t nprob) {
   return t.p < nprob && P.bn >= 16 && P.bn <= 256 && (P.bn & 15u) == 0 && P.nk > 0 &&
-         (t.r + 1) * 128u <= P.a_rows && (t.c + 1) * P.bn <= P.b_rows;
+         (t.r + 1) * 128u <= P.a_rows && (t.c + 1) * P.bn <= P.b_rows && P.a_bytes <= kTgABytes;
 }
+
+// 32 rows (n) from row0 x up to 32 columns (m) from c0 of a swapped tile, staged as
+// [32][33]: the warp walks the block flat, so what a result row has of it is
+// written by neighbouring lanes.  With each lane on a row of its own a store
+// touched 32 sectors, and the epilogue took a fifth of a large group's time.
+__device__ __forceinline__ void store_staged(const TcgProblem &P, uint32_t row0, uint32_t c0, uint32_t left,
+                                             const int32_t *stage, int lane) {
+  if (row0 >= P.N || c0 >= P.M) return;
+  const uint32_t nc = min(32u, min(left, P.M - c0)), nr = min(32u, P.N - row0);
+  int32_t *dst = P.C + (uint64_t)row0 * P.M + c0;
+  if (nc == 32) {
+#pragma unroll 8
+    for (uint32_t r = 0; r < nr; r++) dst[(uint64_t)r * P.M + lane] = stage[r * 33 + lane];
+    return;
+  }
+  const uint32_t magic = 65536u / nc + 1;  // e / nc for e < 1024, nc < 32
+#pragma unroll 4
+  for (uint32_t e = lane; e < nr * nc; e += 32) {
+    const uint32_t r = (e * magic) >> 16, c = e - r * nc;
+    dst[(uint64_t)r * P.M + c] = stage[r * 33 + c];
+  }
+}
+
+// The tiles of one CTA in turn, each with its problem.  The entry of the next tile
+// is asked for when a tile begins and its problem once the tile is under way, so
+// neither load's latency stands between two tiles.
+struct TileWalk {
+  const TcgProblem *probs;
+  const TcgTile *tiles;
+  uint32_t ntiles, nprob, G, b;
+  uint32_t j;
+  bool live, ok, next_live;  // a tile is there; it can be run
+  TcgTile tl, ntl;
+  TcgProblem P, nP;
+
+  __device__ __forceinline__ void fetch_entry(uint32_t at) {
+    const uint32_t t = snake_tile(at, b, G);
+    next_live = t < ntiles;
+    if (next_live) ntl = tiles[t];
+  }
+  __device__ __forceinline__ void fetch_problem() {
+    if (next_live && ntl.p < nprob) nP = probs[ntl.p];
+  }
+  __device__ __forceinline__ void advance() {  // to the fetched tile
+    live = next_live;
+    tl = ntl;
+    P = nP;
+    ok = live && tl.p < nprob && tile_ok(tl, P, nprob);
+    j++;
+    fetch_entry(j);
+  }
+  __device__ __forceinline__ void start() {
+    j = 0;
+    fetch_entry(0);
+    fetch_problem();
+    advance();
+  }
+};
 
 __global__ void __launch_bounds__(kTgThreads, 1)
     gemm_tcg_kernel(const TcgProblem *__restrict__ probs, const CUtensorMap *__restrict__ maps,
@@ -71,11 +148,11 @@ __global__ void __launch_bounds__(kTgThreads, 1)
   const uint32_t acc_empty = acc_full + 16, mma_done = acc_empty + 16;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kTgStages + 5);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-  const uint32_t G = gridDim.x, b = blockIdx.x;
+  TileWalk w{probs, tiles, ntiles, nprob, gridDim.x, blockIdx.x};
   griddep_launch_dependents();
 
   if (tid == 0) {
-    for (int i = 0; i < kTgStages; i++) {
+    for (uint32_t i = 0; i < kTgStages; i++) {
       mbar_init(full + 8 * i, 1);
       mbar_init(empty + 8 * i, 1);
     }
@@ -99,87 +176,112 @@ __global__ void __launch_bounds__(kTgThreads, 1)
   griddep_wait();  // operands and results belong to earlier kernels until here
 
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t it = 0;  // stage loads issued
-      bool stop = false;
-      for (uint32_t j = 0; !stop; j++) {
-        const uint32_t t = snake_tile(j, b, G);
-        if (t >= ntiles) break;
-        const TcgTile tl = tiles[t];
-        if (tl.p >= nprob) continue;
-        const TcgProblem P = probs[tl.p];
-        if (!tile_ok(tl, P, nprob)) continue;
-        const CUtensorMap *ma = maps + 2 * tl.p, *mb = ma + 1;
-        // the maps were written by a host copy: order them for the tensor-map proxy
-        asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(ma) : "memory");
-        asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(mb) : "memory");
-        const uint32_t bytes = kTgABytes + P.bn * 128u;
-        for (uint32_t k = 0; k < P.nk; k++, it++) {
-          const uint32_t s = it % kTgStages, use = it / kTgStages;
-          if (use > 0 && !mbar_wait_err(empty + 8 * s, (use - 1) & 1, abort_flag, err)) {
-            stop = true;
-            break;
+    uint32_t it = 0;  // stage loads issued
+    bool stop = false;
+    // the maps were written by a host copy: order them for the tensor-map proxy
+    auto acquire_maps = [&](uint32_t p) {
+      const CUtensorMap *m = maps + 2 * p;
+      asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(m) : "memory");
+      asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(m + 1) : "memory");
+      asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
+      asm volatile("prefetch.tensormap [%0];" ::"l"(m + 1) : "memory");
+    };
+    w.start();
+    if (w.ok) acquire_maps(w.tl.p);
+    for (; w.live && !stop; w.advance()) {
+      if (!w.ok) {
+        w.fetch_problem();
+        if (w.next_live && w.ntl.p < nprob) acquire_maps(w.ntl.p);
+        continue;
+      }
+      const CUtensorMap *ma = maps + 2 * w.tl.p, *mb = ma + 1;
+      const uint32_t kb = w.P.bn <= kTgTwoRows ? 2u : 1u, nk = w.P.nk, bn = w.P.bn, bytes = w.P.a_bytes + bn * 128u;
+      const uint32_t arow = w.tl.r * 128, brow = w.tl.c * bn;
+      for (uint32_t k = 0; k < nk; k += kb, it++) {
+        const uint32_t s = it % kTgStages, use = it / kTgStages;
+        if (use > 0 && !__all_sync(~0u, mbar_wait_err(empty + 8 * s, (use - 1) & 1, abort_flag, err))) {
+          stop = true;
+          break;
+        }
+        if (elect_one()) {
+          const bool two = kb == 2 && k + 1 < nk;
+          mbar_expect_tx(full + 8 * s, two ? 2 * bytes : bytes);
+          const uint32_t dst = smem_u32(smem + s * kTgSlotBytes), dstb = dst + kb * kTgABytes;
+          tma_load_digits(dst, ma, (int)k, arow, full + 8 * s);
+          tma_load_digits(dstb, mb, (int)k, brow, full + 8 * s);
+          if (two) {
+            tma_load_digits(dst + kTgABytes, ma, (int)k + 1, arow, full + 8 * s);
+            tma_load_digits(dstb + bn * 128u, mb, (int)k + 1, brow, full + 8 * s);
           }
-          mbar_expect_tx(full + 8 * s, bytes);
-          const uint32_t dst = smem_u32(smem + s * kTgSlotBytes);
-          tma_load_digits(dst, ma, (int)k, tl.r * 128, full + 8 * s);
-          tma_load_digits(dst + kTgABytes, mb, (int)k, tl.c * P.bn, full + 8 * s);
+        }
+        __syncwarp();
+        if (k == 0) {  // the first stage is on its way: the next tile's problem and maps
+          w.fetch_problem();
+          if (w.next_live && w.ntl.p < nprob) acquire_maps(w.ntl.p);
         }
       }
-      if (*abort_flag)
-        for (uint32_t q = (it > (uint32_t)kTgStages ? it - kTgStages : 0); q < it; q++)
-          mbar_drain_err(full + 8 * (q % kTgStages), (q / kTgStages) & 1, err);
     }
+    if (lane == 0 && *abort_flag)
+      for (uint32_t q = (it > kTgStages ? it - kTgStages : 0); q < it; q++)
+        mbar_drain_err(full + 8 * (q % kTgStages), (q / kTgStages) & 1, err);
   } else if (warp == 1) {
-    if (lane == 0) {
-      uint32_t it = 0, jt = 0;  // stages consumed, tiles accumulated
-      bool ok = true;
-      for (uint32_t j = 0; ok; j++) {
-        const uint32_t t = snake_tile(j, b, G);
-        if (t >= ntiles) break;
-        const TcgTile tl = tiles[t];
-        if (tl.p >= nprob) continue;
-        const TcgProblem P = probs[tl.p];
-        if (!tile_ok(tl, P, nprob)) continue;
-        const uint32_t a = jt & 1, use = jt >> 1;
-        if (use > 0 && !mbar_wait_err(acc_empty + 8 * a, (use - 1) & 1, abort_flag, err)) {
+    uint32_t it = 0, jt = 0;  // stages consumed, tiles accumulated
+    bool ok = true;
+    for (w.start(); w.live && ok; w.advance()) {
+      if (!w.ok) {
+        w.fetch_problem();
+        continue;
+      }
+      const uint32_t a = jt & 1, use = jt >> 1;
+      if (use > 0 && !__all_sync(~0u, mbar_wait_err(acc_empty + 8 * a, (use - 1) & 1, abort_flag, err))) {
+        ok = false;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const uint32_t d = tmem + a * kTgAccCols;
+      const uint32_t kb = w.P.bn <= kTgTwoRows ? 2u : 1u, nk = w.P.nk, bn = w.P.bn, idesc = w.P.idesc;
+      for (uint32_t k = 0; k < nk; k += kb, it++) {
+        const uint32_t s = it % kTgStages;
+        if (!__all_sync(~0u, mbar_wait_err(full + 8 * s, (it / kTgStages) & 1, abort_flag, err))) {
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t d = tmem + a * kTgAccCols;
-        for (uint32_t k = 0; k < P.nk; k++, it++) {
-          const uint32_t s = it % kTgStages;
-          if (!mbar_wait_err(full + 8 * s, (it / kTgStages) & 1, abort_flag, err)) {
-            ok = false;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;");
-          const uint32_t base = smem_u32(smem + s * kTgSlotBytes);
+        const uint32_t base = smem_u32(smem + s * kTgSlotBytes);
+        const uint64_t da = sw128_desc(base), db = sw128_desc(base + kb * kTgABytes);
+        if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < 4; kk++)
-            mma_f8(d, sw128_desc(base + kk * 32), sw128_desc(base + kTgABytes + kk * 32), P.idesc, (k | kk) != 0);
+          for (int kk = 0; kk < 4; kk++)  // the address field counts 16 bytes
+            mma_f8(d, da + 2 * kk, db + 2 * kk, idesc, (k | kk) != 0);
+          if (kb == 2 && k + 1 < nk) {
+            const uint64_t da1 = da + kTgABytes / 16, db1 = db + bn * 8;
+#pragma unroll
+            for (int kk = 0; kk < 4; kk++) mma_f8(d, da1 + 2 * kk, db1 + 2 * kk, idesc, 1);
+          }
           mma_commit(empty + 8 * s);
         }
-        if (!ok) break;
-        mma_commit(acc_full + 8 * a);
-        jt++;
+        __syncwarp();
+        if (k == 0) w.fetch_problem();
       }
-      if (!ok) {  // issued MMAs finish before TMEM is freed
-        mma_commit(mma_done);
-        mbar_drain_err(mma_done, 0, err);
-      }
+      if (!ok) break;
+      if (elect_one()) mma_commit(acc_full + 8 * a);
+      __syncwarp();
+      jt++;
+    }
+    if (!ok) {  // issued MMAs finish before TMEM is freed
+      if (elect_one()) mma_commit(mma_done);
+      __syncwarp();
+      mbar_drain_err(mma_done, 0, err);
     }
   } else {
     const int q = warp & 3;  // TMEM lanes 32q .. 32q+31 belong to this warp
+    int32_t *stage = reinterpret_cast<int32_t *>(smem + kTgStages * kTgSlotBytes + kTgBarBytes) + (warp - 2) * 32 * 33;
     uint32_t jt = 0;
-    for (uint32_t j = 0;; j++) {
-      const uint32_t t = snake_tile(j, b, G);
-      if (t >= ntiles) break;
-      const TcgTile tl = tiles[t];
-      TcgProblem P;
-      if (tl.p < nprob) P = probs[tl.p];
-      if (tl.p >= nprob || !tile_ok(tl, P, nprob)) {
+    for (w.start(); w.live; w.advance()) {
+      w.fetch_problem();
+      const TcgTile tl = w.tl;
+      TcgProblem P = w.P;
+      if (!w.ok) {
         if (warp == 2 && lane == 0) atomicOr(err, 4u);
         continue;
       }
@@ -187,34 +289,26 @@ __global__ void __launch_bounds__(kTgThreads, 1)
       const uint32_t a = jt & 1, use = jt >> 1;
       if (!__all_sync(0xffffffffu, mbar_wait_err(acc_full + 8 * a, use & 1, abort_flag, err))) break;
       asm volatile("tcgen05.fence::after_thread_sync;");
-      const uint32_t row = tl.r * 128u + (uint32_t)(q * 32 + lane);
+      const uint32_t row0 = tl.r * 128u + (uint32_t)(q * 32);
       const uint32_t taddr = tmem + a * kTgAccCols + ((uint32_t)(q * 32) << 16);
 #pragma unroll 1
-      for (uint32_t col = 0; col < P.bn; col += 16) {
-        uint32_t v[16];
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-            : "r"(taddr + col));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        int32_t o[16];
-#pragma unroll
-        for (int i = 0; i < 16; i++) o[i] = __float2int_rn(__uint_as_float(v[i]));
+      for (uint32_t col = 0; col < P.bn; col += 32) {
+        uint32_t v[32];
+        tmem_ld32(taddr + col, v);
+        tmem_wait_ld(v);
         const uint32_t c0 = tl.c * P.bn + col;
         if (!P.swap) {  // row = m, column = n: lanes write 32 consecutive m of one n
-          store_result_cols<16>(P.C, P.M, P.N, row, c0, o);
-        } else if (row < P.N) {  // row = n, column = m: each lane writes a run of its result row
-          int32_t *dst = P.C + (uint64_t)row * P.M + c0;
-          if ((P.M & 3u) == 0) {
+          int32_t o[2][16];
 #pragma unroll
-            for (int i = 0; i < 16; i += 4)
-              if (c0 + i < P.M) *reinterpret_cast<int4 *>(dst + i) = make_int4(o[i], o[i + 1], o[i + 2], o[i + 3]);
-          } else {
+          for (int i = 0; i < 32; i++) o[i >> 4][i & 15] = __float2int_rn(__uint_as_float(v[i]) * P.scale);
+          store_result_cols<16>(P.C, P.M, P.N, row0 + lane, c0, o[0]);
+          if (col + 16 < P.bn) store_result_cols<16>(P.C, P.M, P.N, row0 + lane, c0 + 16, o[1]);
+        } else {  // row = n, column = m
+          __syncwarp();
 #pragma unroll
-            for (int i = 0; i < 16; i++)
-              if (c0 + i < P.M) dst[i] = o[i];
-          }
+          for (int i = 0; i < 32; i++) stage[lane * 33 + i] = __float2int_rn(__uint_as_float(v[i]) * P.scale);
+          __syncwarp();
+          store_staged(P, row0, c0, P.bn - col, stage, lane);
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;");
@@ -259,30 +353,23 @@ __device__ __forceinline__ void expand_chunk(const ExpandJob &j, uint32_t r, uin
   *reinterpret_cast<uint4 *>(j.digits + digit_offset(r, col0, j.dcols)) = make_uint4(q[0], q[1], q[2], q[3]);
 }
 
-// One thread writes 32 codes (one 16-byte store) of one row of a nibble
-// matrix: the codes of 4 columns as bytes (plane p's nibble spread to bit p
-// of each byte), then two bytes' codes into one (even column low).
+// One thread writes 32 values of one row of a packed matrix: the codes of 4
+// columns as bytes (plane p's 4 bits spread to bit p of each byte), packed.
 template <int CNT>
-__device__ __forceinline__ void expand_nibble_chunk(const ExpandJob &j, uint32_t r, uint32_t col0) {
+__device__ __forceinline__ void expand_packed_chunk(const ExpandJob &j, uint32_t r, uint32_t col0) {
   const uint64_t w = col0 >> 6;
   const int sh = (int)(col0 & 63);
   uint32_t pw[CNT];
 #pragma unroll
   for (int p = 0; p < CNT; p++) pw[p] = (uint32_t)(j.planes[(p * j.nrows_a + r) * j.wpr + w] >> sh);
-  uint32_t o[4];
+  uint32_t c[8];
 #pragma unroll
-  for (int i = 0; i < 4; i++) {  // columns 8i .. 8i + 7
-    uint32_t t[2];
+  for (int i = 0; i < 8; i++) {  // columns 4i .. 4i + 3
+    c[i] = 0;
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      uint32_t c = 0;
-#pragma unroll
-      for (int p = 0; p < CNT; p++) c |= (bfe4(pw[p], 8 * i + 4 * h) * (0x00204081u << p)) & (0x01010101u << p);
-      t[h] = c | (c >> 4);  // bytes 0 and 2: code pairs (even column low)
-    }
-    o[i] = __byte_perm(t[0], t[1], 0x6420u);
+    for (int p = 0; p < CNT; p++) c[i] |= (bfe4(pw[p], 4 * i) * (0x00204081u << p)) & (0x01010101u << p);
   }
-  *reinterpret_cast<uint4 *>(j.digits + nibble_offset(r, col0, j.dcols)) = make_uint4(o[0], o[1], o[2], o[3]);
+  store_packed32(j.digits, r, col0, j.dcols, CNT, (int)j.pform, c);
 }
 
 __device__ __forceinline__ void expand_thread(const ExpandJob &j, uint64_t local) {
@@ -295,13 +382,12 @@ __device__ __forceinline__ void expand_thread(const ExpandJob &j, uint64_t local
     r = (uint32_t)(local / j.chunks);
     col0 = (uint32_t)(local % j.chunks) * 16u;
   }
-  if (j.nib) {
-    col0 *= 2;  // 32 codes per thread
+  if (j.pform) {
+    col0 *= 2;  // 32 values per thread
     switch (j.nbits) {
-      case 1: expand_nibble_chunk<1>(j, r, col0); break;
-      case 2: expand_nibble_chunk<2>(j, r, col0); break;
-      case 3: expand_nibble_chunk<3>(j, r, col0); break;
-      default: expand_nibble_chunk<4>(j, r, col0); break;
+      case 1: expand_packed_chunk<1>(j, r, col0); break;
+      case 2: expand_packed_chunk<2>(j, r, col0); break;
+      default: expand_packed_chunk<3>(j, r, col0); break;
     }
     return;
   }
@@ -321,7 +407,6 @@ __global__ void __launch_bounds__(256) expand_one_kernel(const ExpandJob job) {
 
 // Every job's thread range is a multiple of 256, so all threads of a block
 // belong to one job and the job search below is uniform within the block.
-
 __global__ void __launch_bounds__(256) expand_grouped_kernel(const ExpandJob *__restrict__ jobs, int njobs,
                                                              uint64_t total) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -369,9 +454,9 @@ ExpandJob make_expand_job(const Mat &m, uint8_t *digits) {
   return j;
 }
 
-ExpandJob make_nibble_job(const Mat &m, uint8_t *nibbles) {
-  ExpandJob j = make_expand_job(m, nibbles);
-  j.nib = 1;
+ExpandJob make_packed_job(const Mat &m, uint8_t *packed) {
+  ExpandJob j = make_expand_job(m, packed);
+  j.pform = (uint32_t)m.packed_form();
   j.chunks = (uint32_t)((m.ncols + 31) / 32);
   return j;
 }
@@ -419,13 +504,14 @@ cudaError_t ensure_digit_buffer(gbs_ctx *c, int side, const cudaStream_t *order)
   return e;
 }
 
-// Nibble matrix [drows][dcols / 2] of one side, allocated zeroed on first use.
-cudaError_t ensure_nibble_buffer(gbs_ctx *c, int side, const cudaStream_t *order) {
-  if (c->nibbles[side]) return cudaSuccess;
+// Packed matrix of one side, allocated zeroed on first use.
+cudaError_t ensure_packed_buffer(gbs_ctx *c, int side, const cudaStream_t *order) {
+  if (c->packed[side]) return cudaSuccess;
   const Mat &m = side ? c->rhs : c->lhs;
-  cudaError_t e = alloc_zeroed((void **)&c->nibbles[side], std::max<size_t>(m.drows * m.dcols / 2, 16), order);
+  cudaError_t e = alloc_zeroed((void **)&c->packed[side],
+                               std::max<size_t>(m.drows * m.dcols / 2, 16), order);
   c->plan1_ready = false;
-  c->nibbles_valid[side] = false;
+  c->packed_valid[side] = false;
   return e;
 }
 
@@ -449,11 +535,10 @@ void tcg_plan_free(TcgPlan *p) {
   *p = TcgPlan();
 }
 
-// GBS_TCG_NIBBLES in the environment when a plan is built: 0 keeps it on the
-// digit kernel, 1 puts it on the nibble kernel; unset, the estimate below
-// chooses for groups, and single contexts run on the digits their imports
-// write.  Returns 0, 1 or -1 (choose).
-int tcg_nibbles_mode() {
+// GBS_TCG_NIBBLES in the environment when a plan is built: 0 makes it a digit
+// plan, 1 a packed one; unset, the estimate below chooses for groups, and single
+// contexts run on the digits their imports write.  Returns 0, 1 or -1 (choose).
+int tcg_packed_mode() {
   const char *v = getenv("GBS_TCG_NIBBLES");
   if (v && v[0] == '0') return 0;
   if (v && v[0] == '1') return 1;
@@ -462,50 +547,43 @@ int tcg_nibbles_mode() {
 
 namespace {
 
-// Which persistent kernel serves a plan faster, by an estimate of its
-// critical path.  The nibble kernel reads half a byte per element of each
-// problem's larger side where the digit kernel reads one, but it cuts that
-// side into 256-row tiles (half as many as the digit kernel's 128-row tiles),
-// and its stages move more shared memory (nibbles in, decoded digits out, a
-// 128-row MMA operand however few rows the smaller side has).  Per 128-digit
-// K stage a digit tile costs the longer of its bytes at ~100 GB/s into one SM
-// and its four MMAs (M = 128: ~37 ns up to N = 128, ~68 ns at N = 256), a
-// nibble tile ~0.7 us; the plan costs the longest of its tiles spread over
-// the SMs they can occupy, its largest tile, and its HBM bytes (larger side
-// once, smaller side once, results) at ~5 TB/s.  These constants are fitted
-// to GB300 timings of both kernels on groups of 1 to 397 problems, where the
-// estimate picks the faster kernel every time: groups of about 64 problems or
-// more are HBM-bound and take the nibbles; fewer leave SMs idle and take the
-// digit kernel's finer, cheaper tiles.
-bool plan_prefers_nibbles(gbs_ctx *const *ctxs, int n) {
+// Whether a plan runs faster with its problems' larger sides packed, by an
+// estimate of its critical path: a chunk's boxes enter an SM at 105 bytes/ns (the
+// unpacked side of the TMA, so packing does not help there) while its four MMAs
+// take 0.15-0.27 us, and all tiles together stream their operands at 6 TB/s.
+// Packing pays where HBM sets the pace.  Measured on the tensor cores alone,
+// digits / packed: 4 problems of the 512-problem mix 15.3 / 15.4 us, 16 of them
+// 34.8 / 23.8, 64 103 / 78, all 397 589 / 448; one of 16 x 8192 x 20000 40 / 28,
+// of 128 x 4096 x 20000 28.1 / 27.5, of 256 x 9216 x 4096 19.9 / 20.1.
+bool plan_prefers_packed(gbs_ctx *const *ctxs, int n) {
   const double sms = (double)std::max(1, sm_count());
   double tiles[2] = {0, 0}, work[2] = {0, 0}, longest[2] = {0, 0}, hbm[2] = {0, 0};
   auto mma_ns = [](double bn) { return bn <= 128 ? 37.0 : 37.0 + (bn - 128) * (31.0 / 128); };
   for (int i = 0; i < n; i++) {
     const Mat &L = ctxs[i]->lhs, &R = ctxs[i]->rhs;
-    const double small = (double)std::min(L.nrows, R.nrows), large = (double)std::max(L.nrows, R.nrows);
+    const Mat &A = L.nrows < R.nrows ? R : L;
+    const double small = (double)std::min(L.nrows, R.nrows), large = (double)A.nrows;
     const double nk = (double)((L.ncols + 127) / 128), K = nk * 128;
     if (small == 0 || nk == 0) continue;
     for (int k = 0; k < 2; k++) {
-      const double bn = k ? 256 : std::min(256.0, std::ceil(small / 16) * 16);
-      const double nt = k ? std::ceil(small / 128) * std::ceil(large / 256)
-                          : std::ceil(large / 128) * std::ceil(small / bn);
-      const double t = nk * (k ? 700.0 : std::max((128 * 128 + bn * 128) / 100.0, 4 * mma_ns(bn)));  // ns
+      const double bn = std::min(256.0, std::ceil(small / 16) * 16);
+      const double nt = std::ceil(large / 128) * std::ceil(small / bn);
+      const double t = nk * std::max((128 * 128 + bn * 128) / 105.0, 4 * mma_ns(bn));  // ns
       tiles[k] += nt;
       work[k] += nt * t;
       longest[k] = std::max(longest[k], t);
-      hbm[k] += (k ? large * K / 2 : large * K) + small * K + 4 * small * large;
+      hbm[k] += large * K * (k && A.packable() ? 0.5 : 1.0) + small * K + 4 * small * large;
     }
   }
   double est[2];
   for (int k = 0; k < 2; k++)
-    est[k] = std::max({tiles[k] > 0 ? work[k] / std::min(tiles[k], sms) : 0.0, longest[k], hbm[k] / 5000.0});
-  return est[1] < est[0];
+    est[k] = std::max({tiles[k] > 0 ? work[k] / std::min(tiles[k], sms) : 0.0, longest[k], hbm[k] / 6000.0});
+  return est[1] < 0.95 * est[0];
 }
 
 }  // namespace
 
-// MMA N (tile width over the smaller side) of every problem of a digit plan:
+// MMA N (tile width over the smaller side) of every problem of a plan:
 // the whole smaller side up to 256 rows; while the plan's tiles leave SMs idle,
 // the problem with the longest tiles gets narrower ones (a power of two: the
 // padded rows are whole multiples).  CaffeNet's five GEMMs had 38 tiles, the
@@ -542,16 +620,16 @@ static std::vector<uint32_t> tile_widths(gbs_ctx *const *ctxs, int n) {
 
 int tcg_plan_build(TcgPlan *plan, gbs_ctx *const *ctxs, int n) {
   tcg_plan_free(plan);
-  const int mode = tcg_nibbles_mode();
-  const bool nib = mode < 0 ? plan_prefers_nibbles(ctxs, n) : mode == 1;
-  plan->nibbles = nib;
+  const int mode = tcg_packed_mode();
+  const bool packed = mode < 0 ? plan_prefers_packed(ctxs, n) : mode == 1;
+  plan->packed = packed;
   std::vector<TcgProblem> probs;
   std::vector<CUtensorMap> maps;
   std::vector<TcgTile> tiles;
   std::vector<uint64_t> cost;
   std::vector<ExpandJob> jobs;
   uint64_t threads = 0;
-  const std::vector<uint32_t> widths = nib ? std::vector<uint32_t>() : tile_widths(ctxs, n);
+  const std::vector<uint32_t> widths = tile_widths(ctxs, n);
   for (int i = 0; i < n; i++) {
     gbs_ctx *c = ctxs[i];
     const Mat &L = c->lhs, &R = c->rhs;
@@ -560,17 +638,17 @@ int tcg_plan_build(TcgPlan *plan, gbs_ctx *const *ctxs, int n) {
     P.C = c->res;
     P.M = (uint32_t)L.nrows;
     P.N = (uint32_t)R.nrows;
-    // digit kernel: the larger side is MMA-A; nibble kernel: the smaller side
-    P.swap = nib ? (R.nrows < L.nrows ? 1u : 0u) : (L.nrows < R.nrows ? 1u : 0u);
+    P.swap = L.nrows < R.nrows ? 1u : 0u;        // the larger side is MMA-A
     const int sa = P.swap ? 1 : 0, sb = 1 - sa;  // sides of MMA-A and MMA-B
-    const uint8_t sides = nib ? (uint8_t)((1u << sa) | (4u << sb)) : (uint8_t)3;
+    const bool pa = packed && (sa ? R : L).packable();
+    const uint8_t sides = pa ? (uint8_t)((4u << sa) | (1u << sb)) : (uint8_t)3;
     for (int side = 0; side < 2; side++) {
       cudaError_t e = cudaSuccess;
       if ((sides >> side) & 1) e = ensure_digit_buffer(c, side);
-      if (e == cudaSuccess && ((sides >> (2 + side)) & 1)) e = ensure_nibble_buffer(c, side);
+      if (e == cudaSuccess && ((sides >> (2 + side)) & 1)) e = ensure_packed_buffer(c, side);
       if (e != cudaSuccess) {
         cudaGetLastError();
-        return fail(GBS_ENOMEM, "tensor-core plan: digit or nibble matrix allocation failed");
+        return fail(GBS_ENOMEM, "tensor-core plan: digit or packed matrix allocation failed");
       }
     }
     plan->ctxs.push_back(c);
@@ -580,30 +658,21 @@ int tcg_plan_build(TcgPlan *plan, gbs_ctx *const *ctxs, int n) {
     P.b_rows = (uint32_t)MB.drows;
     P.nk = (uint32_t)((L.ncols + 127) / 128);
     CUtensorMap m2[2];
-    uint32_t rt, ct;
-    if (!nib) {
-      P.bn = widths[i];
-      P.idesc = (1u << 4) | ((P.bn >> 3) << 17) | ((128u >> 4) << 24);
-      if (!tc_map_u8(&m2[0], c->digits[sa], MA.dcols, MA.drows, 128) ||
-          !tc_map_u8(&m2[1], c->digits[sb], MB.dcols, MB.drows, P.bn))
-        return fail(GBS_EUNSUPPORTED, "tensor-core plan: tensor map encoding failed");
-      rt = (uint32_t)((MA.nrows + 127) / 128);
-      ct = (uint32_t)((MB.nrows + P.bn - 1) / P.bn);
+    P.bn = widths[i];
+    P.idesc = (1u << 4) | ((P.bn >> 3) << 17) | ((128u >> 4) << 24);  // fp32 += e4m3 x e4m3
+    P.a_bytes = kTgABytes;
+    P.scale = 1.f;
+    bool ok = tc_map_u8(&m2[1], c->digits[sb], MB.dcols, MB.drows, P.bn);
+    if (pa) {
+      P.idesc |= 5u << 7;  // MMA-A: e2m1
+      P.a_bytes = kTgABytes / 2;
+      P.scale = 2.f;
+      ok = ok && tc_map_packed(&m2[0], c->packed[sa], MA.dcols, MA.drows);
     } else {
-      P.bn = 256;
-      P.idesc = (1u << 4) | ((256u >> 3) << 17) | ((128u >> 4) << 24);
-      P.w4 = MB.nbits > 3 ? 1u : 0u;
-      tc_digit_table(MB, P.tab);
-      // a smaller side of at most 128 rows loads only its rows (16-row blocks) into the
-      // 128-row MMA-A slot: the slot's other rows feed accumulator lanes no store reads
-      const uint32_t a_box = MA.nrows <= 128 ? (uint32_t)std::max<uint64_t>(16, (MA.nrows + 15) / 16 * 16) : 128u;
-      P.a_bytes = a_box * 128u;
-      if (!tc_map_u8(&m2[0], c->digits[sa], MA.dcols, MA.drows, a_box) ||
-          !tc_map_nibbles(&m2[1], c->nibbles[sb], MB.dcols, MB.drows))
-        return fail(GBS_EUNSUPPORTED, "tensor-core plan: tensor map encoding failed");
-      rt = (uint32_t)((MA.nrows + 127) / 128);
-      ct = (uint32_t)((MB.nrows + 255) / 256);
+      ok = ok && tc_map_u8(&m2[0], c->digits[sa], MA.dcols, MA.drows, 128);
     }
+    if (!ok) return fail(GBS_EUNSUPPORTED, "tensor-core plan: tensor map encoding failed");
+    const uint32_t rt = (uint32_t)((MA.nrows + 127) / 128), ct = (uint32_t)((MB.nrows + P.bn - 1) / P.bn);
     maps.push_back(m2[0]);
     maps.push_back(m2[1]);
     for (uint32_t r = 0; r < rt; r++)
@@ -614,9 +683,9 @@ int tcg_plan_build(TcgPlan *plan, gbs_ctx *const *ctxs, int n) {
     probs.push_back(P);
     for (int side = 0; side < 2; side++) {
       const Mat &m = side ? R : L;
-      for (int kind = 0; kind < 2; kind++) {  // digits, nibbles
+      for (int kind = 0; kind < 2; kind++) {  // digits, packed values
         if (!((sides >> (2 * kind + side)) & 1)) continue;
-        ExpandJob j = kind ? make_nibble_job(m, c->nibbles[side]) : make_expand_job(m, c->digits[side]);
+        ExpandJob j = kind ? make_packed_job(m, c->packed[side]) : make_expand_job(m, c->digits[side]);
         j.thread0 = threads;
         threads += ((uint64_t)j.nrows * j.chunks + 255) / 256 * 256;
         if (j.nrows && j.chunks) jobs.push_back(j);
@@ -634,15 +703,12 @@ int tcg_plan_build(TcgPlan *plan, gbs_ctx *const *ctxs, int n) {
   if (e == cudaSuccess) e = upload(&plan->d_tiles, sorted.data(), sorted.size());
   if (e == cudaSuccess) e = upload(&plan->d_jobs, jobs.data(), jobs.size());
   if (e == cudaSuccess)
-    e = nib ? tcgn_prepare()
-            : cudaFuncSetAttribute(gemm_tcg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)tcg_smem_bytes());
+    e = cudaFuncSetAttribute(gemm_tcg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tcg_smem_bytes());
   if (e != cudaSuccess) {
     cudaGetLastError();
     tcg_plan_free(plan);
     return fail(GBS_ENOMEM, "tensor-core plan: table upload failed");
   }
-  plan->nibbles = nib;
   plan->nprob = (uint32_t)probs.size();
   plan->ntiles = (uint32_t)sorted.size();
   plan->njobs = (int)jobs.size();
@@ -662,14 +728,13 @@ cudaError_t tcg_expand(TcgPlan &plan, cudaStream_t s) {
   for (size_t i = 0; i < plan.ctxs.size(); i++)
     for (int side = 0; side < 2; side++) {
       if ((plan.sides[i] >> side) & 1) plan.ctxs[i]->digits_valid[side] = true;
-      if ((plan.sides[i] >> (2 + side)) & 1) plan.ctxs[i]->nibbles_valid[side] = true;
+      if ((plan.sides[i] >> (2 + side)) & 1) plan.ctxs[i]->packed_valid[side] = true;
     }
   return cudaSuccess;
 }
 
 cudaError_t tcg_gemm(const TcgPlan &plan, uint32_t *err, cudaStream_t s, int32_t *out0) {
   if (!plan.ntiles) return cudaSuccess;
-  if (plan.nibbles) return tcgn_gemm(plan, err, s, out0);
   const cudaError_t e = launch_pdl(gemm_tcg_kernel, plan.grid, kTgThreads, tcg_smem_bytes(), s, plan.d_probs,
                                    reinterpret_cast<const CUtensorMap *>(plan.d_maps), plan.d_tiles, plan.ntiles,
                                    plan.nprob, err, out0);

@@ -128,14 +128,14 @@ int build_pack_jobs(gbs_group *g, PackTable &tab, const void *const *lhs, const 
       if (m.nrows && m.ncols && (!src || !device_ptr(src)))
         return fail(GBS_EINVAL, "gbs_group: sources must be device pointers (problem " + std::to_string(p) + ")");
       DigitTarget digits;
-      uint8_t *nibbles = nullptr;
+      uint8_t *packed = nullptr;
       if ((digit_sides >> side) & 1) {  // tensor-core problem: the import writes the digit matrices it reads
         digits.lo = g->ctxs[p]->digits[side];
         digits.lo_bits = (int)m.nbits;
         tc_digit_table(m, digits.tab_lo);
       }
-      if ((digit_sides >> (2 + side)) & 1) nibbles = g->ctxs[p]->nibbles[side];  // ... and nibble matrices
-      PackJob j = make_pack_job(m, src, dt, &digits, nibbles);
+      if ((digit_sides >> (2 + side)) & 1) packed = g->ctxs[p]->packed[side];  // ... and packed matrices
+      PackJob j = make_pack_job(m, src, dt, &digits, packed);
       const int kind = pack_job_direct(j, m) ? 0 : 1;
       units[kind] += pack_job_units(j);
       jobs[kind].push_back(j);
@@ -219,25 +219,25 @@ cudaError_t enqueue_gemm(gbs_group *g, cudaStream_t s) {
   return e;
 }
 
-// True when a digit or nibble matrix some tensor-core problem reads is older than its planes.
+// True when a digit or packed matrix some tensor-core problem reads is older than its planes.
 bool digits_stale(const gbs_group *g) {
   for (size_t i = 0; i < g->tc.ctxs.size(); i++)
     for (int side = 0; side < 2; side++) {
       if (((g->tc.sides[i] >> side) & 1) && !g->tc.ctxs[i]->digits_valid[side]) return true;
-      if (((g->tc.sides[i] >> (2 + side)) & 1) && !g->tc.ctxs[i]->nibbles_valid[side]) return true;
+      if (((g->tc.sides[i] >> (2 + side)) & 1) && !g->tc.ctxs[i]->packed_valid[side]) return true;
     }
   return false;
 }
 
-// After a grouped pack: the digit and nibble matrices it wrote match the new
+// After a grouped pack: the digit and packed matrices it wrote match the new
 // planes, any other of the group's contexts is stale.
 void mark_packed_digits(const gbs_group *g) {
   for (gbs_ctx *c : g->ctxs)
-    for (int side = 0; side < 2; side++) c->digits_valid[side] = c->nibbles_valid[side] = false;
+    for (int side = 0; side < 2; side++) c->digits_valid[side] = c->packed_valid[side] = false;
   for (size_t i = 0; i < g->tc.ctxs.size(); i++)
     for (int side = 0; side < 2; side++) {
       g->tc.ctxs[i]->digits_valid[side] = ((g->tc.sides[i] >> side) & 1) != 0;
-      g->tc.ctxs[i]->nibbles_valid[side] = ((g->tc.sides[i] >> (2 + side)) & 1) != 0;
+      g->tc.ctxs[i]->packed_valid[side] = ((g->tc.sides[i] >> (2 + side)) & 1) != 0;
     }
 }
 
@@ -549,7 +549,7 @@ int gbs_group_split(const gbs_group *g, uint64_t *popc_problems, uint64_t *tc_pr
 int gbs_debug_group_tc_kernel(const gbs_group *g) {
   if (!g) return -fail(GBS_EINVAL, "gbs_debug_group_tc_kernel: group is NULL");  // negative: not a kernel code
   if (!g->tc.ntiles) return 0;
-  return g->tc.nibbles ? 2 : 1;
+  return g->tc.packed ? 2 : 1;
 }
 
 int gbs_debug_group_poison_tile(gbs_group *g, uint32_t tile) {

@@ -30,11 +30,14 @@ constexpr int kMaxBits = 8;
 __host__ __device__ inline uint64_t digit_offset(uint64_t r, uint64_t col, uint64_t ncols_a) {
   return ((r >> 4) * (ncols_a >> 7) + (col >> 7)) * 2048 + ((r & 15) << 7) + (col & 127);
 }
-// The nibble matrix (the tensor-core pipe's compact copy of an operand: each
-// element's plane code in 4 bits, the even column in the low nibble) has the
-// same blocks at half the bytes: [rows/16][cols/128][16][64].  Byte offset
-// of the code pair holding column col (col even).
-__host__ __device__ inline uint64_t nibble_offset(uint64_t r, uint64_t col, uint64_t ncols_a) {
+// The packed matrix, the tensor-core pipe's compact copy of an operand of up to 2
+// bits, or 3 signed ones: each element as a 4-bit float (e2m1), sign and
+// magnitude.  That format runs linearly from 0 to 2 in steps of 1/2 over its first
+// codes, so the code is the magnitude itself and the float half the value.  The
+// TMA unpacks them into the 16-byte groups that tcgen05.mma reads such operands
+// from.  Same blocks as the digits at half the bytes: [rows/16][cols/128][16][64],
+// the even column in the low 4 bits.  Byte offset of column col (a multiple of 2).
+__host__ __device__ inline uint64_t packed_offset(uint64_t r, uint64_t col, uint64_t ncols_a) {
   return ((r >> 4) * (ncols_a >> 7) + (col >> 7)) * 1024 + ((r & 15) << 6) + ((col & 127) >> 1);
 }
 
@@ -50,6 +53,8 @@ struct Mat {
   uint64_t *planes = nullptr;
   bool imported = false;
   bool bipolar() const { return nbits == 1 && issigned; }
+  bool packable() const { return nbits <= 2 || (nbits == 3 && issigned); }
+  int packed_form() const { return bipolar() ? 3 : issigned ? 2 : 1; }  // of a packed matrix's elements
   uint64_t wpr() const { return ncols_a / 64; }
   uint64_t words() const { return nbits * nrows_a * wpr(); }
 };
@@ -112,7 +117,7 @@ struct PackJob {
   uint64_t *planes;
   int32_t *rowsum;
   uint8_t *digits, *digits_hi;
-  uint8_t *nibbles;  // with nibbles set, the import also writes the nibble matrix (codes, 4 bits each)
+  uint8_t *packed;  // with packed set, the import also writes the packed matrix (packed_form pform)
   uint64_t nrows, ncols, nrows_a, wpr, warp0;
   uint64_t dcols;  // digit-matrix columns (a multiple of 256)
   int nbits, issigned, dtype, vec;
@@ -120,28 +125,24 @@ struct PackJob {
   // staged kernels of a grouped import: vec 1 when four elements load as one vector
   uint32_t cpr, magic;  // 32-column chunks per padded row, 2^32 / cpr + 1
   uint32_t dtab[4], dtab_hi[4];
-  int lo_bits, pad;
+  int lo_bits, pform;
 };
 
-// One problem of the persistent tensor-core kernels (device resident).  The
-// MMA's row operand ("MMA-A", 128 rows per tile) is the lhs, or the rhs when
-// swap is set; the other operand gives the MMA's N columns per tile.  The
-// digit kernel (gbs_gemm_tcg.cu) takes the larger side as MMA-A and reads
-// both operands' digit matrices, N = bn; the nibble kernel
-// (gbs_gemm_tcgn.cu) takes the smaller side as MMA-A (digits) and decodes
-// the larger from its nibble matrix, N = 256.
+// One problem of the persistent tensor-core kernel (device resident).  The
+// MMA's row operand ("MMA-A", 128 rows per tile) is the larger side: the lhs, or
+// the rhs when swap is set; the other operand gives the MMA's N columns per
+// tile.  MMA-A is read from its digit matrix, or, in a packed plan and where its
+// values allow it, from its packed matrix; the smaller side always from digits.
 struct TcgProblem {
   int32_t *C;               // result [N][M]
   uint32_t M, N;
-  uint32_t a_rows, b_rows;  // padded rows of the MMA-A digit matrix / the MMA-B digit (nibble) matrix
+  uint32_t a_rows, b_rows;  // padded rows of MMA-A's and MMA-B's matrices
   uint32_t nk;              // K stages of 128 digits
-  uint32_t bn;              // digit kernel: MMA N, a multiple of 16 in [16, 256]
-  uint32_t idesc;           // tcgen05 instruction descriptor for M = 128 and the kernel's N
+  uint32_t bn;              // MMA N, a multiple of 16 in [16, 256]
+  uint32_t idesc;           // tcgen05 instruction descriptor for M = 128, N = bn and the operands' types
   uint32_t swap;            // 1: MMA-A = rhs (tile rows are n), MMA-B = lhs (columns are m)
-  uint32_t w4;              // nibble kernel: MMA-B codes of 4 bits (the two-table lookup)
-  uint32_t tab[4];          // nibble kernel: e4m3 byte of every MMA-B code
-  uint32_t a_bytes;         // nibble kernel: MMA-A bytes loaded per stage (rows of the smaller side, 16-row
-                            // multiples up to 128, x 128 digits; the tile's other rows only feed unstored lanes)
+  uint32_t a_bytes;         // bytes of MMA-A a stage brings: 128 rows x 128 values of 8 or 4 bits
+  float scale;              // result / accumulator (2: MMA-A packed)
 };
 
 // One output tile: problem, 128-row block of MMA-A, bn-column block of MMA-B.
@@ -150,26 +151,25 @@ struct TcgTile {
 };
 
 // One operand of an expansion pass: planes -> e4m3 digit matrix, or planes
-// -> nibble matrix (nib set: the plane codes, 4 bits each).
+// -> packed matrix (pform set: its packed_form).
 struct ExpandJob {
   const uint64_t *planes;
-  uint8_t *digits;   // the digit or nibble matrix
+  uint8_t *digits;   // the digit or packed matrix
   uint64_t nrows_a, wpr, dcols;  // plane rows and words per row; digit-matrix columns
   uint64_t thread0;  // first global thread of this job (16 digits or 32 codes per thread)
   uint32_t nrows, K, chunks, nbits;
   uint32_t tab[4];   // e4m3 byte of every plane code, 4 per word
-  uint32_t nib;
+  uint32_t pform;
 };
 
 // Host-side plan of the persistent tensor-core kernels over some contexts.
 struct TcgPlan {
   std::vector<gbs_ctx *> ctxs;
   // derived matrices each context needs: bit 0 / 1 the lhs / rhs digit
-  // matrix, bit 2 / 3 the lhs / rhs nibble matrix (both digit matrices for
-  // the digit kernel; the smaller side's digits and the larger side's
-  // nibbles for the nibble kernel)
+  // matrix, bit 2 / 3 the lhs / rhs packed matrix (the larger side's in a packed
+  // plan, where that side is packable, instead of its digits)
   std::vector<uint8_t> sides;
-  bool nibbles = false;  // the nibble kernel (gbs_gemm_tcgn.cu) runs the plan
+  bool packed = false;
   TcgProblem *d_probs = nullptr;
   void *d_maps = nullptr;  // CUtensorMap [2 * nprob]: MMA-A map, MMA-B map of each problem
   TcgTile *d_tiles = nullptr;
@@ -223,10 +223,9 @@ struct gbs_ctx {
   // pipe's operands), built from the planes on first use after each import
   uint8_t *digits[2] = {nullptr, nullptr};
   bool digits_valid[2] = {false, false};
-  // nibble matrices [drows][dcols / 2] (4-bit plane codes) of either side, the
-  // larger operand's form for the nibble kernel, built like the digits
-  uint8_t *nibbles[2] = {nullptr, nullptr};
-  bool nibbles_valid[2] = {false, false};
+  // packed matrices of either side, built like the digits
+  uint8_t *packed[2] = {nullptr, nullptr};
+  bool packed_valid[2] = {false, false};
   int host_import = 0;  // GBS_HOST_IMPORT_*: how gbs_import reads host-memory sources
   alignas(64) unsigned char tc_map_da[128];
   alignas(64) unsigned char tc_map_db[128];
@@ -245,7 +244,7 @@ struct gbs_ctx {
   void *split_ws = nullptr;
   uint32_t *split_counters = nullptr;
   gbs::SmallPlan *small = nullptr;  // a side under 256 rows: built on first use
-  // one-problem plan of the persistent nibble kernel, where that is forced on such a context
+  // one-problem packed plan of the persistent kernel, where that is forced on such a context
   gbs::TcgPlan *plan1 = nullptr;
   bool plan1_ready = false;
   gbs::AdjPlan *adj = nullptr;  // tensor-core adjoint workspace, built on first use
@@ -274,8 +273,8 @@ cudaError_t launch_pack(const Mat &m, const void *src, int dtype, int col_major,
 // threshold-quantising import (importRegularAndQuantize); dtype GBS_I8..GBS_F32, thr [nthres][nrows]
 cudaError_t launch_pack_quantize(const Mat &m, const void *src, const void *thr, int nthres, int dtype,
                                  int col_major, const DigitTarget *digits, cudaStream_t s);
-// One operand as a pack job; digits / nibbles may be null.
-PackJob make_pack_job(const Mat &m, const void *src, int dtype, const DigitTarget *digits, uint8_t *nibbles);
+// One operand as a pack job; digits / packed may be null.
+PackJob make_pack_job(const Mat &m, const void *src, int dtype, const DigitTarget *digits, uint8_t *packed);
 // Sets j.vec; true when the direct kernels take the job, false for the staged ones.
 bool pack_job_direct(PackJob &j, const Mat &m);
 uint64_t pack_job_units(const PackJob &j);   // units (32 chunks, one warp) of the job
@@ -363,13 +362,10 @@ cudaError_t tcg_expand(TcgPlan &plan, cudaStream_t s);
 cudaError_t tcg_gemm(const TcgPlan &plan, uint32_t *err, cudaStream_t s, int32_t *out0 = nullptr);
 cudaError_t alloc_zeroed(void **p, size_t bytes, const cudaStream_t *order);
 cudaError_t ensure_digit_buffer(gbs_ctx *c, int side, const cudaStream_t *order = nullptr);
-cudaError_t ensure_nibble_buffer(gbs_ctx *c, int side, const cudaStream_t *order = nullptr);
-// the nibble kernel over a plan built with nibbles set (gbs_gemm_tcgn.cu)
-cudaError_t tcgn_gemm(const TcgPlan &plan, uint32_t *err, cudaStream_t s, int32_t *out0);
-cudaError_t tcgn_prepare();  // kernel attributes, once per plan build
-bool tc_map_nibbles(void *map, const uint8_t *base, uint64_t cols, uint64_t rows);
-// GBS_TCG_NIBBLES in the environment: 0 the digit kernels, 1 the nibble kernel, -1 unset
-int tcg_nibbles_mode();
+cudaError_t ensure_packed_buffer(gbs_ctx *c, int side, const cudaStream_t *order = nullptr);
+bool tc_map_packed(void *map, const uint8_t *base, uint64_t cols, uint64_t rows);
+// GBS_TCG_NIBBLES in the environment: 0 digit plans, 1 packed plans, -1 unset
+int tcg_packed_mode();
 // SM-pair tiles with K split, partial tiles summed through L2 (gbs_gemm_tcp.cu)
 uint32_t pair_gather_splits(uint64_t tiles, uint32_t nstages, uint64_t pairs, double other_us);
 bool ensure_split_workspace(gbs_ctx *c, uint64_t tiles, uint32_t splits, cudaStream_t s);
@@ -388,7 +384,7 @@ int adjoint_tc(gbs_ctx *c, const float *dC, float *dA, float *dB, cudaStream_t s
 bool adjoint_tc_available();
 void adj_plan_free(AdjPlan *p);
 ExpandJob make_expand_job(const Mat &m, uint8_t *digits);
-ExpandJob make_nibble_job(const Mat &m, uint8_t *nibbles);
+ExpandJob make_packed_job(const Mat &m, uint8_t *packed);
 cudaError_t launch_expand(const ExpandJob &job, cudaStream_t s);
 int effective_pipe(const gbs_ctx *c);
 int tuned_variant(const gbs_ctx *c, int pipe);

@@ -12,7 +12,7 @@
 //
 // Every import ends the same way: a lane holds the codes of one "chunk", 32
 // consecutive columns of one row (byte j%4 of q[j/4]), and emits one 32-bit
-// word per plane, 32 bytes of the digit matrix and 16 bytes of the nibble
+// word per plane, 32 bytes of the digit matrix and 16 bytes of the packed
 // matrix.  Chunks are numbered along the padded rows, so chunk c of a plane is
 // its 32-bit word c: a warp's 32 chunks store 128 contiguous bytes per plane
 // whatever the row length, and no lane idles on short rows.
@@ -84,27 +84,9 @@ __device__ __forceinline__ void write_digits32(uint8_t *__restrict__ digits, int
                : "memory");
 }
 
-// The lane's 32 codes into the nibble matrix (dcols columns, blocks of
-// nibble_offset): the low nbits bits of each code byte, two codes a byte
-// (even column low).  Codes past ncols are whatever the source gave: the
-// tensor-core kernel multiplies them by digits that are zero there.
-__device__ __forceinline__ void write_nibbles32(uint8_t *__restrict__ nib, int nbits, uint64_t dcols, uint32_t r,
-                                                uint32_t col0, const uint32_t (&q)[8]) {
-  const uint32_t msk = 0x01010101u * ((1u << nbits) - 1u);
-  uint32_t o[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    uint32_t t0 = q[2 * i] & msk, t1 = q[2 * i + 1] & msk;
-    t0 |= t0 >> 4;  // bytes 0 and 2: code pairs
-    t1 |= t1 >> 4;
-    o[i] = __byte_perm(t0, t1, 0x6420u);
-  }
-  *reinterpret_cast<uint4 *>(nib + nibble_offset(r, col0, dcols)) = make_uint4(o[0], o[1], o[2], o[3]);
-}
-
 // Everything chunk cc of row r writes; idx is its number along the padded
 // rows, derived says whether the row is one of the matrix's own (padding rows
-// have no digits or nibbles).
+// have no digits or packed values).
 __device__ __forceinline__ void emit_chunk(const PackJob &J, uint64_t idx, uint32_t r, uint32_t cc, bool derived,
                                            const uint32_t (&q)[8]) {
   emit_planes32(J.nbits, reinterpret_cast<uint32_t *>(J.planes), J.nrows_a * J.cpr, idx, q);
@@ -119,7 +101,9 @@ __device__ __forceinline__ void emit_chunk(const PackJob &J, uint64_t idx, uint3
     write_digits32(J.digits_hi, J.nbits - J.lo_bits, (uint32_t)J.ncols, J.dcols,
                    make_uint4(J.dtab_hi[0], J.dtab_hi[1], J.dtab_hi[2], J.dtab_hi[3]), r, cc * 32, h);
   }
-  if (J.nibbles) write_nibbles32(J.nibbles, J.nbits, J.dcols, r, cc * 32, q);
+  // columns past ncols hold whatever the codes there give: the tensor-core kernel
+  // multiplies them by digits that are zero
+  if (J.packed) store_packed32(J.packed, r, cc * 32, J.dcols, J.nbits, J.pform, q);
 }
 
 // ---------------------------------------------------------------- chunk numbering
@@ -194,7 +178,8 @@ __device__ __forceinline__ void load_bytes32(const PackJob &J, const UnitBase &b
 __device__ __forceinline__ void codes_of_bytes(int dtype, int bipolar, uint32_t (&q)[8]) {
   if (bipolar && dtype == GBS_I8) {
 #pragma unroll
-    for (int i = 0; i < 8; i++) q[i] = __vcmpgts4(q[i], 0u) & 0x01010101u;
+    for (int i = 0; i < 8; i++)  // 1 where the signed byte is above 0: bits 0-6 not zero, bit 7 clear
+      q[i] = ((((q[i] & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) & ~q[i]) >> 7) & 0x01010101u;
   }
 }
 
@@ -714,7 +699,7 @@ __device__ __forceinline__ int find_job(const PackJob *jobs, int njobs, uint64_t
 // kMaxRun, fewer when the group would leave warps without one); a warp takes
 // runs in a grid stride and keeps kDepth units' loads in flight.
 // HBM-bound on large groups: 7.7 GB of the 512-problem mix (1-byte sources in,
-// planes and nibble or digit matrices out) in 1.23 ms, 0.92 of the copy rate;
+// planes and packed or digit matrices out) in 1.23 ms, 0.92 of the copy rate;
 // one strided pair of 16-byte loads per lane, a unit to a row segment and a
 // binary search per run took 2.17 ms.
 constexpr int kMaxRun = 8;
@@ -903,12 +888,13 @@ inline unsigned blocks_for(uint64_t threads, unsigned per_block) {
 
 }  // namespace
 
-PackJob make_pack_job(const Mat &m, const void *src, int dtype, const DigitTarget *digits, uint8_t *nibbles) {
+PackJob make_pack_job(const Mat &m, const void *src, int dtype, const DigitTarget *digits, uint8_t *packed) {
   PackJob j;
   memset(&j, 0, sizeof(j));
   j.src = src;
   j.planes = m.planes;
-  j.nibbles = nibbles;
+  j.packed = packed;
+  j.pform = m.packed_form();
   j.nrows = m.nrows;
   j.ncols = m.ncols;
   j.nrows_a = m.nrows_a;

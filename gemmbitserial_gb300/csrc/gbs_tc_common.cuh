@@ -198,6 +198,12 @@ __device__ __forceinline__ void mma_f8(uint32_t tmem, uint64_t adesc, uint64_t b
       " tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc));
 }
+// One lane of a converged warp: true there.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+  return one != 0;
+}
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                : "memory");
@@ -207,6 +213,31 @@ __device__ __forceinline__ uint32_t bfe4(uint32_t x, int sh) {
   uint32_t r;
   asm("bfe.u32 %0, %1, %2, 4;" : "=r"(r) : "r"(x), "r"(sh));
   return r;
+}
+
+// 32 columns of row r of a packed matrix, from their codes (a byte each in q,
+// bits above nbits ignored): even and odd columns gathered by byte, then eight
+// elements at a time, with multiply-adds where they save integer instructions,
+// which run at half their rate.
+__device__ __forceinline__ void store_packed32(uint8_t *base, uint32_t r, uint32_t col0, uint64_t dcols, int nbits,
+                                               int form, const uint32_t (&q)[8]) {
+  const uint32_t ones = (1u << nbits) - 1u, msk = 0x01010101u * ones;
+  uint32_t o[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+    o[i] = (__byte_perm(q[2 * i], q[2 * i + 1], 0x7531u) & msk) * 16u +
+           (__byte_perm(q[2 * i], q[2 * i + 1], 0x6420u) & msk);
+  if (form == 2) {  // two's complement: magnitude (x ^ ones) + 1 and the sign bit, 8
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const uint32_t neg = (o[i] >> (nbits - 1)) & 0x11111111u;
+      o[i] = (o[i] ^ (neg * ones)) + neg * 9u;
+    }
+  } else if (form == 3) {  // 0: -1 (9), 1: +1
+#pragma unroll
+    for (int i = 0; i < 4; i++) o[i] = 0x99999999u - o[i] * 8u;
+  }
+  *reinterpret_cast<uint4 *>(base + packed_offset(r, col0, dcols)) = make_uint4(o[0], o[1], o[2], o[3]);
 }
 
 // e4m3 bytes of 4 consecutive columns of one tile row: codes from the tile's

@@ -45,8 +45,8 @@ struct WidePlan {
   int lo_bits[2] = {0, 0};  // bits of a side's low part (the high part's weight is 2^lo_bits)
   // Each form has its own [side][part] digit matrices (a captured graph of one
   // must not find the other's): the fused form's match the planes while the
-  // context's digits_valid says so, the separate form's while its nibbles_valid
-  // does (a wide context has no nibble matrices of its own).
+  // context's digits_valid says so, the separate form's while its packed_valid
+  // does (a wide context has no packed matrices of its own).
   uint8_t *sep[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
   gbs_ctx *sub[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [lhs part][rhs part], separate form
   int fused_splits = 0;  // K splits of the fused kernel, 0: the separate form only
@@ -436,7 +436,7 @@ cudaError_t launch_fused(const gbs_ctx *c, const WidePlan &p, const WideArgs &a,
 
 // The digit matrices of one form, rebuilt from the planes where they are older.
 cudaError_t expand_parts(gbs_ctx *c, const WidePlan &p, bool fused, cudaStream_t s) {
-  bool(&valid)[2] = fused ? c->digits_valid : c->nibbles_valid;
+  bool(&valid)[2] = fused ? c->digits_valid : c->packed_valid;
   for (int side = 0; side < 2; side++) {
     if (valid[side]) continue;
     for (int k = 0; k < p.parts[side]; k++) {
@@ -445,10 +445,10 @@ cudaError_t expand_parts(gbs_ctx *c, const WidePlan &p, bool fused, cudaStream_t
       cudaError_t e = launch_expand(job, s);
       if (e != cudaSuccess) return e;
     }
-    if (!fused)  // the parts' own nibble matrices (one-problem plans) are stale too
+    if (!fused)  // the parts' own packed matrices (one-problem plans) are stale too
       for (auto &row : p.sub)
         for (gbs_ctx *sub : row)
-          if (sub) sub->nibbles_valid[side] = false;
+          if (sub) sub->packed_valid[side] = false;
     valid[side] = true;
   }
   return cudaSuccess;
@@ -493,8 +493,8 @@ void wide_plan_free(WidePlan *p) {
       if (s->sk_ws) cudaFree(s->sk_ws);
       if (s->split_ws) cudaFree(s->split_ws);
       if (s->sk_flags) cudaFree(s->sk_flags);
-      for (uint8_t *nb : s->nibbles)
-        if (nb) cudaFree(nb);
+      for (uint8_t *pk : s->packed)
+        if (pk) cudaFree(pk);
       delete s;  // its planes alias the parent's, its digit matrices are the plan's
     }
   for (auto &form : {&p->digits, &p->sep})

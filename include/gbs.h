@@ -388,13 +388,12 @@ GBS_API uint32_t gbs_debug_tc_error(void);
  * exercise the grouped kernel's descriptor validation (host-side injection). */
 GBS_API int gbs_debug_group_poison_tile(gbs_group *g, uint32_t tile);
 
-/* Which persistent tensor-core kernel runs a group's tensor-core problems:
- * 0 none, 1 the digit kernel (both operands as e4m3 digit matrices), 2 the
- * nibble kernel (the larger operand as 4-bit codes, decoded to digits in
- * shared memory).  By default an estimate of both kernels' critical paths
- * chooses (hundreds of problems: nibbles; one or a few: digits);
- * GBS_TCG_NIBBLES=0 or 1 in the environment at gbs_group_create forces the
- * digit or the nibble kernel.  Negative on a NULL group. */
+/* How a group's tensor-core problems hold their larger operands: 0 there are no
+ * such problems, 1 as e4m3 digits, 2 ("nibbles") as 4-bit floats where their
+ * values allow it, which the TMA unpacks.  By default an estimate of both plans'
+ * critical paths chooses (hundreds of problems: packed; one or a few: digits);
+ * GBS_TCG_NIBBLES=0 or 1 in the environment at gbs_group_create forces one.
+ * Negative on a NULL group. */
 GBS_API int gbs_debug_group_tc_kernel(const gbs_group *g);
 
 /* Exercises the tensor-core kernels' bounded waits without a GPU fault: one
