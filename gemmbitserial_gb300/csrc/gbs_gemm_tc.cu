@@ -346,42 +346,45 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t issued = 0;
-      for (uint32_t k = 0; k < a.nstages; k++) {
-        const uint32_t s = k % a.stages, use = k / a.stages;
-        if (use > 0 && !mbar_wait(empty + 8 * s, (use - 1) & 1, abort_flag)) break;
+    uint32_t issued = 0;
+    for (uint32_t k = 0; k < a.nstages; k++) {
+      const uint32_t s = k % a.stages, use = k / a.stages;
+      if (use > 0 && !__all_sync(0xffffffffu, mbar_wait(empty + 8 * s, (use - 1) & 1, abort_flag))) break;
+      if (elect_one()) {
         mbar_expect_tx(full + 8 * s, stage_bytes);
         const uint32_t dst = smem_u32(smem + s * stage_bytes);
         tma_load_digits(dst, &tmA, (int)k, (uint32_t)m0, full + 8 * s);
         for (int h = 0; h < BN / 128; h++)
           tma_load_digits(dst + a_bytes + h * 128 * kRowB, &tmB, (int)k, (uint32_t)(n0 + 128 * h), full + 8 * s);
-        issued = k + 1;
       }
-      if (*abort_flag) {
-        for (uint32_t k = (issued > (uint32_t)a.stages ? issued - a.stages : 0); k < issued; k++)
-          mbar_drain(full + 8 * (k % a.stages), (k / a.stages) & 1);
-      }
+      __syncwarp();
+      issued = k + 1;
+    }
+    if (lane == 0 && *abort_flag) {
+      for (uint32_t k = (issued > (uint32_t)a.stages ? issued - a.stages : 0); k < issued; k++)
+        mbar_drain(full + 8 * (k % a.stages), (k / a.stages) & 1);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      bool ok = true;
-      for (uint32_t k = 0; k < a.nstages && ok; k++) {
-        const uint32_t s = k % a.stages;
-        if (!mbar_wait(full + 8 * s, (k / a.stages) & 1, abort_flag)) {
-          ok = false;
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t base = smem_u32(smem + s * stage_bytes);
+    bool ok = true;
+    for (uint32_t k = 0; k < a.nstages && ok; k++) {
+      const uint32_t s = k % a.stages;
+      if (!__all_sync(0xffffffffu, mbar_wait(full + 8 * s, (k / a.stages) & 1, abort_flag))) {
+        ok = false;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const uint32_t base = smem_u32(smem + s * stage_bytes);
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < 4; kk++)
           mma_f8(tmem, sw128_desc(base + kk * 32), sw128_desc(base + a_bytes + kk * 32), a.idesc, (k | kk) != 0);
         mma_commit(empty + 8 * s);
       }
-      mma_commit(ok ? acc_full : mma_done);
-      if (!ok) mbar_drain(mma_done, 0);
+      __syncwarp();
     }
+    if (elect_one()) mma_commit(ok ? acc_full : mma_done);
+    __syncwarp();
+    if (!ok) mbar_drain(mma_done, 0);
   } else {
     if (__all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag))) {
       asm volatile("tcgen05.fence::after_thread_sync;");
@@ -516,52 +519,60 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     // full barrier.  Each CTA loading its own halves onto that barrier puts a
     // cross-SM completion on every stage's critical path, which measured about
     // twice as slow per stage as the one-issuer ring.  (The test hook loads nothing.)
-    if (lane == 0 && peer == 0 && a.wait_limit == 0) {
+    if (peer == 0 && a.wait_limit == 0) {
       uint32_t issued = 0;
       for (uint32_t k = 0; k < nk; k++) {
         const uint32_t s = k % a.stages, use = k / a.stages;
-        if (use > 0 && !mbar_wait(empty + 8 * s, (use - 1) & 1, abort_flag)) break;
-        const uint32_t fb = map_to_rank(full + 8 * s, lead);
-        mbar_expect_tx(full + 8 * s, 2 * stage_bytes);
-        const uint32_t dst = smem_u32(smem + s * stage_bytes), pdst = map_to_rank(dst, lead + 1);
-        const int kc = (int)(k_lo + k);
-        tma_load_digits_pair(dst, &tmA, kc, (uint32_t)pair_m0, fb);
-        tma_load_digits_pair(dst + kPairHalfBytes, &tmB, kc, (uint32_t)n0, fb);
-        tma_load_digits_pair(pdst, &tmA, kc, (uint32_t)(pair_m0 + 128), fb);
-        tma_load_digits_pair(pdst + kPairHalfBytes, &tmB, kc, (uint32_t)(n0 + BN / 2), fb);
+        if (use > 0 && !__all_sync(0xffffffffu, mbar_wait(empty + 8 * s, (use - 1) & 1, abort_flag))) break;
+        if (elect_one()) {
+          const uint32_t fb = map_to_rank(full + 8 * s, lead);
+          mbar_expect_tx(full + 8 * s, 2 * stage_bytes);
+          const uint32_t dst = smem_u32(smem + s * stage_bytes), pdst = map_to_rank(dst, lead + 1);
+          const int kc = (int)(k_lo + k);
+          tma_load_digits_pair(dst, &tmA, kc, (uint32_t)pair_m0, fb);
+          tma_load_digits_pair(dst + kPairHalfBytes, &tmB, kc, (uint32_t)n0, fb);
+          tma_load_digits_pair(pdst, &tmA, kc, (uint32_t)(pair_m0 + 128), fb);
+          tma_load_digits_pair(pdst + kPairHalfBytes, &tmB, kc, (uint32_t)(n0 + BN / 2), fb);
+        }
+        __syncwarp();
         issued = k + 1;
       }
       // after an abort, wait (bounded) for the loads the barriers still expect
       // (the peer's shared memory is written until then; the closing cluster
       // barrier keeps the peer resident)
-      if (*abort_flag) {
+      if (lane == 0 && *abort_flag) {
         for (uint32_t k = (issued > (uint32_t)a.stages ? issued - a.stages : 0); k < issued; k++)
           mbar_drain(full + 8 * (k % a.stages), (k / a.stages) & 1);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && peer == 0) {
+    if (peer == 0) {
       // test hook: nothing was loaded, so this wait runs out (no copy or MMA in flight)
-      bool ok = a.wait_limit == 0 || mbar_wait_rounds(full, 0, abort_flag, a.wait_limit);
+      bool ok = a.wait_limit == 0 ||
+                __all_sync(0xffffffffu, mbar_wait_rounds(full, 0, abort_flag, a.wait_limit));
       for (uint32_t k = 0; k < nk && ok; k++) {
         const uint32_t s = k % a.stages;
-        if (!mbar_wait(full + 8 * s, (k / a.stages) & 1, abort_flag)) {
+        if (!__all_sync(0xffffffffu, mbar_wait(full + 8 * s, (k / a.stages) & 1, abort_flag))) {
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;");
         const uint32_t base = smem_u32(smem + s * stage_bytes);
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < 4; kk++)
-          mma_f8_pair(tmem, sw128_desc(base + kk * 32), sw128_desc(base + kPairHalfBytes + kk * 32), a.idesc,
-                      (k | kk) != 0);
-        mma_commit_pair(empty + 8 * s, pair_mask);
+          for (int kk = 0; kk < 4; kk++)
+            mma_f8_pair(tmem, sw128_desc(base + kk * 32), sw128_desc(base + kPairHalfBytes + kk * 32), a.idesc,
+                        (k | kk) != 0);
+          mma_commit_pair(empty + 8 * s, pair_mask);
+        }
+        __syncwarp();
       }
       if (ok) {
-        mma_commit_pair(acc_full, pair_mask);
+        if (elect_one()) mma_commit_pair(acc_full, pair_mask);
+        __syncwarp();
       } else {  // issued MMAs finish before TMEM is freed
-        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mma_done)
-                     : "memory");
+        if (elect_one()) mma_commit_done(mma_done);
+        __syncwarp();
         mbar_drain(mma_done, 0);
       }
     }
@@ -718,60 +729,67 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   griddep_wait();  // operands and result belong to the previous kernels until here
 
   if (warp == 0) {
-    if (lane == 0 && peer == 0) {  // the leader's TMA: both CTAs' halves of every stage
+    if (peer == 0) {  // the leader's TMA: both CTAs' halves of every stage
       uint32_t g = 0;
       bool stop = false;
       for (uint32_t t = pid; t < ntiles && !stop; t += npairs) {
         const uint32_t m0 = (t % mt) * 256u, n0 = (t / mt) * 256u;
         for (uint32_t k = 0; k < nk; k++, g++) {
           const uint32_t s = g % a.stages, use = g / a.stages;
-          if (use > 0 && !mbar_wait(empty + 8 * s, (use - 1) & 1, abort_flag)) {
+          if (use > 0 && !__all_sync(0xffffffffu, mbar_wait(empty + 8 * s, (use - 1) & 1, abort_flag))) {
             stop = true;
             break;
           }
-          const uint32_t fb = map_to_rank(full + 8 * s, 0);
-          mbar_expect_tx(full + 8 * s, 2 * stage_bytes);
-          const uint32_t dst = smem_u32(smem + s * stage_bytes), pdst = map_to_rank(dst, 1);
-          tma_load_digits_pair(dst, &tmA, (int)k, m0, fb);
-          tma_load_digits_pair(dst + kPairHalfBytes, &tmB, (int)k, n0, fb);
-          tma_load_digits_pair(pdst, &tmA, (int)k, m0 + 128, fb);
-          tma_load_digits_pair(pdst + kPairHalfBytes, &tmB, (int)k, n0 + 128, fb);
+          if (elect_one()) {
+            const uint32_t fb = map_to_rank(full + 8 * s, 0);
+            mbar_expect_tx(full + 8 * s, 2 * stage_bytes);
+            const uint32_t dst = smem_u32(smem + s * stage_bytes), pdst = map_to_rank(dst, 1);
+            tma_load_digits_pair(dst, &tmA, (int)k, m0, fb);
+            tma_load_digits_pair(dst + kPairHalfBytes, &tmB, (int)k, n0, fb);
+            tma_load_digits_pair(pdst, &tmA, (int)k, m0 + 128, fb);
+            tma_load_digits_pair(pdst + kPairHalfBytes, &tmB, (int)k, n0 + 128, fb);
+          }
+          __syncwarp();
         }
       }
-      if (*abort_flag)  // wait (bounded) for the loads the barriers still expect
+      if (lane == 0 && *abort_flag)  // wait (bounded) for the loads the barriers still expect
         for (uint32_t q = (g > (uint32_t)a.stages ? g - a.stages : 0); q < g; q++)
           mbar_drain(full + 8 * (q % a.stages), (q / a.stages) & 1);
     }
   } else if (warp == 1) {
-    if (lane == 0 && peer == 0) {  // the leader issues the pair's MMAs
+    if (peer == 0) {  // the leader issues the pair's MMAs
       bool ok = true;
       uint32_t g = 0, j = 0;
       for (uint32_t t = pid; t < ntiles && ok; t += npairs, j++) {
         const uint32_t b = j & 1u, dacc = tmem + b * 256u;
-        if (j >= 2 && !mbar_wait(acc_empty + 8 * b, ((j >> 1) - 1) & 1, abort_flag)) {
+        if (j >= 2 && !__all_sync(0xffffffffu, mbar_wait(acc_empty + 8 * b, ((j >> 1) - 1) & 1, abort_flag))) {
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;");
         for (uint32_t k = 0; k < nk; k++, g++) {
           const uint32_t s = g % a.stages;
-          if (!mbar_wait(full + 8 * s, (g / a.stages) & 1, abort_flag)) {
+          if (!__all_sync(0xffffffffu, mbar_wait(full + 8 * s, (g / a.stages) & 1, abort_flag))) {
             ok = false;
             break;
           }
           asm volatile("tcgen05.fence::after_thread_sync;");
           const uint32_t base = smem_u32(smem + s * stage_bytes);
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < 4; kk++)
-            mma_f8_pair(dacc, sw128_desc(base + kk * 32), sw128_desc(base + kPairHalfBytes + kk * 32), a.idesc,
-                        (k | kk) != 0);
-          mma_commit_pair(empty + 8 * s, kPairMask);
+            for (int kk = 0; kk < 4; kk++)
+              mma_f8_pair(dacc, sw128_desc(base + kk * 32), sw128_desc(base + kPairHalfBytes + kk * 32), a.idesc,
+                          (k | kk) != 0);
+            mma_commit_pair(empty + 8 * s, kPairMask);
+          }
+          __syncwarp();
         }
-        if (ok) mma_commit_pair(acc_full + 8 * b, kPairMask);
+        if (ok && elect_one()) mma_commit_pair(acc_full + 8 * b, kPairMask);
+        __syncwarp();
       }
       if (!ok) {  // issued MMAs finish before TMEM is freed
-        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mma_done)
-                     : "memory");
+        if (elect_one()) mma_commit_done(mma_done);
+        __syncwarp();
         mbar_drain(mma_done, 0);
       }
     }
@@ -922,7 +940,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   griddep_wait();  // operands, result and workspace belong to the previous kernels until here
 
   if (warp == 0) {
-    if (lane == 0 && peer == 0) {  // the leader's TMA: both CTAs' halves of every stage
+    if (peer == 0) {  // the leader's TMA: both CTAs' halves of every stage
       uint32_t g = 0, u = u1;
       bool stop = false;
       SkSeg sg;
@@ -930,55 +948,62 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         const uint32_t m0 = (sg.t % a.mt) * 256u, n0 = (sg.t / a.mt) * 256u;
         for (uint32_t k = sg.k0; k < sg.k1; k++, g++) {
           const uint32_t s = g % a.stages, use = g / a.stages;
-          if (use > 0 && !mbar_wait(empty + 8 * s, (use - 1) & 1, abort_flag)) {
+          if (use > 0 && !__all_sync(0xffffffffu, mbar_wait(empty + 8 * s, (use - 1) & 1, abort_flag))) {
             stop = true;
             break;
           }
-          const uint32_t fb = map_to_rank(full + 8 * s, 0);
-          mbar_expect_tx(full + 8 * s, 2 * stage_bytes);
-          const uint32_t dst = smem_u32(smem + s * stage_bytes), pdst = map_to_rank(dst, 1);
-          tma_load_digits_pair(dst, &tmA, (int)k, m0, fb);
-          tma_load_digits_pair(dst + kPairHalfBytes, &tmB, (int)k, n0, fb);
-          tma_load_digits_pair(pdst, &tmA, (int)k, m0 + 128, fb);
-          tma_load_digits_pair(pdst + kPairHalfBytes, &tmB, (int)k, n0 + 128, fb);
+          if (elect_one()) {
+            const uint32_t fb = map_to_rank(full + 8 * s, 0);
+            mbar_expect_tx(full + 8 * s, 2 * stage_bytes);
+            const uint32_t dst = smem_u32(smem + s * stage_bytes), pdst = map_to_rank(dst, 1);
+            tma_load_digits_pair(dst, &tmA, (int)k, m0, fb);
+            tma_load_digits_pair(dst + kPairHalfBytes, &tmB, (int)k, n0, fb);
+            tma_load_digits_pair(pdst, &tmA, (int)k, m0 + 128, fb);
+            tma_load_digits_pair(pdst + kPairHalfBytes, &tmB, (int)k, n0 + 128, fb);
+          }
+          __syncwarp();
         }
       }
-      if (*abort_flag)  // wait (bounded) for the loads the barriers still expect
+      if (lane == 0 && *abort_flag)  // wait (bounded) for the loads the barriers still expect
         for (uint32_t q = (g > (uint32_t)a.stages ? g - a.stages : 0); q < g; q++)
           mbar_drain(full + 8 * (q % a.stages), (q / a.stages) & 1);
     }
   } else if (warp == 1) {
-    if (lane == 0 && peer == 0) {  // the leader issues the pair's MMAs
+    if (peer == 0) {  // the leader issues the pair's MMAs
       bool ok = true;
       uint32_t g = 0, j = 0, u = u1;
       SkSeg sg;
       while (ok && sk_next(u, u0, nk, sg)) {
         const uint32_t b = j & 1u, dacc = tmem + b * 256u;
-        if (j >= 2 && !mbar_wait(acc_empty + 8 * b, ((j >> 1) - 1) & 1, abort_flag)) {
+        if (j >= 2 && !__all_sync(0xffffffffu, mbar_wait(acc_empty + 8 * b, ((j >> 1) - 1) & 1, abort_flag))) {
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;");
         for (uint32_t k = sg.k0; k < sg.k1; k++, g++) {
           const uint32_t s = g % a.stages;
-          if (!mbar_wait(full + 8 * s, (g / a.stages) & 1, abort_flag)) {
+          if (!__all_sync(0xffffffffu, mbar_wait(full + 8 * s, (g / a.stages) & 1, abort_flag))) {
             ok = false;
             break;
           }
           asm volatile("tcgen05.fence::after_thread_sync;");
           const uint32_t base = smem_u32(smem + s * stage_bytes);
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < 4; kk++)
-            mma_f8_pair(dacc, sw128_desc(base + kk * 32), sw128_desc(base + kPairHalfBytes + kk * 32), a.idesc,
-                        (k != sg.k0 || kk != 0) ? 1u : 0u);
-          mma_commit_pair(empty + 8 * s, kPairMask);
+            for (int kk = 0; kk < 4; kk++)
+              mma_f8_pair(dacc, sw128_desc(base + kk * 32), sw128_desc(base + kPairHalfBytes + kk * 32), a.idesc,
+                          (k != sg.k0 || kk != 0) ? 1u : 0u);
+            mma_commit_pair(empty + 8 * s, kPairMask);
+          }
+          __syncwarp();
         }
-        if (ok) mma_commit_pair(acc_full + 8 * b, kPairMask);
+        if (ok && elect_one()) mma_commit_pair(acc_full + 8 * b, kPairMask);
+        __syncwarp();
         j++;
       }
       if (!ok) {  // issued MMAs finish before TMEM is freed
-        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mma_done)
-                     : "memory");
+        if (elect_one()) mma_commit_done(mma_done);
+        __syncwarp();
         mbar_drain(mma_done, 0);
       }
     }

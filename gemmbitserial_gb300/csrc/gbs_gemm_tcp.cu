@@ -90,46 +90,53 @@ __global__ void __launch_bounds__(kSpThreads, 1)
   griddep_wait();  // operands, result and workspace belong to earlier kernels until here
 
   if (warp == 0) {
-    if (lane == 0 && peer == 0) {  // the leader's TMA: both CTAs' halves of every stage
+    if (peer == 0) {  // the leader's TMA: both CTAs' halves of every stage
       uint32_t k = 0;
       for (; k < nk; k++) {
         const uint32_t s = k % kSpStages, use = k / kSpStages;
-        if (use > 0 && !mbar_wait_err(empty + 8 * s, (use - 1) & 1, abort_flag, err)) break;
-        const uint32_t fb = map_to_rank(full + 8 * s, 0);
-        mbar_expect_tx(full + 8 * s, 2 * kSpStageBytes);
-        const uint32_t dst = smem_u32(smem + s * kSpStageBytes);
+        if (use > 0 && !__all_sync(0xffffffffu, mbar_wait_err(empty + 8 * s, (use - 1) & 1, abort_flag, err))) break;
+        if (elect_one()) {
+          const uint32_t fb = map_to_rank(full + 8 * s, 0);
+          mbar_expect_tx(full + 8 * s, 2 * kSpStageBytes);
+          const uint32_t dst = smem_u32(smem + s * kSpStageBytes);
 #pragma unroll
-        for (uint32_t h = 0; h < 2; h++) {
-          const uint32_t d = h ? map_to_rank(dst, 1) : dst;
-          tma_load_digits_pair(d, &tmA, (int)(k_lo + k), m0 + 128 * h, fb);
-          tma_load_digits_pair(d + kSpHalf, &tmB, (int)(k_lo + k), n0 + 128 * h, fb);
+          for (uint32_t h = 0; h < 2; h++) {
+            const uint32_t d = h ? map_to_rank(dst, 1) : dst;
+            tma_load_digits_pair(d, &tmA, (int)(k_lo + k), m0 + 128 * h, fb);
+            tma_load_digits_pair(d + kSpHalf, &tmB, (int)(k_lo + k), n0 + 128 * h, fb);
+          }
         }
+        __syncwarp();
       }
-      if (*abort_flag)  // wait (bounded) for the loads the barriers still expect, in the peer's memory too
+      if (lane == 0 && *abort_flag)  // wait (bounded) for the loads the barriers still expect, in the peer's memory too
         for (uint32_t i = (k > (uint32_t)kSpStages ? k - kSpStages : 0); i < k; i++)
           mbar_drain_err(full + 8 * (i % kSpStages), (i / kSpStages) & 1, err);
     }
   } else if (warp == 1) {
-    if (lane == 0 && peer == 0) {
+    if (peer == 0) {
       bool ok = true;
       for (uint32_t k = 0; k < nk; k++) {
         const uint32_t s = k % kSpStages;
-        if (!mbar_wait_err(full + 8 * s, (k / kSpStages) & 1, abort_flag, err)) {
+        if (!__all_sync(0xffffffffu, mbar_wait_err(full + 8 * s, (k / kSpStages) & 1, abort_flag, err))) {
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;");
         const uint32_t base = smem_u32(smem + s * kSpStageBytes);
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < 4; kk++)
-          mma_f8_pair(tmem, sw128_desc(base + kk * 32), sw128_desc(base + kSpHalf + kk * 32), a.idesc, (k | kk) != 0);
-        mma_commit_pair(empty + 8 * s, 3);
+          for (int kk = 0; kk < 4; kk++)
+            mma_f8_pair(tmem, sw128_desc(base + kk * 32), sw128_desc(base + kSpHalf + kk * 32), a.idesc, (k | kk) != 0);
+          mma_commit_pair(empty + 8 * s, 3);
+        }
+        __syncwarp();
       }
       if (ok) {
-        mma_commit_pair(acc_full, 3);
+        if (elect_one()) mma_commit_pair(acc_full, 3);
+        __syncwarp();
       } else {  // issued MMAs finish before TMEM is freed
-        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mma_done)
-                     : "memory");
+        if (elect_one()) mma_commit_done(mma_done);
+        __syncwarp();
         mbar_drain_err(mma_done, 0, err);
       }
     }
@@ -137,7 +144,7 @@ __global__ void __launch_bounds__(kSpThreads, 1)
     asm volatile("tcgen05.fence::after_thread_sync;");
     constexpr uint32_t kShare = 256 / SPLITS;  // columns of a share
     constexpr int kBatch = SPLITS - 1 < 3 ? SPLITS - 1 : 3;  // others' columns in flight
-    const uint32_t q = warp & 3, taddr = tmem + ((q * 32) << 16), lane = threadIdx.x & 31;
+    const uint32_t q = warp & 3, taddr = tmem + ((q * 32) << 16);
     const uint64_t gm = m0 + 128 * peer + q * 32 + lane;
     const uint32_t tile = (blockIdx.x >> 1) * gridDim.y + blockIdx.y;
     // this warp's slots: split s's columns at ws + s * stride

@@ -135,42 +135,46 @@ __global__ void __launch_bounds__(kSmThreads, 1)
   const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16);
   float4 *part = reinterpret_cast<float4 *>(smem) + q * 32 + lane;  // partial tile [bn / 4][128 rows][4 columns]
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t k = 0;
-      for (; k < nk; k++) {
-        const uint32_t s = k % stages, use = k / stages;
-        if (use > 0 && !mbar_wait_err(empty + 8 * s, (use - 1) & 1, abort_flag, err)) break;
+    uint32_t k = 0;
+    for (; k < nk; k++) {
+      const uint32_t s = k % stages, use = k / stages;
+      if (use > 0 && !__all_sync(0xffffffffu, mbar_wait_err(empty + 8 * s, (use - 1) & 1, abort_flag, err))) break;
+      if (elect_one()) {
         mbar_expect_tx(full + 8 * s, slot);
         const uint32_t dst = smem_u32(smem + s * slot);
         tma_load_digits(dst, &tmA, (int)(k_lo + k), r0, full + 8 * s);
         tma_load_digits(dst + kSmABytes, &tmB, (int)(k_lo + k), c0, full + 8 * s);
       }
-      if (*abort_flag)
-        for (uint32_t i = (k > stages ? k - stages : 0); i < k; i++)
-          mbar_drain_err(full + 8 * (i % stages), (i / stages) & 1, err);
+      __syncwarp();
     }
+    if (lane == 0 && *abort_flag)
+      for (uint32_t i = (k > stages ? k - stages : 0); i < k; i++)
+        mbar_drain_err(full + 8 * (i % stages), (i / stages) & 1, err);
   } else if (warp == 1) {
-    if (lane == 0) {
-      bool ok = true;
-      for (uint32_t k = 0; k < nk; k++) {
-        const uint32_t s = k % stages;
-        if (!mbar_wait_err(full + 8 * s, (k / stages) & 1, abort_flag, err)) {
-          ok = false;
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t base = smem_u32(smem + s * slot);
+    bool ok = true;
+    for (uint32_t k = 0; k < nk; k++) {
+      const uint32_t s = k % stages;
+      if (!__all_sync(0xffffffffu, mbar_wait_err(full + 8 * s, (k / stages) & 1, abort_flag, err))) {
+        ok = false;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const uint32_t base = smem_u32(smem + s * slot);
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < 4; kk++)
           mma_f8(tmem, sw128_desc(base + kk * 32), sw128_desc(base + kSmABytes + kk * 32), a.idesc, (k | kk) != 0);
         mma_commit(empty + 8 * s);
       }
-      if (ok) {
-        mma_commit(acc_full);
-      } else {  // issued MMAs finish before TMEM is freed
-        mma_commit(mma_done);
-        mbar_drain_err(mma_done, 0, err);
-      }
+      __syncwarp();
+    }
+    if (ok) {
+      if (elect_one()) mma_commit(acc_full);
+      __syncwarp();
+    } else {  // issued MMAs finish before TMEM is freed
+      if (elect_one()) mma_commit(mma_done);
+      __syncwarp();
+      mbar_drain_err(mma_done, 0, err);
     }
   } else {
     done = __all_sync(0xffffffffu, mbar_wait_err(acc_full, 0, abort_flag, err));
