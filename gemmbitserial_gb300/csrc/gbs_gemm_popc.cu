@@ -315,27 +315,39 @@ __global__ void __launch_bounds__(NT, 2) gemm_popc_tiled(TileArgs g) {
   popc_tile<BM, BN, KC, XOR>(g, (uint64_t)blockIdx.x * BM, (uint64_t)blockIdx.y * BN, smem);
 }
 
-// One output's weighted popcounts over every plane pair, this lane's share:
-// words lane, lane + 32, ... of lhs row a0 and rhs row b0 (planes a_plane /
-// b_plane words apart).  Each step loads U x 32 words of every plane first --
-// independent loads, one memory latency per step rather than one per plane
-// pair and 32 words -- then counts.  WM >= max(wa, wb) sizes the register
-// arrays.  Words past wpr count as zero (AND and XOR alike).
-template <int WM, int U, typename Alpha>
+// V consecutive plane words of a row by one load: 2 where rows start on 16 bytes.
+template <int V>
+__device__ __forceinline__ void ldg_words(const uint64_t *p, bool in, uint64_t *v) {
+  if (V == 2) {
+    const ulonglong2 x = in ? __ldg(reinterpret_cast<const ulonglong2 *>(p)) : make_ulonglong2(0ull, 0ull);
+    v[0] = x.x;
+    v[V - 1] = x.y;
+  } else {
+    v[0] = in ? __ldg(p) : 0ull;
+  }
+}
+
+// One output's weighted popcounts over every plane pair, this lane's share: V
+// words from V * lane on, then 32 * V further, ... of lhs row a0 and rhs row b0
+// (planes a_plane / b_plane words apart).  Each step loads U x 32 x V words of
+// every plane first -- independent loads, one memory latency per step rather than
+// one per plane pair and 32 words -- then counts.  WM >= max(wa, wb) sizes the
+// register arrays.  Words past wpr count as zero (AND and XOR alike).
+template <int WM, int U, int V, typename Alpha>
 __device__ __forceinline__ uint32_t skinny_lane_sum_t(const uint64_t *__restrict__ a0, uint64_t a_plane,
                                                       const uint64_t *__restrict__ b0, uint64_t b_plane, uint64_t wpr,
                                                       int wa, int wb, bool use_xor, int lane, Alpha alpha) {
   uint32_t acc = 0;
-  for (uint64_t w0 = 0; w0 < wpr; w0 += 32 * U) {
-    uint64_t av[WM][U], bv[WM][U];
+  for (uint64_t w0 = 0; w0 < wpr; w0 += 32 * U * V) {
+    uint64_t av[WM][U * V], bv[WM][U * V];
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      const uint64_t w = w0 + (uint64_t)(32 * u + lane);
+      const uint64_t w = w0 + (uint64_t)(V * (32 * u + lane));
       const bool in = w < wpr;
 #pragma unroll
-      for (int i = 0; i < WM; i++) av[i][u] = (in && i < wa) ? __ldg(a0 + i * a_plane + w) : 0ull;
+      for (int i = 0; i < WM; i++) ldg_words<V>(a0 + i * a_plane + w, in && i < wa, av[i] + V * u);
 #pragma unroll
-      for (int j = 0; j < WM; j++) bv[j][u] = (in && j < wb) ? __ldg(b0 + j * b_plane + w) : 0ull;
+      for (int j = 0; j < WM; j++) ldg_words<V>(b0 + j * b_plane + w, in && j < wb, bv[j] + V * u);
     }
 #pragma unroll
     for (int i = 0; i < WM; i++) {
@@ -345,7 +357,8 @@ __device__ __forceinline__ uint32_t skinny_lane_sum_t(const uint64_t *__restrict
         if (j >= wb) break;
         uint32_t c = 0;
 #pragma unroll
-        for (int u = 0; u < U; u++) c += (uint32_t)(use_xor ? __popcll(av[i][u] ^ bv[j][u]) : __popcll(av[i][u] & bv[j][u]));
+        for (int u = 0; u < U * V; u++)
+          c += (uint32_t)(use_xor ? __popcll(av[i][u] ^ bv[j][u]) : __popcll(av[i][u] & bv[j][u]));
         acc += c * alpha(i, j);
       }
     }
@@ -353,21 +366,37 @@ __device__ __forceinline__ uint32_t skinny_lane_sum_t(const uint64_t *__restrict
   return acc;
 }
 
+// Rows of an even number of words from a 16-byte boundary load two words at a
+// time: rows of 9216 columns then take one step, not two, and half the loads.
 template <typename Alpha>
 __device__ __forceinline__ uint32_t skinny_lane_sum(const uint64_t *__restrict__ a0, uint64_t a_plane,
                                                     const uint64_t *__restrict__ b0, uint64_t b_plane, uint64_t wpr,
                                                     int wa, int wb, bool use_xor, int lane, Alpha alpha) {
   const int wm = wa > wb ? wa : wb;
-  if (wm <= 1) return skinny_lane_sum_t<1, 4>(a0, a_plane, b0, b_plane, wpr, wa, wb, use_xor, lane, alpha);
-  if (wm <= 2) return skinny_lane_sum_t<2, 4>(a0, a_plane, b0, b_plane, wpr, wa, wb, use_xor, lane, alpha);
-  if (wm <= 4) return skinny_lane_sum_t<4, 2>(a0, a_plane, b0, b_plane, wpr, wa, wb, use_xor, lane, alpha);
-  return skinny_lane_sum_t<kMaxBits, 1>(a0, a_plane, b0, b_plane, wpr, wa, wb, use_xor, lane, alpha);
+  const bool two = ((wpr | a_plane | b_plane) & 1) == 0 && (((uintptr_t)a0 | (uintptr_t)b0) & 15) == 0;
+  if (wm <= 1) {
+    if (two) return skinny_lane_sum_t<1, 4, 2>(a0, a_plane, b0, b_plane, wpr, wa, wb, use_xor, lane, alpha);
+    return skinny_lane_sum_t<1, 4, 1>(a0, a_plane, b0, b_plane, wpr, wa, wb, use_xor, lane, alpha);
+  }
+  if (wm <= 2) {
+    if (two) return skinny_lane_sum_t<2, 3, 2>(a0, a_plane, b0, b_plane, wpr, wa, wb, use_xor, lane, alpha);
+    return skinny_lane_sum_t<2, 4, 1>(a0, a_plane, b0, b_plane, wpr, wa, wb, use_xor, lane, alpha);
+  }
+  if (wm <= 4) return skinny_lane_sum_t<4, 2, 1>(a0, a_plane, b0, b_plane, wpr, wa, wb, use_xor, lane, alpha);
+  return skinny_lane_sum_t<kMaxBits, 1, 1>(a0, a_plane, b0, b_plane, wpr, wa, wb, use_xor, lane, alpha);
 }
 
 // One output (m, n) of a grouped problem by one warp, lanes over the K words
 // (the skinny tile class: matrix-vector and other small-output problems).
 __device__ __forceinline__ void grouped_skinny_output(const GroupProblem &P, uint64_t o, int lane) {
-  const uint64_t n = o / P.M, m = o % P.M;
+  uint64_t n, m;
+  if (o <= 0xFFFFFFFFull && P.M <= 0xFFFFFFFFull) {  // 32-bit division in the common case
+    n = (uint32_t)o / (uint32_t)P.M;
+    m = (uint32_t)o - (uint32_t)n * (uint32_t)P.M;
+  } else {
+    n = o / P.M;
+    m = o - n * P.M;
+  }
   uint32_t acc = skinny_lane_sum(P.A + m * P.wpr, P.a_plane, P.B + n * P.wpr, P.b_plane, P.wpr, P.wa, P.wb,
                                  P.use_xor != 0, lane,
                                  [&](int i, int j) { return alpha_of(i, j, P.neg_i, P.neg_j, P.shift, P.use_xor); });

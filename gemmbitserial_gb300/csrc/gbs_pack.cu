@@ -695,8 +695,7 @@ __device__ __forceinline__ int find_job(const PackJob *jobs, int njobs, uint64_t
 }
 
 // One launch packs every operand of a grouped GEMM whose rows are 1-byte and
-// 16-byte aligned.  A run is `run` units of one job (pack_run_units: up to
-// kMaxRun, fewer when the group would leave warps without one); a warp takes
+// 16-byte aligned.  A run is `run` units of one job (pack_run_units); a warp takes
 // runs in a grid stride and keeps kDepth units' loads in flight.
 // HBM-bound on large groups: 7.7 GB of the 512-problem mix (1-byte sources in,
 // planes and packed or digit matrices out) in 1.23 ms, 0.92 of the copy rate;
@@ -941,11 +940,13 @@ bool pack_job_direct(PackJob &j, const Mat &m) {
 
 uint64_t pack_job_units(const PackJob &j) { return (j.nrows_a * j.cpr + 31) / 32; }
 
-// Units per run of a grouped import of `units` units: four runs for each of 32
-// warps on 152 SMs before a run grows past one unit (CaffeNet's 1.2 M unaligned
-// bytes in runs of 8 were 147 warps and 48 us).
+// Units per run of a grouped import of `units` units: two runs for each of 32
+// warps on 152 SMs, whole pairs of units up to kMaxRun; finding a run's job and
+// first row costs as much as two units.  CaffeNet's 61 K units take 19.7 us in runs
+// of 8, 21.8 in runs of 3, and 23.8 in runs of 14, one to a warp.
 uint32_t pack_run_units(uint64_t units) {
-  return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(kMaxRun, units / (4 * 152 * 32)));
+  const uint64_t each = (units + 152 * 64 - 1) / (152 * 64);
+  return (uint32_t)(each <= 1 ? 1 : std::min<uint64_t>(kMaxRun, (each + kDepth - 1) / kDepth * kDepth));
 }
 
 namespace {

@@ -1,10 +1,10 @@
-"""Packed plans of a group's tensor-core problems: every width and encoding of the larger side as 4- or 6-bit floats,
+"""Matrix-vector problems of the popcount kernels, and packed plans of a group's tensor-core problems: every width and encoding of the larger side as 4- or 6-bit floats,
 written by the grouped import and by the expansion of planes that single imports left, at the tiles' edges."""
 import numpy as np
 import pytest
 
 from gemmbitserial_gb300 import _capi, datagen
-from gemmbitserial_gb300.api import allocGEMMContext, deallocGEMMContext
+from gemmbitserial_gb300.api import allocGEMMContext, deallocGEMMContext, gemmBitSerial
 from gemmbitserial_gb300.grouped import Group
 
 pytestmark = pytest.mark.gpu
@@ -52,6 +52,36 @@ def test_packed_plan(bits, enc, expanded, monkeypatch):
         assert g.status() == _capi.GBS_OK
         for c, (a, b) in zip(ctxs, ops):
             want = b.astype(np.int64) @ a.astype(np.int64).T
+            assert np.array_equal(c.res.reshape(want.shape), want)
+    finally:
+        g.free()
+        for c in ctxs:
+            deallocGEMMContext(c)
+
+
+@pytest.mark.parametrize("bits", [(1, 1), (2, 2), (1, 2), (3, 1)])
+@pytest.mark.parametrize("K", [1, 255, 8192, 12288, 12289, 24600])
+def test_matrix_vector(bits, K):
+    """Steps of two words a lane at their edges, in the grouped kernel and the single one."""
+    import torch
+    wa, wb = bits
+    rng = np.random.default_rng(K)
+    dims, ops, ctxs = [(1, 1), (37, 1), (3, 2)], [], []
+    for M, N in dims:
+        ops.append((rng.integers(0, 1 << wa, (M, K)).astype(np.int8), rng.integers(0, 1 << wb, (N, K)).astype(np.int8)))
+        ctxs.append(allocGEMMContext(M, K, N, wa, wb, False, False))
+    g = Group(ctxs)
+    try:
+        dev = [(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()) for a, b in ops]
+        g.import_([a for a, _ in dev], [b for _, b in dev])
+        g.gemm()
+        torch.cuda.synchronize()
+        assert g.status() == _capi.GBS_OK
+        for c, (a, b) in zip(ctxs, ops):
+            want = b.astype(np.int64) @ a.astype(np.int64).T
+            assert np.array_equal(c.res.reshape(want.shape), want)
+            c.set_pipe(_capi.GBS_PIPE_POPC)
+            gemmBitSerial(c)
             assert np.array_equal(c.res.reshape(want.shape), want)
     finally:
         g.free()
