@@ -448,8 +448,12 @@ __device__ __forceinline__ void store_cols(const TmaArgs &a, const uint32_t (&v)
   store_result_cols<32>(a.C, a.M, a.N, gm, n0, o);
 }
 
+// Eight epilogue warps where a whole tile is stored at the kernel's end, half its
+// columns each.
+constexpr int pair_threads(int splits) { return splits == 1 ? 64 + 8 * 32 : kPairThreads; }
+
 template <int SPLITS, int BN>
-__global__ void __launch_bounds__(kPairThreads, 1)
+__global__ void __launch_bounds__(pair_threads(SPLITS), 1)
     gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, TmaArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -585,20 +589,17 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       const uint64_t gm = m0 + q * 32 + lane;
       const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16);
       if (SPLITS == 1) {
-        // four 32-column TMEM loads behind one wait: tcgen05.wait::ld waits
-        // for all of a thread's loads, so the latency is paid once per 128
-        // columns
-#pragma unroll 1
-        for (int col = 0; col < BN; col += 128) {
-          uint32_t v[4][32];
+        // the warp's 32-column TMEM loads behind one wait: tcgen05.wait::ld
+        // waits for all of a thread's loads, so the latency is paid once
+        const int col = ((warp - 2) >> 2) * (BN / 2);
+        uint32_t v[BN / 64][32];
 #pragma unroll
-          for (int i = 0; i < 4; i++) tmem_ld32(taddr + (uint32_t)(col + 32 * i), v[i]);
-          tmem_wait_ld(v[0]);
+        for (int i = 0; i < BN / 64; i++) tmem_ld32(taddr + (uint32_t)(col + 32 * i), v[i]);
+        tmem_wait_ld(v[0]);
 #pragma unroll
-          for (int i = 1; i < 4; i++) tmem_after_wait(v[i]);
+        for (int i = 1; i < BN / 64; i++) tmem_after_wait(v[i]);
 #pragma unroll
-          for (int i = 0; i < 4; i++) store_cols(a, v[i], gm, n0 + col + 32 * i);
-        }
+        for (int i = 0; i < BN / 64; i++) store_cols(a, v[i], gm, n0 + col + 32 * i);
       } else {
         // the columns the other K chunks reduce go into the drained ring as
         // [64 column quads][128 rows][4 columns] fp32: each lane (row) writes,
@@ -1420,7 +1421,7 @@ void pair_launch_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&attr)[2],
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
   cfg = cudaLaunchConfig_t{};
-  cfg.blockDim = dim3(kPairThreads);
+  cfg.blockDim = dim3(pair_threads(splits));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   attr[0].id = cudaLaunchAttributeClusterDimension;
