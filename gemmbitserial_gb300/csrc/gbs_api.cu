@@ -130,7 +130,7 @@ void free_ctx_buffers(gbs_ctx *c) {
   small_plan_free(c->small);
   wide_plan_free(c->wide);
   if (c->sk_ws) cudaFree(c->sk_ws);
-  if (c->split_ws) cudaFree(c->split_ws);
+  if (c->split_owned) cudaFree(c->split_owned);
   if (c->sk_flags) cudaFree(c->sk_flags);
   if (c->digits[0]) cudaFree(c->digits[0]);
   if (c->digits[1]) cudaFree(c->digits[1]);

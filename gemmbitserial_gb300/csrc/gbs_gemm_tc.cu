@@ -1607,6 +1607,53 @@ bool pdl_for(cudaStream_t s) {
   return st == cudaStreamCaptureStatusNone;
 }
 
+namespace {
+
+// Tile width, K split inside a cluster, and K split over independent pairs (1:
+// none; otherwise it is taken instead, on 256-column tiles) of an M x N GEMM.
+struct PairRule {
+  int bn, splits;
+  uint32_t gather;
+};
+
+// A split inside a cluster sums partials over distributed shared memory, which
+// costs more the more chunks there are: candidates in order of preference, the
+// first that keeps at least half the SM pairs busy in one wave wins, else the one
+// that keeps the most busy.  (An M=256 N=128 pair MMA takes as long as an N=256
+// one, so narrow tiles only pay where they replace a wider split.)
+PairRule pair_rule(uint64_t M, uint64_t N, uint32_t nstages) {
+  static const int cand[6][2] = {{256, 1}, {256, 2}, {128, 1}, {128, 2}, {256, 4}, {128, 4}};
+  const uint64_t mt = (M + 255) / 256, pairs = (uint64_t)sm_count_cached() / 2;
+  PairRule r{256, 1, 1};
+  uint64_t best_used = 0;
+  for (const auto &cv : cand) {
+    const int cb = cv[0], cs = cv[1];
+    const uint64_t tiles = mt * ((N + cb - 1) / cb);
+    if (cs > 1 && (nstages / cs < 8 || tiles > (uint64_t)pair_max_clusters(cs, cb))) continue;
+    const uint64_t used = std::min<uint64_t>(tiles * cs, pairs);
+    if (used > best_used) {
+      best_used = used;
+      r.bn = cb;
+      r.splits = cs;
+    }
+    if (2 * used >= pairs) break;
+  }
+  // Few tiles and a long K: 256 x 256 tiles split over independent pairs, where
+  // that is estimated faster than the choice above (measured: 0.35 us a stage,
+  // whatever the width, and 6 us a launch, split in a cluster or not)
+  const uint64_t chosen = mt * ((N + r.bn - 1) / r.bn) * r.splits;
+  const double us = (double)((chosen + pairs - 1) / pairs) * 0.35 * (nstages / r.splits) + 6.0;
+  r.gather = pair_gather_splits(mt * ((N + 255) / 256), nstages, pairs, us);
+  return r;
+}
+
+}  // namespace
+
+uint32_t pair_gather_choice(const gbs_ctx *c) {
+  if (c->lhs.nrows < 256 || c->rhs.nrows < 256) return 1;
+  return pair_rule(c->lhs.nrows, c->rhs.nrows, (uint32_t)(c->lhs.dcols / 128)).gather;
+}
+
 cudaError_t launch_gemm_tc_hbm(gbs_ctx *c, cudaStream_t s, int bn_req) {
   const bool small = bn_req < 0 && (c->lhs.nrows < 256 || c->rhs.nrows < 256);
   if (small && (c->plan1_ready || tcg_packed_mode() == 1)) {
@@ -1650,12 +1697,6 @@ cudaError_t launch_gemm_tc_hbm(gbs_ctx *c, cudaStream_t s, int bn_req) {
   if (bn_req == kPairVariant || bn_req == kPairVariant128 || bn_req == kPairVariantPersistent || bn_req < 0 ||
       pair_split_variant(bn_req)) {
     // 256 x BN tiles on SM pairs
-    // Tile width and K split.  A split sums partials over distributed shared
-    // memory, which costs more the more chunks there are: candidates in order
-    // of preference, the first that keeps at least half the SM pairs busy in
-    // one wave wins, else the one that keeps the most busy.  (An M=256 N=128
-    // pair MMA takes as long as an N=256 one, so narrow tiles only pay where
-    // they replace a wider split.)
     const uint64_t mt = (a.M + 255) / 256;
     int bn = bn_req == kPairVariant128 ? 128 : 256;
     int splits = pair_splits(mt * ((a.N + bn - 1) / bn), a.nstages, bn);
@@ -1667,36 +1708,15 @@ cudaError_t launch_gemm_tc_hbm(gbs_ctx *c, cudaStream_t s, int bn_req) {
         splits = 1;  // every K chunk needs a stage, and all clusters of the grid must fit at once
     }
     if (bn_req < 0) {
-      const uint64_t pairs = (uint64_t)sm_count_cached() / 2;
-      static const int cand[6][2] = {{256, 1}, {256, 2}, {128, 1}, {128, 2}, {256, 4}, {128, 4}};
-      uint64_t best_used = 0;
-      for (const auto &cv : cand) {
-        const int cb = cv[0], cs = cv[1];
-        const uint64_t tiles = mt * ((a.N + cb - 1) / cb);
-        if (cs > 1 && (a.nstages / cs < 8 || tiles > (uint64_t)pair_max_clusters(cs, cb))) continue;
-        const uint64_t used = std::min<uint64_t>(tiles * cs, pairs);
-        if (used > best_used) {
-          best_used = used;
-          bn = cb;
-          splits = cs;
-        }
-        if (2 * used >= pairs) break;
-      }
-    }
-    if (bn_req < 0) {
-      // Few tiles and a long K: 256 x 256 tiles split over independent pairs, where
-      // that is estimated faster than the choice above (measured: 0.35 us a stage,
-      // whatever the width, and 6 us a launch, split in a cluster or not)
-      const uint64_t pairs = (uint64_t)sm_count_cached() / 2, tiles = mt * ((a.N + 255) / 256);
-      const uint64_t chosen = mt * ((a.N + bn - 1) / bn) * splits;
-      const double us = (double)((chosen + pairs - 1) / pairs) * 0.35 * (a.nstages / splits) + 6.0;
-      const uint32_t gather = pair_gather_splits(tiles, a.nstages, pairs, us);
-      if (gather > 1 && ensure_split_workspace(c, tiles, gather, s)) {
+      const PairRule r = pair_rule(a.M, a.N, a.nstages);
+      bn = r.bn;
+      splits = r.splits;
+      if (r.gather > 1 && ensure_split_workspace(c, r.gather, s)) {
         c->last_pair_bn = 256;
-        c->last_pair_splits = (int)gather;
+        c->last_pair_splits = (int)r.gather;
         c->last_pair_persistent = false;
         c->last_pair_streamk = 0;
-        return launch_pair_gather(c, c->tc_map_da, c->tc_map_db, gather, s);
+        return launch_pair_gather(c, c->tc_map_da, c->tc_map_db, r.gather, s);
       }
     }
     if (bn == 128 && !c->digit_map_b64_ready) {

@@ -469,12 +469,12 @@ cudaError_t launch_expand(const ExpandJob &job, cudaStream_t s) {
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-// Allocates a zeroed buffer.  With a stream (order) the zeroing is queued there,
+// Allocates a zeroed buffer (and `more` bytes behind it, as they come).  With a stream (order) the zeroing is queued there,
 // before whatever that stream does with the buffer next; into a capture, where it
 // would be recorded instead, and without a stream it is done before returning.
 // (Waiting for the device on each buffer was most of a new context's first call.)
-cudaError_t alloc_zeroed(void **p, size_t bytes, const cudaStream_t *order) {
-  cudaError_t e = dev_alloc(p, bytes);
+cudaError_t alloc_zeroed(void **p, size_t bytes, const cudaStream_t *order, size_t more) {
+  cudaError_t e = dev_alloc(p, bytes + more);
   if (e != cudaSuccess) return e;
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusActive;
   if (order && cudaStreamIsCapturing(*order, &st) != cudaSuccess) cudaGetLastError();
@@ -492,11 +492,15 @@ cudaError_t alloc_zeroed(void **p, size_t bytes, const cudaStream_t *order) {
 }
 
 // Digit matrix [drows][dcols] of one side, allocated zeroed on first use
-// (order: alloc_zeroed).
+// (order: alloc_zeroed); the first of a context's two also holds the workspace of
+// its K-split GEMM, where it will run one (not for a group's plan, without order).
 cudaError_t ensure_digit_buffer(gbs_ctx *c, int side, const cudaStream_t *order) {
   if (c->digits[side]) return cudaSuccess;
   const Mat &m = side ? c->rhs : c->lhs;
-  cudaError_t e = alloc_zeroed((void **)&c->digits[side], std::max<size_t>(m.drows * m.dcols, 16), order);
+  const size_t digits = std::max<size_t>(m.drows * m.dcols, 16);
+  const size_t ws = order && !c->split_ws ? split_workspace_bytes(c) : 0, zeroed = ws ? split_workspace_zeroed(c) : 0;
+  cudaError_t e = alloc_zeroed((void **)&c->digits[side], digits + zeroed, order, ws - zeroed);
+  if (e == cudaSuccess && ws) set_split_workspace(c, c->digits[side] + digits);
   c->digit_maps_ready = false;
   c->digit_map_b64_ready = false;
   c->plan1_ready = false;

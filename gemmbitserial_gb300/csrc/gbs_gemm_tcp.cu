@@ -244,6 +244,11 @@ __global__ void __launch_bounds__(kSpThreads, 1)
   }
 }
 
+uint64_t split_tiles(const gbs_ctx *c) { return ((c->lhs.nrows + 255) / 256) * ((c->rhs.nrows + 255) / 256); }
+size_t split_counter_bytes(const gbs_ctx *c, uint32_t splits) {
+  return (split_tiles(c) * 8 * splits * sizeof(uint32_t) + 255) / 256 * 256;
+}
+
 template <int SPLITS>
 cudaError_t launch(const CUtensorMap &ma, const CUtensorMap &mb, const SplitArgs &a, cudaStream_t s) {
   uint32_t *err = tc_error_ptr();
@@ -292,26 +297,38 @@ uint32_t pair_gather_splits(uint64_t tiles, uint32_t nstages, uint64_t pairs, do
   return best;
 }
 
-// The context's workspace for `tiles` tiles in `splits`, allocated (counters
-// zeroed) on first use; false when it cannot be, as into a capture.
-bool ensure_split_workspace(gbs_ctx *c, uint64_t tiles, uint32_t splits, cudaStream_t s) {
+// Bytes of a context's workspace, the arrival counters first; 0 where the rule does
+// not split its K.  It is laid out behind the first digit matrix the context
+// allocates: an allocation of its own cost the context's first GEMM 45 us.
+size_t split_workspace_bytes(const gbs_ctx *c) {
+  const uint32_t splits = pair_gather_choice(c);
+  return splits > 1 ? split_counter_bytes(c, splits) + split_tiles(c) * splits * 8 * 2048 * sizeof(float4) : 0;
+}
+size_t split_workspace_zeroed(const gbs_ctx *c) { return split_counter_bytes(c, pair_gather_choice(c)); }
+void set_split_workspace(gbs_ctx *c, void *p) {
+  c->split_counters = static_cast<uint32_t *>(p);
+  c->split_ws = static_cast<uint8_t *>(p) + split_counter_bytes(c, pair_gather_choice(c));
+}
+
+// The same for a context whose digits are another's (a part of a wide operand's):
+// false when it cannot be allocated, as into a capture.
+bool ensure_split_workspace(gbs_ctx *c, uint32_t splits, cudaStream_t s) {
   if (c->split_ws) return true;  // a context keeps its shape, and the rule its choice
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
     cudaGetLastError();
     return false;
   }
-  const size_t ws = tiles * splits * 8 * 2048 * sizeof(float4), counters = tiles * 8 * splits * sizeof(uint32_t);
   void *p = nullptr;  // not a capture: the zeroing below is queued before the GEMM that counts
-  cudaError_t e = dev_alloc(&p, ws + counters);
-  if (e == cudaSuccess) e = cudaMemsetAsync(static_cast<uint8_t *>(p) + ws, 0, counters, s);
+  cudaError_t e = dev_alloc(&p, split_workspace_bytes(c));
+  if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, split_counter_bytes(c, splits), s);
   if (e != cudaSuccess) {
     cudaGetLastError();
     if (p) cudaFree(p);
     return false;
   }
-  c->split_ws = p;
-  c->split_counters = reinterpret_cast<uint32_t *>(static_cast<uint8_t *>(p) + ws);
+  c->split_owned = p;
+  set_split_workspace(c, p);
   return true;
 }
 

@@ -240,9 +240,11 @@ struct gbs_ctx {
   float *sk_ws = nullptr;
   uint32_t *sk_flags = nullptr;
   uint32_t sk_pairs = 0, sk_epoch = 0;
-  // K-split SM pairs (gbs_gemm_tcp.cu): partial columns, and the arrival counters after them
+  // K-split SM pairs (gbs_gemm_tcp.cu): partial columns and arrival counters, behind a digit
+  // matrix or in an allocation of their own (split_owned)
   void *split_ws = nullptr;
   uint32_t *split_counters = nullptr;
+  void *split_owned = nullptr;
   gbs::SmallPlan *small = nullptr;  // a side under 256 rows: built on first use
   // one-problem packed plan of the persistent kernel, where that is forced on such a context
   gbs::TcgPlan *plan1 = nullptr;
@@ -360,7 +362,7 @@ int tcg_plan_build(TcgPlan *plan, gbs_ctx *const *ctxs, int n);
 void tcg_plan_free(TcgPlan *plan);
 cudaError_t tcg_expand(TcgPlan &plan, cudaStream_t s);
 cudaError_t tcg_gemm(const TcgPlan &plan, uint32_t *err, cudaStream_t s, int32_t *out0 = nullptr);
-cudaError_t alloc_zeroed(void **p, size_t bytes, const cudaStream_t *order);
+cudaError_t alloc_zeroed(void **p, size_t bytes, const cudaStream_t *order, size_t more = 0);
 cudaError_t ensure_digit_buffer(gbs_ctx *c, int side, const cudaStream_t *order = nullptr);
 cudaError_t ensure_packed_buffer(gbs_ctx *c, int side, const cudaStream_t *order = nullptr);
 bool tc_map_packed(void *map, const uint8_t *base, uint64_t cols, uint64_t rows);
@@ -368,7 +370,11 @@ bool tc_map_packed(void *map, const uint8_t *base, uint64_t cols, uint64_t rows)
 int tcg_packed_mode();
 // SM-pair tiles with K split, partial tiles summed through L2 (gbs_gemm_tcp.cu)
 uint32_t pair_gather_splits(uint64_t tiles, uint32_t nstages, uint64_t pairs, double other_us);
-bool ensure_split_workspace(gbs_ctx *c, uint64_t tiles, uint32_t splits, cudaStream_t s);
+uint32_t pair_gather_choice(const gbs_ctx *c);  // of the context's built-in rule, 1: none
+size_t split_workspace_bytes(const gbs_ctx *c);
+size_t split_workspace_zeroed(const gbs_ctx *c);  // of those, at the start, zero before the first GEMM
+void set_split_workspace(gbs_ctx *c, void *p);
+bool ensure_split_workspace(gbs_ctx *c, uint32_t splits, cudaStream_t s);
 cudaError_t launch_pair_gather(gbs_ctx *c, const void *map_a, const void *map_b, uint32_t splits, cudaStream_t s);
 // one context with a side under 256 rows on its digit matrices (gbs_gemm_tcs.cu)
 cudaError_t launch_gemm_tcs(gbs_ctx *c, cudaStream_t s);

@@ -491,7 +491,7 @@ void wide_plan_free(WidePlan *p) {
       }
       small_plan_free(s->small);
       if (s->sk_ws) cudaFree(s->sk_ws);
-      if (s->split_ws) cudaFree(s->split_ws);
+      if (s->split_owned) cudaFree(s->split_owned);
       if (s->sk_flags) cudaFree(s->sk_flags);
       for (uint8_t *pk : s->packed)
         if (pk) cudaFree(pk);
