@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // TMA-fed GEMM on digit matrices: 128 x BN output tile per CTA.
 //   warp 0     TMA: A box 128 rows x 128 bytes, B boxes 128 rows x 128 bytes
 //              (BN/128 of them), 128-byte swizzle = the MMA's K-major layout
-//   warp 1     TMEM allocation; lane 0 issues 4 tcgen05.mma (K = 32) per stage
+//   warp 1     TMEM allocation; an elected lane issues 4 tcgen05.mma (K = 32) per stage
 //   warps 2-9  epilogue: TMEM -> int32 -> res[n*M + m]
 constexpr int kTmaStagesMax = 4;
 constexpr int kTmaThreads = 320;
@@ -429,10 +429,10 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
 // 128-column tiles double the tile count for shapes with few tiles.
 //   warp 0     in the leader: TMA of both CTAs' halves of every stage onto
 //              the leader's full barrier (the peer's into its shared memory)
-//   warp 1     TMEM allocation (both CTAs, collectively); in the leader, lane
-//              0 issues the MMAs and commits to the empty / accumulator
-//              barriers of both CTAs (multicast)
-//   warps 2-5  epilogue of this CTA's 128 rows
+//   warp 1     TMEM allocation (both CTAs, collectively); in the leader, an
+//              elected lane issues the MMAs and commits to the empty /
+//              accumulator barriers of both CTAs (multicast)
+//   warps 2-5  epilogue of this CTA's 128 rows (2-9 without a K split)
 // A cluster barrier closes the kernel, so no CTA frees TMEM or exits while
 // its peer may still signal its barriers or write its accumulator.
 constexpr int kPairStagesMax = 9;
@@ -449,7 +449,7 @@ __device__ __forceinline__ void store_cols(const TmaArgs &a, const uint32_t (&v)
 }
 
 // Eight epilogue warps where a whole tile is stored at the kernel's end, half its
-// columns each.
+// columns each: 2048 x 4096 x 2048 back to back 17.1 -> 16.8 us.
 constexpr int pair_threads(int splits) { return splits == 1 ? 64 + 8 * 32 : kPairThreads; }
 
 template <int SPLITS, int BN>

@@ -469,9 +469,10 @@ cudaError_t launch_expand(const ExpandJob &job, cudaStream_t s) {
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-// Allocates a zeroed buffer (and `more` bytes behind it, as they come).  With a stream (order) the zeroing is queued there,
-// before whatever that stream does with the buffer next; into a capture, where it
-// would be recorded instead, and without a stream it is done before returning.
+// Allocates a zeroed buffer (and `more` bytes behind it, as they come).  With a
+// stream (order) the zeroing is queued there, before whatever that stream does with
+// the buffer next; into a capture, where it would be recorded instead, and without a
+// stream it is done before returning.
 // (Waiting for the device on each buffer was most of a new context's first call.)
 cudaError_t alloc_zeroed(void **p, size_t bytes, const cudaStream_t *order, size_t more) {
   cudaError_t e = dev_alloc(p, bytes + more);

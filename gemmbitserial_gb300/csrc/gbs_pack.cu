@@ -697,10 +697,11 @@ __device__ __forceinline__ int find_job(const PackJob *jobs, int njobs, uint64_t
 // One launch packs every operand of a grouped GEMM whose rows are 1-byte and
 // 16-byte aligned.  A run is `run` units of one job (pack_run_units); a warp takes
 // runs in a grid stride and keeps kDepth units' loads in flight.
-// HBM-bound on large groups: 7.7 GB of the 512-problem mix (1-byte sources in,
-// planes and packed or digit matrices out) in 1.23 ms, 0.92 of the copy rate;
-// one strided pair of 16-byte loads per lane, a unit to a row segment and a
-// binary search per run took 2.17 ms.
+// Bound by integer instructions beside HBM on large groups: 8.1 GB of the
+// 512-problem mix (1-byte sources in, planes and packed or digit matrices out) in
+// 1.34 ms, 0.9 of the copy rate, 0.69 instructions a cycle and scheduler; one strided
+// pair of 16-byte loads per lane, a unit to a row segment and a binary search per run
+// took 2.17 ms.
 constexpr int kMaxRun = 8;
 constexpr int kDepth = 2;
 
@@ -974,8 +975,8 @@ cudaError_t run_staged(const PackJob &j, const void *thr, int nthres, bool quant
   with_source(j.dtype, aligned, [&](auto t, auto al) {
     using T = decltype(t);
     constexpr bool A = decltype(al)::value;
-    e = launch_pdl(quant ? pack_staged<T, true, A> : pack_staged<T, false, A>, blocks_for(units * 32, 256), 256, 0, s, j,
-                   (const T *)thr, nthres, r0, r1, units);
+    const auto kern = quant ? pack_staged<T, true, A> : pack_staged<T, false, A>;
+    e = launch_pdl(kern, blocks_for(units * 32, 256), 256, 0, s, j, (const T *)thr, nthres, r0, r1, units);
   });
   count_launch();
   return e != cudaSuccess ? e : cudaGetLastError();
@@ -988,8 +989,8 @@ cudaError_t run_colmajor(const PackJob &j, const void *thr, int nthres, bool qua
   with_source(j.dtype, aligned4(j.src, j.dtype, j.nrows), [&](auto t, auto al) {
     using T = decltype(t);
     constexpr bool A = decltype(al)::value;
-    e = launch_pdl(quant ? pack_colmajor<T, true, A> : pack_colmajor<T, false, A>, (unsigned)blocks, kCmThreads, 0, s, j,
-                   (const T *)thr, nthres);
+    const auto kern = quant ? pack_colmajor<T, true, A> : pack_colmajor<T, false, A>;
+    e = launch_pdl(kern, (unsigned)blocks, kCmThreads, 0, s, j, (const T *)thr, nthres);
   });
   count_launch();
   return e != cudaSuccess ? e : cudaGetLastError();
@@ -1049,7 +1050,7 @@ cudaError_t launch_rowsum_grouped(const PackJob *jobs, int njobs, uint64_t total
   if (total_warps == 0 || njobs == 0) return cudaSuccess;
   const uint64_t blocks = (total_warps + 7) / 8;
   const cudaError_t e =
-      launch_pdl(rowsum_grouped, (unsigned)(blocks < 152 * 64 ? blocks : 152 * 64), 256, 0, s, jobs, njobs, total_warps);
+      launch_pdl(rowsum_grouped, (unsigned)std::min<uint64_t>(blocks, 152 * 64), 256, 0, s, jobs, njobs, total_warps);
   count_launch();
   return e != cudaSuccess ? e : cudaGetLastError();
 }

@@ -11,18 +11,23 @@ prints "ok <case>".  The kernels each case launches:
   gemm_popc       the same on the CUDA cores (gemm_popc_tiled)
   gemm_bmma       the same on b1 mma.sync (gemm_bmma_kernel)
   gemm_tc_smem    the same, planes decoded in shared memory (gemm_tc_kernel)
+  gemm_split      256x9216x4096 bp x bp, the library's choice (gemm_tc_pair_split_kernel)
+  gemm_two        4096x2048x2048 u2 x bp, the library's choice (gemm_tc_pair_persistent_kernel)
+  gemm_wide       2048x4096x2048 s8 x s8, the library's choice (gemm_wide_pair_kernel)
+  gemm_small      384 x 2304 x 169 u2 x u2, the library's choice (gemm_tcs_kernel)
   gemm_skinny     8x8192x8 u1 x u1 (gemm_popc_skinny)
   gemm_rows       9 x 8192 x 32768, 1-bit unsigned x 2-bit signed on the CUDA cores (gemm_popc_rows: at most
                   16 lhs rows, 64 rhs rows x every lhs row per CTA)
-  import_device   importRegular of the 2048x4096 int8 lhs from device memory, planes + digits (pack_rowmajor)
-  import_host     the same from pinned host memory, read over the host link (pack_rowmajor)
+  import_device   importRegular of the 2048x4096 int8 lhs from device memory, planes + digits (pack_bytes)
+  import_host     the same from pinned host memory, read over the host link (pack_bytes)
   import_colmajor the same operand read column-major (pack_colmajor)
-  import_quantize importRegularAndQuantize of a 2048x4096 float lhs, 7 thresholds per row (pack_quantize_kernel)
-  expand          column-major imports, then a forward that first expands the planes (expand_one_kernel)
+  import_quantize importRegularAndQuantize of a 2048x4096 float lhs, 7 thresholds per row (pack_staged)
+  expand          imports for the CUDA cores, then a tensor-core forward that first expands the planes
+                  (expand_one_kernel)
   group           the 512-problem mix as one group: import, row sums, GEMMs (pack_grouped, rowsum_grouped,
                   gemm_tcg_kernel, gemm_popc_grouped)
   group_small     the same on a 96-problem mix of the same distribution (a few hundred MB on the device)
-  adjoint         A 4096x2048 u2, B 2048x2048 bipolar, dC ~ N(0,1) (split_kernel, values_t_kernel, adjoint_tc_kernel)
+  adjoint         A 4096x2048 u2, B 2048x2048 bipolar, dC ~ N(0,1) (adjoint_prepare, adjoint_tc_kernel)
   adjoint_simt    the same on the CUDA cores (adjoint_kernel)
 """
 from __future__ import annotations
@@ -32,9 +37,9 @@ import ctypes as C
 import os
 import sys
 
-CASES = ["gemm", "gemm_streamk", "gemm_popc", "gemm_bmma", "gemm_tc_smem", "gemm_skinny", "gemm_rows", "import_device",
-         "import_host", "import_colmajor", "import_quantize", "expand", "group", "group_small", "adjoint",
-         "adjoint_simt"]
+CASES = ["gemm", "gemm_streamk", "gemm_popc", "gemm_bmma", "gemm_tc_smem", "gemm_split", "gemm_two", "gemm_wide",
+         "gemm_small", "gemm_skinny", "gemm_rows", "import_device", "import_host", "import_colmajor", "import_quantize",
+         "expand", "group", "group_small", "adjoint", "adjoint_simt"]
 
 
 def main() -> None:
@@ -74,9 +79,19 @@ def main() -> None:
             pipe = _capi.GBS_PIPE_BMMA
         elif case == "gemm_tc_smem":
             pipe, variant = _capi.GBS_PIPE_TC_SMEM, 256
+        elif case == "gemm_split":
+            name = "gemm_256x9216x4096_bpbp"
+        elif case == "gemm_two":
+            name = "gemm_4096x2048x2048_u2bp"
+        elif case == "gemm_wide":
+            name = "gemm_2048x4096x2048_s8s8"
         elif case == "gemm_skinny":
             name = "gemm_8x8192x8_u1u1"
-        if case == "gemm_rows":
+        if case == "gemm_small":
+            c = allocGEMMContext(384, 2304, 169, 2, 2, False, False)
+            dA = torch.from_numpy(datagen.operand(datagen.SEED_BASE + 63, 384, 2304, 2, "u")).to(dev)
+            dB = torch.from_numpy(datagen.operand(datagen.SEED_BASE + 64, 169, 2304, 2, "u")).to(dev)
+        elif case == "gemm_rows":
             c = allocGEMMContext(9, 8192, 32768, 1, 2, False, True)
             c.set_pipe(_capi.GBS_PIPE_POPC)
             dA = torch.from_numpy(datagen.operand(datagen.SEED_BASE + 61, 9, 8192, 1, "u")).to(dev)
@@ -108,11 +123,12 @@ def main() -> None:
                                                               C.c_void_p(T.data_ptr()), 7, _capi.GBS_F32, 0, sh))
     elif case == "expand":
         c, dA, dB = ctx_of("gemm_2048x4096x2048_u3s2")
-        aT, bT = dA.t().contiguous(), dB.t().contiguous()
 
-        def run():  # column-major imports write no digits: the forward expands them first
-            _capi.check(lib.gbs_import(c._h, 0, C.c_void_p(aT.data_ptr()), _capi.GBS_I8, 1, sh))
-            _capi.check(lib.gbs_import(c._h, 1, C.c_void_p(bT.data_ptr()), _capi.GBS_I8, 1, sh))
+        def run():  # imports for another pipe write no digits: the forward expands them first
+            c.set_pipe(_capi.GBS_PIPE_POPC)
+            _capi.check(lib.gbs_import(c._h, 0, C.c_void_p(dA.data_ptr()), _capi.GBS_I8, 0, sh))
+            _capi.check(lib.gbs_import(c._h, 1, C.c_void_p(dB.data_ptr()), _capi.GBS_I8, 0, sh))
+            c.set_pipe(_capi.GBS_PIPE_TC)
             _capi.check(lib.gbs_gemm(c._h, sh))
     elif case in ("group", "group_small"):
         from gemmbitserial_gb300.grouped import Group

@@ -1,5 +1,6 @@
-"""Matrix-vector problems of the popcount kernels, and packed plans of a group's tensor-core problems: every width and encoding of the larger side as 4- or 6-bit floats,
-written by the grouped import and by the expansion of planes that single imports left, at the tiles' edges."""
+"""Packed plans of a group's tensor-core problems: every width and encoding of the larger side, as 4-bit floats where
+they allow it, written by the grouped import and by the expansion of planes that single imports left, at the tiles'
+edges; and the popcount kernels' matrix-vector outputs."""
 import numpy as np
 import pytest
 
