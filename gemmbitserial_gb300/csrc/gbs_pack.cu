@@ -50,18 +50,31 @@ __device__ __forceinline__ void emit_planes32(int nbits, uint32_t *__restrict__ 
   }
 }
 
-// e4m3 digits of 4 codes (one per byte): the code's low nbits bits index the
-// 16-entry byte table tab (byte-permute lookup; PRMT reads only 3 index bits,
-// so 4-bit codes take the high half of the table when bit 3 is set).
-__device__ __forceinline__ uint32_t digits4(uint32_t x, int nbits, uint4 tab) {
-  const uint32_t xm = x & (0x01010101u * ((1u << nbits) - 1u));
-  const uint32_t t = xm | (xm >> 4);                  // byte 0 = c0 | c1 << 4, byte 2 = c2 | c3 << 4
-  const uint32_t sel = __byte_perm(t, 0u, 0x0020u);   // nibbles c0 c1 c2 c3
-  if (nbits <= 3) return __byte_perm(tab.x, tab.y, sel);
-  const uint32_t lo = __byte_perm(tab.x, tab.y, sel & 0x7777u);
-  const uint32_t hi = __byte_perm(tab.z, tab.w, sel & 0x7777u);
-  const uint32_t m = ((xm >> 3) & 0x01010101u) * 0xFFu;
-  return (lo & ~m) | (hi & m);
+// Byte permute by 4-bit selectors: bit 3 of one gives the sign bit of the byte it
+// names, eight times.
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+  return r;
+}
+
+// e4m3 digits of 8 codes (bytes of q0 and q1, bits above nbits ignored) out of the
+// 16-entry byte table tab.  The codes' low bits, gathered eight to a word, are the
+// selectors of a byte permute.  Of 4-bit codes the permute of the low half of the
+// table, all of it positive, leaves 0 where bit 3 is set, the permute of the high
+// half without its signs by the inverted bit 3 leaves 0 elsewhere, and the signs, one
+// for the half, follow bit 3.
+__device__ __forceinline__ void digits8(uint32_t q0, uint32_t q1, int nbits, uint32_t msk, uint4 tab, uint32_t &d0,
+                                        uint32_t &d1) {
+  const uint32_t sel = (__byte_perm(q0, q1, 0x7531u) & msk) * 16u + (__byte_perm(q0, q1, 0x6420u) & msk);
+  d0 = prmt(tab.x, tab.y, sel);
+  d1 = prmt(tab.x, tab.y, sel >> 16);
+  if (nbits > 3) {
+    const uint32_t inv = sel ^ 0x88888888u, sign = tab.z & 0x80808080u;
+    const uint32_t z = tab.z & 0x7F7F7F7Fu, w = tab.w & 0x7F7F7F7Fu;
+    d0 |= prmt(z, w, inv) | (q0 * 16u & sign);
+    d1 |= prmt(z, w, inv >> 16) | (q1 * 16u & sign);
+  }
 }
 
 // The lane's 32 digits (0 past ncols) into the digit matrix (dcols columns,
@@ -69,9 +82,10 @@ __device__ __forceinline__ uint32_t digits4(uint32_t x, int nbits, uint4 tab) {
 // and columns past the planes' padded width stay as allocated: zero.
 __device__ __forceinline__ void write_digits32(uint8_t *__restrict__ digits, int nbits, uint32_t ncols, uint64_t dcols,
                                                uint4 tab, uint32_t r, uint32_t col0, const uint32_t (&q)[8]) {
+  const uint32_t msk = 0x01010101u * ((1u << nbits) - 1u);
   uint32_t d[8];
 #pragma unroll
-  for (int i = 0; i < 8; i++) d[i] = digits4(q[i], nbits, tab);
+  for (int i = 0; i < 8; i += 2) digits8(q[i], q[i + 1], nbits, msk, tab, d[i], d[i + 1]);
   if (col0 + 32 > ncols) {
 #pragma unroll
     for (int i = 0; i < 8; i++) {
