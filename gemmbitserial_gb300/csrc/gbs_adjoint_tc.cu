@@ -601,7 +601,7 @@ struct AdjPlan {
   __nv_bfloat16 *split = nullptr;  // [3][N][pM]
   __nv_bfloat16 *val[2] = {};      // lhs values [M][pK], rhs values [N][pK]
   CUtensorMap xk, xmn, va, vb;
-  float *part = nullptr;      // split tiles' sums and flags (AdjTcArgs), when a deal splits
+  float *part = nullptr;      // split tiles' sums and flags (AdjTcArgs), behind the operands, when a deal splits
   uint32_t *flags = nullptr;
   uint32_t nflags = 0;
   AdjDeal deal[4];            // by the wanted gradients: bit 0 dB, bit 1 dA
@@ -610,8 +610,6 @@ struct AdjPlan {
 void adj_plan_free(AdjPlan *p) {
   if (!p) return;
   if (p->ws) cudaFree(p->ws);
-  if (p->part) cudaFree(p->part);
-  if (p->flags) cudaFree(p->flags);
   delete p;
 }
 
@@ -711,28 +709,6 @@ int build_plan(gbs_ctx *c) {
   const uint64_t M = c->lhs.nrows, N = c->rhs.nrows, K = c->lhs.ncols;
   const uint64_t pM = pitch64(M), pK = pitch64(K), term = N * pM;
   AdjPlan *p = new AdjPlan();
-  // every array starts on a 128-byte boundary: the pitches are multiples of 64 values
-  const size_t bytes = (3 * term + (M + N) * pK) * sizeof(__nv_bfloat16);
-  if (dev_alloc((void **)&p->ws, bytes) != cudaSuccess) {
-    cudaGetLastError();
-    delete p;
-    return fail(GBS_ENOMEM, "gbs_adjoint: workspace allocation failed");
-  }
-  p->split = p->ws;
-  p->val[0] = p->ws + 3 * term;
-  p->val[1] = p->val[0] + M * pK;
-  // dB: rows n, contraction m (contiguous); the true M and N bound the boxes, past them reads are 0
-  const cuuint64_t dk[3] = {M, N, 3}, sk[2] = {pM * 2, term * 2};
-  const cuuint32_t bk[3] = {(cuuint32_t)kAdjKs, 128, 3};
-  // dA: rows m (contiguous, 64 at a time), contraction n
-  const cuuint64_t dmn[4] = {64, N, pM / 64, 3}, smn[3] = {pM * 2, 128, term * 2};
-  const cuuint32_t bmn[4] = {64, (cuuint32_t)kAdjKs, 2, 3};
-  if (!bf16_map(&p->xk, p->split, 3, dk, sk, bk, CU_TENSOR_MAP_SWIZZLE_128B) ||
-      !bf16_map(&p->xmn, p->split, 4, dmn, smn, bmn, CU_TENSOR_MAP_SWIZZLE_128B) ||
-      !values_map(&p->va, p->val[0], M, pK) || !values_map(&p->vb, p->val[1], N, pK)) {
-    adj_plan_free(p);
-    return fail(GBS_EUNSUPPORTED, "gbs_adjoint: tensor map encoding failed");
-  }
   const int max_pairs = adj_max_pairs();
   if (!max_pairs) {
     adj_plan_free(p);
@@ -749,14 +725,34 @@ int build_plan(gbs_ctx *c) {
     p->deal[want] = deal_tiles(first, n[first], cost[first], n[1 - first], cost[1 - first], pairs);
     if (p->deal[want].pieces > 1 || p->deal[want].fpieces > 1) split_pairs = std::max(split_pairs, pairs);
   }
+  p->nflags = 2 * split_pairs * 2 * kAdjEpiWarps;
+  // One allocation: operands (every array starts on a 128-byte boundary: the pitches are multiples of 64 values),
+  // then the split tiles' sums and flags
+  const size_t bytes = ((3 * term + (M + N) * pK) * sizeof(__nv_bfloat16) + 255) / 256 * 256;
+  const size_t sums = (size_t)p->nflags * 4096 * sizeof(float);
+  if (dev_alloc((void **)&p->ws, bytes + sums + p->nflags * sizeof(uint32_t)) != cudaSuccess) {
+    cudaGetLastError();
+    delete p;
+    return fail(GBS_ENOMEM, "gbs_adjoint: workspace allocation failed");
+  }
   if (split_pairs) {
-    p->nflags = 2 * split_pairs * 2 * kAdjEpiWarps;
-    if (dev_alloc((void **)&p->part, (size_t)p->nflags * 4096 * sizeof(float)) != cudaSuccess ||
-        dev_alloc((void **)&p->flags, (size_t)p->nflags * sizeof(uint32_t)) != cudaSuccess) {
-      cudaGetLastError();
-      adj_plan_free(p);
-      return fail(GBS_ENOMEM, "gbs_adjoint: workspace allocation failed");
-    }
+    p->part = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(p->ws) + bytes);
+    p->flags = reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>(p->part) + sums);
+  }
+  p->split = p->ws;
+  p->val[0] = p->ws + 3 * term;
+  p->val[1] = p->val[0] + M * pK;
+  // dB: rows n, contraction m (contiguous); the true M and N bound the boxes, past them reads are 0
+  const cuuint64_t dk[3] = {M, N, 3}, sk[2] = {pM * 2, term * 2};
+  const cuuint32_t bk[3] = {(cuuint32_t)kAdjKs, 128, 3};
+  // dA: rows m (contiguous, 64 at a time), contraction n
+  const cuuint64_t dmn[4] = {64, N, pM / 64, 3}, smn[3] = {pM * 2, 128, term * 2};
+  const cuuint32_t bmn[4] = {64, (cuuint32_t)kAdjKs, 2, 3};
+  if (!bf16_map(&p->xk, p->split, 3, dk, sk, bk, CU_TENSOR_MAP_SWIZZLE_128B) ||
+      !bf16_map(&p->xmn, p->split, 4, dmn, smn, bmn, CU_TENSOR_MAP_SWIZZLE_128B) ||
+      !values_map(&p->va, p->val[0], M, pK) || !values_map(&p->vb, p->val[1], N, pK)) {
+    adj_plan_free(p);
+    return fail(GBS_EUNSUPPORTED, "gbs_adjoint: tensor map encoding failed");
   }
   c->adj = p;
   return GBS_OK;

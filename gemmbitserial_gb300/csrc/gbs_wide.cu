@@ -338,18 +338,22 @@ void scale_table(uint32_t (&tab)[4], int power) {
 }
 
 cudaError_t alloc_parts(const gbs_ctx *c, const WidePlan &p, uint8_t *(&digits)[2][2]) {
-  // (both sides' buffers at once, which the two imports may write on different streams: zeroed before returning)
+  // (both sides' buffers at once, which the two imports may write on different streams: zeroed before returning;
+  // one allocation, whose start is the lhs's first part)
+  if (digits[0][0]) return cudaSuccess;
+  size_t bytes[2], total = 0;
   for (int side = 0; side < 2; side++) {
     const Mat &m = side ? c->rhs : c->lhs;
-    const size_t bytes = std::max<size_t>(m.drows * m.dcols, 16);
-    for (int k = 0; k < p.parts[side]; k++) {
-      if (digits[side][k]) continue;
-      if (alloc_zeroed((void **)&digits[side][k], bytes, nullptr) != cudaSuccess) {
-        cudaGetLastError();
-        return cudaErrorMemoryAllocation;
-      }
-    }
+    bytes[side] = std::max<size_t>(m.drows * m.dcols, 256);
+    total += p.parts[side] * bytes[side];
   }
+  uint8_t *at = nullptr;
+  if (alloc_zeroed((void **)&at, total, nullptr) != cudaSuccess) {
+    cudaGetLastError();
+    return cudaErrorMemoryAllocation;
+  }
+  for (int side = 0; side < 2; side++)
+    for (int k = 0; k < p.parts[side]; k++, at += bytes[side]) digits[side][k] = at;
   return cudaSuccess;
 }
 
@@ -497,10 +501,8 @@ void wide_plan_free(WidePlan *p) {
         if (pk) cudaFree(pk);
       delete s;  // its planes alias the parent's, its digit matrices are the plan's
     }
-  for (auto &form : {&p->digits, &p->sep})
-    for (auto &side : *form)
-      for (uint8_t *d : side)
-        if (d) cudaFree(d);
+  for (uint8_t *d : {p->digits[0][0], p->sep[0][0]})  // each form's one allocation
+    if (d) cudaFree(d);
   if (p->partial) cudaFree(p->partial);
   delete p;
 }
