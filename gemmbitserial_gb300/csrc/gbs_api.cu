@@ -465,6 +465,7 @@ int gbs_import(gbs_ctx *c, int side, const void *src, int dtype, int col_major, 
   cudaStream_t s = as_stream(stream);
   c->digits_valid[side] = c->packed_valid[side] = false;
   c->vt_valid[side] = false;
+  release_split_workspace(c, s);
   DigitTarget target;
   const DigitTarget *digits = import_digit_target(c, side, target, s) ? &target : nullptr;
   cudaError_t e = cudaSuccess;
@@ -553,6 +554,7 @@ int gbs_import_quantize(gbs_ctx *c, int side, const void *src, const void *thres
   cudaStream_t s = as_stream(stream);
   c->digits_valid[side] = c->packed_valid[side] = false;
   c->vt_valid[side] = false;
+  release_split_workspace(c, s);
   DigitTarget target;
   const DigitTarget *digits = import_digit_target(c, side, target, s) ? &target : nullptr;
   bool host = false;

@@ -12,10 +12,15 @@
 // pairs of a tile are independent: each leaves its partial columns in a
 // workspace (L2), and for every share of the columns the pair that arrives last
 // adds the others' to its own, still in TMEM, and stores the result.  Nobody
-// depends on anybody's progress, so any number of such GEMMs may run at once; but
-// a pair looks at its own share for 2 us before leaving that too, so pairs in
+// depends on anybody's progress, so any number of contexts' GEMMs may run at once;
+// but a pair looks at its own share for 2 us before leaving that too, so pairs in
 // step each sum their own.  (A fence, a counter and a look per share, one after
 // the other, cost 2.7 us more.)
+//
+// The workspace is the context's, so two such GEMMs of one context must not
+// overlap: one stream at a time owns it (ensure_split_workspace), and a GEMM on
+// another stream, or recorded into a graph, splits inside clusters instead, which
+// keeps nothing outside the launch.
 #include <algorithm>
 #include <cstring>
 
@@ -310,16 +315,31 @@ void set_split_workspace(gbs_ctx *c, void *p) {
   c->split_ws = static_cast<uint8_t *>(p) + split_counter_bytes(c, pair_gather_choice(c));
 }
 
-// The same for a context whose digits are another's (a part of a wide operand's):
-// false when it cannot be allocated, as into a capture.
-bool ensure_split_workspace(gbs_ctx *c, uint32_t splits, cudaStream_t s) {
-  if (c->split_ws) return true;  // a context keeps its shape, and the rule its choice
+static bool in_capture(cudaStream_t s) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
+  if (cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone) return false;
+  cudaGetLastError();
+  return true;
+}
+
+// The context's workspace for a GEMM on s; false where it has none, or where a
+// GEMM that may still run holds it.  Launches of one stream follow each other, so
+// the stream that first takes the workspace keeps it (by its id: a handle may be
+// another stream's later) until an import gives it back.  A graph replays on any
+// stream, so none is recorded with it.  A context whose digits are another's (a
+// part of a wide operand's) gets an allocation of its own here.
+bool ensure_split_workspace(gbs_ctx *c, uint32_t splits, cudaStream_t s) {
+  unsigned long long id = 0;
+  if (in_capture(s)) return false;
+  if (cudaStreamGetId(s, &id) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  void *p = nullptr;  // not a capture: the zeroing below is queued before the GEMM that counts
+  if (c->split_taken && c->split_stream != id) return false;
+  c->split_taken = true;
+  c->split_stream = id;
+  if (c->split_ws) return true;  // a context keeps its shape, and the rule its choice
+  void *p = nullptr;             // the zeroing below is queued before the GEMM that counts
   cudaError_t e = dev_alloc(&p, split_workspace_bytes(c));
   if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, split_counter_bytes(c, splits), s);
   if (e != cudaSuccess) {
@@ -330,6 +350,13 @@ bool ensure_split_workspace(gbs_ctx *c, uint32_t splits, cudaStream_t s) {
   c->split_owned = p;
   set_split_workspace(c, p);
   return true;
+}
+
+// An import on s: it overwrites what the context's earlier GEMMs read, so it is
+// ordered after them, and the GEMMs of what it imports after it.  Their stream may
+// be another.
+void release_split_workspace(gbs_ctx *c, cudaStream_t s) {
+  if (c->split_taken && !in_capture(s)) c->split_taken = false;
 }
 
 cudaError_t launch_pair_gather(gbs_ctx *c, const void *map_a, const void *map_b, uint32_t splits, cudaStream_t s) {

@@ -245,6 +245,8 @@ struct gbs_ctx {
   void *split_ws = nullptr;
   uint32_t *split_counters = nullptr;
   void *split_owned = nullptr;
+  bool split_taken = false;  // a GEMM since the last import uses them, on the stream of id split_stream
+  unsigned long long split_stream = 0;
   gbs::SmallPlan *small = nullptr;  // a side under 256 rows: built on first use
   // one-problem packed plan of the persistent kernel, where that is forced on such a context
   gbs::TcgPlan *plan1 = nullptr;
@@ -375,6 +377,7 @@ size_t split_workspace_bytes(const gbs_ctx *c);
 size_t split_workspace_zeroed(const gbs_ctx *c);  // of those, at the start, zero before the first GEMM
 void set_split_workspace(gbs_ctx *c, void *p);
 bool ensure_split_workspace(gbs_ctx *c, uint32_t splits, cudaStream_t s);
+void release_split_workspace(gbs_ctx *c, cudaStream_t s);
 cudaError_t launch_pair_gather(gbs_ctx *c, const void *map_a, const void *map_b, uint32_t splits, cudaStream_t s);
 // one context with a side under 256 rows on its digit matrices (gbs_gemm_tcs.cu)
 cudaError_t launch_gemm_tcs(gbs_ctx *c, cudaStream_t s);

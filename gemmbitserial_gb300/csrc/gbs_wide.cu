@@ -452,7 +452,10 @@ cudaError_t expand_parts(gbs_ctx *c, const WidePlan &p, bool fused, cudaStream_t
     if (!fused)  // the parts' own packed matrices (one-problem plans) are stale too
       for (auto &row : p.sub)
         for (gbs_ctx *sub : row)
-          if (sub) sub->packed_valid[side] = false;
+          if (sub) {
+            sub->packed_valid[side] = false;
+            release_split_workspace(sub, s);
+          }
     valid[side] = true;
   }
   return cudaSuccess;
