@@ -77,13 +77,7 @@ __device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) { mbar
 // mbar_wait with a given number of rounds (the test hook's short limit)
 __device__ __forceinline__ bool mbar_wait_rounds(uint32_t bar, uint32_t parity, volatile int *abort_flag,
                                                  uint32_t rounds) {
-  for (uint32_t it = 0; it < rounds; ++it) {
-    if (mbar_try(bar, parity)) return true;
-    if (*abort_flag) return false;
-  }
-  *abort_flag = 1;
-  atomicOr(&g_tc_error, 1u);
-  return false;
+  return mbar_wait_rounds_err(bar, parity, abort_flag, &g_tc_error, rounds);
 }
 
 // One tile row of one stage: CNT planes (16 bytes each, `pstride` apart) ->
@@ -1898,42 +1892,64 @@ uint32_t tc_error_word() {
 
 using namespace gbs;
 
-// Test hook of the tensor-core kernels' bounded waits: one launch of the
-// SM-pair kernel that loads and multiplies nothing, so its first wait gives up
-// after `rounds` try_wait rounds; the kernel then takes its abort path (error
-// bit, bounded drains, TMEM freed, clean exit) and the host reads the error.
-extern "C" int gbs_debug_tc_timeout(gbs_ctx *c, uint32_t rounds, void *stream) {
-  if (!c || rounds == 0) return fail(GBS_EINVAL, "gbs_debug_tc_timeout: NULL context or zero rounds");
-  if (!c->lhs.imported || !c->rhs.imported) return fail(GBS_ESTATE, "gbs_debug_tc_timeout: import both operands first");
-  if (!tc_exact(c, GBS_PIPE_TC) || c->lhs.nrows < 256 || c->rhs.nrows < 256)
-    return fail(GBS_EUNSUPPORTED, "gbs_debug_tc_timeout: needs a context the SM-pair kernel runs (M, N >= 256)");
+// Test hooks of the tensor-core kernels' bounded waits: `launch` issues one
+// kernel some or all of whose pairs load and multiply nothing, so their first wait
+// gives up after `rounds` try_wait rounds; they then take the kernel's abort path
+// (error bit, bounded drains, TMEM freed, clean exit) and the host reads the error.
+template <typename F>
+static int timeout_probe(gbs_ctx *c, uint32_t rounds, void *stream, const char *who, F launch) {
+  const std::string name(who);
   int prev = -1;
   if (cudaGetDevice(&prev) != cudaSuccess || cudaSetDevice(c->device) != cudaSuccess)
-    return cuda_fail(cudaGetLastError(), "gbs_debug_tc_timeout: cudaSetDevice");
+    return cuda_fail(cudaGetLastError(), (name + ": cudaSetDevice").c_str());
   cudaStream_t s = (cudaStream_t)stream;
   const uint32_t zero = 0;
   cudaError_t e = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_tc_error, &zero, sizeof(zero));
-  const int saved_pipe = c->pipe, saved_variant = c->variant;
   int rc = GBS_OK;
   if (e == cudaSuccess) {
-    c->pipe = GBS_PIPE_TC;
-    c->variant = 2561;  // one 256 x 256 tile per SM pair, no K split
     c->debug_wait_limit = rounds;
-    rc = gbs_gemm(c, stream);
+    rc = launch(s);
     c->debug_wait_limit = 0;
-    c->pipe = saved_pipe;
-    c->variant = saved_variant;
     e = cudaStreamSynchronize(s);
   }
   uint32_t err = 0;
   if (e == cudaSuccess) e = cudaMemcpyFromSymbol(&err, g_tc_error, sizeof(err));
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_tc_error, &zero, sizeof(zero));
   if (prev >= 0) cudaSetDevice(prev);
-  if (e != cudaSuccess) return cuda_fail(e, "gbs_debug_tc_timeout");
+  if (e != cudaSuccess) return cuda_fail(e, who);
   if (rc != GBS_OK) return rc;
-  if (err) return fail(GBS_ETIMEOUT, "gbs_debug_tc_timeout: the kernel's bounded wait gave up (error bits " +
-                                         std::to_string(err) + "); it drained, freed TMEM and returned");
-  return fail(GBS_EINVAL, "gbs_debug_tc_timeout: the wait did not run out");
+  if (err) return fail(GBS_ETIMEOUT, name + ": the kernel's bounded wait gave up (error bits " + std::to_string(err) +
+                                         "); it drained, freed TMEM and returned");
+  return fail(GBS_EINVAL, name + ": the wait did not run out");
 }
 
+extern "C" int gbs_debug_tc_timeout(gbs_ctx *c, uint32_t rounds, void *stream) {
+  if (!c || rounds == 0) return fail(GBS_EINVAL, "gbs_debug_tc_timeout: NULL context or zero rounds");
+  if (!c->lhs.imported || !c->rhs.imported) return fail(GBS_ESTATE, "gbs_debug_tc_timeout: import both operands first");
+  if (!tc_exact(c, GBS_PIPE_TC) || c->lhs.nrows < 256 || c->rhs.nrows < 256)
+    return fail(GBS_EUNSUPPORTED, "gbs_debug_tc_timeout: needs a context the SM-pair kernel runs (M, N >= 256)");
+  return timeout_probe(c, rounds, stream, "gbs_debug_tc_timeout", [&](cudaStream_t) {
+    const int saved_pipe = c->pipe, saved_variant = c->variant;
+    c->pipe = GBS_PIPE_TC;
+    c->variant = 2561;  // one 256 x 256 tile per SM pair, no K split
+    const int rc = gbs_gemm(c, stream);
+    c->pipe = saved_pipe;
+    c->variant = saved_variant;
+    return rc;
+  });
+}
+
+extern "C" int gbs_debug_split_timeout(gbs_ctx *c, uint32_t rounds, void *stream) {
+  if (!c || rounds == 0) return fail(GBS_EINVAL, "gbs_debug_split_timeout: NULL context or zero rounds");
+  if (!c->lhs.imported || !c->rhs.imported)
+    return fail(GBS_ESTATE, "gbs_debug_split_timeout: import both operands first");
+  return timeout_probe(c, rounds, stream, "gbs_debug_split_timeout", [&](cudaStream_t s) {
+    const uint32_t splits = tc_exact(c, GBS_PIPE_TC) ? pair_gather_choice(c) : 1;
+    if (splits == 1 || !ensure_split_workspace(c, splits, s))
+      return fail(GBS_EUNSUPPORTED, "gbs_debug_split_timeout: the context's GEMM on this stream does not split K over "
+                                    "independent SM pairs");
+    const cudaError_t e = launch_gemm_tc_hbm(c, s, -1);
+    return e == cudaSuccess ? GBS_OK : cuda_fail(e, "gbs_debug_split_timeout");
+  });
+}

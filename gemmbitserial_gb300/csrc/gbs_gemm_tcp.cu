@@ -44,6 +44,7 @@ struct SplitArgs {
   uint32_t nstages, idesc;
   float4 *ws;          // [tile][split][CTA][warp][64 column quads][32 rows]
   uint32_t *arrived;   // [tile][CTA][warp][share]: pairs that have left or hold their columns; 0 between launches
+  uint32_t wait_limit; // test hook: the pairs of split 0 load nothing and wait this many rounds (0: normal launches)
 };
 
 template <int SPLITS>
@@ -61,6 +62,7 @@ __global__ void __launch_bounds__(kSpThreads, 1)
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   const uint32_t m0 = (blockIdx.x >> 1) * 256, n0 = blockIdx.y * 256, split = blockIdx.z;
   const uint32_t k_lo = split * a.nstages / SPLITS, nk = (split + 1) * a.nstages / SPLITS - k_lo;
+  const bool idle = a.wait_limit != 0 && split == 0;  // of the test hook
   griddep_launch_dependents();
   if (tid == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmA)) : "memory");
@@ -95,7 +97,7 @@ __global__ void __launch_bounds__(kSpThreads, 1)
   griddep_wait();  // operands, result and workspace belong to earlier kernels until here
 
   if (warp == 0) {
-    if (peer == 0) {  // the leader's TMA: both CTAs' halves of every stage
+    if (peer == 0 && !idle) {  // the leader's TMA: both CTAs' halves of every stage
       uint32_t k = 0;
       for (; k < nk; k++) {
         const uint32_t s = k % kSpStages, use = k / kSpStages;
@@ -119,8 +121,8 @@ __global__ void __launch_bounds__(kSpThreads, 1)
     }
   } else if (warp == 1) {
     if (peer == 0) {
-      bool ok = true;
-      for (uint32_t k = 0; k < nk; k++) {
+      bool ok = !idle || __all_sync(0xffffffffu, mbar_wait_rounds_err(full, 0, abort_flag, err, a.wait_limit));
+      for (uint32_t k = 0; k < nk && ok; k++) {
         const uint32_t s = k % kSpStages;
         if (!__all_sync(0xffffffffu, mbar_wait_err(full + 8 * s, (k / kSpStages) & 1, abort_flag, err))) {
           ok = false;
@@ -145,7 +147,11 @@ __global__ void __launch_bounds__(kSpThreads, 1)
         mbar_drain_err(mma_done, 0, err);
       }
     }
-  } else if (__all_sync(0xffffffffu, mbar_wait_err(acc_full, 0, abort_flag, err))) {
+  } else {
+    // A pair whose wait gave up counts in all the same, with nothing left or stored: the counters end at 0, and only
+    // this launch's results, which the error word disowns, are wrong.
+    const bool done = __all_sync(0xffffffffu, idle ? mbar_wait_rounds_err(acc_full, 0, abort_flag, err, a.wait_limit)
+                                                   : mbar_wait_err(acc_full, 0, abort_flag, err));
     asm volatile("tcgen05.fence::after_thread_sync;");
     constexpr uint32_t kShare = 256 / SPLITS;  // columns of a share
     constexpr int kBatch = SPLITS - 1 < 3 ? SPLITS - 1 : 3;  // others' columns in flight
@@ -170,7 +176,7 @@ __global__ void __launch_bounds__(kSpThreads, 1)
       }
     };
 #pragma unroll 1
-    for (uint32_t j = 1; j < SPLITS; j++) leave((split + j) % SPLITS);
+    for (uint32_t j = 1; j < SPLITS && done; j++) leave((split + j) % SPLITS);
     __threadfence();
     __syncwarp();
     // lane l counts this pair in for share l, all shares but its own at once
@@ -186,7 +192,7 @@ __global__ void __launch_bounds__(kSpThreads, 1)
       }
     __syncwarp();
     if (__shfl_sync(0xffffffffu, count, split) != SPLITS - 1) {
-      leave(split);
+      if (done) leave(split);
       __threadfence();
       __syncwarp();
       if (lane == split) count = atomicAdd(arrived + lane, 1u);
@@ -198,6 +204,7 @@ __global__ void __launch_bounds__(kSpThreads, 1)
       const uint32_t share = __ffs(mine) - 1;
       mine &= mine - 1;
       if (lane == 0) arrived[share] = 0u;  // ready for the next launch
+      if (!done) continue;
 #pragma unroll 1
       for (uint32_t c = share * kShare; c < (share + 1) * kShare; c += 32) {
         float4 r[kBatch][8];  // the others' loads first
@@ -368,6 +375,7 @@ cudaError_t launch_pair_gather(gbs_ctx *c, const void *map_a, const void *map_b,
   a.idesc = (1u << 4) | ((256u >> 3) << 17) | ((256u >> 4) << 24);
   a.ws = static_cast<float4 *>(c->split_ws);
   a.arrived = c->split_counters;
+  a.wait_limit = c->debug_wait_limit;
   const CUtensorMap &ma = *reinterpret_cast<const CUtensorMap *>(map_a);
   const CUtensorMap &mb = *reinterpret_cast<const CUtensorMap *>(map_b);
   if (splits == 8) return launch<8>(ma, mb, a, s);

@@ -32,16 +32,21 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 // Bounded wait: true when the phase completed; false on abort or timeout.
-// A timeout raises the CTA's abort flag and sets bit 0 of *err.
-__device__ __forceinline__ bool mbar_wait_err(uint32_t bar, uint32_t parity, volatile int *abort_flag,
-                                              uint32_t *err) {
-  for (uint32_t it = 0; it < kTcWaitLimit; ++it) {
+// A timeout raises the CTA's abort flag and sets bit 0 of *err.  The number of
+// rounds is kTcWaitLimit but for the test hooks'.
+__device__ __forceinline__ bool mbar_wait_rounds_err(uint32_t bar, uint32_t parity, volatile int *abort_flag,
+                                                     uint32_t *err, uint32_t rounds) {
+  for (uint32_t it = 0; it < rounds; ++it) {
     if (mbar_try(bar, parity)) return true;
     if (*abort_flag) return false;
   }
   *abort_flag = 1;
   atomicOr(err, 1u);
   return false;
+}
+__device__ __forceinline__ bool mbar_wait_err(uint32_t bar, uint32_t parity, volatile int *abort_flag,
+                                              uint32_t *err) {
+  return mbar_wait_rounds_err(bar, parity, abort_flag, err, kTcWaitLimit);
 }
 // Bounded wait that ignores the abort flag: drains work this thread issued.
 // A timeout sets bit 1 of *err.

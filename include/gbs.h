@@ -406,6 +406,14 @@ GBS_API int gbs_debug_group_tc_kernel(const gbs_group *g);
  * result buffer is not written.  No reference counterpart. */
 GBS_API int gbs_debug_tc_timeout(gbs_ctx *ctx, uint32_t rounds, void *stream);
 
+/* The same for the kernel that splits K over independent SM pairs (few 256 x
+ * 256 tiles and a long K, by the built-in rule): the pairs of the first K part
+ * load nothing and give up, the others run.  The result buffer's contents are
+ * undefined until the next GEMM, which is as good as any.  GBS_EUNSUPPORTED
+ * where the context's GEMM on `stream` is another kernel's.  No reference
+ * counterpart. */
+GBS_API int gbs_debug_split_timeout(gbs_ctx *ctx, uint32_t rounds, void *stream);
+
 /* Number of kernel launches the library has issued since load (all entry points). */
 GBS_API uint64_t gbs_debug_launch_count(void);
 
