@@ -50,7 +50,8 @@ struct gbs_group {
   uint64_t rs_warps = 0;
   PackTable imports, captured;  // of gbs_group_import, and of the captured graph (which keeps reading it)
   std::vector<gbs::PackJob *> foreign;  // tables of imports recorded into a caller's own capture
-  cudaEvent_t packed = nullptr;  // the last import's pack: its table may be written again
+  cudaEvent_t packed = nullptr;  // after the last pack that read imports.jobs: that table may be written again
+  bool packed_set = false;       // it has been recorded, which no capture ever does
   size_t smem = 0;
   int grid = 0;
   cudaGraph_t graph = nullptr;
@@ -168,6 +169,7 @@ int build_pack_jobs(gbs_group *g, PackTable &tab, const void *const *lhs, const 
     }
   } else if (e == cudaSuccess && tab.host.size() <= (size_t)kInlinePackJobs) {
     tab.with_launch = true;
+    tab.recorded = nullptr;
   } else if (e == cudaSuccess) {
     if (tab.capacity < bytes) {
       if (tab.jobs) cudaFree(tab.jobs);  // waits for the device: nothing reads the old table any more
@@ -175,7 +177,7 @@ int build_pack_jobs(gbs_group *g, PackTable &tab, const void *const *lhs, const 
       tab.capacity = 0;
       e = dev_alloc((void **)&tab.jobs, bytes);
       if (e == cudaSuccess) tab.capacity = bytes;
-    } else {
+    } else if (g->packed_set) {
       e = cudaStreamWaitEvent(s, g->packed, 0);
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(tab.jobs, tab.host.data(), bytes, cudaMemcpyHostToDevice, s);
@@ -433,7 +435,10 @@ int gbs_group_import(gbs_group *g, const void *const *lhs_srcs, const void *cons
   int rc = build_pack_jobs(g, g->imports, lhs_srcs, rhs_srcs, dtypes, (cudaStream_t)stream);
   if (rc != GBS_OK) return rc;
   cudaError_t e = enqueue_pack(g->imports, (cudaStream_t)stream);
-  if (e == cudaSuccess) e = cudaEventRecord(g->packed, (cudaStream_t)stream);
+  if (e == cudaSuccess && !g->imports.with_launch && !g->imports.recorded) {
+    e = cudaEventRecord(g->packed, (cudaStream_t)stream);
+    g->packed_set = e == cudaSuccess;
+  }
   if (e != cudaSuccess) return cuda_fail(e, "gbs_group_import: pack kernel");
   for (gbs_ctx *c : g->ctxs) {
     c->lhs.imported = c->rhs.imported = true;
