@@ -466,6 +466,11 @@ int gbs_group_capture(gbs_group *g, const void *const *lhs_srcs, const void *con
   if (!stream)  // CUDA cannot capture the legacy default stream
     return fail(GBS_EINVAL, "gbs_group_capture: capture needs a created stream, not the legacy default stream");
   const bool with_pack = lhs_srcs && rhs_srcs;
+  // a stream under capture cannot begin another, and waiting for it below would end the caller's
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  cudaError_t ce = cudaStreamIsCapturing((cudaStream_t)stream, &st);
+  if (ce == cudaSuccess && st != cudaStreamCaptureStatusNone) ce = cudaErrorIllegalState;
+  if (ce != cudaSuccess) return cuda_fail(ce, "gbs_group_capture: the stream is being captured");
   if (with_pack) {
     // a graph captured before may still run and read its table; the new table is there before any replay
     cudaError_t se = g->captured.jobs ? cudaDeviceSynchronize() : cudaSuccess;
