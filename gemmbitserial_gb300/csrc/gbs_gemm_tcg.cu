@@ -472,20 +472,30 @@ cudaError_t launch_expand(const ExpandJob &job, cudaStream_t s) {
 // Allocates a zeroed buffer (and `more` bytes behind it, as they come).  With a
 // stream (order) the zeroing is queued there, before whatever that stream does with
 // the buffer next; into a capture, where it would be recorded instead, and without a
-// stream it is done before returning.
+// stream it is done before returning, on a stream of its own: neither the device nor
+// the default stream can be waited for while some stream is captured.  The thread's
+// capture mode is relaxed meanwhile: an allocation is part of no capture and
+// disturbs none.
 // (Waiting for the device on each buffer was most of a new context's first call.)
 cudaError_t alloc_zeroed(void **p, size_t bytes, const cudaStream_t *order, size_t more) {
-  cudaError_t e = dev_alloc(p, bytes + more);
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
   if (e != cudaSuccess) return e;
+  e = dev_alloc(p, bytes + more);
+  const bool allocated = e == cudaSuccess;
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusActive;
   if (order && cudaStreamIsCapturing(*order, &st) != cudaSuccess) cudaGetLastError();
-  if (order && st == cudaStreamCaptureStatusNone) {
+  if (allocated && order && st == cudaStreamCaptureStatusNone) {
     e = cudaMemsetAsync(*p, 0, bytes, *order);
-  } else {
-    e = cudaMemset(*p, 0, bytes);
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  } else if (allocated) {
+    cudaStream_t own = nullptr;
+    e = cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMemsetAsync(*p, 0, bytes, own);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(own);
+    if (own) cudaStreamDestroy(own);
   }
-  if (e != cudaSuccess) {
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (allocated && e != cudaSuccess) {
     cudaFree(*p);
     *p = nullptr;
   }
