@@ -511,7 +511,12 @@ cudaError_t ensure_digit_buffer(gbs_ctx *c, int side, const cudaStream_t *order)
   const size_t digits = std::max<size_t>(m.drows * m.dcols, 16);
   const size_t ws = order && !c->split_ws ? split_workspace_bytes(c) : 0, zeroed = ws ? split_workspace_zeroed(c) : 0;
   cudaError_t e = alloc_zeroed((void **)&c->digits[side], digits + zeroed, order, ws - zeroed);
-  if (e == cudaSuccess && ws) set_split_workspace(c, c->digits[side] + digits);
+  if (e == cudaSuccess && ws) {
+    set_split_workspace(c, c->digits[side] + digits);
+  } else if (e != cudaSuccess && ws) {
+    cudaGetLastError();
+    e = alloc_zeroed((void **)&c->digits[side], digits, order);
+  }
   c->digit_maps_ready = false;
   c->digit_map_b64_ready = false;
   c->plan1_ready = false;
