@@ -465,34 +465,6 @@ __device__ __forceinline__ uint32_t row_threshold_codes4(const Raw4<T> &x, T t0,
   }
 }
 
-// Four rows r .. r + 3 of one column, each against its own thresholds (a row
-// past nrows, whose code is not wanted, reads the last row's).
-template <typename T>
-__device__ __forceinline__ uint32_t col_threshold_codes4(const Raw4<T> &x, const T *__restrict__ thr, int nthres,
-                                                         uint64_t r, uint64_t nrows) {
-  const T *p[4];
-  T v[4];
-  bool over[4];
-  uint32_t c[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    p[i] = thr + (r + i < nrows ? r + i : nrows - 1);
-    v[i] = elem_of<T>(x, i);
-    over[i] = true;
-    c[i] = 0u;
-  }
-#pragma unroll 4
-  for (int t = 0; t < nthres; t++) {
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      over[i] = over[i] && !(v[i] <= p[i][(uint64_t)t * nrows]);
-      c[i] += over[i] ? 1u : 0u;
-    }
-    if ((t & 7) == 7 && !(over[0] || over[1] || over[2] || over[3])) break;
-  }
-  return pack4(c[0], c[1], c[2], c[3]);
-}
-
 // Row-major sources of any element type and alignment.  A warp loads the unit's
 // 1024 columns four elements a lane, 8 lanes to a chunk, so that its loads
 // are contiguous whatever the element size (a lane loading the 32 columns it
@@ -641,9 +613,8 @@ __global__ void __launch_bounds__(256) pack_staged(const __grid_constant__ PackJ
 constexpr int kCmRows = 64, kCmCols = 256, kCmThreads = 512;
 constexpr int kCmWords = kCmCols * 17 + 4 * (kCmCols / 32);
 
-template <typename T, bool QUANT, bool ALIGNED>
-__global__ void __launch_bounds__(kCmThreads) pack_colmajor(const __grid_constant__ PackJob J,
-                                                            const T *__restrict__ thr, int nthres) {
+template <typename T, bool ALIGNED>
+__global__ void __launch_bounds__(kCmThreads) pack_colmajor(const __grid_constant__ PackJob J) {
   __shared__ uint32_t st[kCmWords];
   griddep_launch_dependents();
   griddep_wait();  // source, planes and digits belong to earlier kernels until here
@@ -665,16 +636,7 @@ __global__ void __launch_bounds__(kCmThreads) pack_colmajor(const __grid_constan
 #pragma unroll
   for (int i = 0; i < kLoads; i++) {
     const uint32_t t = i * kCmThreads + tid, col = t >> 4, g = t & 15;
-    uint32_t w;
-    if (QUANT) {
-      const uint64_t c = c0 + col, r = r0 + 4 * g;
-      const uint32_t n = (c < J.ncols && r < J.nrows) ? (uint32_t)min((uint64_t)4, J.nrows - r) : 0u;
-      w = n == 0 ? 0u : nthres == 0 ? own_codes4<T>(x[i]) : col_threshold_codes4<T>(x[i], thr, nthres, r, J.nrows);
-      if (n < 4) w &= (1u << (8 * n)) - 1u;
-    } else {
-      w = codes4<T>(x[i], bip, J.issigned, J.nbits);
-    }
-    st[col * 17 + 4 * (col >> 5) + g] = w;
+    st[col * 17 + 4 * (col >> 5) + g] = codes4<T>(x[i], bip, J.issigned, J.nbits);
   }
   __syncthreads();
   // a thread per (row, chunk): lanes 0..7 of a row its 8 chunks, four rows of a quadruple a warp
@@ -689,6 +651,54 @@ __global__ void __launch_bounds__(kCmThreads) pack_colmajor(const __grid_constan
     q[w] = __byte_perm(__byte_perm(p[(4 * w) * 17], p[(4 * w + 1) * 17], sel),
                        __byte_perm(p[(4 * w + 2) * 17], p[(4 * w + 3) * 17], sel), 0x5410u);
   emit_chunk(J, r * J.cpr + cc, (uint32_t)r, (uint32_t)cc, r < J.nrows, q);
+}
+
+// Threshold imports: a warp takes 32 rows x 32 columns, a lane a row, so a column's
+// loads are contiguous, all 32 are in flight at once, and each threshold of a row is
+// read once for its 32 columns.  In the tiles above, each thread with the thresholds of
+// four rows, one load after the other: 8192 x 8192 int32 against 3 thresholds 151 us, 92
+// this way, 2048 x 4096 24 and 14, 1048576 x 1 (tiles mostly empty) 277 and 53,
+// 1 x 1048576 132 and 42.
+template <typename T>
+__global__ void __launch_bounds__(256) pack_colmajor_quant(const __grid_constant__ PackJob J,
+                                                          const T *__restrict__ thr, int nthres) {
+  griddep_launch_dependents();
+  griddep_wait();  // source, planes and digits belong to earlier kernels until here
+  const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint64_t r = w / J.cpr * 32 + (threadIdx.x & 31);
+  const uint32_t cc = (uint32_t)(w % J.cpr);
+  if (r >= J.nrows_a) return;  // no warp-wide step follows
+  uint32_t q[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+  const uint64_t c0 = (uint64_t)cc * 32;
+  if (r < J.nrows && c0 < J.ncols) {
+    const uint32_t n = (uint32_t)min((uint64_t)32, J.ncols - c0);
+    const T *src = (const T *)J.src + c0 * J.nrows + r;
+    T x[32];
+#pragma unroll
+    for (int j = 0; j < 32; j++) x[j] = (uint32_t)j < n ? src[(uint64_t)j * J.nrows] : (T)0;
+    if (nthres == 0) {
+#pragma unroll
+      for (int j = 0; j < 32; j++)
+        q[j >> 2] |= (std::is_same<T, float>::value ? low_byte((float)x[j]) : (uint32_t)x[j] & 0xffu) << (8 * (j & 3));
+    } else {
+      uint32_t over = n == 32 ? kFull : (1u << n) - 1u;  // columns above every threshold so far
+      for (int t = 0; t < nthres && over; t++) {
+        const T th = thr[(uint64_t)t * J.nrows + r];
+        uint32_t above = 0u;
+#pragma unroll
+        for (int g = 0; g < 32; g += 8)
+          if (g < (int)n) {  // the last columns of a row, or its only ones, are few
+#pragma unroll
+            for (int j = g; j < g + 8; j++) above |= !(x[j] <= th) ? 1u << j : 0u;
+          }
+        over &= above;
+#pragma unroll
+        for (int i = 0; i < 8; i++)  // one more in the bytes of those columns (mod 256, as the reference's cast)
+          if (4 * i < (int)n) q[i] = __vadd4(q[i], (((over >> (4 * i)) & 15u) * 0x00204081u) & 0x01010101u);
+      }
+    }
+  }
+  emit_chunk(J, r * J.cpr + cc, (uint32_t)r, cc, r < J.nrows, q);
 }
 
 // ---------------------------------------------------------------- grouped import
@@ -996,15 +1006,24 @@ cudaError_t run_staged(const PackJob &j, const void *thr, int nthres, bool quant
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-cudaError_t run_colmajor(const PackJob &j, const void *thr, int nthres, bool quant, cudaStream_t s) {
+cudaError_t run_colmajor(const PackJob &j, cudaStream_t s) {
   const uint64_t blocks = ((j.nrows_a + kCmRows - 1) / kCmRows) * ((j.wpr * 64 + kCmCols - 1) / kCmCols);
   if (blocks > 0x7FFFFFFFull) return cudaErrorInvalidConfiguration;
   cudaError_t e = cudaSuccess;
   with_source(j.dtype, aligned4(j.src, j.dtype, j.nrows), [&](auto t, auto al) {
+    e = launch_pdl(pack_colmajor<decltype(t), decltype(al)::value>, (unsigned)blocks, kCmThreads, 0, s, j);
+  });
+  count_launch();
+  return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+cudaError_t run_colmajor_quant(const PackJob &j, const void *thr, int nthres, cudaStream_t s) {
+  const uint64_t blocks = ((j.nrows_a + 31) / 32 * j.cpr + 7) / 8;
+  if (blocks > 0x7FFFFFFFull) return cudaErrorInvalidConfiguration;
+  cudaError_t e = cudaSuccess;
+  with_source(j.dtype, false, [&](auto t, auto) {
     using T = decltype(t);
-    constexpr bool A = decltype(al)::value;
-    const auto kern = quant ? pack_colmajor<T, true, A> : pack_colmajor<T, false, A>;
-    e = launch_pdl(kern, (unsigned)blocks, kCmThreads, 0, s, j, (const T *)thr, nthres);
+    e = launch_pdl(pack_colmajor_quant<T>, (unsigned)blocks, 256, 0, s, j, (const T *)thr, nthres);
   });
   count_launch();
   return e != cudaSuccess ? e : cudaGetLastError();
@@ -1028,7 +1047,7 @@ cudaError_t launch_pack_quantize(const Mat &m, const void *src, const void *thr,
                                  int col_major, const DigitTarget *digits, cudaStream_t s) {
   if (m.nrows_a == 0 || m.wpr() == 0) return cudaSuccess;
   const PackJob j = make_pack_job(m, src, dtype, digits, nullptr);
-  if (col_major) return run_colmajor(j, thr, nthres, true, s);
+  if (col_major) return run_colmajor_quant(j, thr, nthres, s);
   return run_staged(j, thr, nthres, true, aligned4(src, dtype, m.ncols), 0, m.nrows_a, s);
 }
 
@@ -1036,7 +1055,7 @@ cudaError_t launch_pack(const Mat &m, const void *src, int dtype, int col_major,
                         cudaStream_t s) {
   if (m.nrows_a == 0 || m.wpr() == 0) return cudaSuccess;
   if (!col_major) return launch_pack_rows(m, src, dtype, 0, m.nrows_a, digits, s);
-  return run_colmajor(make_pack_job(m, src, dtype, digits, nullptr), nullptr, 0, false, s);
+  return run_colmajor(make_pack_job(m, src, dtype, digits, nullptr), s);
 }
 
 cudaError_t launch_pack_grouped(const PackJob *host, const PackJob *jobs, const int (&n)[2], const uint64_t (&runs)[2],
