@@ -1643,6 +1643,13 @@ PairRule pair_rule(uint64_t M, uint64_t N, uint32_t nstages) {
 
 }  // namespace
 
+static bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone) return false;
+  cudaGetLastError();
+  return true;
+}
+
 uint32_t pair_gather_choice(const gbs_ctx *c) {
   if (c->lhs.nrows < 256 || c->rhs.nrows < 256) return 1;
   return pair_rule(c->lhs.nrows, c->rhs.nrows, (uint32_t)(c->lhs.dcols / 128)).gather;
@@ -1650,14 +1657,15 @@ uint32_t pair_gather_choice(const gbs_ctx *c) {
 
 cudaError_t launch_gemm_tc_hbm(gbs_ctx *c, cudaStream_t s, int bn_req) {
   const bool small = bn_req < 0 && (c->lhs.nrows < 256 || c->rhs.nrows < 256);
-  if (small && (c->plan1_ready || tcg_packed_mode() == 1)) {
-    // packed plans forced on a side of fewer than 256 rows: a one-problem plan
-    if (!c->plan1_ready) {
-      if (!c->plan1) c->plan1 = new TcgPlan();
-      gbs_ctx *one[1] = {c};
-      if (tcg_plan_build(c->plan1, one, 1) != GBS_OK) return cudaErrorInvalidValue;
-      c->plan1_ready = true;
-    }
+  const TcgForm *form = small && tcg_packed_mode() != 1 ? small_persistent(c) : nullptr;
+  if (small && !c->plan1_ready && (tcg_packed_mode() == 1 || (form && !capturing(s)))) {
+    // a side of fewer than 256 rows and many tiles or a long K, or packed plans forced: a one-problem plan
+    if (!c->plan1) c->plan1 = new TcgPlan();
+    gbs_ctx *one[1] = {c};
+    c->plan1_ready = tcg_plan_build(c->plan1, one, 1, form) == GBS_OK;
+    if (!c->plan1_ready && !form) return cudaErrorInvalidValue;  // (otherwise gemm_tcs_kernel takes it)
+  }
+  if (small && c->plan1_ready) {
     for (int side = 0; side < 2; side++) {  // the digit and packed matrices the plan reads
       cudaError_t e = cudaSuccess;
       if (((c->plan1->sides[0] >> side) & 1) && !c->digits_valid[side]) e = expand_side(c, side, s);

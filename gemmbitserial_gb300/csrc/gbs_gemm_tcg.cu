@@ -16,7 +16,8 @@
 // order, no atomics).  A tile is 128 rows of the MMA-A operand x bn rows of
 // the MMA-B operand; per problem the larger side is MMA-A ("swap" when that
 // is the rhs), so a problem with few lhs rows uses an MMA N as small as 16
-// instead of padding M to 128.
+// instead of padding M to 128.  A plan of one context's own GEMM may give MMA-A to the
+// smaller lhs (TcgForm): its rows are consecutive in the result.
 //
 // Large groups read HBM once per element of the larger sides, so a "packed" plan
 // holds those that allow it as 4-bit floats (packed_offset): the TMA unpacks them
@@ -638,10 +639,11 @@ static std::vector<uint32_t> tile_widths(gbs_ctx *const *ctxs, int n) {
   return bn;
 }
 
-int tcg_plan_build(TcgPlan *plan, gbs_ctx *const *ctxs, int n) {
+// The plan of some contexts; `form` gives the tiles of a one-problem plan on digits.
+int tcg_plan_build(TcgPlan *plan, gbs_ctx *const *ctxs, int n, const TcgForm *form) {
   tcg_plan_free(plan);
   const int mode = tcg_packed_mode();
-  const bool packed = mode < 0 ? plan_prefers_packed(ctxs, n) : mode == 1;
+  const bool packed = form ? false : mode < 0 ? plan_prefers_packed(ctxs, n) : mode == 1;
   plan->packed = packed;
   std::vector<TcgProblem> probs;
   std::vector<CUtensorMap> maps;
@@ -658,7 +660,8 @@ int tcg_plan_build(TcgPlan *plan, gbs_ctx *const *ctxs, int n) {
     P.C = c->res;
     P.M = (uint32_t)L.nrows;
     P.N = (uint32_t)R.nrows;
-    P.swap = L.nrows < R.nrows ? 1u : 0u;        // the larger side is MMA-A
+    const uint32_t large = L.nrows < R.nrows ? 1u : 0u;
+    P.swap = form ? form->swap : large;          // the larger side is MMA-A, unless the form says otherwise
     const int sa = P.swap ? 1 : 0, sb = 1 - sa;  // sides of MMA-A and MMA-B
     const bool pa = packed && (sa ? R : L).packable();
     const uint8_t sides = pa ? (uint8_t)((4u << sa) | (1u << sb)) : (uint8_t)3;
@@ -678,7 +681,7 @@ int tcg_plan_build(TcgPlan *plan, gbs_ctx *const *ctxs, int n) {
     P.b_rows = (uint32_t)MB.drows;
     P.nk = (uint32_t)((L.ncols + 127) / 128);
     CUtensorMap m2[2];
-    P.bn = widths[i];
+    P.bn = form ? form->bn : widths[i];
     P.idesc = (1u << 4) | ((P.bn >> 3) << 17) | ((128u >> 4) << 24);  // fp32 += e4m3 x e4m3
     P.a_bytes = kTgABytes;
     P.scale = 1.f;
@@ -695,11 +698,11 @@ int tcg_plan_build(TcgPlan *plan, gbs_ctx *const *ctxs, int n) {
     const uint32_t rt = (uint32_t)((MA.nrows + 127) / 128), ct = (uint32_t)((MB.nrows + P.bn - 1) / P.bn);
     maps.push_back(m2[0]);
     maps.push_back(m2[1]);
-    for (uint32_t r = 0; r < rt; r++)
-      for (uint32_t cc = 0; cc < ct; cc++) {
-        tiles.push_back(TcgTile{(uint32_t)probs.size(), r, cc, 0u});
-        cost.push_back((uint64_t)P.nk * (128 + P.bn));
-      }
+    for (uint32_t t = 0; t < rt * ct; t++) {  // the tiles that share the larger side's rows in turn
+      tiles.push_back(P.swap == large ? TcgTile{(uint32_t)probs.size(), t / ct, t % ct, 0u}
+                                      : TcgTile{(uint32_t)probs.size(), t % rt, t / rt, 0u});
+      cost.push_back((uint64_t)P.nk * (128 + P.bn));
+    }
     probs.push_back(P);
     for (int side = 0; side < 2; side++) {
       const Mat &m = side ? R : L;

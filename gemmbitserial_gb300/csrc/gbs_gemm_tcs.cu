@@ -7,20 +7,23 @@
 // The persistent kernel over a problem table (gbs_gemm_tcg.cu) gives such a
 // context one tile per 128 rows of its larger side, as wide as the smaller
 // side: 3 of 152 SMs for 384 x 2304 x 169, each streaming 18 stages of 38 KB.
-// Here the tiles are as narrow as it pays (MMA N = bn, 16 to 256) and K is
-// split over the CTAs of a cluster, chosen by an estimate of the critical
-// path (plan below); the maps and the problem are launch parameters, so no
-// table is read before the first load.
-//   warp 0     lane 0: TMA, 128 x 128 digits of the larger side and bn x 128 of
-//              the smaller per stage, into a ring of as many stages as fit
-//   warp 1     TMEM allocation; lane 0 issues 4 tcgen05.mma (M = 128, N = bn,
-//              K = 32) per stage
+// Here the tiles are as narrow as it pays (MMA N = bn, 16 to 256), either side
+// gives the MMA's 128 rows, and K is split over the CTAs of a cluster, chosen by an
+// estimate of the critical path (choose_tiles); the maps and the problem are launch
+// parameters, so no table is read before the first load.  Where the tiles take
+// several waves, or a long K its narrow stages, the persistent kernel is the faster
+// one and runs the context (small_persistent).
+//   warp 0     TMA, 128 x 128 digits of the side that gives the rows and bn x 128 of
+//              the other per stage, into a ring of as many stages as fit
+//   warp 1     TMEM allocation; 4 tcgen05.mma (M = 128, N = bn, K = 32) per stage
 //   warps 2-5  epilogue; with K split, the CTAs leave their fp32 partial tiles in
 //              the drained ring and each sums its share of the columns over
 //              distributed shared memory (integers below 2^24: exact)
+// Warps 0 and 1 issue from an elected lane.
 // Every mbarrier wait is bounded; on timeout the CTA sets a bit in the error
 // word, stops issuing, drains what it issued and frees TMEM.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 
@@ -31,7 +34,10 @@ namespace gbs {
 
 struct SmallPlan {
   CUtensorMap ma, mb;
+  bool maps = false;
   uint32_t bn, splits, swap, rt, ct;
+  bool persistent = false;  // the persistent kernel is estimated faster
+  TcgForm form;
 };
 
 namespace {
@@ -43,7 +49,7 @@ constexpr int kSmStagesMax = 8;
 
 struct SmallArgs {
   int32_t *C;
-  uint32_t M, N, nk, bn, splits, swap, ct, stages, idesc, cols;  // cols: TMEM columns allocated
+  uint32_t M, N, nk, bn, splits, swap, rt, ct, stages, idesc, cols;  // cols: TMEM columns allocated
 };
 
 constexpr size_t small_smem(uint32_t bn, int stages) {
@@ -104,7 +110,9 @@ __global__ void __launch_bounds__(kSmThreads, 1)
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * stages + 2);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   const uint32_t split = blockIdx.x % a.splits, tile = blockIdx.x / a.splits;
-  const uint32_t r0 = tile / a.ct * 128u, c0 = tile % a.ct * a.bn;
+  // neighbouring tiles share the rows or columns of the side with more of them
+  const bool byrow = a.rt <= a.ct;
+  const uint32_t r0 = (byrow ? tile % a.rt : tile / a.ct) * 128u, c0 = (byrow ? tile / a.rt : tile % a.ct) * a.bn;
   const uint32_t k_lo = split * a.nk / a.splits, nk = (split + 1) * a.nk / a.splits - k_lo;
   griddep_launch_dependents();
   if (tid == 0) {
@@ -241,55 +249,125 @@ __global__ void __launch_bounds__(kSmThreads, 1)
   }
 }
 
-// Tile width and K split with the least estimated time: a stage costs the
-// longer of its bytes at ~105 GB/s into one SM and its four MMAs (~37 ns each up
-// to N = 128, 68 ns at 256); a wave of CTAs 2.5 us of setup, first load and
-// stores; a split 1.5 us of cluster barriers and its remote reads at ~15 GB/s.
-void choose_tiles(uint64_t large, uint64_t small, uint32_t nk, uint32_t &bn, uint32_t &splits) {
-  double best = 0.0;
-  bn = 0;
-  const uint32_t whole = (uint32_t)std::min<uint64_t>(256, (small + 15) / 16 * 16);
-  for (uint32_t w : {whole, 128u, 64u, 32u, 16u}) {  // the others divide 256, the rows' padding
-    if (w > whole || (w == whole && bn)) continue;
-    for (uint32_t s : {1u, 2u, 4u, 8u}) {
-      if (s > 1 && (nk / s < 4 || w < 4 * s)) break;
-      const double tiles = std::ceil((double)large / 128) * std::ceil((double)small / w);
-      const double mma = w <= 128 ? 37.0 : 37.0 + (w - 128) * (31.0 / 128);
-      const double stage = std::max((16384.0 + 128.0 * w) / 105.0, 4 * mma);
-      const double waves = std::ceil(tiles * s / 152.0);
-      const double ns = waves * (std::ceil((double)nk / s) * stage + 2500.0) +
-                        (s > 1 ? 1500.0 + 512.0 * w * (s - 1) / s / 15.0 : 0.0);
-      if (!bn || ns < best) {
-        best = ns;
-        bn = w;
-        splits = s;
+// CTAs of a cluster of `splits` that the GPU holds at once, one to an SM, cached per device.
+double cluster_ctas(uint32_t splits) {
+  static std::atomic<int> cache[64][4];
+  const int i = splits == 1 ? 0 : splits == 2 ? 1 : splits == 4 ? 2 : 3;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1.0;
+  int v = cache[dev][i].load(std::memory_order_relaxed);
+  if (v == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(splits);
+    cfg.blockDim = dim3(kSmThreads);
+    cfg.dynamicSmemBytes = kSmSmemCap;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    cudaError_t e = cudaFuncSetAttribute(gemm_tcs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmSmemCap);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, gemm_tcs_kernel, &cfg);
+    if (e != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      return 1.0;
+    }
+    v = n * (int)splits;
+    cache[dev][i].store(v, std::memory_order_relaxed);
+  }
+  return v;
+}
+
+// Which side gives the MMA's 128 rows, the tile width and the K split with the least
+// estimated time, and whether the persistent kernel, with a table of the context's
+// tiles, beats it.  In ns, fitted to both kernels' times over 9 to 255 x 64 to 8192 x
+// 300 to 100000 and the same transposed: a stage costs its bytes at 105 GB/s into one
+// SM and no less than 345 here, 115 GB/s and 300 there (205 up to 64 columns, where two
+// chunks share a stage).  A wave of CTAs here adds 1700 and its stores: 16 a column where the
+// tile's rows are lhs rows (the lanes write consecutive elements of the result), 22
+// where they are rhs rows and the result's rows are 16-byte aligned, 73 where they are
+// not; a split, of one wave at most, 2900 of cluster barriers and its remote reads at 15
+// GB/s.  There a tile is stored while the next is multiplied, in 1600 + 10.7 a column,
+// or 1400 + 27 staged for rhs rows, 2400 at least, and the first takes 1900 more, 4000
+// with others after it.  A larger lhs gives the rows itself: the result's rows are then
+// long, and rhs rows of a tile far apart.
+// With the larger side's rows and this kernel in every case 255 x 256 x 100000 took 126
+// us (35 so), 128 x 1024 x 100000 46 (32), 20000 x 8192 x 255 94 (60), 255 x 64 x 10000
+// 22.5 (6.4).
+void choose_tiles(const gbs_ctx *c, SmallPlan &p) {
+  const uint64_t M = c->lhs.nrows, N = c->rhs.nrows;
+  const double nk = (double)((c->lhs.ncols + 127) / 128), sms = cluster_ctas(1);
+  double best = 0.0, other = 0.0;
+  p.bn = p.form.bn = 0;
+  auto bytes = [](double w) { return 16384.0 + 128.0 * w; };
+  for (uint32_t swap = 0; swap < (M < N ? 2u : 1u); swap++) {
+    const uint64_t rows = swap ? N : M, cols = swap ? M : N;
+    const double rt = std::ceil((double)rows / 128);
+    const uint32_t whole = (uint32_t)std::min<uint64_t>(256, (cols + 15) / 16 * 16);
+    for (uint32_t w : {whole, 128u, 64u, 32u, 16u}) {  // the others divide 256, the rows' padding
+      if (w > whole) continue;
+      const double ct = std::ceil((double)cols / w), used = std::min<double>(w, (double)cols);
+      const double store = used * (!swap ? 16.0 : (M & 3) == 0 ? 22.0 : 73.0);
+      for (uint32_t s : {1u, 2u, 4u, 8u}) {
+        if (s > 1 && (nk / s < 4 || w < 4 * s || rt * ct * s > cluster_ctas(s))) break;
+        const double waves = std::ceil(rt * ct * s / sms);
+        const double ns = waves * (std::ceil(nk / s) * std::max(345.0, bytes(w) / 105.0) + 1700.0 + store / s) +
+                          (s > 1 ? 2900.0 + 512.0 * w * (s - 1) / s / 15.0 : 0.0);
+        if (!p.bn || ns < best) {
+          best = ns;
+          p.bn = w;
+          p.splits = s;
+          p.swap = swap;
+        }
+      }
+      const double mul = nk * std::max(w <= 64 ? 205.0 : 300.0, bytes(w) / 115.0);
+      const double epi = std::max(2400.0, swap ? 1400.0 + 27.0 * used : 1600.0 + 10.7 * used);
+      const double rounds = std::ceil(rt * ct / sms);
+      const double ns = (rounds > 1.0 ? 4000.0 : 1900.0) + (rounds - 1.0) * std::max(mul, epi) + mul + epi;
+      if (!p.form.bn || ns < other) {
+        other = ns;
+        p.form.bn = w;
+        p.form.swap = swap;
       }
     }
   }
+  p.rt = (uint32_t)(((p.swap ? N : M) + 127) / 128);
+  p.ct = (uint32_t)(((p.swap ? M : N) + p.bn - 1) / p.bn);
+  p.persistent = other < 0.95 * best;
+}
+
+// The context's tiles, chosen on first use.
+SmallPlan &small_plan(gbs_ctx *c) {
+  if (!c->small) {
+    c->small = new SmallPlan();
+    choose_tiles(c, *c->small);
+  }
+  return *c->small;
 }
 
 }  // namespace
 
 void small_plan_free(SmallPlan *p) { delete p; }
 
+const TcgForm *small_persistent(gbs_ctx *c) {
+  const SmallPlan &p = small_plan(c);
+  return p.persistent ? &p.form : nullptr;
+}
+
 // The GEMM of a context whose digit matrices are built and current.
 cudaError_t launch_gemm_tcs(gbs_ctx *c, cudaStream_t s) {
   const Mat &L = c->lhs, &R = c->rhs;
-  if (!c->small) {
-    SmallPlan *p = new SmallPlan();
-    p->swap = L.nrows < R.nrows ? 1u : 0u;  // the larger side is the MMA's 128-row operand
-    const Mat &A = p->swap ? R : L, &B = p->swap ? L : R;
-    choose_tiles(A.nrows, B.nrows, (uint32_t)((L.ncols + 127) / 128), p->bn, p->splits);
-    p->rt = (uint32_t)((A.nrows + 127) / 128);
-    p->ct = (uint32_t)((B.nrows + p->bn - 1) / p->bn);
-    if (!tc_map_u8(&p->ma, c->digits[p->swap ? 1 : 0], A.dcols, A.drows, 128) ||
-        !tc_map_u8(&p->mb, c->digits[p->swap ? 0 : 1], B.dcols, B.drows, p->bn)) {
-      delete p;
+  SmallPlan &p = small_plan(c);
+  if (!p.maps) {
+    const Mat &A = p.swap ? R : L, &B = p.swap ? L : R;
+    if (!tc_map_u8(&p.ma, c->digits[p.swap ? 1 : 0], A.dcols, A.drows, 128) ||
+        !tc_map_u8(&p.mb, c->digits[p.swap ? 0 : 1], B.dcols, B.drows, p.bn))
       return cudaErrorInvalidValue;
-    }
-    c->small = p;
+    p.maps = true;
   }
-  const SmallPlan &p = *c->small;
   SmallArgs a;
   a.C = result_ptr(c);
   a.M = (uint32_t)L.nrows;
@@ -298,6 +376,7 @@ cudaError_t launch_gemm_tcs(gbs_ctx *c, cudaStream_t s) {
   a.bn = p.bn;
   a.splits = p.splits;
   a.swap = p.swap;
+  a.rt = p.rt;
   a.ct = p.ct;
   a.stages = (uint32_t)small_stages(p.bn);
   a.idesc = (1u << 4) | ((p.bn >> 3) << 17) | ((128u >> 4) << 24);

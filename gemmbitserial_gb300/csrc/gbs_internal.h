@@ -162,6 +162,11 @@ struct ExpandJob {
   uint32_t pform;
 };
 
+// Tiles of a one-problem plan on digits: MMA-A is the lhs, or the rhs (swap), MMA N = bn.
+struct TcgForm {
+  uint32_t swap, bn;
+};
+
 // Host-side plan of the persistent tensor-core kernels over some contexts.
 struct TcgPlan {
   std::vector<gbs_ctx *> ctxs;
@@ -360,7 +365,7 @@ bool tc_encoder_available();
 // persistent tensor-core kernel over a table of problems (gbs_gemm_tcg.cu)
 bool tcg_eligible(const gbs_ctx *c);
 bool tcg_preferred(const gbs_ctx *c);
-int tcg_plan_build(TcgPlan *plan, gbs_ctx *const *ctxs, int n);
+int tcg_plan_build(TcgPlan *plan, gbs_ctx *const *ctxs, int n, const TcgForm *form = nullptr);
 void tcg_plan_free(TcgPlan *plan);
 cudaError_t tcg_expand(TcgPlan &plan, cudaStream_t s);
 cudaError_t tcg_gemm(const TcgPlan &plan, uint32_t *err, cudaStream_t s, int32_t *out0 = nullptr);
@@ -382,6 +387,7 @@ cudaError_t launch_pair_gather(gbs_ctx *c, const void *map_a, const void *map_b,
 // one context with a side under 256 rows on its digit matrices (gbs_gemm_tcs.cu)
 cudaError_t launch_gemm_tcs(gbs_ctx *c, cudaStream_t s);
 void small_plan_free(SmallPlan *p);
+const TcgForm *small_persistent(gbs_ctx *c);  // of a plan of the persistent kernel to run instead, or null
 // tensor-core pipe for 5-8-bit operands (gbs_wide.cu): operands split into parts of <= 4 bits
 bool tc_wide(const gbs_ctx *c);
 cudaError_t launch_gemm_wide(gbs_ctx *c, cudaStream_t s, int variant);
