@@ -655,48 +655,71 @@ int adj_max_pairs() {
 // least kMinPiece stages.  4096 x 2048 x 2048: 64 tiles of 64 stages and 128 of
 // 32 over 76 pairs; whole tiles only would end with 28 pairs a tile (26 us)
 // behind the rest, halves of those 28 end half a tile behind.  Few long tiles (a
-// large batch against a small layer) are split too, down to an even share of
-// all the work.  A part costs its sums' way through L2, about 3 us: kMinPiece
-// stages of 0.8 us keep it worth while.
-constexpr uint32_t kMinPiece = 6, kMaxPieces = 8;
+// large batch against a small layer) are split too, in as many parts as end soonest.
+// A part costs its sums' way through L2, about 3 us: kMinPiece stages of 0.8 us keep
+// it worth while.  A tile takes about 4 us, kTileStages stages, for its stores however short
+// its contraction: counted by their stages alone, the 256 one-stage tiles of dA at 4096
+// x 4096 x 1 all went to the 12 pairs that dB's long ones had left idle (109 us, 69 so;
+// 4096 x 4096 x 64 86 and 45).
+constexpr uint32_t kMinPiece = 6, kMaxPieces = 8, kTileStages = 5, kPieceStages = 4;
 
-AdjDeal deal_tiles(uint32_t first, uint64_t nfirst, uint64_t cfirst, uint64_t nother, uint64_t cother,
-                   uint32_t pairs) {
+// The deal with the first gradient's tiles in fpieces parts, and the stages until it ends.
+AdjDeal deal_parts(uint32_t first, uint64_t nfirst, uint64_t cfirst, uint64_t nother, uint64_t cother, uint32_t pairs,
+                   uint32_t fpieces, uint64_t &span) {
   AdjDeal d;
   memset(&d, 0, sizeof(d));
   d.first = first;
   d.pairs = pairs;
-  d.pieces = d.fpieces = 1;
-  const uint64_t share = std::max<uint64_t>((nfirst * cfirst + nother * cother) / pairs, kMinPiece);
-  if (nfirst && 2 * nfirst <= pairs && cfirst >= 2 * share)
-    d.fpieces = (uint32_t)std::min<uint64_t>(std::min<uint64_t>(kMaxPieces, pairs / nfirst), cfirst / share);
-  const bool split = d.fpieces > 1;
-  d.a = (uint32_t)(split ? nfirst * d.fpieces : nfirst % pairs);
+  d.pieces = 1;
+  d.fpieces = fpieces;
+  const bool split = fpieces > 1;
+  d.a = (uint32_t)(split ? nfirst * fpieces : nfirst % pairs);
+  const uint64_t tfirst = std::max<uint64_t>(cfirst, kTileStages), tother = std::max<uint64_t>(cother, kTileStages);
   const uint64_t size[2] = {d.a, pairs - d.a};
-  uint64_t load[2] = {split ? cfirst / d.fpieces : (nfirst / pairs + 1) * cfirst,
-                      split ? 0 : nfirst / pairs * cfirst};
+  uint64_t load[2] = {split ? (cfirst + fpieces - 1) / fpieces + kPieceStages : (nfirst / pairs + 1) * tfirst,
+                      split ? 0 : nfirst / pairs * tfirst};
   uint64_t s[2] = {0, 0}, takers = pairs;
+  int g = 0;
   while (nother) {
-    const bool all = !size[0] || !size[1] || load[0] == load[1];
-    const int g = load[0] < load[1] ? 0 : 1;
+    // (the last few whole tiles, where both are equal, to the pairs that had no long ones)
+    const bool all = !size[0] || !size[1] ||
+                     (load[0] == load[1] && (nother > size[1] || cother >= 2 * kMinPiece));
+    g = load[0] < load[1] ? 0 : 1;
     takers = all ? pairs : size[g];
     d.p0 = all || g == 0 ? 0 : d.a;
     if (nother < takers) break;
     for (int i = 0; i < 2; i++)
       if (all || i == g) {
         s[i]++;
-        load[i] += cother;
+        load[i] += tother;
       }
     nother -= takers;
   }
   d.sa = (uint32_t)s[0];
   d.sb = (uint32_t)s[1];
   d.rem = (uint32_t)nother;
-  if (nother)
+  if (nother) {
     d.pieces = (uint32_t)std::max<uint64_t>(
         1, std::min<uint64_t>(std::min<uint64_t>(kMaxPieces, takers / nother), cother / kMinPiece));
+    load[g] += d.pieces > 1 ? (cother + d.pieces - 1) / d.pieces + kPieceStages : tother;
+  }
+  span = std::max(size[0] ? load[0] : 0, size[1] ? load[1] : 0);
+  return d;
+}
+
+AdjDeal deal_tiles(uint32_t first, uint64_t nfirst, uint64_t cfirst, uint64_t nother, uint64_t cother,
+                   uint32_t pairs) {
+  uint64_t best = 0, span = 0;
+  AdjDeal d = deal_parts(first, nfirst, cfirst, nother, cother, pairs, 1, best);
+  for (uint32_t f = 2; nfirst && f <= kMaxPieces && nfirst * f <= pairs && cfirst / f >= kMinPiece; f++) {
+    const AdjDeal e = deal_parts(first, nfirst, cfirst, nother, cother, pairs, f, span);
+    if (10 * span < 9 * best) {  // parts of long tiles, unless a tenth is all they save
+      best = span;
+      d = e;
+    }
+  }
   AdjTile w;
-  for (d.grid = pairs; d.grid > 1 && !dealt_tile(d, (uint32_t)(split || nfirst < pairs ? nfirst : pairs),
+  for (d.grid = pairs; d.grid > 1 && !dealt_tile(d, (uint32_t)(d.fpieces > 1 || nfirst < pairs ? nfirst : pairs),
                                                  d.grid - 1, 0, w);)
     d.grid--;
   return d;
