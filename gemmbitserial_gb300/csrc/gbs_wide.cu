@@ -20,9 +20,9 @@
 //   A.B = 2^l X + 2^l Y
 // and for one wide operand X = ah.b, Y = al.b, A.B = 2^lo X + Y (parts
 // unscaled).  X and Y are exact while K times the largest |term| sum stays
-// below 2^24 (X in units of 1, Y in units of 2^-l); longer K splits over
-// kMaxSplit launches' worth of CTAs, whose int32 partial results the combine
-// kernel adds.  8 x 8 bits at 2048 x 4096 x 2048: four part GEMMs and their
+// below 2^24 (X in units of 1, Y in units of 2^-l); longer K splits in two or
+// four over as many times the CTAs, whose int32 partial results the combine kernel
+// adds.  8 x 8 bits at 2048 x 4096 x 2048: four part GEMMs and their
 // combination took 87 us and re-read both operands twice.
 //
 // Separate form (a side under 256 rows, K beyond the splits, forced
@@ -37,8 +37,6 @@
 #include "gbs_tc_common.cuh"
 
 namespace gbs {
-
-constexpr int kMaxSplit = 4;
 
 struct WidePlan {
   int parts[2] = {1, 1};    // parts per side (1 or 2)
