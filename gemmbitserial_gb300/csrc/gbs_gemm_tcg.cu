@@ -24,11 +24,11 @@
 // on the way into shared memory and the MMA takes them as they land there (e2m1
 // against the other side's e4m3), so nothing is decoded by threads.
 //
-//   warp 0     lane 0: TMA producer -- A box 128 x 128 values and B box
+//   warp 0     TMA producer -- A box 128 x 128 values and B box
 //              bn x 128 bytes, 128-byte swizzle, one or two of each a stage,
 //              into a 4-slot ring that runs across tile boundaries
 //   warp 1     allocates all 512 TMEM columns (two 256-column accumulators);
-//              lane 0 issues 4 or 8 tcgen05.mma (K = 32) per stage and commits the
+//              issues 4 or 8 tcgen05.mma (K = 32) per stage and commits the
 //              accumulator of each tile
 //   warps 2-5  epilogue of tile j while the MMAs of tile j+1 run: tcgen05.ld
 //              32 lanes x 32 columns, fp32 -> int32, stores into res[n*M + m]

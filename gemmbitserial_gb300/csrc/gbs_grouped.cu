@@ -13,8 +13,9 @@
 // Problems go to one of two persistent kernels: the tensor-core kernel over
 // e4m3 digit matrices (gbs_gemm_tcg.cu) where it is exact and cheaper, the
 // CUDA-core popcount kernel otherwise.  GBS_GROUP_PIPE=popc or =tc in the
-// environment forces one kernel (tc: wherever it is exact).  Digit matrices
-// are rebuilt by one grouped expansion launch after every import.
+// environment forces one kernel (tc: wherever it is exact).  The grouped import
+// writes the digit and packed matrices with the planes; where the planes came another
+// way, one grouped expansion launch rebuilds them before the GEMM.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>

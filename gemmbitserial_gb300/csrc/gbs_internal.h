@@ -258,7 +258,7 @@ struct gbs_ctx {
   bool plan1_ready = false;
   gbs::AdjPlan *adj = nullptr;  // tensor-core adjoint workspace, built on first use
   gbs::WidePlan *wide = nullptr;  // tensor-core parts of 5-8-bit operands, built on first use
-  bool vt_valid[2] = {false, false};  // its transposed bf16 operand values match the planes
+  bool vt_valid[2] = {false, false};  // its bf16 operand values match the planes
 };
 
 namespace gbs {

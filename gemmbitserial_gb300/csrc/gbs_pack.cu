@@ -125,8 +125,9 @@ __device__ __forceinline__ void emit_chunk(const PackJob &J, uint64_t idx, uint3
 // A unit is 32 chunks, a lane each.  The unit's first chunk is located once, in
 // 64 bits: its row r, its chunk of the row cc, and how many rows from r on are
 // the matrix's own (rows) and to be written (rows_a).  The lanes then work in
-// 32 bits (integer arithmetic at half the rate of the other instructions is what
-// bounds these kernels once their loads are contiguous): chunk i is dr rows
+// 32 bits, integer arithmetic being at half the rate of the other instructions (the
+// grouped import issues 0.69 instructions a cycle and scheduler; a single operand's is a
+// wave or two that wait on memory): chunk i is dr rows
 // further, t = cc + i divided by cpr through a multiply-high by magic = 2^32 /
 // cpr + 1 (exact while t * cpr < 2^32, i < 32 (kMaxRun + 1)), or, for rows of
 // 65000 chunks and more, 0 or 1.
@@ -410,8 +411,9 @@ struct RowThresholds {
 // 22 us, bound by integer instructions).  A block that does not is scanned for
 // its first crossing.  Elements past every threshold of a block of 8 go on to
 // the next.  2048 x 4096 int32 against 7 thresholds: 58 us loading a column
-// run per lane, 15 us now (33.5 MB in, 11.5 MB out: 6.6 us at the copy rate;
-// integer instructions bound it).  (A NaN exceeds the fill value too: counts are cut to the
+// run per lane, 15 us now (33.5 MB in, 11.5 MB out: 6.6 us at the copy rate).  No unit is
+// busy there, SM 37 %, DRAM 28 %: 80 registers and the staging leave 24 warps an SM,
+// 2.25 waves of them, and those wait on memory.  (A NaN exceeds the fill value too: counts are cut to the
 // thresholds there are.)  Every lane of the warp calls it.
 template <typename T, int LEVELS>
 __device__ __forceinline__ uint32_t row_threshold_codes4(const Raw4<T> &x, T t0, const T *__restrict__ thr, int nthres,

@@ -206,7 +206,7 @@ __device__ __forceinline__ void mma_f8(uint32_t tmem, uint64_t adesc, uint64_t b
 // One lane of a converged warp, always the same: true there.  Warps that load or
 // multiply walk their stages whole and issue from this lane: issued by lane 0 of a
 // diverged warp, a stage of four MMAs takes 0.27 us to issue, as long as the four
-// take on 256 columns (0.264), elected 0.19.  The persistent pair kernel on
+// take on 256 columns (0.264), elected 0.19.  The one-tile pair kernel on
 // 2048 x 4096 x 2048 went from 0.287 us a stage to that rate, 17.9 -> 17.1 us.
 __device__ __forceinline__ bool elect_one() {
   uint32_t one;

@@ -8,6 +8,7 @@ prints "ok <case>".  The kernels each case launches:
 
   gemm            2048x4096x2048 u3 x s2 forward, the library's choice (gemm_tc_pair_kernel)
   gemm_streamk    the same on the stream-K SM-pair kernel (gemm_tc_pair_streamk_kernel)
+  gemm_tma        the same on single SMs (gemm_tc_tma_kernel<256>)
   gemm_popc       the same on the CUDA cores (gemm_popc_tiled)
   gemm_bmma       the same on b1 mma.sync (gemm_bmma_kernel)
   gemm_tc_smem    the same, planes decoded in shared memory (gemm_tc_kernel)
@@ -15,6 +16,7 @@ prints "ok <case>".  The kernels each case launches:
   gemm_two        4096x2048x2048 u2 x bp, the library's choice (gemm_tc_pair_persistent_kernel)
   gemm_wide       2048x4096x2048 s8 x s8, the library's choice (gemm_wide_pair_kernel)
   gemm_small      384 x 2304 x 169 u2 x u2, the library's choice (gemm_tcs_kernel)
+  gemm_many       128 x 1024 x 100000 u2 x s2, the library's choice (gemm_tcg_kernel over one problem)
   gemm_skinny     8x8192x8 u1 x u1 (gemm_popc_skinny)
   gemm_rows       9 x 8192 x 32768, 1-bit unsigned x 2-bit signed on the CUDA cores (gemm_popc_rows: at most
                   16 lhs rows, 64 rhs rows x every lhs row per CTA)
@@ -22,6 +24,7 @@ prints "ok <case>".  The kernels each case launches:
   import_host     the same from pinned host memory, read over the host link (pack_bytes)
   import_colmajor the same operand read column-major (pack_colmajor)
   import_quantize importRegularAndQuantize of a 2048x4096 float lhs, 7 thresholds per row (pack_staged)
+  import_quantize_colmajor  the same read column-major (pack_colmajor_quant)
   expand          imports for the CUDA cores, then a tensor-core forward that first expands the planes
                   (expand_one_kernel)
   group           the 512-problem mix as one group: import, row sums, GEMMs (pack_grouped, rowsum_grouped,
@@ -37,9 +40,10 @@ import ctypes as C
 import os
 import sys
 
-CASES = ["gemm", "gemm_streamk", "gemm_popc", "gemm_bmma", "gemm_tc_smem", "gemm_split", "gemm_two", "gemm_wide",
-         "gemm_small", "gemm_skinny", "gemm_rows", "import_device", "import_host", "import_colmajor", "import_quantize",
-         "expand", "group", "group_small", "adjoint", "adjoint_simt"]
+CASES = ["gemm", "gemm_streamk", "gemm_tma", "gemm_popc", "gemm_bmma", "gemm_tc_smem", "gemm_split", "gemm_two",
+         "gemm_wide", "gemm_small", "gemm_many", "gemm_skinny", "gemm_rows", "import_device", "import_host",
+         "import_colmajor", "import_quantize", "import_quantize_colmajor", "expand", "group", "group_small", "adjoint",
+         "adjoint_simt"]
 
 
 def main() -> None:
@@ -73,6 +77,8 @@ def main() -> None:
         pipe, variant, name = None, None, "gemm_2048x4096x2048_u3s2"
         if case == "gemm_streamk":
             pipe, variant = _capi.GBS_PIPE_TC, 515
+        elif case == "gemm_tma":
+            pipe, variant = _capi.GBS_PIPE_TC, 256
         elif case == "gemm_popc":
             pipe = _capi.GBS_PIPE_POPC
         elif case == "gemm_bmma":
@@ -91,6 +97,10 @@ def main() -> None:
             c = allocGEMMContext(384, 2304, 169, 2, 2, False, False)
             dA = torch.from_numpy(datagen.operand(datagen.SEED_BASE + 63, 384, 2304, 2, "u")).to(dev)
             dB = torch.from_numpy(datagen.operand(datagen.SEED_BASE + 64, 169, 2304, 2, "u")).to(dev)
+        elif case == "gemm_many":
+            c = allocGEMMContext(128, 1024, 100000, 2, 2, False, True)
+            dA = torch.from_numpy(datagen.operand(datagen.SEED_BASE + 65, 128, 1024, 2, "u")).to(dev)
+            dB = torch.from_numpy(datagen.operand(datagen.SEED_BASE + 66, 100000, 1024, 2, "s")).to(dev)
         elif case == "gemm_rows":
             c = allocGEMMContext(9, 8192, 32768, 1, 2, False, True)
             c.set_pipe(_capi.GBS_PIPE_POPC)
@@ -119,8 +129,10 @@ def main() -> None:
             g.manual_seed(5)
             X = torch.randn(2048, 4096, generator=g, device=dev)
             T = torch.sort(torch.randn(7, 2048, generator=g, device=dev), dim=0).values.contiguous()
+            col = int(case == "import_quantize_colmajor")
+            X = X.t().contiguous() if col else X
             run = lambda: _capi.check(lib.gbs_import_quantize(c._h, 0, C.c_void_p(X.data_ptr()),  # noqa: E731
-                                                              C.c_void_p(T.data_ptr()), 7, _capi.GBS_F32, 0, sh))
+                                                              C.c_void_p(T.data_ptr()), 7, _capi.GBS_F32, col, sh))
     elif case == "expand":
         c, dA, dB = ctx_of("gemm_2048x4096x2048_u3s2")
 

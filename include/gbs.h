@@ -417,7 +417,7 @@ GBS_API int gbs_debug_split_timeout(gbs_ctx *ctx, uint32_t rounds, void *stream)
 /* Number of kernel launches the library has issued since load (all entry points). */
 GBS_API uint64_t gbs_debug_launch_count(void);
 
-/* Tile width (256 or 128), K split (1, 2 or 4; for the stream-K kernel the
+/* Tile width (256 or 128), K split (1, 2, 4 or 8; for the stream-K kernel the
  * number of SM pairs it ran on) and which SM-pair kernel ran for the last
  * SM-pair launch of ctx: 0 one tile per pair, 1 the persistent kernel, 2 the
  * stream-K kernel; all 0 if none was. */
